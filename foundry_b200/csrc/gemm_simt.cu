@@ -4,10 +4,11 @@
 //
 // A projection is `x * W^T` with W stored [out, in] row-major and no bias
 // (src/nn/linear.rs:19-36); accumulation is 32-bit in the reference too
-// (src/metal/kernels/matmul.metal:42-64). Every output element sums its K
-// products in the same order whatever M is, so a row's result does not depend
-// on what else is in the batch.
+// (src/metal/kernels/matmul.metal:42-64). Every output element of this kernel sums
+// its K products in order, whatever M is. Operands in 32 bits that 16-byte loads can
+// address take the kernels of gemm_f32.cu instead (see there for how they sum).
 #include "common.cuh"
+#include "gemm_f32.h"
 
 namespace {
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
@@ -79,6 +80,11 @@ FB_API int fb_gemm_simt(const void* x, const void* w, void* out, int M, int N, i
   FB_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_simt: bad sizes M=%d N=%d K=%d", M, N, K);
   FB_REQUIRE(ldx >= K && ldw >= K && ldo >= N, "gemm_simt: a leading dimension is too small");
   if (M == 0) return 0;
+  if (in_dtype == FB_F32 && out_dtype == FB_F32) {
+    const FbGemmF32 p = {(const float*)x, (const float*)w, (float*)out, M, N, K, ldx, ldw, ldo,
+                         1, 0, 0, 0};
+    if (fb_gemm_f32_fits(p)) return fb_gemm_f32_launch(p, stream);
+  }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   FB_REQUIRE(grid.y <= 65535, "gemm_simt: M=%d exceeds the grid limit", M);
   FB_DISPATCH_DTYPE(in_dtype, TI, FB_DISPATCH_DTYPE(out_dtype, TO, (
@@ -97,6 +103,11 @@ FB_API int fb_gemm_simt_batched(const void* x, const void* w, void* out, int M, 
              "gemm_simt_batched: bad sizes M=%d N=%d K=%d count=%d", M, N, K, count);
   FB_REQUIRE(ldx >= K && ldw >= K && ldo >= N, "gemm_simt_batched: a leading dimension is too small");
   if (M == 0) return 0;
+  if (in_dtype == FB_F32 && out_dtype == FB_F32) {
+    const FbGemmF32 p = {(const float*)x, (const float*)w, (float*)out, M, N, K, ldx, ldw, ldo,
+                         count, bx, bw, bo};
+    if (fb_gemm_f32_fits(p)) return fb_gemm_f32_launch(p, stream);
+  }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, count);
   FB_REQUIRE(grid.y <= 65535, "gemm_simt_batched: M=%d exceeds the grid limit", M);
   FB_DISPATCH_DTYPE(in_dtype, TI, FB_DISPATCH_DTYPE(out_dtype, TO, (
