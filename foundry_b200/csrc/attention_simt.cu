@@ -1,6 +1,7 @@
 // Causal grouped-query attention over the paged cache on the CUDA cores, in
-// 32-bit arithmetic: the attention of the 32-bit path (prompts and single
-// tokens alike) and the plain check of the tensor-core kernels.
+// 32-bit arithmetic: the plain check of the tensor-core kernels, and the attention
+// of the 32-bit path where the kernels of attention_f32.cu do not fit (head sizes
+// other than 32, 64 and 128, rows that 16-byte loads cannot address).
 //
 // Formulas (reference, by its path in stratorys/foundry):
 //   query head a reads key-value head a / (A / Kh)       (src/nn/attention.rs:40-44)
@@ -19,6 +20,7 @@
 // lanes own head elements lane, lane+32, ...
 // Queries, keys and values are read with coherent (L2) loads: the kernel that
 // wrote this step's rows may have overlapped this kernel's start.
+#include "attention_f32.h"
 #include "common.cuh"
 
 namespace {
@@ -130,8 +132,9 @@ attention_simt_kernel(const T* q, long long q_stride, T* __restrict__ out,
 
 FB_API int fb_attention_simt(const void* q, long long q_stride, void* out, long long out_stride,
                              int dtype, const int* positions, const int* seq_of_token,
-                             const int* page_table, int max_pages, const void* k_cache,
-                             const void* v_cache, long long page_stride, long long head_stride,
+                             const int* page_table, int max_pages, int n_seqs,
+                             const void* k_cache, const void* v_cache, long long page_stride,
+                             long long head_stride,
                              int ring_pages, int window, int T, int A, int Kh, int D, float scale,
                              cudaStream_t stream) {
   FB_REQUIRE(T >= 0 && A > 0 && Kh > 0 && D > 0, "attention: bad sizes T=%d A=%d Kh=%d D=%d", T, A,
@@ -144,6 +147,13 @@ FB_API int fb_attention_simt(const void* q, long long q_stride, void* out, long 
              "attention: a row stride is too small");
   FB_REQUIRE(T <= 0x7fffffff / 1 && max_pages > 0, "attention: bad page table");
   if (T == 0) return 0;
+  if (dtype == FB_F32) {
+    const FbAttentionF32 p = {(const float*)q, q_stride, (float*)out, out_stride, positions,
+                              seq_of_token, page_table, max_pages, n_seqs, (const float*)k_cache,
+                              (const float*)v_cache, page_stride, head_stride, ring_pages, window,
+                              T, A, Kh, D, scale};
+    if (fb_attention_f32_fits(p)) return fb_attention_f32_launch(p, stream);
+  }
   dim3 grid(T, (A + WARPS - 1) / WARPS);
   FB_DISPATCH_DTYPE(dtype, E, (fb_launch(attention_simt_kernel<E>, dim3(grid), dim3(WARPS * 32), 0, stream, 
       (const E*)q, q_stride, (E*)out, out_stride, positions, seq_of_token, page_table, max_pages,

@@ -50,7 +50,7 @@ _SIGNATURES = {
     "fb_gemm_simt_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_ll,
                              c_int, c_ll, c_ll, c_ll, c_int, c_int, c_void_p],
     "fb_attention_simt": [c_void_p, c_ll, c_void_p, c_ll, c_int, c_void_p, c_void_p, c_void_p,
-                          c_int, c_void_p, c_void_p, c_ll, c_ll, c_int, c_int, c_int, c_int, c_int,
+                          c_int, c_int, c_void_p, c_void_p, c_ll, c_ll, c_int, c_int, c_int, c_int, c_int,
                           c_int, c_float, c_void_p],
     "fb_sum_planes": [c_void_p, c_int, c_ll, c_ll, c_void_p, c_int, c_void_p],
     "fb_gemm_tc_grouped": [c_void_p, c_ll, c_int, c_void_p, c_ll, c_int, c_int, c_void_p, c_int,
@@ -1734,9 +1734,9 @@ def attention_simt(q: torch.Tensor, out: torch.Tensor, positions: torch.Tensor,
     _call("fb_attention_simt", _dev(q, "q", contiguous=False), _rows(q, "q"),
           _dev(out, "out", contiguous=False), _rows(out, "out"), code_of(q.dtype),
           _dev(positions, "positions", torch.int32), _dev(seq_of_token, "seq_of_token", torch.int32),
-          _dev(page_table, "page_table", torch.int32), page_table.shape[1], k_cache.data_ptr(),
-          v_cache.data_ptr(), k_cache.stride(0), k_cache.stride(1), ring_pages, window, T,
-          num_heads, num_kv_heads, head_dim, float(scale), _stream())
+          _dev(page_table, "page_table", torch.int32), page_table.shape[1], page_table.shape[0],
+          k_cache.data_ptr(), v_cache.data_ptr(), k_cache.stride(0), k_cache.stride(1), ring_pages,
+          window, T, num_heads, num_kv_heads, head_dim, float(scale), _stream())
     return out
 
 

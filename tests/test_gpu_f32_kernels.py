@@ -63,3 +63,78 @@ def test_batched_products(ops, M, K):
     ops.gemm_simt_batched(x, w, out)
     for b in range(3):
         check_product(x[:, b], w[b], out[:, b])
+
+
+def paged_case(runs, Kh, G, D, ring=0, seed=5):
+    """`runs`: (sequence, first position, tokens) in token order; -1 = padding rows."""
+    n_seqs = max(s for s, _, _ in runs) + 1
+    longest = max(a + n for _, a, n in runs)
+    width = ring or (longest + PAGE - 1) // PAGE
+    order = torch.randperm(n_seqs * width, generator=torch.Generator().manual_seed(seed))
+    table = order.view(n_seqs, width).to(torch.int32).to(DEV)
+    k, v = rnd(n_seqs * width, Kh, PAGE, D, seed=6), rnd(n_seqs * width, Kh, PAGE, D, seed=7)
+    seq = torch.cat([torch.full((n,), s, dtype=torch.int32) for s, _, n in runs]).to(DEV)
+    pos = torch.cat([torch.arange(a, a + n, dtype=torch.int32) for _, a, n in runs]).to(DEV)
+    return dict(q=rnd(seq.numel(), Kh * G * D, seed=8), table=table, k=k, v=v, seq=seq, pos=pos)
+
+
+def check_attention(ops, case, Kh, G, D, window=0, ring=0):
+    T = case["seq"].numel()
+    out = torch.full((T, Kh * G * D), 9.0, device=DEV)
+    scale = D ** -0.5
+    ops.attention_simt(case["q"], out, case["pos"], case["seq"], case["table"], case["k"], case["v"],
+                       Kh * G, Kh, D, scale, window, ring)
+    q = case["q"].double().view(T, Kh * G, D)
+    worst = 0.0
+    for t in range(T):
+        s, p = int(case["seq"][t]), int(case["pos"][t])
+        if s < 0:
+            assert bool((out[t] == 0).all())
+            continue
+        j = torch.arange(max(0, p - window + 1) if window else 0, p + 1, device=DEV)
+        page = j // PAGE % ring if ring else j // PAGE
+        pages = case["table"][s][page].long()
+        k, v = case["k"][pages, :, j % PAGE].double(), case["v"][pages, :, j % PAGE].double()
+        k, v = k.repeat_interleave(G, 1), v.repeat_interleave(G, 1)  # [keys, heads, D]
+        w = torch.softmax(torch.einsum("hd,jhd->hj", q[t], k) * scale, -1)
+        want = torch.einsum("hj,jhd->hd", w, v)
+        worst = max(worst, float((out[t].double().view(-1, D) - want).abs().max()))
+    # scores of a few units, off by D * 2^-24 of |q||k| * scale <= 30; weights by as much; their sums
+    # by the number of keys * 2^-24 of |v| <= 5
+    assert worst < (30 * D + 5 * 600) * 2.0 ** -24, worst
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("G", [1, 3, 4, 6])
+def test_attention_of_single_tokens(ops, D, G):
+    runs = [(0, 0, 1), (1, 599, 1), (2, 63, 1), (-1, 0, 1), (3, 64, 1), (4, 15, 1)]
+    check_attention(ops, paged_case(runs, 2, G, D), 2, G, D)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("runs", [
+    [(0, 0, 130)],                                                     # blocks' and tiles' edges
+    [(0, 37, 64), (1, 0, 65)],                                         # continued; ends in a block
+    [(0, 0, 17), (1, 200, 20), (2, 3, 16), (3, 0, 40), (-1, 0, 30)],   # runs in one block, padding
+])
+def test_attention_of_prompts(ops, D, runs):
+    check_attention(ops, paged_case(runs, 2, 2, D), 2, 2, D)
+
+
+@pytest.mark.parametrize("runs", [[(0, 0, 1), (1, 250, 1)], [(0, 180, 70)]])
+@pytest.mark.parametrize("window", [1, 20, 90])
+def test_attention_with_a_window_on_a_ring(ops, runs, window):
+    ring = (window + PAGE - 1) // PAGE + 2
+    check_attention(ops, paged_case(runs, 1, 2, 64, ring=ring), 1, 2, 64, window, ring)
+
+
+@pytest.mark.parametrize("tokens", [100, 12])  # tiles; ranges
+def test_a_later_token_that_is_no_number_does_not_reach_earlier_ones(ops, tokens):
+    case = paged_case([(0, 0, tokens)], 1, 1, 64)
+    bad = tokens * 7 // 10
+    for name in ("k", "v"):
+        case[name][case["table"][0][bad // PAGE].long(), 0, bad % PAGE] = float("nan")
+    out = torch.empty(tokens, 64, device=DEV)
+    ops.attention_simt(case["q"], out, case["pos"], case["seq"], case["table"], case["k"], case["v"],
+                       1, 1, 64, 0.125)
+    assert bool(torch.isfinite(out[:bad]).all()) and bool(torch.isnan(out[bad:]).all())
