@@ -460,7 +460,10 @@ __global__ void __launch_bounds__(256) scan_kernel(ScanArgs a, int tc) {
 // pairs through the two-wide fma. Row groups lie over the warps' lanes and the warps; their
 // shares of a token's outputs meet by shuffles and, once per tile of tokens, in shared memory.
 // PASS 1: the chunk's contribution and the product of its decays; 2: its outputs. RG: row
-// groups (8 RG >= dim). GS: one decay a head.
+// groups (8 RG >= dim). GS: one decay a head. WKV: the outputs of that recurrence, which reads
+// the state before its token's decay and adds the token times a bonus (1,500 tokens, 24 heads of
+// 128 x 128: 737 us with the scan above in either pass, 204 here; 32 of
+// 64 x 64, 2,048 tokens: 247 and 100).
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack2(float x, float y) {
   f32x2 r;
@@ -496,7 +499,7 @@ struct LcShape {
   static constexpr int WG = RG / RW;                           // shares that meet in shared memory
 };
 
-template <int PASS, int RG, bool GS>
+template <int PASS, int RG, bool GS, bool WKV = false>
 __global__ void __launch_bounds__(LcShape<RG>::THREADS) linear_chunk_kernel(ScanArgs a) {
   using Sh = LcShape<RG>;
   constexpr int LC_TOKENS = Sh::TOKENS, DP = RG * 8, COLS = Sh::COLS, CG = Sh::CG, RW = Sh::RW, WG = Sh::WG;
@@ -564,8 +567,14 @@ __global__ void __launch_bounds__(LcShape<RG>::THREADS) linear_chunk_kernel(Scan
 
   const long long unit = ((long long)blockIdx.x * a.H + h) * dim;  // this chunk's place in wg, ws
   float* S_chunk = a.ws + unit * vdim;
-  const float skip = (PASS == 2 && a.bonus != nullptr) ? a.bonus[h] : 0.f;
+  const float skip = (PASS == 2 && !WKV && a.bonus != nullptr) ? a.bonus[h] : 0.f;
   f32x2 s[4][4], decayed[4];  // [row pair][column]
+  f32x2 bonus[4];
+#pragma unroll
+  for (int p = 0; WKV && p < 4; ++p) {
+    const float* row = a.bonus + (long long)h * dim + row0 + 2 * p;
+    bonus[p] = row0 + 2 * p < dim ? pack2(row[0], row[1]) : pack2(0.f, 0.f);  // (whole fours)
+  }
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
     float4 r[2];
@@ -611,13 +620,15 @@ __global__ void __launch_bounds__(LcShape<RG>::THREADS) linear_chunk_kernel(Scan
         for (int i = 0; i < 2; ++i) {
           const int p = half * 2 + i;
           const f32x2 k = i ? k4.y : k4.x, g = i ? g4.y : g4.x;
+          const f32x2 q = PASS == 2 ? (i ? q4.y : q4.x) : 0ull;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) s[p][c] = fma2(g, s[p][c], mul2(k, v2[c]));
-          if (PASS == 2) {
-            const f32x2 q = i ? q4.y : q4.x;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) o[c] = fma2(q, s[p][c], o[c]);
-          } else {
+          for (int c = 0; c < 4; ++c) {
+            const f32x2 kv = mul2(k, v2[c]);
+            if (WKV) o[c] = fma2(q, fma2(bonus[p], kv, s[p][c]), o[c]);
+            s[p][c] = fma2(g, s[p][c], kv);
+            if (PASS == 2 && !WKV) o[c] = fma2(q, s[p][c], o[c]);
+          }
+          if (PASS == 1) {
             decayed[p] = mul2(decayed[p], g);
           }
         }
@@ -692,24 +703,27 @@ bool linear_chunks_fit(const ScanArgs& a) {
 }
 
 template <int PASS, int RG>
-void launch_linear_chunks(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
+void launch_linear_chunks(const ScanArgs& a, bool wkv, int n_seqs, cudaStream_t stream) {
   const dim3 grid(n_seqs * a.n_chunks, a.H, (a.vdim + LcShape<RG>::COLS - 1) / LcShape<RG>::COLS);
   const dim3 block(LcShape<RG>::THREADS);
   // (pass 1 as a launch without the dependent mark, like any long scan: see launch_scan)
   if (PASS == 1) {
     if (a.g_scalar) fb_launch_serial(linear_chunk_kernel<1, RG, true>, grid, block, 0, stream, a);
     else fb_launch_serial(linear_chunk_kernel<1, RG, false>, grid, block, 0, stream, a);
+  } else if (wkv) {
+    if (a.g_scalar) fb_launch(linear_chunk_kernel<2, RG, true, true>, grid, block, 0, stream, a);
+    else fb_launch(linear_chunk_kernel<2, RG, false, true>, grid, block, 0, stream, a);
   } else {
     if (a.g_scalar) fb_launch(linear_chunk_kernel<2, RG, true>, grid, block, 0, stream, a);
     else fb_launch(linear_chunk_kernel<2, RG, false>, grid, block, 0, stream, a);
   }
 }
 template <int PASS>
-void launch_linear_pass(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
-  if (a.dim <= 32) launch_linear_chunks<PASS, 4>(a, n_seqs, stream);
-  else if (a.dim <= 64) launch_linear_chunks<PASS, 8>(a, n_seqs, stream);
-  else if (a.dim <= 128) launch_linear_chunks<PASS, 16>(a, n_seqs, stream);
-  else launch_linear_chunks<PASS, 32>(a, n_seqs, stream);
+void launch_linear_pass(const ScanArgs& a, bool wkv, int n_seqs, cudaStream_t stream) {
+  if (a.dim <= 32) launch_linear_chunks<PASS, 4>(a, wkv, n_seqs, stream);
+  else if (a.dim <= 64) launch_linear_chunks<PASS, 8>(a, wkv, n_seqs, stream);
+  else if (a.dim <= 128) launch_linear_chunks<PASS, 16>(a, wkv, n_seqs, stream);
+  else launch_linear_chunks<PASS, 32>(a, wkv, n_seqs, stream);
 }
 
 // From the chunks' contributions to their starting states, in place: one thread V neighbouring
@@ -1044,11 +1058,12 @@ FB_API int fb_state_scan(int mode, const float* q, long long q_ld, const float* 
   ScanArgs a{q, q_ld, k, k_ld, v, v_ld, g, g_ld, beta, beta_ld, bonus, state, state_stride,
              s_offset, out, cu_tokens, slots, H, rep, dim, vdim, g_scalar ? 1 : 0, out_scale,
              n_chunks, chunk, ws, wg};
-  if (mode == 2 && n_chunks > 1 && linear_chunks_fit(a)) {
-    launch_linear_pass<1>(a, n_seqs, stream);
+  // (mode 1 reads no step sizes)
+  if (mode != 0 && n_chunks > 1 && linear_chunks_fit(a) && (mode == 2 || beta == nullptr)) {
+    launch_linear_pass<1>(a, mode == 1, n_seqs, stream);
     fb_launch(scan_chunk_starts_kernel<4>, dim3(n_seqs, H, (dim * vdim / 4 + 127) / 128), dim3(128), 0,
               stream, a);
-    launch_linear_pass<2>(a, n_seqs, stream);
+    launch_linear_pass<2>(a, mode == 1, n_seqs, stream);
     return fb_check_launch("state_scan");
   }
   // a column is shared by kp lanes: eight key rows a lane where the head allows it
