@@ -183,6 +183,10 @@ _SIGNATURES = {
                       c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_ll, c_void_p, c_void_p, c_void_p,
                       c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
                       c_void_p, c_int, c_void_p],
+    "fb_chunk_scan": [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p,
+                      c_ll, c_void_p, c_ll, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                      c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p],
+    "fb_chunk_scan_unit": [c_int, c_int, c_int],
     "fb_linear_step_fits": [c_int, c_int, c_int],
     "fb_linear_step": [c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
                        c_void_p, c_int, c_void_p, c_ll, c_ll, c_void_p, c_ll, c_int, c_void_p,
@@ -2785,6 +2789,36 @@ def scan_chunks(ctx, mode: int, H: int, dim: int, vdim: int):
     return (longest + chunk - 1) // chunk, chunk
 
 
+# The delta rule over prompts whose heads have 64 or 128 key channels goes 32 tokens at a time as
+# small matrix products (csrc/chunk_scan.cu) where sequences bring about this many tokens and more
+# (one of 128 tokens, 32 heads of 64 x 64: 26 us against 47 token by token; eight of 60: 72 and 68).
+# Tokens and sequences count as a replayed step pads them, so that both forms of a step take the
+# same path. The workspace holds at most so many floats (256 MB); longer steps are worked in parts.
+CHUNK_SCAN_LEAST = 96
+CHUNK_SCAN_TOKENS, CHUNK_SCAN_ROOM = 32, 1 << 26
+
+
+def _padded(n: int, least: int) -> int:
+    while least < n:
+        least *= 2
+    return least
+
+
+def chunk_scan_unit(ctx, mode: int, T: int, H: int, dim: int, vdim: int, rows, state: StateRows,
+                    field: str) -> int:
+    """Floats of workspace a chunk takes, or 0 where `chunk_scan.cu` does not fit: another
+    recurrence, single tokens, few of them, other sizes, `rows` that no 16-byte piece can address."""
+    if mode != SCAN_DELTA or ctx.is_decode or SCAN_CHUNK_TOKENS <= 0:
+        return 0
+    tokens = _padded(T, 16) if T <= 128 else (T + 127) // 128 * 128
+    if tokens < CHUNK_SCAN_LEAST * _padded(ctx.n_seqs, 1):
+        return 0
+    if any(t.data_ptr() % 16 or t.stride(0) % 4 for t in rows) or state.stride % 4 or \
+            (state.rows.data_ptr() + 4 * state.offset[field]) % 16:
+        return 0
+    return _fn("fb_chunk_scan_unit")(H, dim, vdim)
+
+
 def low_rank_decay(low: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, tau: float,
                    out: torch.Tensor) -> torch.Tensor:
     """out[t, c] = sigmoid(low[t] . weight[c] + bias[c])^(1 / tau), in 32-bit: `low` float32 rows
@@ -2813,6 +2847,22 @@ def state_scan(ctx, mode: int, q, k, v, g, state: StateRows, field: str, out: to
     if out.shape != (T, H * vdim) or out.dtype != torch.float32 or not out.is_contiguous():
         raise KernelError("state_scan: out must be contiguous float32 [T, heads * vdim]")
     f32 = torch.float32
+    unit = chunk_scan_unit(ctx, mode, T, H, dim, vdim, (q, k, out) if decay_per_head else
+                           (q, k, out, g), state, field)
+    if unit:
+        total = T // CHUNK_SCAN_TOKENS + ctx.n_seqs
+        room = min(total, max(1, CHUNK_SCAN_ROOM // unit))
+        ws = torch.empty(room * unit, dtype=f32, device=out.device)
+        _call("fb_chunk_scan", _dev(q, "q", f32, contiguous=False), _rows(q, "q"),
+              _dev(k, "k", f32, contiguous=False), _rows(k, "k"),
+              _dev(v, "v", f32, contiguous=False), _rows(v, "v"),
+              _dev(g, "g", f32, contiguous=False), _rows(g, "g"),
+              _dev(beta, "beta", f32, contiguous=False), _rows(beta, "beta"),
+              state.rows.data_ptr(), state.stride, state.offset[field], out.data_ptr(),
+              _dev(ctx.cu_tokens, "cu_tokens", torch.int32), _dev(ctx.slots, "slots", torch.int32),
+              ctx.n_seqs, H, rep, dim, vdim, 1 if decay_per_head else 0, ws.data_ptr(), total, room,
+              _stream(), tag=("t{} {}x{}", T, dim, vdim))
+        return out
     n_chunks, chunk = scan_chunks(ctx, mode, H, dim, vdim)
     starts = decays = None
     if n_chunks > 1:

@@ -1,0 +1,102 @@
+"""The delta rule in chunks of 32 tokens (csrc/chunk_scan.cu) against the rule token by token in
+float64: sizes, decays a head and a channel, sequences that end inside a chunk or lie side by side,
+steps worked in parts, states that nobody else may touch."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from foundry_b200.kernels import ops as o
+    return o
+
+
+def plain(q, k, v, g, beta, S):
+    """One sequence: q, k [T, H, d]; v [T, H, e]; g [T, H, d or 1]; beta [T, H]; S [H, d, e]."""
+    out = []
+    for t in range(q.shape[0]):
+        S = S * g[t, :, :, None]
+        u = torch.sigmoid(beta[t])[:, None] * (v[t] - torch.einsum("hd,hde->he", k[t], S))
+        S = S + k[t, :, :, None] * u[:, None]
+        out.append(torch.einsum("hd,hde->he", q[t], S))
+    return torch.stack(out), S
+
+
+def run(ops, lens, H, G, d, e, channels, decay, seed=0, nan_at=None):
+    gen = torch.Generator().manual_seed(seed)
+    T, n = sum(lens), len(lens)
+    wide = torch.randn(T, 2 * G * d + H * e, generator=gen).to(DEV)  # q | k | v of one product
+    for a in (0, G * d):
+        part = wide[:, a:a + G * d].view(T, G, d)
+        part /= part.norm(dim=-1, keepdim=True)
+    if nan_at is not None:
+        wide[nan_at] = float("nan")
+    g = decay(torch.rand(T, H * d if channels else H, generator=gen)).to(DEV)
+    beta = torch.randn(T, H + 3, generator=gen).to(DEV)[:, 3:]
+    slots = torch.randperm(n + 2, generator=gen)[:n]
+    rows = (0.3 * torch.randn(n + 3, 4 + H * d * e, generator=gen)).to(DEV)
+    before = rows.clone()
+    cu = [0]
+    for x in lens:
+        cu.append(cu[-1] + x)
+    ctx = types.SimpleNamespace(
+        is_decode=False, n_seqs=n, max_q_len=max(lens), slots=slots.to(torch.int32).to(DEV),
+        cu_tokens=torch.tensor(cu, dtype=torch.int32, device=DEV))
+    state = ops.StateRows(rows, [("tail", 4), ("S", H * d * e)])
+    out = torch.full((T, H * e), 9.0, device=DEV)
+    q, k, v = wide, wide[:, G * d:], wide[:, 2 * G * d:]
+    assert ops.chunk_scan_unit(ctx, ops.SCAN_DELTA, T, H, d, e, (q, k, out), state, "S") > 0
+    ops.state_scan(ctx, ops.SCAN_DELTA, q, k, v, g, state, "S", out, H, H // G, d, e, beta=beta,
+                   decay_per_head=not channels)
+    heads = [wide[:, a:a + G * d].double().view(T, G, d).repeat_interleave(H // G, 1)
+             for a in (0, G * d)]
+    values = wide[:, 2 * G * d:].double().view(T, H, e)
+    want, states = [], before[:, 4:].double().view(n + 3, H, d, e).clone()
+    for s, a, b in zip(slots.tolist(), cu, cu[1:]):
+        part, states[s] = plain(heads[0][a:b], heads[1][a:b], values[a:b],
+                                g[a:b].double().view(b - a, H, -1), beta[a:b].double(), states[s])
+        want.append(part)
+    assert torch.equal(rows[:, :4], before[:, :4])
+    return out.double().view(T, H, e), torch.cat(want), rows[:, 4:].double().view_as(states), states
+
+
+def near(a, b):
+    # sums of up to 128 + 32 products and a substitution of 32 steps, each off by 2^-24 of its
+    # terms: about sqrt(32) * 2^-24 = 3.4e-7 in the 2-norm where they are off independently
+    assert float((a - b).norm() / b.norm()) < 1e-6
+
+
+DECAYS = {"slow": lambda x: 1.0 - 0.05 * x, "any": lambda x: torch.exp(-torch.exp(8.0 * x - 5.0)),
+          "gone": lambda x: torch.where(x < 0.3, 0.0, x)}
+
+
+@pytest.mark.parametrize("decay", list(DECAYS))
+@pytest.mark.parametrize("channels", [False, True])
+@pytest.mark.parametrize("H,G,d,e", [(4, 2, 64, 64), (2, 2, 128, 128), (3, 1, 64, 16), (2, 1, 128, 48)])
+def test_chunks_equal_token_by_token(ops, H, G, d, e, channels, decay):
+    for lens in ([97], [128], [300, 96, 161]):
+        out, want, rows, states = run(ops, lens, H, G, d, e, channels, DECAYS[decay], seed=d + e)
+        near(out, want)
+        near(rows, states)  # every slot's: the sequences' moved on, the others as they were
+
+
+@pytest.mark.parametrize("room", [1, 2, 5])
+def test_steps_in_parts(ops, room, monkeypatch):
+    """A workspace of so many chunks: parts that begin and end inside sequences."""
+    unit = ops._fn("fb_chunk_scan_unit")(2, 64, 32)
+    monkeypatch.setattr(ops, "CHUNK_SCAN_ROOM", room * unit)
+    out, want, rows, states = run(ops, [200, 96, 130], 2, 1, 64, 32, True, DECAYS["any"])
+    near(out, want)
+    near(rows, states)
+
+
+def test_a_later_token_that_is_no_number_does_not_reach_earlier_ones(ops):
+    out, want, _, _ = run(ops, [128], 2, 2, 64, 64, True, DECAYS["slow"], nan_at=70)
+    assert bool(torch.isfinite(out[:70]).all()) and bool(torch.isnan(out[70:]).all())
+    near(out[:70], want[:70])
