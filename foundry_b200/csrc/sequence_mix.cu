@@ -71,6 +71,72 @@ __global__ void token_shift_mix_kernel(const T* h, float* state, long long state
   }
 }
 
+// The same 16 bytes of a row at a time, a run of tokens a thread (their mixing weights are read
+// once). Bound by its bytes.
+template <typename T, int MIXES>
+__global__ void __launch_bounds__(128)
+token_shift_rows_kernel(const T* h, float* state, long long state_stride, long long prev_offset,
+                        const float* __restrict__ mu, T* __restrict__ out,
+                        const int* __restrict__ seq_of_token, const int* __restrict__ cu_tokens,
+                        const int* __restrict__ slots, int T_, int W, int run, int single) {
+  constexpr int V = 16 / sizeof(T);
+  fb_pdl_launch();
+  const int i = (blockIdx.y * blockDim.x + threadIdx.x) * V;
+  if (i >= W) {
+    fb_pdl_wait();
+    return;
+  }
+  float m[MIXES][V];
+#pragma unroll
+  for (int k = 0; k < MIXES; ++k)
+#pragma unroll
+    for (int e = 0; e < V; ++e) m[k][e] = mu[(long long)k * W + i + e];
+  fb_pdl_wait();
+  auto load = [](const T* p, float (&v)[V]) {
+    __align__(16) T raw[V];
+    *reinterpret_cast<uint4*>(raw) = __ldcg(reinterpret_cast<const uint4*>(p));
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = fb_to_float<T>(raw[e]);
+  };
+  const int t0 = blockIdx.x * run, t1 = min(T_, t0 + run);
+  float before[V], x[V];
+  int last_seq = -1;
+  for (int t = t0; t < t1; ++t) {
+    const int seq = seq_of_token[t];
+    if (seq < 0) {
+#pragma unroll
+      for (int k = 0; k < MIXES; ++k)
+        *reinterpret_cast<uint4*>(out + ((long long)k * T_ + t) * W + i) = make_uint4(0u, 0u, 0u, 0u);
+      last_seq = -1;
+      continue;
+    }
+    float* prev_state = state + (long long)slots[seq] * state_stride + prev_offset + i;
+    load(h + (long long)t * W + i, x);
+    if (seq != last_seq) {
+      if (t == cu_tokens[seq]) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) before[e] = __ldcg(prev_state + e);
+      } else {
+        load(h + (long long)(t - 1) * W + i, before);
+      }
+      last_seq = seq;
+    }
+#pragma unroll
+    for (int k = 0; k < MIXES; ++k) {
+      __align__(16) T raw[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) raw[e] = fb_from_float<T>(x[e] + (before[e] - x[e]) * m[k][e]);
+      *reinterpret_cast<uint4*>(out + ((long long)k * T_ + t) * W + i) =
+          *reinterpret_cast<const uint4*>(raw);
+    }
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      before[e] = x[e];
+      if (single) prev_state[e] = x[e];  // (no other thread reads the sequence's row there)
+    }
+  }
+}
+
 // ------------------------------------------------------- tail of the inputs
 // state tail [n_tail, C] <- the last n_tail rows of (old tail ++ this step's rows).
 template <typename T>
@@ -143,6 +209,98 @@ __global__ void conv_silu_unit_kernel(const float* x, long long ld, const float*
   }
   __syncthreads();
   for (int c = threadIdx.x; c < C; c += blockDim.x) out[(size_t)t * C + c] = y[c];
+}
+
+// The same for channels in groups of 32 * V (V = 2 or 4; unit heads are one group each): a warp
+// takes a group and a run of tokens, a lane V neighbouring channels, so a token's row is read
+// once, in whole lines, and the taps' inputs stay in registers. Bound by its bytes (the block a
+// token above reads every input for each of its taps and every channel's taps again).
+template <int V, int TAPS>
+__global__ void __launch_bounds__(256)
+conv_groups_kernel(const float* x, long long ld, const float* __restrict__ w,
+                   const float* __restrict__ bias, float* state, long long state_stride,
+                   long long tail_offset, float* __restrict__ out, int C, int T_,
+                   const int* __restrict__ seq_of_token, const int* __restrict__ cu_tokens,
+                   const int* __restrict__ slots, int n_unit, int n_scaled, float extra,
+                   float unit_eps, int run, int single) {
+  fb_pdl_launch();
+  const int lane = threadIdx.x & 31;
+  const int group = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int c = group * 32 * V + lane * V;
+  if (c >= C) {
+    fb_pdl_wait();
+    return;
+  }
+  auto load = [](const float* p, float (&v)[V]) {
+    if constexpr (V == 4) {
+      const float4 f = __ldcg(reinterpret_cast<const float4*>(p));
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else {
+      const float2 f = __ldcg(reinterpret_cast<const float2*>(p));
+      v[0] = f.x; v[1] = f.y;
+    }
+  };
+  auto store = [](float* p, const float (&v)[V]) {
+    if constexpr (V == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+  };
+  float taps[TAPS][V], b[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    b[e] = bias != nullptr ? bias[c + e] : 0.f;
+#pragma unroll
+    for (int a = 0; a < TAPS; ++a) taps[a][e] = w[(long long)(c + e) * TAPS + a];
+  }
+  fb_pdl_wait();
+  const int t0 = blockIdx.x * run, t1 = min(T_, t0 + run);
+  float hist[TAPS][V];  // the inputs of the last TAPS - 1 tokens, then this one's
+  int last_seq = -1;
+  for (int t = t0; t < t1; ++t) {
+    const int seq = seq_of_token[t];
+    float y[V];
+    if (seq < 0) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) y[e] = 0.f;
+      store(out + (long long)t * C + c, y);
+      last_seq = -1;
+      continue;
+    }
+    float* tail = state + (long long)slots[seq] * state_stride + tail_offset + c;
+    load(x + (long long)t * ld + c, hist[TAPS - 1]);
+    if (seq != last_seq) {  // the run's first token, or a sequence's
+      const int start = cu_tokens[seq];
+#pragma unroll
+      for (int a = 0; a < TAPS - 1; ++a) {
+        const int idx = t - (TAPS - 1 - a) - start;  // row of the step, negative: the tail
+        load(idx >= 0 ? x + (long long)(start + idx) * ld + c : tail + (long long)(TAPS - 1 + idx) * C,
+             hist[a]);
+      }
+      last_seq = seq;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      float acc = 0.f;
+#pragma unroll
+      for (int a = 0; a < TAPS; ++a) acc = fmaf(taps[a][e], hist[a][e], acc);
+      if (bias != nullptr) acc += b[e];
+      y[e] = acc * sigmoidf_(acc);
+      ss = fmaf(y[e], y[e], ss);
+    }
+    if (group < n_unit) {
+      const float r = (group < n_scaled ? extra : 1.0f) / sqrtf(fb_warp_sum(ss) + unit_eps);
+#pragma unroll
+      for (int e = 0; e < V; ++e) y[e] *= r;
+    }
+    store(out + (long long)t * C + c, y);
+    // (a lane reads and writes its own channels of the tail alone)
+#pragma unroll
+    for (int a = 0; a < TAPS - 1; ++a) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) hist[a][e] = hist[a + 1][e];
+      if (single) store(tail + (long long)a * C, hist[a]);
+    }
+  }
 }
 
 // The same without unit heads: nothing ties a token's channels together, so they are
@@ -905,6 +1063,69 @@ __global__ void low_rank_decay_kernel(const float* low, long long ld, const T* _
       out[(size_t)(t0 + t) * n + c] = expf((fminf(z[t], 0.f) - logf(1.0f + expf(-fabsf(z[t])))) * inv_tau);
 }
 
+// ------------------------- a low-rank projection between its two roundings, one kernel
+// out[t, c] = last(sum_r act(in[t, r]) w[c, r]): act (identity or tanh) rounded to the type that
+// the weights are stored in, as the input of a product is, 32-bit sums; last: 0 none, 1 a decay
+// exp(-exp(A[head]) softplus(z + bias[c])), 2 a decay exp(-exp(z + bias[c])). Three launches as
+// cast, product, decay. A block takes up to TOKENS rows, staged in shared memory; a thread a
+// channel, whose weights it reads once for all of them. Bound by issue (an FMA a token and rank,
+// a 16-byte shared-memory read for four of them) from some hundred tokens on, by its launch below.
+constexpr int LOW_RANK = 8;  // weights a thread holds at a time
+template <typename T, int TOKENS, int ACT, int LAST>
+__global__ void __launch_bounds__(128)
+low_rank_kernel(const float* in, long long ld, const T* __restrict__ w, int rank,
+                const float* __restrict__ A, int per_head, const float* __restrict__ bias,
+                float* __restrict__ out, int T_, int n) {
+  fb_pdl_launch();
+  extern __shared__ __align__(16) float rows[];  // [rank][TOKENS]
+  const int t0 = blockIdx.x * TOKENS, c = blockIdx.y * blockDim.x + threadIdx.x;
+  const T* wr = w + (long long)(c < n ? c : 0) * rank;
+  __align__(16) T raw[LOW_RANK];
+  auto weights = [&](int r0) {
+#pragma unroll
+    for (int i = 0; i < (int)(LOW_RANK * sizeof(T) / 16); ++i)
+      reinterpret_cast<uint4*>(raw)[i] = __ldg(reinterpret_cast<const uint4*>(wr + r0) + i);
+  };
+  weights(0);  // constants: asked for before the wait
+  fb_pdl_wait();
+  for (int i = threadIdx.x; i < rank * TOKENS; i += blockDim.x) {
+    const int t = i / rank, r = i - t * rank;
+    const float v = t0 + t < T_ ? __ldcg(in + (long long)(t0 + t) * ld + r) : 0.f;
+    rows[r * TOKENS + t] = fb_to_float<T>(fb_from_float<T>(ACT == 1 ? tanhf(v) : v));
+  }
+  __syncthreads();
+  float z[TOKENS];
+#pragma unroll
+  for (int t = 0; t < TOKENS; ++t) z[t] = 0.f;
+  for (int r0 = 0; r0 < rank; r0 += LOW_RANK) {
+    float v[LOW_RANK];
+#pragma unroll
+    for (int i = 0; i < LOW_RANK; ++i) v[i] = fb_to_float<T>(raw[i]);
+    if (r0 + LOW_RANK < rank) weights(r0 + LOW_RANK);
+#pragma unroll
+    for (int i = 0; i < LOW_RANK; ++i) {
+      const float4* x = reinterpret_cast<const float4*>(rows + (r0 + i) * TOKENS);
+#pragma unroll
+      for (int t = 0; t < TOKENS; t += 4) {
+        const float4 f = x[t / 4];
+        z[t] = fmaf(f.x, v[i], z[t]);
+        z[t + 1] = fmaf(f.y, v[i], z[t + 1]);
+        z[t + 2] = fmaf(f.z, v[i], z[t + 2]);
+        z[t + 3] = fmaf(f.w, v[i], z[t + 3]);
+      }
+    }
+  }
+  if (c >= n) return;
+  const float rate = LAST == 1 ? expf(A[c / per_head]) : 0.f, b = LAST != 0 ? bias[c] : 0.f;
+#pragma unroll
+  for (int t = 0; t < TOKENS; ++t) {
+    if (t0 + t >= T_) break;
+    const float y = z[t] + b;
+    out[(long long)(t0 + t) * n + c] =
+        LAST == 0 ? y : LAST == 1 ? expf(-rate * softplusf_(y)) : expf(-expf(y));
+  }
+}
+
 // out = act(in) rounded to the activation type; act: 0 identity, 1 tanh, 2 the square of relu
 template <typename T>
 __global__ void unary_cast_kernel(const float* in, long long ld, T* __restrict__ out, int n,
@@ -945,6 +1166,48 @@ FB_API int fb_sigmoid_gate(void* x, int dtype, long long ldx, const float* gate,
   return fb_check_launch("sigmoid_gate");
 }
 
+namespace {
+template <typename T, int TOKENS>
+void launch_low_rank(const float* in, long long ld, int act, const T* w, int rank, const float* A,
+                     int per_head, const float* bias, int last, float* out, int T_, int n,
+                     cudaStream_t stream) {
+  // few tokens: small blocks, so that the channels cover more SMs
+  const dim3 block(TOKENS < 16 ? 64 : 128);
+  const dim3 grid((T_ + TOKENS - 1) / TOKENS, (n + block.x - 1) / block.x);
+  const size_t smem = (size_t)rank * TOKENS * 4;
+  auto go = [&](auto kernel) {
+    fb_launch(kernel, grid, block, smem, stream, in, ld, w, rank, A, per_head, bias, out, T_, n);
+  };
+  if (act == 1) {
+    if (last == 0) go(low_rank_kernel<T, TOKENS, 1, 0>);
+    else if (last == 1) go(low_rank_kernel<T, TOKENS, 1, 1>);
+    else go(low_rank_kernel<T, TOKENS, 1, 2>);
+  } else {
+    if (last == 0) go(low_rank_kernel<T, TOKENS, 0, 0>);
+    else if (last == 1) go(low_rank_kernel<T, TOKENS, 0, 1>);
+    else go(low_rank_kernel<T, TOKENS, 0, 2>);
+  }
+}
+}  // namespace
+
+// act: 0 identity, 1 tanh; last: 0 none, 1 the decay with A (one a head of per_head channels), 2
+// the decay without; `w` [n, rank] of whole 16-byte pieces.
+FB_API int fb_low_rank(const float* in, long long ld, int act, const void* w, int w_dtype, int rank,
+                       const float* A, int per_head, const float* bias, int last, float* out, int T,
+                       int n, cudaStream_t stream) {
+  FB_REQUIRE(T >= 0 && n > 0 && rank > 0 && rank % LOW_RANK == 0 && ld >= rank && (act == 0 || act == 1) &&
+                 last >= 0 && last <= 2 && ((uintptr_t)w % 16) == 0, "low_rank: bad arguments");
+  FB_REQUIRE((last == 0 || bias != nullptr) && (last != 1 || (A != nullptr && per_head > 0)),
+             "low_rank: a decay needs its bias and its rates");
+  FB_REQUIRE((size_t)rank * 16 * 4 <= 48 * 1024, "low_rank: rank %d exceeds 768", rank);
+  if (T == 0) return 0;
+  FB_DISPATCH_DTYPE(w_dtype, E, {
+    if (T <= 8) launch_low_rank<E, 8>(in, ld, act, (const E*)w, rank, A, per_head, bias, last, out, T, n, stream);
+    else launch_low_rank<E, 16>(in, ld, act, (const E*)w, rank, A, per_head, bias, last, out, T, n, stream);
+  });
+  return fb_check_launch("low_rank");
+}
+
 FB_API int fb_low_rank_decay(const float* low, long long ld, const void* w, int w_dtype,
                              const float* bias, float tau, float* out, int T, int rank, int n,
                              cudaStream_t stream) {
@@ -964,6 +1227,17 @@ FB_API int fb_token_shift_mix(const void* h, int dtype, float* state, long long 
                               int T, int W, int n_mix, int single, cudaStream_t stream) {
   FB_REQUIRE(T >= 0 && W > 0 && n_mix > 0, "token_shift_mix: bad sizes");
   if (T == 0) return 0;
+  if (n_mix == 5 && W % (dtype == FB_BF16 ? 8 : 4) == 0 && ((uintptr_t)h % 16) == 0 &&
+      ((uintptr_t)out % 16) == 0) {
+    const int run = single ? 1 : T >= 512 ? 4 : 1;
+    FB_DISPATCH_DTYPE(dtype, E, {
+      const int pieces = W / (16 / (int)sizeof(E));
+      fb_launch(token_shift_rows_kernel<E, 5>, dim3((T + run - 1) / run, (pieces + 127) / 128),
+                dim3(128), 0, stream, (const E*)h, state, state_stride, prev_offset, mu, (E*)out,
+                seq_of_token, cu_tokens, slots, T, W, run, single);
+    });
+    return fb_check_launch("token_shift_rows");
+  }
   FB_DISPATCH_DTYPE(dtype, E, (fb_launch(token_shift_mix_kernel<E>, dim3(T), dim3(256), 0, stream,
       (const E*)h, state, state_stride, prev_offset, mu, (E*)out, seq_of_token, cu_tokens, slots,
       T, W, n_mix, single)));
@@ -993,6 +1267,30 @@ FB_API int fb_conv_silu_unit(const float* x, long long ld, const float* w, const
   FB_REQUIRE(n_unit == 0 || (size_t)C * 4 <= 200 * 1024,
              "conv_silu_unit: %d channels do not fit shared memory", C);
   if (T == 0) return 0;
+  // groups of a warp's 16- or 8-byte pieces; runs of 8 tokens, each of which reads the taps - 1
+  // inputs in front of it again (few tokens: shorter runs, more warps)
+  const int width = n_unit > 0 ? dim : C % 128 == 0 ? 128 : 64;
+  if ((width == 64 || width == 128) && C % width == 0 && taps >= 2 && taps <= 4 && ld % 4 == 0 &&
+      state_stride % 4 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)out % 16) == 0 &&
+      ((uintptr_t)(state + tail_offset) % 16) == 0) {
+    const int run = single ? 1 : T >= 512 ? 8 : T >= 64 ? 4 : 2;
+    const dim3 grid((T + run - 1) / run, (C / width + 7) / 8);
+    auto go = [&](auto kernel) {
+      fb_launch(kernel, grid, dim3(256), 0, stream, x, ld, w, bias, state, state_stride, tail_offset,
+                out, C, T, seq_of_token, cu_tokens, slots, n_unit, n_scaled, extra, unit_eps, run,
+                single);
+    };
+    if (width == 64) {
+      if (taps == 2) go(conv_groups_kernel<2, 2>);
+      else if (taps == 3) go(conv_groups_kernel<2, 3>);
+      else go(conv_groups_kernel<2, 4>);
+    } else {
+      if (taps == 2) go(conv_groups_kernel<4, 2>);
+      else if (taps == 3) go(conv_groups_kernel<4, 3>);
+      else go(conv_groups_kernel<4, 4>);
+    }
+    return fb_check_launch("conv_groups");
+  }
   if (n_unit == 0) {
     fb_launch(conv_silu_kernel, dim3(T, (C + 255) / 256), dim3(256), 0, stream, x, ld, w, bias, taps,
               state, state_stride, tail_offset, out, C, seq_of_token, cu_tokens, slots, single);

@@ -183,6 +183,8 @@ _SIGNATURES = {
                       c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_ll, c_void_p, c_void_p, c_void_p,
                       c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
                       c_void_p, c_int, c_void_p],
+    "fb_low_rank": [c_void_p, c_ll, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int,
+                    c_void_p, c_int, c_int, c_void_p],
     "fb_chunk_scan": [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p,
                       c_ll, c_void_p, c_ll, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                       c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p],
@@ -2817,6 +2819,29 @@ def chunk_scan_unit(ctx, mode: int, T: int, H: int, dim: int, vdim: int, rows, s
             (state.rows.data_ptr() + 4 * state.offset[field]) % 16:
         return 0
     return _fn("fb_chunk_scan_unit")(H, dim, vdim)
+
+
+def low_rank(x: torch.Tensor, weight: torch.Tensor, act: str = "identity",
+             bias: Optional[torch.Tensor] = None, A: Optional[torch.Tensor] = None,
+             per_head: int = 1) -> Optional[torch.Tensor]:
+    """float32 [T, n] = act(x) weight^T, `x` float32 rows [T, rank] (possibly strided) rounded to
+    the weights' type in front of the product; with `bias` the sums become decays, exp(-exp(A)
+    softplus(z + bias)) or, without `A`, exp(-exp(z + bias)). None where one kernel does not fit
+    (ranks of no whole 16-byte pieces): the caller then goes cast, product, decay."""
+    T, rank = x.shape
+    n = weight.shape[0]
+    if rank % 8 or rank > 512 or weight.data_ptr() % 16 or not weight.is_contiguous():
+        return None
+    if weight.shape[1] != rank or (bias is not None and bias.numel() != n):
+        raise KernelError(f"low_rank: {tuple(x.shape)} x {tuple(weight.shape)}")
+    out = torch.empty((T, n), dtype=torch.float32, device=x.device)
+    _call("fb_low_rank", _dev(x, "x", torch.float32, contiguous=False), _rows(x, "x"),
+          {"identity": 0, "tanh": 1}[act], _dev(weight, "weight"), code_of(weight.dtype), rank,
+          0 if A is None else _dev(A, "A", torch.float32), per_head,
+          0 if bias is None else _dev(bias, "bias", torch.float32),
+          0 if bias is None else 1 if A is not None else 2, out.data_ptr(), T, n, _stream(),
+          tag=("t{} r{} n{}", T, rank, n))
+    return out
 
 
 def low_rank_decay(low: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, tau: float,

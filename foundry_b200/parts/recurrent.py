@@ -121,11 +121,15 @@ class GatedDeltaChannel(Part):
         if not ops.conv_silu_unit(ctx, p, self.conv, state, "tail", qkv, C, n_unit=2 * G, dim=d,
                                   n_scaled=G, extra=d ** -0.5, unit_eps=self.unit_eps):
             ops.state_tail_update(ctx, p, state, "tail", self.taps - 1, C)
-        low = torch.empty((T, self.decay_rank + self.gate_rank), dtype=x.dtype, device=x.device)
-        ops.unary_cast(p[:, C + H:], low)
-        decay = product_f32(low[:, :self.decay_rank], self.a2)
-        gate = product_f32(low[:, self.decay_rank:], self.g2)
-        ops.decay_gate(decay, d, self.dt_bias, self.A_log)
+        at = C + H + self.decay_rank
+        decay = ops.low_rank(p[:, C + H:at], self.a2, bias=self.dt_bias, A=self.A_log, per_head=d)
+        gate = ops.low_rank(p[:, at:at + self.gate_rank], self.g2)
+        if decay is None or gate is None:
+            low = torch.empty((T, self.decay_rank + self.gate_rank), dtype=x.dtype, device=x.device)
+            ops.unary_cast(p[:, C + H:], low)
+            decay = product_f32(low[:, :self.decay_rank], self.a2)
+            gate = product_f32(low[:, self.decay_rank:], self.g2)
+            ops.decay_gate(decay, d, self.dt_bias, self.A_log)
         o = torch.empty((T, H * v), **f32)
         ops.state_scan(ctx, ops.SCAN_DELTA, qkv, qkv[:, G * d:], qkv[:, 2 * G * d:], decay, state,
                        "S", o, H, H // G, d, v, beta=p[:, C:])
@@ -326,10 +330,13 @@ class WkvTimeMix(Part):
             ops.state_tail_update(ctx, x, state, "prev", 1, W)
         r, k, v, g = (product_f32(mixes[i], w) for i, w in
                       enumerate((self.r, self.k, self.v, self.g)))
-        low = torch.empty((T, self.decay_rank), dtype=x.dtype, device=x.device)
-        ops.unary_cast(product_f32(mixes[4], self.w1), low, "tanh")
-        decay = product_f32(low, self.w2)
-        ops.decay_gate(decay, d, self.w0, None)
+        raw = product_f32(mixes[4], self.w1)
+        decay = ops.low_rank(raw, self.w2, "tanh", bias=self.w0)
+        if decay is None:
+            low = torch.empty((T, self.decay_rank), dtype=x.dtype, device=x.device)
+            ops.unary_cast(raw, low, "tanh")
+            decay = product_f32(low, self.w2)
+            ops.decay_gate(decay, d, self.w0, None)
         o = torch.empty((T, H * d), dtype=torch.float32, device=x.device)
         ops.state_scan(ctx, ops.SCAN_WKV, r, k, v, decay, state, "S", o, H, 1, d, d, bonus=self.u)
         y = torch.empty((T, H * d), dtype=x.dtype, device=x.device)

@@ -1,0 +1,113 @@
+"""The per-token pieces around the recurrences that read whole 16-byte pieces or take several steps
+in one kernel, at the edges of their runs and blocks, against plain statements of the same work."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from foundry_b200.kernels import ops as o
+    return o
+
+
+def step_of(runs, n_slots, decode=False):
+    """A context of `runs` = tokens of each sequence, three padding rows behind them."""
+    seq, cu = [], [0]
+    for i, n in enumerate(runs):
+        seq += [i] * n
+        cu.append(cu[-1] + n)
+    seq += [-1] * 3
+    as_int = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    slots = torch.randperm(n_slots, generator=torch.Generator().manual_seed(3))[:len(runs)].tolist()
+    return types.SimpleNamespace(is_decode=decode, n_seqs=len(runs), seq_of_token=as_int(seq),
+                                 cu_tokens=as_int(cu), slots=as_int(slots)), slots, cu, len(seq)
+
+
+@pytest.mark.parametrize("runs", [[1, 1, 1, 1, 1], [1], [3, 70, 1, 2], [530, 9]])
+@pytest.mark.parametrize("dim,taps", [(64, 2), (64, 4), (128, 3), (128, 4), (96, 4)])
+def test_convolution(ops, runs, dim, taps):
+    decode = max(runs) == 1
+    ctx, slots, cu, T = step_of(runs, 7, decode)
+    n_unit, n_scaled, heads, extra = 3, 1, 5, 0.3
+    C = heads * dim
+    gen = torch.Generator().manual_seed(dim + taps)
+    x = torch.randn(T, C + 8, generator=gen).to(DEV)[:, 4:C + 4]
+    w, bias = torch.randn(C, taps, generator=gen).to(DEV), torch.randn(C, generator=gen).to(DEV)
+    for b, unit in ((None, n_unit), (bias, n_unit), (bias, 0)):
+        rows = torch.randn(8, 8 + (taps - 1) * C, generator=torch.Generator().manual_seed(9)).to(DEV)
+        before = rows.clone()
+        state = ops.StateRows(rows, [("other", 8), ("tail", (taps - 1) * C)])
+        out = torch.full((T, C), 9.0, device=DEV)
+        moved = ops.conv_silu_unit(ctx, x, w, state, "tail", out, C, n_unit=unit, dim=dim,
+                                   n_scaled=n_scaled if unit else 0, extra=extra, unit_eps=1e-6, bias=b)
+        assert moved == decode
+        for s, slot in enumerate(slots):
+            past = before[slot, 8:].view(taps - 1, C).double()
+            full = torch.cat([past, x[cu[s]:cu[s + 1]].double()])
+            n = cu[s + 1] - cu[s]
+            y = sum(full[a:a + n] * w[:, a].double() for a in range(taps)) + (0 if b is None else b.double())
+            y = (y * torch.sigmoid(y)).view(n, heads, dim)
+            if unit:
+                r = 1.0 / torch.sqrt((y[:, :unit] ** 2).sum(-1, keepdim=True) + 1e-6)
+                r[:, :n_scaled] *= extra
+                y[:, :unit] *= r
+            # four products, an exponential and a root: a few 2^-23 of values of up to ten
+            assert float((out[cu[s]:cu[s + 1]].double() - y.view(n, C)).abs().max()) < 2e-5
+            want = full[-(taps - 1):] if decode else past
+            assert torch.equal(rows[slot, 8:].view(taps - 1, C), want.float())
+        assert bool((out[cu[-1]:] == 0).all()) and torch.equal(rows[:, :8], before[:, :8])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("runs", [[1, 1, 1], [5, 1, 3], [517, 2]])
+@pytest.mark.parametrize("W", [64, 2056, 100])
+def test_token_shift(ops, runs, W, dtype):
+    decode = max(runs) == 1
+    ctx, slots, cu, T = step_of(runs, 5, decode)
+    gen = torch.Generator().manual_seed(W)
+    h = torch.randn(T, W, generator=gen).to(dtype).to(DEV)
+    mu = torch.rand(5, W, generator=gen).to(DEV)
+    rows = torch.randn(6, 4 + W, generator=gen).to(DEV)
+    before = rows.clone()
+    out = torch.full((5, T, W), 9.0, dtype=dtype, device=DEV)
+    ops.token_shift_mix(ctx, h, ops.StateRows(rows, [("other", 4), ("prev", W)]), "prev", mu, out)
+    for s, slot in enumerate(slots):
+        x = h[cu[s]:cu[s + 1]].float()
+        prev = torch.cat([before[slot, 4:][None], x[:-1]])
+        want = (x + (prev - x) * mu[:, None]).to(dtype)
+        assert float((out[:, cu[s]:cu[s + 1]].float() - want.float()).abs().max()) < \
+            (0.04 if dtype == torch.bfloat16 else 1e-6)  # a rounding of values of up to five
+        assert torch.equal(rows[slot, 4:], x[-1] if decode else before[slot, 4:])
+    assert bool((out[:, cu[-1]:] == 0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 16, 17, 50])
+@pytest.mark.parametrize("rank,n", [(8, 5), (64, 200), (40, 129)])
+def test_low_rank(ops, T, rank, n, dtype):
+    gen = torch.Generator().manual_seed(T + rank)
+    x = torch.randn(T, rank + 7, generator=gen).to(DEV)[:, 3:3 + rank]
+    w = (torch.randn(n, rank, generator=gen) / rank ** 0.5).to(dtype).to(DEV)
+    bias = torch.randn(n, generator=gen).to(DEV)
+    per_head = 1 if n % 5 else 5
+    A = torch.randn(n // per_head, generator=gen).to(DEV)
+    for act in ("identity", "tanh"):
+        rounded = (torch.tanh(x) if act == "tanh" else x).to(dtype).double()
+        z = rounded @ w.double().T
+        rate = torch.exp(A.double()).repeat_interleave(per_head)
+        y = z + bias.double()
+        for kw, want in ((dict(), z), (dict(bias=bias), torch.exp(-torch.exp(y))),
+                         (dict(bias=bias, A=A, per_head=per_head),
+                          torch.exp(-rate * torch.nn.functional.softplus(y)))):
+            got = ops.low_rank(x, w, act, **kw)
+            # sums of `rank` products near one; a decay moves by no more than its exponent does
+            # (a hyperbolic tangent next to a rounding edge may round the other way)
+            bound = 4e-3 if act == "tanh" and dtype == torch.bfloat16 else 2e-5
+            assert float((got.double() - want).abs().max()) < bound
+    assert ops.low_rank(x[:, :rank - 1], w[:, :rank - 1].contiguous()) is None
