@@ -116,8 +116,9 @@ struct ResidualSink {
 template <bool ROPE> struct RopeArg { using type = NoRope; };
 template <> struct RopeArg<true> { using type = RopeWrite; };
 struct NoSink {};
-// The second product of a pair: CTAs from `first` on work it (float32 out, plain epilogue).
-struct SecondProduct {
+// Further products of the same tokens in the grid: CTAs from `first` on work one (float32 out,
+// plain epilogue).
+struct OneMore {
   const __nv_bfloat16* x;
   long long ldx;
   const __nv_bfloat16* w;
@@ -126,14 +127,19 @@ struct SecondProduct {
   long long ldo;
   int N, K, first;
 };
-struct NoSecond {};
-template <bool PAIR> struct PairArg { using type = NoSecond; };
-template <> struct PairArg<true> { using type = SecondProduct; };
+constexpr int FB_SKINNY_MOST_PRODUCTS = 6;
+struct MoreProducts {
+  int count;
+  OneMore of[FB_SKINNY_MOST_PRODUCTS - 1];
+};
+struct NoMore {};
+template <bool MANY> struct MoreArg { using type = NoMore; };
+template <> struct MoreArg<true> { using type = MoreProducts; };
 // what a kernel instance ends with
 constexpr int MODE_PLAIN = 0;  // store, or SiLU(gate) * up
 constexpr int MODE_ROPE = 1;   // rotate and write queries, keys, values
 constexpr int MODE_SINK = 2;   // add into the residual rows in front of a norm
-constexpr int MODE_PAIR = 3;   // store; the grid holds two products
+constexpr int MODE_MANY = 3;   // store; the grid holds several products
 constexpr int MODE_CLAMP = 4;  // (gate, up) pairs with clamped halves and biases
 template <int MODE> struct EndArg { using type = NoSink; };
 template <> struct EndArg<MODE_SINK> { using type = ResidualSink; };
@@ -158,7 +164,7 @@ gemm_skinny_kernel(const __nv_bfloat16* x, long long ldx,
                    const typename RopeArg<MODE == MODE_ROPE>::type rw,
                    const RowScale scale,
                    const typename EndArg<MODE>::type sink,
-                   const typename PairArg<MODE == MODE_PAIR>::type second) {
+                   const typename MoreArg<MODE == MODE_MANY>::type more) {
   constexpr bool ROPE = MODE == MODE_ROPE, SINK = MODE == MODE_SINK;
   __shared__ float red[WARPS][16][8 * NT + 1];
   __shared__ float scale_part[4][16];
@@ -166,13 +172,16 @@ gemm_skinny_kernel(const __nv_bfloat16* x, long long ldx,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   int group = blockIdx.x;
-  if constexpr (MODE == MODE_PAIR) {
-    if (group >= second.first) {
-      group -= second.first;
-      x = second.x; ldx = second.ldx;
-      w = second.w; ldw = second.ldw;
-      out = second.out; ldo = second.ldo;
-      N = second.N; K = second.K;
+  if constexpr (MODE == MODE_MANY) {
+#pragma unroll
+    for (int i = 0; i < FB_SKINNY_MOST_PRODUCTS - 1; ++i) {
+      if (i < more.count && (int)blockIdx.x >= more.of[i].first) {
+        group = blockIdx.x - more.of[i].first;
+        x = more.of[i].x; ldx = more.of[i].ldx;
+        w = more.of[i].w; ldw = more.of[i].ldw;
+        out = more.of[i].out; ldo = more.of[i].ldo;
+        N = more.of[i].N; K = more.of[i].K;
+      }
     }
   }
   const int n0 = group * 16;
@@ -529,7 +538,7 @@ int launch_skinny(const void* x, long long ldx, const void* w, long long ldw, vo
                   long long next_bytes, int ksplit, long long plane_stride, int warps,
                   int late_trigger, const RopeWrite& rw, const RowScale& scale,
                   const ResidualSink& sink, cudaStream_t stream,
-                  SecondProduct second = SecondProduct{}, const FbGluClamp& clamp = FbGluClamp{}) {
+                  MoreProducts more = MoreProducts{}, const FbGluClamp& clamp = FbGluClamp{}) {
   FB_REQUIRE(next_bytes >= 0 && next_bytes % 16 == 0 && ((uintptr_t)next % 16) == 0,
              "gemm_skinny: the prefetch range must be 16-byte aligned and a multiple of 16 bytes");
   FB_REQUIRE(T > 0 && T <= 16 && N > 0 && K > 0, "gemm_skinny: bad sizes T=%d N=%d K=%d", T, N, K);
@@ -553,13 +562,16 @@ int launch_skinny(const void* x, long long ldx, const void* w, long long ldw, vo
                                sink.ldr >= N && sink.ldxg >= N && sink.ss_stride >= T),
              "gemm_skinny: the residual sink needs its four arrays, rows of %d and shares of %d",
              N, T);
-  second.first = (N + 15) / 16;
-  const int blocks = second.first + (second.w != nullptr ? (second.N + 15) / 16 : 0);
+  int blocks = (N + 15) / 16, longest = K;
+  for (int i = 0; i < more.count; ++i) {
+    more.of[i].first = blocks;
+    blocks += (more.of[i].N + 15) / 16;
+    longest = more.of[i].K > longest ? more.of[i].K : longest;
+  }
   // Warps per CTA: as many as still let every CTA of the grid be resident at
   // once (one CTA of 16 warps, two of 8 or five of 4 fit an SM). A second, thin
   // round of CTAs costs a whole round's latency: measured on the 3B decode step,
   // 192 CTAs of 16 warps (148 + 44) were 4 us a call slower than 192 of 8.
-  const int longest = second.w != nullptr && second.K > K ? second.K : K;
   const int chunks = ((longest + CHUNK - 1) / CHUNK + ksplit - 1) / ksplit;
   if (warps == 0) {
     const long long ctas = (long long)blocks * ksplit;
@@ -570,19 +582,19 @@ int launch_skinny(const void* x, long long ldx, const void* w, long long ldw, vo
   const int unroll = per >= 4 ? 4 : per >= 3 ? 3 : 2;
   // CTAs from this one on are the last half round of the grid (16 / warps CTAs fit an SM)
   const int early_from = blocks * ksplit - (16 / warps) * (sm_count() / 2);
-#define FB_SKINNY_R(NT, W, U, MODE, ROPE_ARG, SINK_ARG, PAIR_ARG)                                       \
+#define FB_SKINNY_R(NT, W, U, MODE, ROPE_ARG, SINK_ARG, MORE_ARG)                                       \
   do {                                                                                         \
   fb_launch(gemm_skinny_kernel<NT, W, U, MODE>, dim3(blocks, ksplit), dim3(W * 32),            \
             shares_bytes, stream, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, ldw,   \
             out, ldo, out_f32, T, N, K, epilogue, next, next_bytes, plane_stride,               \
-            late_trigger, early_from, ROPE_ARG, scale, SINK_ARG, PAIR_ARG); } while (0)
+            late_trigger, early_from, ROPE_ARG, scale, SINK_ARG, MORE_ARG); } while (0)
 #define FB_SKINNY(NT, W, U)                                                      \
   do {                                                                           \
-    if (epilogue == 2) FB_SKINNY_R(NT, W, U, MODE_ROPE, rw, NoSink{}, NoSecond{});            \
-    else if (epilogue == 3) FB_SKINNY_R(NT, W, U, MODE_SINK, NoRope{}, sink, NoSecond{});     \
-    else if (epilogue == 6) FB_SKINNY_R(NT, W, U, MODE_CLAMP, NoRope{}, clamp, NoSecond{});   \
-    else if (second.w != nullptr) FB_SKINNY_R(NT, W, U, MODE_PAIR, NoRope{}, NoSink{}, second); \
-    else FB_SKINNY_R(NT, W, U, MODE_PLAIN, NoRope{}, NoSink{}, NoSecond{});                   \
+    if (epilogue == 2) FB_SKINNY_R(NT, W, U, MODE_ROPE, rw, NoSink{}, NoMore{});            \
+    else if (epilogue == 3) FB_SKINNY_R(NT, W, U, MODE_SINK, NoRope{}, sink, NoMore{});     \
+    else if (epilogue == 6) FB_SKINNY_R(NT, W, U, MODE_CLAMP, NoRope{}, clamp, NoMore{});   \
+    else if (more.count > 0) FB_SKINNY_R(NT, W, U, MODE_MANY, NoRope{}, NoSink{}, more);      \
+    else FB_SKINNY_R(NT, W, U, MODE_PLAIN, NoRope{}, NoSink{}, NoMore{});                   \
   } while (0)
 #define FB_SKINNY_U(NT, W)                                    \
   do {                                                        \
@@ -634,7 +646,7 @@ FB_API int fb_gemm_skinny(const void* x, long long ldx, const void* w, long long
                        scale_dim > 0 ? 1.0f / (float)scale_dim : 0.f, scale_eps};
   return launch_skinny(x, ldx, w, ldw, out, ldo, out_f32, T, N, K, epilogue, next, next_bytes,
                        ksplit, plane_stride, warps, 1, RopeWrite{}, scale, ResidualSink{}, stream,
-                       SecondProduct{}, FbGluClamp{glu_limit, glu_alpha, glu_shift, glu_bias});
+                       MoreProducts{}, FbGluClamp{glu_limit, glu_alpha, glu_shift, glu_bias});
 }
 
 // Two products of the same T tokens in one launch, float32 out: out1 = x1 w1^T ([T, N1]) and
@@ -647,10 +659,34 @@ FB_API int fb_gemm_skinny_pair(const void* x1, long long ldx1, const void* w1, l
   FB_REQUIRE(N2 > 0 && K2 > 0 && K2 % 8 == 0 && ldx2 % 8 == 0 && ldw2 % 8 == 0 && w2 != nullptr &&
                  ((uintptr_t)x2 % 16) == 0 && ((uintptr_t)w2 % 16) == 0,
              "gemm_skinny_pair: the second product's sizes must keep 16-byte alignment");
-  const SecondProduct second{(const __nv_bfloat16*)x2, ldx2, (const __nv_bfloat16*)w2, ldw2, out2,
-                             ldo2, N2, K2, 0};
+  MoreProducts more{};
+  more.count = 1;
+  more.of[0] = OneMore{(const __nv_bfloat16*)x2, ldx2, (const __nv_bfloat16*)w2, ldw2, out2, ldo2,
+                       N2, K2, 0};
   return launch_skinny(x1, ldx1, w1, ldw1, out1, ldo1, 1, T, N1, K1, 0, next, next_bytes, 1, 0, 0, 1,
-                       RopeWrite{}, RowScale{}, ResidualSink{}, stream, second);
+                       RopeWrite{}, RowScale{}, ResidualSink{}, stream, more);
+}
+
+// Several products of the same T tokens in one launch, float32 out: out_i = x_i w_i^T ([T, N_i]).
+// `products`: on the host, eight numbers each: x, ldx, w, ldw, out, ldo, N, K.
+FB_API int fb_gemm_skinny_many(const long long* products, int count, int T, const void* next,
+                               long long next_bytes, cudaStream_t stream) {
+  FB_REQUIRE(count >= 1 && count <= FB_SKINNY_MOST_PRODUCTS, "gemm_skinny_many: %d products", count);
+  MoreProducts more{};
+  more.count = count - 1;
+  for (int i = 1; i < count; ++i) {
+    const long long* p = products + 8 * i;
+    OneMore& m = more.of[i - 1];
+    m = OneMore{(const __nv_bfloat16*)p[0], p[1], (const __nv_bfloat16*)p[2], p[3], (float*)p[4],
+                p[5], (int)p[6], (int)p[7], 0};
+    FB_REQUIRE(m.N > 0 && m.K > 0 && m.K % 8 == 0 && m.ldx % 8 == 0 && m.ldw % 8 == 0 &&
+                   m.w != nullptr && ((uintptr_t)m.x % 16) == 0 && ((uintptr_t)m.w % 16) == 0,
+               "gemm_skinny_many: product %d's sizes must keep 16-byte alignment", i);
+  }
+  return launch_skinny((const void*)products[0], products[1], (const void*)products[2], products[3],
+                       (void*)products[4], products[5], 1, T, (int)products[6], (int)products[7], 0,
+                       next, next_bytes, 1, 0, 0, 1, RopeWrite{}, RowScale{}, ResidualSink{}, stream,
+                       more);
 }
 
 // The projection in front of a norm (see the top of the file): resid [T, N]

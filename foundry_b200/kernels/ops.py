@@ -67,6 +67,7 @@ _SIGNATURES = {
     "fb_rope_table": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
     "fb_gemm_tc_status": [c_void_p],
     "fb_gemm_tc_pair_status": [c_void_p],
+    "fb_gemm_skinny_many": [c_void_p, c_int, c_int, c_void_p, c_ll, c_void_p],
     "fb_gemm_skinny_pair": [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_int, c_int, c_void_p,
                             c_ll, c_void_p, c_ll, c_void_p, c_ll, c_int, c_int, c_int, c_void_p, c_ll,
                             c_void_p],
@@ -904,6 +905,39 @@ def gemm_skinny_pair(x1: torch.Tensor, w1: torch.Tensor, x2: torch.Tensor, w2: t
     _call("fb_gemm_skinny_pair", *args, M, *_prefetch_range(then_reads), _stream(),
           tag=("m{} k{}+{} n{}+{}", M, w1.shape[1], w2.shape[1], w1.shape[0], w2.shape[0]))
     return tuple(outs)
+
+
+SKINNY_MOST_PRODUCTS = 6
+
+
+def skinny_many_fits(pairs) -> bool:
+    """Whether `gemm_skinny_many` takes these (x, w) products."""
+    rows = pairs[0][0].shape[0]
+    return (len(pairs) <= SKINNY_MOST_PRODUCTS and 0 < rows <= SKINNY_ROWS
+            and all(x.dtype == w.dtype == torch.bfloat16 and x.shape[0] == rows
+                    and _tc_usable(x, w, x) for x, w in pairs))
+
+
+def gemm_skinny_many(pairs, then_reads: Optional[torch.Tensor] = None):
+    """[x w^T for (x, w) in pairs] in float32 for up to 16 token rows each, one launch of the
+    weight-streaming kernel for all of them (a launch of its own and its ramp are 4 to 5 us of a
+    replayed step, as much as streaming 30 MB)."""
+    M = pairs[0][0].shape[0]
+    outs, numbers = [], []
+    for x, w in pairs:
+        if x.shape != (M, w.shape[1]):
+            raise KernelError(f"gemm_skinny_many: x {tuple(x.shape)}, w {tuple(w.shape)}")
+        out = torch.empty((M, w.shape[0]), dtype=torch.float32, device=x.device)
+        outs.append(out)
+        numbers += [_dev(x, "x", torch.bfloat16, contiguous=False), _rows(x, "x"),
+                    _dev(w, "w", torch.bfloat16, contiguous=False), _rows(w, "w"), out.data_ptr(),
+                    w.shape[0], w.shape[0], w.shape[1]]
+    table = (ctypes.c_longlong * len(numbers))(*numbers)
+    _call("fb_gemm_skinny_many", ctypes.addressof(table), len(pairs), M,
+          *_prefetch_range(then_reads), _stream(),
+          tag=("m{} k{} n{} x{}", M, pairs[0][1].shape[1], sum(w.shape[0] for _, w in pairs),
+               len(pairs)))
+    return outs
 
 
 def gemm_skinny_residual(x: torch.Tensor, w: torch.Tensor, sink: ResidualSink,

@@ -40,6 +40,14 @@ def product_pair(x1: torch.Tensor, w1: torch.Tensor, x2: torch.Tensor, w2: torch
     return product_planes(x1, w1, then_reads=w2), product_planes(x2, w2, then_reads=then_reads)
 
 
+def products_f32(pairs):
+    """[x w^T for (x, w) in pairs], each as `product_f32` gives it; a handful of tokens takes one
+    launch for all of them."""
+    if min(x.shape[1] for x, _ in pairs) >= SMALL_K and ops.skinny_many_fits(pairs):
+        return ops.gemm_skinny_many(pairs)
+    return [product_f32(x, w) for x, w in pairs]
+
+
 def product_to_residual(ctx, x: torch.Tensor, w: torch.Tensor):
     """A part's last product, whose result joins the residual: float32 as
     `product_f32` gives it, or, where the block offers the next norm's sink

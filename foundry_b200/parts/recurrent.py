@@ -61,7 +61,7 @@ from ..cache.store import StateRequest, StateView
 from ..kernels import ops
 from ..weights.loader import ExpectedTensor
 from .base import Fetch, Part, register_mixer
-from .products import product_f32, product_to_residual
+from .products import product_f32, product_to_residual, products_f32
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
@@ -328,9 +328,8 @@ class WkvTimeMix(Part):
         mixes = torch.empty((len(self.MIXES), T, W), dtype=x.dtype, device=x.device)
         if not ops.token_shift_mix(ctx, x, state, "prev", self.mu, mixes):
             ops.state_tail_update(ctx, x, state, "prev", 1, W)
-        r, k, v, g = (product_f32(mixes[i], w) for i, w in
-                      enumerate((self.r, self.k, self.v, self.g)))
-        raw = product_f32(mixes[4], self.w1)
+        r, k, v, g, raw = products_f32([(mixes[i], w) for i, w in enumerate(
+            (self.r, self.k, self.v, self.g, self.w1))])
         decay = ops.low_rank(raw, self.w2, "tanh", bias=self.w0)
         if decay is None:
             low = torch.empty((T, self.decay_rank), dtype=x.dtype, device=x.device)

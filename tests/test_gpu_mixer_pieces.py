@@ -111,3 +111,18 @@ def test_low_rank(ops, T, rank, n, dtype):
             bound = 4e-3 if act == "tanh" and dtype == torch.bfloat16 else 2e-5
             assert float((got.double() - want).abs().max()) < bound
     assert ops.low_rank(x[:, :rank - 1], w[:, :rank - 1].contiguous()) is None
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 16])
+def test_several_products_in_one_launch(ops, T):
+    gen = torch.Generator().manual_seed(T)
+    sizes = [(128, 40), (128, 16), (256, 7), (64, 300), (128, 33), (72, 64)]
+    pairs = [(torch.randn(T, k, generator=gen).to(torch.bfloat16).to(DEV),
+              torch.randn(n, k, generator=gen).to(torch.bfloat16).to(DEV)) for k, n in sizes]
+    for count in range(1, 7):
+        assert ops.skinny_many_fits(pairs[:count])
+        for (x, w), out in zip(pairs, ops.gemm_skinny_many(pairs[:count])):
+            want = x.double() @ w.double().T
+            size = x.double().abs() @ w.double().abs().T
+            assert bool(((out.double() - want).abs() <= x.shape[1] * 2.0 ** -23 * size).all())
+    assert not ops.skinny_many_fits(pairs + pairs[:1])
