@@ -299,55 +299,97 @@ FB_API int fb_moe_experts_rows(const void* h, int dtype, const void* gate_up, co
 //                     order of c, so the sum does not depend on the sorting
 namespace {
 
+// One block of WARPS warps sorts the pairs, an expert's in the order of their indices: a warp takes
+// a run of neighbouring pairs, 32 at a time; lanes with the same expert find one another by a
+// match, so that a warp counts its run's pairs without atomics (pass 1), the runs' counts become
+// first places (pass 2), and the run is placed (pass 3). 4,000 pairs of 16 experts on 32 warps end
+// 2 us behind the choice that they wait for; a warp an expert, each reading all the pairs, took 24.
+template <int WARPS>
 __device__ __forceinline__ void sort_pairs(const int* chosen, int n_pairs, int E,
                                            int* __restrict__ counts, int* __restrict__ starts,
                                            int* __restrict__ place, int* __restrict__ pair_at) {
-  // one block; counts and starts live in shared memory (E <= 256)
-  __shared__ int cnt[256], start[257];
-  for (int e = threadIdx.x; e < 256; e += blockDim.x) cnt[e] = 0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int e = chosen[i];
-    if (e >= 0 && e < E) atomicAdd(&cnt[e], 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0;
-    for (int e = 0; e < E; ++e) { start[e] = at; at += cnt[e]; }
-    start[E] = at;
-  }
-  __syncthreads();
-  // a warp places the pairs of an expert in the order of their indices (a fixed
-  // order): 32 pairs at a time, each lane's place from a ballot of the matching lanes
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  for (int e = warp; e < E; e += nwarps) {
-    int at = start[e];
-    for (int base = 0; base < n_pairs; base += 32) {
-      const int i = base + lane;
-      const bool mine = i < n_pairs && chosen[i] == e;
-      const unsigned hits = __ballot_sync(0xffffffffu, mine);
-      if (mine) {
-        const int where = at + __popc(hits & ((1u << lane) - 1u));
-        place[i] = where;
-        pair_at[where] = i;
+  __shared__ int held[WARPS][256];  // E <= 256
+  __shared__ int start[256];
+  constexpr int AHEAD = 4;  // loads of a run under way together
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int run = (n_pairs + WARPS * 32 - 1) / (WARPS * 32) * 32;
+  const int first = warp * run, last = min(n_pairs, first + run);
+  for (int e = lane; e < E; e += 32) held[warp][e] = 0;
+  __syncwarp();
+  auto walk = [&](auto each) {
+    for (int base = first; base < last; base += 32 * AHEAD) {
+      int e[AHEAD];
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k) {
+        const int i = base + 32 * k + lane;
+        e[k] = i < last ? __ldcg(chosen + i) : -2;
       }
-      at += __popc(hits);
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k) {
+        if (base + 32 * k >= last) break;
+        const bool has = e[k] >= 0 && e[k] < E;
+        const unsigned same = __match_any_sync(0xffffffffu, has ? e[k] : -1);
+        each(base + 32 * k + lane, e[k], has, same, __popc(same & ((1u << lane) - 1u)));
+        __syncwarp();
+      }
     }
-    if (lane == 0) { counts[e] = cnt[e]; starts[e] = start[e]; }
+  };
+  walk([&](int, int e, bool has, unsigned same, int rank) {
+    if (has && rank == 0) held[warp][e] += __popc(same);
+  });
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += WARPS * 32) {
+    int at = 0;
+#pragma unroll 8
+    for (int w = 0; w < WARPS; ++w) {
+      const int n = held[w][e];
+      held[w][e] = at;
+      at += n;
+    }
+    counts[e] = start[e] = at;
   }
-  if (threadIdx.x == 0) starts[E] = start[E];
-  // pairs without an expert among the first E (identity experts) are put nowhere
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int e = chosen[i];
-    if (e < 0 || e >= E) place[i] = -1;
+  __syncthreads();
+  if (warp == 0) {  // counts to first places, a lane eight neighbouring experts
+    int own[8], sum = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      own[k] = lane * 8 + k < E ? start[lane * 8 + k] : 0;
+      sum += own[k];
+    }
+    int at = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+      const int x = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += x;
+    }
+    if (lane == 31) starts[E] = at;
+    at -= sum;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (lane * 8 + k < E) {
+        start[lane * 8 + k] = at;
+        starts[lane * 8 + k] = at;
+      }
+      at += own[k];
+    }
   }
+  __syncthreads();
+  walk([&](int i, int e, bool has, unsigned same, int rank) {
+    const int where = has ? start[e] + held[warp][e] + rank : -1;
+    __syncwarp();
+    if (has && rank == 0) held[warp][e] += __popc(same);
+    if (has) pair_at[where] = i;
+    // pairs without an expert among the first E (identity experts) are put nowhere
+    if (e != -2) place[i] = where;
+  });
 }
 
-__global__ void moe_sort_kernel(const int* chosen, int n_pairs, int E, int* __restrict__ counts,
+constexpr int SORT_WARPS = 32;
+__global__ void __launch_bounds__(SORT_WARPS * 32) moe_sort_kernel(const int* chosen, int n_pairs, int E, int* __restrict__ counts,
                                 int* __restrict__ starts, int* __restrict__ place,
                                 int* __restrict__ pair_at) {
   fb_pdl_wait();
-  sort_pairs(chosen, n_pairs, E, counts, starts, place, pair_at);
+  sort_pairs<SORT_WARPS>(chosen, n_pairs, E, counts, starts, place, pair_at);
 }
 
 // Choice and sort in one block, for the few tokens of a single-token step: eight warps
@@ -372,7 +414,7 @@ moe_route_sort_kernel(const float* z, long long ld, const float* __restrict__ bi
                 sum_floor, weight_scale, group_best, t, lane, s_all[warp], s_group[warp],
                 s_plain[warp]);
   __syncthreads();  // the block's own writes of `chosen` are visible to all its threads
-  sort_pairs(chosen, T * top, experts, counts, starts, place, pair_at);
+  sort_pairs<ROUTE_SORT_WARPS>(chosen, T * top, experts, counts, starts, place, pair_at);
 }
 
 template <typename T>
@@ -384,6 +426,18 @@ __global__ void moe_gather_kernel(const T* x, const int* pair_at, const int* sta
   if (at >= starts[E]) return;
   const int t = pair_at[at] / top;
   for (int i = threadIdx.x; i < W; i += blockDim.x) out[(size_t)at * W + i] = x[(size_t)t * W + i];
+}
+
+// The same for rows of whole 16-byte pieces.
+__global__ void __launch_bounds__(256)
+moe_gather_rows_kernel(const uint4* x, const int* pair_at, const int* starts, int E, int top,
+                       uint4* __restrict__ out, int pieces) {
+  fb_pdl_launch();
+  fb_pdl_wait();
+  const int at = blockIdx.x;
+  if (at >= __ldcg(starts + E)) return;
+  const uint4* row = x + (size_t)(__ldcg(pair_at + at) / top) * pieces;
+  for (int i = threadIdx.x; i < pieces; i += blockDim.x) out[(size_t)at * pieces + i] = __ldcg(row + i);
 }
 
 __device__ __forceinline__ float glu_act(float g, float u, float limit, float alpha, float shift) {
@@ -647,12 +701,174 @@ __global__ void moe_combine_kernel(const float* y, const int* place, const float
     out[t * W + i] = acc;
   }
 }
+
+// The same for rows of whole fours, a thread four neighbouring channels: bound by its bytes (2,000
+// tokens of 3,072, two choices, 74 MB: 13.6 us; a channel a thread 30).
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_combine_rows_kernel(const float* y, const int* place, const float* weights, int top,
+                        float* __restrict__ out, int W, const float* addend, const T* h) {
+  fb_pdl_launch();
+  fb_pdl_wait();
+  const size_t t = blockIdx.x;
+  const int i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (i >= W) return;
+  float acc[4] = {};
+  for (int c0 = 0; c0 < top; c0 += 2) {  // two choices' rows under way together
+    int at[2];
+    float wt[2];
+    float4 row[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const bool on = c0 + k < top;
+      at[k] = on ? __ldcg(place + t * top + c0 + k) : -1;
+      wt[k] = on ? __ldcg(weights + t * top + c0 + k) : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (at[k] >= 0) {
+        row[k] = __ldcg(reinterpret_cast<const float4*>(y + (size_t)at[k] * W + i));
+      } else if (h != nullptr) {
+        row[k] = make_float4(fb_load_coherent<T>(h + t * W + i), fb_load_coherent<T>(h + t * W + i + 1),
+                             fb_load_coherent<T>(h + t * W + i + 2), fb_load_coherent<T>(h + t * W + i + 3));
+      } else {
+        row[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (c0 + k >= top) break;
+      acc[0] = fmaf(wt[k], row[k].x, acc[0]);
+      acc[1] = fmaf(wt[k], row[k].y, acc[1]);
+      acc[2] = fmaf(wt[k], row[k].z, acc[2]);
+      acc[3] = fmaf(wt[k], row[k].w, acc[3]);
+    }
+  }
+  if (addend != nullptr) {
+    const float4 f = __ldcg(reinterpret_cast<const float4*>(addend + t * W + i));
+    acc[0] += f.x; acc[1] += f.y; acc[2] += f.z; acc[3] += f.w;
+  }
+  *reinterpret_cast<float4*>(out + t * W + i) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
+// The router's product and the choice in one kernel, for rows of whole 64s in 16 bits and up to 64
+// outputs: a block takes 16 tokens, its eight warps share K, token rows and router rows go
+// straight from memory into mma.sync fragments (K permuted within 64 so that a thread's fragment is
+// 16-byte pieces, as in gemm_skinny.cu), the warps' sums meet in shared memory in order, and the
+// tokens' logits are routed where they were made. Bound by its loads' latency: 2,000 tokens of
+// 3,072, 16 outputs 21 us; the product alone took 27 on the tcgen05 kernel, whose 16 tiles
+// walk all of K on 16 SMs, and the choice 6.
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                          uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+constexpr int ROUTER_WARPS = 8, ROUTER_TOKENS = 16;
+template <int NT>
+__global__ void __launch_bounds__(ROUTER_WARPS * 32)
+moe_router_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __restrict__ w,
+                  long long ldw, int K, float* z, const float* __restrict__ bias, int E, int top,
+                  int* __restrict__ chosen, float* __restrict__ weights, int score, int groups,
+                  int keep, const float* __restrict__ correction, int normalise, float sum_floor,
+                  float weight_scale, int group_best, int T) {
+  fb_pdl_launch();
+  __shared__ float part[ROUTER_WARPS][ROUTER_TOKENS][8 * NT + 1];
+  __shared__ float s_all[ROUTER_WARPS][8 * NT], s_group[ROUTER_WARPS][8 * NT],
+      s_plain[ROUTER_WARPS][8 * NT];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int t0 = blockIdx.x * ROUTER_TOKENS;
+  const __nv_bfloat16* rows[2] = {x + (long long)min(t0 + g, T - 1) * ldx + q * 8,
+                                  x + (long long)min(t0 + g + 8, T - 1) * ldx + q * 8};
+  const __nv_bfloat16* out_rows[NT];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) out_rows[j] = w + (long long)min(j * 8 + g, E - 1) * ldw + q * 8;
+  float acc[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+  fb_pdl_wait();
+#pragma unroll 2
+  for (int c = warp; c < K / 64; c += ROUTER_WARPS) {
+    uint4 a[2][2], b[NT][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+        a[r][half] = __ldcg(reinterpret_cast<const uint4*>(rows[r] + c * 64 + half * 32));
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+        b[j][half] = __ldg(reinterpret_cast<const uint4*>(out_rows[j] + c * 64 + half * 32));
+    const uint32_t* lo = reinterpret_cast<const uint32_t*>(&a[0][0]);
+    const uint32_t* hi = reinterpret_cast<const uint32_t*>(&a[1][0]);
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const uint32_t* y = reinterpret_cast<const uint32_t*>(&b[j][0]);
+        mma_16816(acc[j], lo[2 * s], hi[2 * s], lo[2 * s + 1], hi[2 * s + 1], y[2 * s], y[2 * s + 1]);
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) part[warp][g + (i >> 1) * 8][j * 8 + 2 * q + (i & 1)] = acc[j][i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < ROUTER_TOKENS * 8 * NT; i += ROUTER_WARPS * 32) {
+    const int t = i / (8 * NT), e = i % (8 * NT);
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < ROUTER_WARPS; ++k) sum += part[k][t][e];
+    if (t0 + t < T && e < E) z[(long long)(t0 + t) * E + e] = sum;
+  }
+  __syncthreads();  // the block's own writes of z are visible to all its threads
+  for (int t = t0 + warp; t < min(T, t0 + ROUTER_TOKENS); t += ROUTER_WARPS)
+    route_token(z, E, bias, E, top, chosen, weights, score, groups, keep, correction, normalise,
+                sum_floor, weight_scale, group_best, t, lane, s_all[warp], s_group[warp],
+                s_plain[warp]);
+}
 }  // namespace
+
+// fb_moe_route behind its product: z [T, E] = x router^T in 32 bits, then the choice.
+FB_API int fb_moe_router(const void* x, long long ldx, const void* w, long long ldw, int K, float* z,
+                         const float* bias, int E, int top, int* chosen, float* weights, int T,
+                         int score, int groups, int keep, const float* correction, int normalise,
+                         float sum_floor, float weight_scale, int group_best, cudaStream_t stream) {
+  FB_REQUIRE(T >= 0 && E > 0 && E <= 64 && top > 0 && top <= E && top <= 32,
+             "moe_router: %d experts (at most 64), %d chosen (at most 32)", E, top);
+  FB_REQUIRE(K > 0 && K % 64 == 0 && ldx % 8 == 0 && ldw % 8 == 0 && ((uintptr_t)x % 16) == 0 &&
+                 ((uintptr_t)w % 16) == 0,
+             "moe_router: K must be a multiple of 64 and the rows 16-byte aligned");
+  FB_REQUIRE(score >= 0 && score <= 2 && (group_best == 1 || group_best == 2),
+             "moe_router: unknown scoring rule %d (groups by their best %d)", score, group_best);
+  FB_REQUIRE(groups >= 1 && E % groups == 0 && keep >= 1 && keep <= groups &&
+             (long long)keep * (E / groups) >= top,
+             "moe_router: %d groups of %d experts, %d kept, %d chosen", groups, E, keep, top);
+  FB_REQUIRE(score != 0 || (groups == 1 && correction == nullptr && !normalise &&
+                            weight_scale == 1.0f),
+             "moe_router: groups, a correction, shares of the sum and a constant on the weights need "
+             "scores of their own");
+  if (T == 0) return 0;
+  auto go = [&](auto kernel) {
+    fb_launch(kernel, dim3((T + ROUTER_TOKENS - 1) / ROUTER_TOKENS), dim3(ROUTER_WARPS * 32), 0, stream,
+              (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, ldw, K, z, bias, E, top, chosen,
+              weights, score, groups, keep, correction, normalise, sum_floor, weight_scale,
+              group_best, T);
+  };
+  if (E <= 8) go(moe_router_kernel<1>);
+  else if (E <= 16) go(moe_router_kernel<2>);
+  else if (E <= 32) go(moe_router_kernel<4>);
+  else go(moe_router_kernel<8>);
+  return fb_check_launch("moe_router");
+}
 
 FB_API int fb_moe_sort(const int* chosen, int n_pairs, int E, int* counts, int* starts, int* place,
                        int* pair_at, cudaStream_t stream) {
   FB_REQUIRE(n_pairs >= 0 && E > 0 && E <= 256, "moe_sort: %d experts (at most 256)", E);
-  fb_launch(moe_sort_kernel, dim3(1), dim3(256), 0, stream, chosen, n_pairs, E, counts, starts,
+  fb_launch(moe_sort_kernel, dim3(1), dim3(SORT_WARPS * 32), 0, stream, chosen, n_pairs, E, counts, starts,
             place, pair_at);
   return fb_check_launch("moe_sort");
 }
@@ -686,6 +902,14 @@ FB_API int fb_moe_gather(const void* x, int dtype, const int* pair_at, const int
                          int top, void* out, int n_pairs, int W, cudaStream_t stream) {
   FB_REQUIRE(n_pairs >= 0 && W > 0 && top > 0, "moe_gather: bad sizes");
   if (n_pairs == 0) return 0;
+  const size_t bytes = (size_t)W * (dtype == FB_BF16 ? 2 : 4);
+  if ((dtype == FB_BF16 || dtype == FB_F32) && bytes % 16 == 0 && ((uintptr_t)x % 16) == 0 &&
+      ((uintptr_t)out % 16) == 0) {
+    const int pieces = (int)(bytes / 16);
+    fb_launch(moe_gather_rows_kernel, dim3(n_pairs), dim3(pieces < 256 ? (pieces + 31) / 32 * 32 : 256),
+              0, stream, (const uint4*)x, pair_at, starts, E, top, (uint4*)out, pieces);
+    return fb_check_launch("moe_gather");
+  }
   FB_DISPATCH_DTYPE(dtype, T_, (fb_launch(moe_gather_kernel<T_>, dim3(n_pairs), dim3(256), 0,
       stream, (const T_*)x, pair_at, starts, E, top, (T_*)out, W)));
   return fb_check_launch("moe_gather");
@@ -782,6 +1006,14 @@ FB_API int fb_moe_combine(const float* y, const int* place, const float* weights
                           int h_dtype, cudaStream_t stream) {
   FB_REQUIRE(T >= 0 && W > 0 && top > 0, "moe_combine: bad sizes");
   if (T == 0) return 0;
+  if (W % 4 == 0 && ((uintptr_t)y % 16) == 0 && ((uintptr_t)out % 16) == 0 &&
+      ((uintptr_t)addend % 16) == 0) {
+    const int threads = T <= 64 ? 64 : 256;  // few tokens: a row's columns go to several blocks
+    FB_DISPATCH_DTYPE(h_dtype, E, (fb_launch(moe_combine_rows_kernel<E>,
+        dim3(T, (W / 4 + threads - 1) / threads), dim3(threads), 0, stream, y, place, weights, top,
+        out, W, addend, (const E*)h)));
+    return fb_check_launch("moe_combine");
+  }
   const int want = (W + 255) / 256;  // few tokens: a row's columns go to several blocks
   const int parts = T <= 256 ? (want < 32 ? want : 32) : 1;
   FB_DISPATCH_DTYPE(h_dtype, E, (fb_launch(moe_combine_kernel<E>, dim3(T, parts), dim3(256), 0,

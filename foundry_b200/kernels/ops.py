@@ -202,6 +202,9 @@ _SIGNATURES = {
     "fb_unary_cast": [c_void_p, c_ll, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "fb_add_into": [c_void_p, c_void_p, c_ll, c_void_p],
     "fb_sigmoid_gate": [c_void_p, c_int, c_ll, c_void_p, c_ll, c_int, c_int, c_void_p],
+    "fb_moe_router": [c_void_p, c_ll, c_void_p, c_ll, c_int, c_void_p, c_void_p, c_int, c_int,
+                      c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float,
+                      c_float, c_int, c_void_p],
     "fb_moe_route_sort": [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
                           c_int, c_int, c_void_p, c_int, c_float, c_float, c_int, c_int, c_void_p,
                           c_void_p, c_void_p, c_void_p, c_void_p],
@@ -3105,6 +3108,40 @@ def moe_route_sorted(z: torch.Tensor, bias: Optional[torch.Tensor], top: int, ch
           order.counts.data_ptr(),
           order.starts.data_ptr(), order.place.data_ptr(), order.pair_at.data_ptr(), _stream())
     return order
+
+
+def moe_router_fits(x, router: torch.Tensor) -> bool:
+    """Whether `moe_router_sorted` takes these rows: 16-bit rows of whole 64s, up to 64 outputs,
+    more tokens than the one-block choice takes (up to there the weight-streaming product, which
+    also applies a norm's pending scale, and that block are two launches, too)."""
+    return (isinstance(x, torch.Tensor) and x.shape[0] > MOE_ROUTE_SORT_ROWS
+            and x.dtype == router.dtype == torch.bfloat16 and router.shape[0] <= 64
+            and x.shape[1] % 64 == 0 and x.stride(1) == router.stride(1) == 1
+            and x.stride(0) % 8 == 0 and router.stride(0) % 8 == 0
+            and x.data_ptr() % 16 == 0 and router.data_ptr() % 16 == 0)
+
+
+def moe_router_sorted(x: torch.Tensor, router: torch.Tensor, bias: Optional[torch.Tensor], top: int,
+                      chosen: torch.Tensor, weights: torch.Tensor, experts: int,
+                      score: str = "softmax_chosen", groups: int = 1, keep: int = 1,
+                      correction: Optional[torch.Tensor] = None, normalise: bool = False,
+                      sum_floor: float = 0.0, weight_scale: float = 1.0,
+                      group_best: int = 2) -> ExpertOrder:
+    """The router's product in 32 bits, the choice (`moe_route`) and the sort of the chosen pairs."""
+    T, K = x.shape
+    E = router.shape[0]
+    if correction is not None and tuple(correction.shape) != (E,):
+        raise KernelError(f"moe_router: a correction of {tuple(correction.shape)} for {E} experts")
+    z = torch.empty((T, E), dtype=torch.float32, device=x.device)
+    _call("fb_moe_router", _dev(x, "x", contiguous=False), x.stride(0),
+          _dev(router, "router", contiguous=False), router.stride(0), K, z.data_ptr(),
+          0 if bias is None else _dev(bias, "bias", torch.float32), E, top,
+          _dev(chosen, "chosen", torch.int32), _dev(weights, "weights", torch.float32), T,
+          MOE_SCORES[score], int(groups), int(keep),
+          0 if correction is None else _dev(correction, "correction", torch.float32),
+          1 if normalise else 0, float(sum_floor), float(weight_scale), int(group_best), _stream(),
+          tag=("t{} k{} e{}", T, K, E))
+    return ExpertOrder(chosen, experts)
 
 
 def moe_gather(x: torch.Tensor, order: ExpertOrder) -> torch.Tensor:

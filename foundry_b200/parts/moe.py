@@ -120,7 +120,6 @@ class RoutedExperts(Part):
         """`addend` (float32 [T, width]): rows that join the sum where the chosen experts'
         rows are combined (the result of a part that ran beside this one)."""
         T = x.shape[0]
-        z = product_f32(x, self.router)
         chosen = torch.empty((T, self.top), dtype=torch.int32, device=x.device)
         weights = torch.empty((T, self.top), dtype=torch.float32, device=x.device)
         rule = dict(score=self.score, groups=self.groups, keep=self.keep,
@@ -129,11 +128,15 @@ class RoutedExperts(Part):
                     group_best=self.group_best)
         own = ops.plain(x) if self.identity else None  # what an identity expert gives
         grouped = ops.moe_grouped_fits(self.width) and ops.moe_grouped_fits(self.ff)
-        if grouped:  # the choice, and the pairs sorted by expert
-            order = ops.moe_route_sorted(z, self.router_bias, self.top, chosen, weights,
-                                         experts=self.experts, **rule)
+        if grouped and ops.moe_router_fits(x, self.router):
+            order = ops.moe_router_sorted(x, self.router, self.router_bias, self.top, chosen,
+                                          weights, self.experts, **rule)
+        elif grouped:  # the choice, and the pairs sorted by expert
+            order = ops.moe_route_sorted(product_f32(x, self.router), self.router_bias, self.top,
+                                         chosen, weights, experts=self.experts, **rule)
         else:
-            ops.moe_route(z, self.router_bias, self.top, chosen, weights, **rule)
+            ops.moe_route(product_f32(x, self.router), self.router_bias, self.top, chosen, weights,
+                          **rule)
         # the shared expert's rows join the sum where the chosen experts' rows are combined
         shared = addend
         if self.shared is not None:
