@@ -60,6 +60,8 @@ class StepContext:
     # the step's own rows (a mixer may then work on those rows instead of the cache);
     # in a replayed step it is fixed when the step is captured
     fresh: bool = False
+    # The wanted rows are all rows, in their order (fixed when a step is captured)
+    wants_every_row: bool = False
     _tables: Dict[int, torch.Tensor] = field(default_factory=dict)
     # The weight that the step streams after the part being run (a prefetch
     # hint, set by the model and the blocks as they go; None = unknown).

@@ -74,7 +74,8 @@ class DecodeRunner:
             n_tokens=b, n_seqs=b, n_want=b, token_ids=part[0], positions=part[1],
             seq_of_token=part[2], want_rows=part[3], slots=part[4], cu_tokens=part[5],
             kv_lens=part[6], slots_host=None, cu_tokens_host=None, kv_lens_host=None,
-            is_decode=True, max_q_len=1, max_kv_len=width * PAGE, unequal_lengths=unequal)
+            is_decode=True, max_q_len=1, max_kv_len=width * PAGE, unequal_lengths=unequal,
+            wants_every_row=True)
         for i, group in enumerate(groups):
             self.ctx._tables[id(group)] = part[7 + i].view(b, width)
         self.h_tables = [self.h[7 + i].reshape(b, width) for i in range(len(groups))]
@@ -95,12 +96,11 @@ class DecodeRunner:
 
     def _body(self) -> None:
         engine = self.engine
+        b = self.bucket
         with ops.scratch_owner(engine.scratch):
             self.logits = engine.model.forward(self.ctx, engine.cache)
-        b = self.bucket
-        ops.select_tokens(self.logits, self.next_tokens, self.temperature, self.meta64[:b],
-                          self.meta64[b:])
-        self.ctx.token_ids.copy_(self.next_tokens)
+            ops.select_tokens(self.logits, self.next_tokens, self.temperature, self.meta64[:b],
+                              self.meta64[b:], also=self.ctx.token_ids)
 
     def run(self) -> None:
         """One step over the buffers' current contents."""

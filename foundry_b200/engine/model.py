@@ -192,6 +192,8 @@ class Model:
             return self._logits(normed, logits)
         if isinstance(delta, ops.DepthMix):  # the last stream is a sum over the kept ones
             delta = delta.settle(resid)
+        if ctx.wants_every_row:  # each row in its place (single-token steps): nothing to gather
+            return self._logits(self.final_norm.add_norm(resid, delta), logits)
         rows = torch.empty((n, spec.hidden_size), dtype=torch.float32, device=self.device)
         ops.gather_rows(resid, ctx.want_rows, rows)
         rows_delta = None

@@ -103,7 +103,7 @@ _SIGNATURES = {
     "fb_gemm_rows_status": [c_void_p],
     "fb_row_scales": [c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p],
     "fb_select_tokens": [c_void_p, c_ll, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-                         c_int, c_void_p, c_void_p, c_void_p],
+                         c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
     "fb_ln_add_ln": [c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p,
                      c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_int,
                      c_void_p],
@@ -1786,27 +1786,32 @@ def attention_simt(q: torch.Tensor, out: torch.Tensor, positions: torch.Tensor,
 # ------------------------------------------------------------------- sampling
 def select_tokens(logits: torch.Tensor, out: torch.Tensor, temperature: Optional[torch.Tensor],
                   streams: Optional[torch.Tensor] = None,
-                  steps: Optional[torch.Tensor] = None) -> torch.Tensor:
+                  steps: Optional[torch.Tensor] = None,
+                  also: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Greedy where temperature is 0 (or None), Gumbel-max sampling elsewhere.
     `streams[r]` is the row's random stream (`sampling.stream_key(seed, key)`),
     `steps[r]` how many tokens its sequence has generated. Large vocabularies
-    are scanned by several blocks per row and merged by a second small kernel."""
+    are scanned by several blocks per row and merged by a second small kernel, or,
+    with `also` (a second place for the tokens, the next step's input), by the
+    block of a row that arrives last (counters of the scratch owner's)."""
     n, V = logits.shape
-    if out.numel() != n:
+    if out.numel() != n or (also is not None and also.numel() != n):
         raise KernelError("select_tokens: out does not hold one token per row")
     chunks = 1 if V < 16384 else min(64, (V + 2047) // 2048)
     part_val = part_idx = None
     if chunks > 1:
         part_val = torch.empty(n * chunks, dtype=torch.float32, device=logits.device)
         part_idx = torch.empty(n * chunks, dtype=torch.int32, device=logits.device)
-        _COUNT[0] += 1  # the merge kernel
+        if also is None:
+            _COUNT[0] += 1  # the merge kernel
     _call("fb_select_tokens", _dev(logits, "logits", torch.float32, contiguous=False),
           _rows(logits, "logits"), n, V,
           0 if temperature is None else _dev(temperature, "temperature", torch.float32),
           0 if streams is None else _dev(streams, "streams", torch.int64),
           0 if steps is None else _dev(steps, "steps", torch.int64),
-          _dev(out, "out", torch.int32), chunks,
-          0 if part_val is None else part_val.data_ptr(),
+          _dev(out, "out", torch.int32), 0 if also is None else _dev(also, "also", torch.int32),
+          _arrival_counters(logits.device, n).data_ptr() if also is not None and chunks > 1 else 0,
+          chunks, 0 if part_val is None else part_val.data_ptr(),
           0 if part_idx is None else part_idx.data_ptr(), _stream())
     return out
 
