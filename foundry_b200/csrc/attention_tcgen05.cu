@@ -47,6 +47,13 @@
 // first tokens, whose pages are walked in front of it; and the heads' outputs may be
 // multiplied by the sigmoid of a gate before they are rounded.
 //
+// The form over rows (ROWS): keys and values are rows of the step's own tokens, for steps in which
+// every sequence begins at its first token, a head's key from two sources (whole 64s of its own
+// and up to 64 elements that all heads share): the latent attention of a prompt, whose keys and
+// values are expanded for it. A tile of keys may reach into the next sequence's rows: scores there
+// are masked, and the softmax warps put zeros over the values before the product reads them.
+// 2,048 tokens, 32 heads of 64 + 32 and 64: 44 us against 172 on mma.sync (attention_maps_mma.cu).
+//
 // Shared memory (96 KB at head size 128) and tensor memory (256 columns) are
 // sized so that two CTAs share an SM: the second CTA's warps fill the gaps that
 // a row's long dependent chain leaves on the schedulers and the tensor pipe.
@@ -94,6 +101,8 @@ struct FaParams {
   long long ks_page, ks_head;
   const float* gate;                // float32 rows, A * DV elements, or null
   long long gate_stride;
+  // The form over rows: elements from one head's key (value) to the next in a row.
+  int k_head, v_head;
 };
 constexpr int TABLE_FRONT = 192;  // a query row may lie 127 in front of a page, a key 63 into it
 constexpr int TABLE_BACK = 96;    // a warp's rows span 32, a page 64 keys
@@ -144,14 +153,16 @@ struct FaSmem {
   // never three CTAs on an SM: they would need more tensor memory than it has
   static constexpr int LEAST = 77 * 1024;
   static constexpr int BYTES = USED > LEAST ? USED : LEAST;
-  static_assert(BYTES <= LIMIT, "two CTAs must fit an SM");
+  // (three blocks along a key take the SM for one CTA)
+  static_assert(BYTES <= LIMIT || KS > 2, "two CTAs must fit an SM");
 };
 
-template <int KS, int VS, bool ONE>
+template <int KS, int VS, bool ONE, bool ROWS = false>
 __global__ void __launch_bounds__(THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                        const __grid_constant__ CUtensorMap map_k,
-                       const __grid_constant__ CUtensorMap map_v, const FaParams p) {
+                       const __grid_constant__ CUtensorMap map_v,
+                       const __grid_constant__ CUtensorMap map_shared, const FaParams p) {
   using Smem = FaSmem<KS, VS, ONE>;
   constexpr int RING = Smem::RING;
   constexpr int Q_SUB = BQ * 128;              // bytes of one query sub-tile
@@ -254,6 +265,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
       for (int j = 0; j < n_pages; ++j) {
         const int s = j % RING;
         const uint32_t parity = (uint32_t)((j / RING) & 1) ^ 1u;
+        if constexpr (ROWS) {  // (rows beyond the step's last come as zeros)
+          const int key_row = tok0 + page_at(j) * FB_PAGE;
+          if (!mbar_wait(&k_empty[s], parity, abort_flag, 11, j)) break;
+          mbar_expect_tx(&k_full[s], Smem::K_BYTES);
+#pragma unroll
+          for (int sb = 0; sb < KS; ++sb) {
+            uint8_t* dst = sK + s * Smem::K_BYTES + sb * KV_SUB;
+            if (sb + 1 < KS) tma_load_2d(dst, &map_k, &k_full[s], head * p.k_head + sb * 64, key_row);
+            else tma_load_2d(dst, &map_shared, &k_full[s], 0, key_row);
+          }
+          if (!mbar_wait(&v_empty[s], parity, abort_flag, 10, j)) break;
+          mbar_expect_tx(&v_full[s], Smem::V_BYTES);
+#pragma unroll
+          for (int sb = 0; sb < VS; ++sb)
+            tma_load_2d(sV + s * Smem::V_BYTES + sb * KV_SUB, &map_v, &v_full[s],
+                        head * p.v_head + sb * 64, key_row);
+          continue;
+        }
         const int page = pages[page_at(j)];
         if (!mbar_wait(&k_empty[s], parity, abort_flag, 11, j)) break;
         mbar_expect_tx(&k_full[s], Smem::K_BYTES);
@@ -474,6 +503,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         packed[c] = *reinterpret_cast<const uint32_t*>(&h);
       }
       l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+      if (ROWS && key0 + FB_PAGE > kv_len) {
+        // values behind the sequence's last token may be anybody's, and no numbers: a weight of
+        // zero is not enough (whole rows of a tile, so its swizzle does not matter)
+        ok = mbar_wait(&v_full[j % ST], (uint32_t)((j / ST) & 1), abort_flag, 17, j);
+        if (!ok) break;
+        if (row < FB_PAGE && key0 + row >= kv_len) {
+#pragma unroll
+          for (int sb = 0; sb < VS; ++sb) {
+            uint4* at = reinterpret_cast<uint4*>(sV + (j % ST) * Smem::V_BYTES + sb * KV_SUB + row * 128);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) at[e] = make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
       tmem_st32(tmem_base + lane_base + (uint32_t)(b * FB_PAGE), packed);
       tmem_st_wait();
       tc_fence_before();
@@ -573,9 +617,9 @@ int make_map(CUtensorMap* map, const void* ptr, int rank, const long long* dims,
   return 0;
 }
 
-template <int KS, int VS, bool ONE = false>
-int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FaParams& p,
-           int q_blocks, cudaStream_t stream) {
+template <int KS, int VS, bool ONE = false, bool ROWS = false>
+int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+           const CUtensorMap& shared, const FaParams& p, int q_blocks, cudaStream_t stream) {
   using Smem = FaSmem<KS, VS, ONE>;
   int bytes = Smem::BYTES;
   if (ONE && p.table != nullptr && p.table_pitch <= Smem::TABLE_ROOM &&
@@ -583,13 +627,13 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
     bytes = Smem::USED + p.table_pitch * 4;
   static bool configured[64] = {};
   if (fb_first_use_on_device(configured)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<KS, VS, ONE>,
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<KS, VS, ONE, ROWS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          ONE ? Smem::LIMIT : Smem::BYTES);
     if (e != cudaSuccess) return fb_fail(2, "attention_tc: %s", cudaGetErrorString(e));
   }
-  fb_launch(attn_prefill_tc_kernel<KS, VS, ONE>, dim3(p.A, q_blocks), dim3(THREADS), bytes, stream,
-            mq, mk, mv, p);
+  fb_launch(attn_prefill_tc_kernel<KS, VS, ONE, ROWS>, dim3(p.A, q_blocks), dim3(THREADS), bytes,
+            stream, mq, mk, mv, shared, p);
   return fb_check_launch("attention_prefill_tc");
 }
 
@@ -642,10 +686,55 @@ FB_API int fb_attention_prefill_tc(const void* q, long long q_stride, int T, voi
   p.D = D; p.DV = DV; p.window = window;
   p.scale_log2 = scale * LOG2E;
   p.sink_logits = sink_logits;
-  if (D <= 64) return DV <= 64 ? launch<1, 1>(mq, mk, mv, p, q_blocks, stream)
-                               : launch<1, 2>(mq, mk, mv, p, q_blocks, stream);
-  return DV <= 64 ? launch<2, 1>(mq, mk, mv, p, q_blocks, stream)
-                  : launch<2, 2>(mq, mk, mv, p, q_blocks, stream);
+  if (D <= 64) return DV <= 64 ? launch<1, 1>(mq, mk, mv, mk, p, q_blocks, stream)
+                               : launch<1, 2>(mq, mk, mv, mk, p, q_blocks, stream);
+  return DV <= 64 ? launch<2, 1>(mq, mk, mv, mk, p, q_blocks, stream)
+                  : launch<2, 2>(mq, mk, mv, mk, p, q_blocks, stream);
+}
+
+// The form over rows (see the file's notes): q [T, A * (K1 + K2)] rows; a head's K1 key elements at
+// `k` + head * k_head in rows k_row apart, the other K2 at `k_shared` for every head, its DV value
+// elements at `v` + head * v_head. K1: 64 or 128; K2: a multiple of 8 up to 64.
+FB_API int fb_attention_prefill_rows(const void* q, long long q_stride, int T, void* out,
+                                     long long out_stride, const int* cu_tokens, const int* kv_lens,
+                                     const void* k, long long k_row, int k_head,
+                                     const void* k_shared, long long ks_row, const void* v,
+                                     long long v_row, int v_head, int n_seqs, int q_blocks, int A,
+                                     int K1, int K2, int DV, float scale, const float* sink_logits,
+                                     cudaStream_t stream) {
+  FB_REQUIRE((K1 == 64 || K1 == 128) && K2 > 0 && K2 <= 64 && K2 % 8 == 0 && DV > 0 && DV <= 128 &&
+                 DV % 8 == 0,
+             "attention_rows: keys of %d + %d and values of %d elements are not built", K1, K2, DV);
+  FB_REQUIRE(n_seqs > 0 && A > 0 && T > 0, "attention_rows: bad sizes");
+  FB_REQUIRE(q_stride % 8 == 0 && out_stride % 8 == 0 && k_row % 8 == 0 && ks_row % 8 == 0 &&
+                 v_row % 8 == 0 && k_head % 8 == 0 && v_head % 8 == 0 && k_head >= K1 && v_head >= DV &&
+                 ((uintptr_t)q % 16) == 0 && ((uintptr_t)out % 16) == 0 && ((uintptr_t)k % 16) == 0 &&
+                 ((uintptr_t)k_shared % 16) == 0 && ((uintptr_t)v % 16) == 0,
+             "attention_rows: pointers and strides must keep 16-byte alignment");
+  if (q_blocks <= 0) return 0;
+  bind_status_mirror(stream);
+  CUtensorMap mq, mk, ms, mv;
+  const auto rows_map = [&](CUtensorMap* map, const void* at, long long width, long long stride, int rows) {
+    const long long dims[2] = {width, T}, strides[1] = {stride};
+    const int box[2] = {64, rows};
+    return make_map(map, at, 2, dims, strides, box);
+  };
+  int rc = rows_map(&mq, q, (long long)A * (K1 + K2), q_stride, BQ);
+  if (!rc) rc = rows_map(&mk, k, (long long)(A - 1) * k_head + K1, k_row, FB_PAGE);
+  if (!rc) rc = rows_map(&ms, k_shared, K2, ks_row, FB_PAGE);
+  if (!rc) rc = rows_map(&mv, v, (long long)(A - 1) * v_head + DV, v_row, FB_PAGE);
+  if (rc) return rc;
+  FaParams p{};
+  p.out = (__nv_bfloat16*)out; p.out_stride = out_stride;
+  p.cu_tokens = cu_tokens; p.kv_lens = kv_lens;
+  p.n_seqs = n_seqs; p.A = A; p.Kh = A;
+  p.D = K1 + K2; p.DV = DV; p.k_head = k_head; p.v_head = v_head;
+  p.scale_log2 = scale * LOG2E;
+  p.sink_logits = sink_logits;
+  if (K1 == 64) return DV <= 64 ? launch<2, 1, false, true>(mq, mk, mv, ms, p, q_blocks, stream)
+                                : launch<2, 2, false, true>(mq, mk, mv, ms, p, q_blocks, stream);
+  return DV <= 64 ? launch<3, 1, false, true>(mq, mk, mv, ms, p, q_blocks, stream)
+                  : launch<3, 2, false, true>(mq, mk, mv, ms, p, q_blocks, stream);
 }
 
 // The form with shared rows (see the file's notes): `rows` are one cache entry's
@@ -701,8 +790,8 @@ FB_API int fb_attention_prefill_shared(const void* q, long long q_stride, int T,
   p.table = table; p.table_last = table_last; p.table_pitch = table_pitch;
   p.key_scale = key_scale; p.ks_page = ks_page; p.ks_head = ks_head;
   p.gate = gate; p.gate_stride = gate_stride;
-  if (D <= 64) return launch<1, 1, true>(mq, mk, mk, p, q_blocks, stream);
-  return launch<2, 2, true>(mq, mk, mk, p, q_blocks, stream);
+  if (D <= 64) return launch<1, 1, true>(mq, mk, mk, mk, p, q_blocks, stream);
+  return launch<2, 2, true>(mq, mk, mk, mk, p, q_blocks, stream);
 }
 
 // As fb_gemm_tc_status, for the attention kernel of this file.

@@ -158,6 +158,9 @@ _SIGNATURES = {
                           c_void_p, c_void_p, c_void_p, c_ll, c_ll, c_ll, c_ll, c_ll, c_ll, c_ll,
                           c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                           c_float, c_void_p, c_float, c_float, c_float, c_void_p],
+    "fb_attention_prefill_rows": [c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_void_p,
+                                  c_ll, c_int, c_void_p, c_ll, c_void_p, c_ll, c_int, c_int, c_int,
+                                  c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
     "fb_attention_prefill_shared": [c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_void_p,
                                     c_void_p, c_int, c_void_p, c_ll, c_void_p, c_ll, c_ll, c_int,
                                     c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
@@ -2550,19 +2553,47 @@ def attention_maps_paged(ctx, q, out, page_table, k_cache, v_cache, H: int, G: i
     return out
 
 
+def _tc_rows_blocks(ctx, q, out, k, k_shared, v, k1: int, k2: int, vdim: int, softcap: float) -> int:
+    """128-row query blocks of a step that the tcgen05 kernel over rows takes, else 0: some
+    sequence brings 64 tokens or more, keys of 64 or 128 elements and up to 64 shared ones, no
+    soft cap, and 16-byte rows throughout."""
+    if not PREFILL_TC or softcap or k_shared is None or k1 not in (64, 128) or not 0 < k2 <= 64 \
+            or k2 % 8 or vdim % 8 or vdim > 128:
+        return 0
+    for t in (q, out, k, k_shared, v):
+        if t.data_ptr() % 16 or any(n % 8 for n in t.stride()[:-1]):
+            return 0
+    if ctx.cu_tokens_host is None:  # a replayed step: bounds that its bucket gives
+        return (ctx.query_blocks_bound + 1) // 2 + ctx.n_seqs if ctx.long_queries else 0
+    lens = [b - a for a, b in zip(ctx.cu_tokens_host, ctx.cu_tokens_host[1:])]
+    return sum((n + 127) // 128 for n in lens) if max(lens) >= 64 else 0
+
+
 def attention_maps_rows(ctx, q: torch.Tensor, out: torch.Tensor, k: torch.Tensor,
                         k_shared: Optional[torch.Tensor], v: torch.Tensor, H: int, dim: int,
                         vdim: int, scale: float, softcap: float = 0.0,
                         sink_logits: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The same kernel over the step's own rows, for a step in which every sequence
     begins at its first token: k [T, H, k1] (a view; a head's own key elements),
-    k_shared [T, dim - k1] (a view; the rest of every head's key), v [T, H, vdim] (a view)."""
+    k_shared [T, dim - k1] (a view; the rest of every head's key), v [T, H, vdim] (a view).
+    Where it fits, the tcgen05 kernel in its form over rows (csrc/attention_tcgen05.cu)."""
     T = q.shape[0]
     k1 = k.shape[2]
     if k.shape[:2] != (T, H) or v.shape != (T, H, vdim) or (k1 != dim) != (k_shared is not None) \
             or k.stride(2) != 1 or v.stride(2) != 1 or (k_shared is not None and (
                 tuple(k_shared.shape) != (T, dim - k1) or k_shared.stride(1) != 1)):
         raise KernelError("attention_maps_rows: shapes differ")
+    blocks128 = _tc_rows_blocks(ctx, q, out, k, k_shared, v, k1, dim - k1, vdim, softcap)
+    if blocks128:
+        _call("fb_attention_prefill_rows", _dev(q, "q", torch.bfloat16, contiguous=False), _rows(q, "q"),
+              T, _dev(out, "out", torch.bfloat16, contiguous=False), _rows(out, "out"),
+              _dev(ctx.cu_tokens, "cu_tokens", torch.int32), _dev(ctx.kv_lens, "kv_lens", torch.int32),
+              k.data_ptr(), k.stride(0), k.stride(1), k_shared.data_ptr(), k_shared.stride(0),
+              v.data_ptr(), v.stride(0), v.stride(1), ctx.n_seqs, blocks128, H, k1, dim - k1, vdim,
+              float(scale),
+              0 if sink_logits is None else _dev(sink_logits, "sink_logits", torch.float32),
+              _stream())
+        return out
     _call("fb_attention_maps", _dev(q, "q", torch.bfloat16, contiguous=False), _rows(q, "q"),
           _dev(out, "out", torch.bfloat16, contiguous=False), _rows(out, "out"),
           _dev(ctx.cu_tokens, "cu_tokens", torch.int32), _dev(ctx.kv_lens, "kv_lens", torch.int32),
