@@ -179,12 +179,28 @@ __device__ __forceinline__ __nv_bfloat16 fb_from_float<__nv_bfloat16>(float v) {
   return __float2bfloat16_rn(v);
 }
 
+// n / d for d >= 1, without the branch that the division operator takes for scaled operands: the
+// hardware's reciprocal, one Newton step, and the quotient corrected by its own remainder
+// (Markstein's method), within an ulp; what no correction fits (infinities, NaN) keeps the plain
+// product. The branch kept the epilogues of the gated products from overlapping one element's
+// latency with the next one's: 2,048 rows of 2,048 -> 2 x 8,192 102.2 -> 100.4 us (300 rows: 52 ->
+// 44), 16 experts of 250 rows of 3,072 -> 2 x 2,048 142 -> 115 us (1,000 rows each: 462 -> 375).
+__device__ __forceinline__ float fb_quotient(float n, float d) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float plain = n * r;
+  r = fmaf(r, fmaf(-d, r, 1.0f), r);
+  float q = n * r;
+  q = fmaf(r, fmaf(-d, q, n), q);
+  return q == q ? q : plain;
+}
+
 // The activation of a gated feed-forward on its gate: 0 SiLU, g / (1 + exp(-g));
 // 1 the tanh form of GELU, 0.5 g (1 + tanh(u)) with u = sqrt(2/pi) (g + 0.044715 g^3),
 // which is g / (1 + exp(-2u)).
 __device__ __forceinline__ float fb_glu_act(float g, int act) {
   const float z = act == 0 ? g : 1.5957691216057308f * (g + 0.044715f * g * g * g);
-  return g / (1.0f + __expf(-z));
+  return fb_quotient(g, 1.0f + __expf(-z));
 }
 
 // A gated feed-forward with clamped halves: g = min(gate + b, limit), u = clamp(up + b, -limit,

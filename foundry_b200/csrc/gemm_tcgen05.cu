@@ -350,7 +350,7 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap map_a,
                   const float gate = fminf(__uint_as_float(g[e + 2 * q + h]), glu.limit);
                   const float up =
                       fminf(fmaxf(__uint_as_float(u[e + 2 * q + h]), -glu.limit), glu.limit);
-                  r2[h] = gate * (1.0f / (1.0f + __expf(-glu.alpha * gate))) * (up + glu.shift);
+                  r2[h] = fb_quotient(gate, 1.0f + __expf(-glu.alpha * gate)) * (up + glu.shift);
                 }
                 const __nv_bfloat162 h2 = __floats2bfloat162_rn(r2[0], r2[1]);
                 pk[q] = *reinterpret_cast<const uint32_t*>(&h2);
@@ -571,7 +571,7 @@ gemm_tc_grouped_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                   const float gate = fminf(__uint_as_float(g[e + 2 * q + h]), glu.limit);
                   const float up =
                       fminf(fmaxf(__uint_as_float(u[e + 2 * q + h]), -glu.limit), glu.limit);
-                  r2[h] = gate * (1.0f / (1.0f + __expf(-glu.alpha * gate))) * (up + glu.shift);
+                  r2[h] = fb_quotient(gate, 1.0f + __expf(-glu.alpha * gate)) * (up + glu.shift);
                 }
                 const __nv_bfloat162 h2 = __floats2bfloat162_rn(r2[0], r2[1]);
                 pk[q] = *reinterpret_cast<const uint32_t*>(&h2);
