@@ -880,7 +880,8 @@ int launch_grouped_persistent(const CUtensorMap& ma, const CUtensorMap& mb, cons
 // over groups of ceil(rows of the group / 128); rows_a / 128 + groups always is.
 // glu 1: a group's rows are rows_b / 2 gate rows, then as many up rows; out is bf16
 // [rows_a, rows_b / 2] = act(gate) * up with the rule of `gemm_tc_grouped_kernel`.
-// persistent 1: the form with one CTA an SM and two accumulators, where it applies.
+// persistent 1: the form with one CTA an SM and two accumulators, where it applies; 2: the
+// form with two SMs on a tile (gemm_tcgen05_pair.cu), where it applies, else as 1.
 FB_API int fb_gemm_tc_grouped(const void* a, long long lda, int rows_a, const void* b,
                               long long ldb, int rows_b, int K, const int* starts, int groups,
                               int slots, void* out, long long ldo, int out_f32, int glu,
@@ -897,6 +898,9 @@ FB_API int fb_gemm_tc_grouped(const void* a, long long lda, int rows_a, const vo
              ldo);
   FB_REQUIRE(!glu || (!out_f32 && ldo % 8 == 0 && ((uintptr_t)out % 16) == 0),
              "gemm_tc_grouped: the gated form writes bfloat16 rows on 16-byte boundaries");
+  if (persistent == 2 && fb_grouped_pair_takes(rows_a, rows_b, groups))
+    return fb_gemm_tc_grouped_pair(a, lda, rows_a, b, ldb, rows_b, K, starts, groups, out, ldo,
+                                   out_f32, glu, limit, alpha, shift, stream);
   bind_status_mirror(stream);
   // the widest tile that divides a group's features: a tile never spans two groups
   // (gated: a tile is BN / 2 features wide, their gate rows and their up rows)

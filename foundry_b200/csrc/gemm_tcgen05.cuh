@@ -77,6 +77,12 @@ int fb_gemm_tc_pair(const void* a, long long lda, int rows_a, const void* b, lon
                     int rows_b, int bn, const FbGemmParams& p, void* workspace,
                     long long workspace_bytes, int* counters, int counters_len,
                     int share_min_kblocks, cudaStream_t stream);
+// The grouped product in pairs (the same file), called by fb_gemm_tc_grouped.
+bool fb_grouped_pair_takes(int rows_a, int rows_b, int groups);
+int fb_gemm_tc_grouped_pair(const void* a, long long lda, int rows_a, const void* b, long long ldb,
+                            int rows_b, int K, const int* starts, int groups, void* out,
+                            long long ldo, int out_f32, int glu, float limit, float alpha,
+                            float shift, cudaStream_t stream);
 
 namespace {
 

@@ -473,7 +473,333 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& 
   return fb_check_launch("gemm_tc_pair");
 }
 
+// ---------------------------------------------------------------- grouped pairs
+// The grouped product (gemm_tcgen05.cu has the task) with two SMs on a tile, and with the
+// weights as the instruction's 256 rows and a group's tokens as its N. Why: what an expert
+// gets is any number of tokens, and N goes in steps of 32 where rows go in steps of 128 (250
+// tokens: one tile of 256; 270: two of 160 and 110), and a pair takes half the bytes from L2
+// for a weight tile that a CTA by itself takes, which bounds the one-CTA form (96 bytes per
+// cycle and SM wanted, about 60 to be had). A group's tokens are cut into the fewest tiles of
+// at most 256, of about equal size; a unit is (token tile, 256 weight rows), a pair walks the
+// units cluster, cluster + clusters, ... with two accumulators as the dense form above. The
+// accumulator has features as lanes and tokens as columns, so a warp's store is 32 features
+// of a token. GLU: a CTA's 128 weight rows are 64 gate rows and the up rows of the same
+// features, so a feature's two sums sit 64 lanes apart: the sums take a turn through shared
+// memory, 16 tokens at a time, and a thread stores four features of a token.
+// 16 experts over 3,072 -> 2 x 2,048, gated: 500 rows each 164 us against 192 for one CTA an SM
+// (1.23 PFLOP/s), 1,000 rows 299 against 383; back, 2,048 -> 3,072: 97 against 119, 168 against
+// 216. Below about 128 rows an expert the weights' bytes bound both forms (ops.gemm_tc_grouped).
+constexpr int GROUPED_PAIR_SLOTS = 512;
+
+struct SmemGroupedPair {
+  static constexpr int A_BYTES = BM * BK * 2;
+  static constexpr int STAGE_BYTES = 2 * A_BYTES;
+  static constexpr int STAGES = 6;
+  static constexpr int EXCHANGE = 2 * 16 * BM * 4;  // two halves of 16 tokens
+  static constexpr int BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 + EXCHANGE;
+};
+
+// Token maps by the rows of their boxes (a CTA loads half of a tile's tokens).
+struct TokenMaps {
+  CUtensorMap rows128, rows64, rows32;
+};
+
+struct GroupedGlu {
+  float limit, alpha, shift;
+};
+
+// Whether all four epilogue warps are well (each comes here whatever became of its wait).
+__device__ __forceinline__ bool epilogue_all(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
+      "barrier.cta.red.and.aligned.pred p, 5, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(all) : "r"((uint32_t)ok) : "memory");
+  return all != 0;
+}
+
+template <bool GLU>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w,
+                            const __grid_constant__ TokenMaps maps, const int* starts, int groups,
+                            int rows_w, int K, void* out, long long ldo, int out_f32,
+                            const GroupedGlu glu) {
+  using S = SmemGroupedPair;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  float* exchange = (float*)(tiles + S::STAGES * S::STAGE_BYTES);
+  uint64_t* full = (uint64_t*)((uint8_t*)exchange + S::EXCHANGE);  // used in the leader
+  uint64_t* empty = full + S::STAGES;
+  uint64_t* acc_full = empty + S::STAGES;  // [2]
+  uint64_t* acc_empty = acc_full + 2;      // [2], used in the leader
+  uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  __shared__ int s_starts[257];
+  __shared__ int s_group[GROUPED_PAIR_SLOTS], s_row0[GROUPED_PAIR_SLOTS], s_rows[GROUPED_PAIR_SLOTS];
+  __shared__ int s_slots;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_cta_rank();
+  const bool leader = rank == 0;
+  const int cluster = (int)(blockIdx.x >> 1), clusters = (int)(gridDim.x >> 1);
+  const int nkb = (K + BK - 1) / BK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 8);  // the four epilogue warps of both CTAs
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fb_pdl_wait();  // `starts` is the work of an earlier kernel
+  for (int g = threadIdx.x; g <= groups; g += blockDim.x) s_starts[g] = __ldcg(starts + g);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int n = 0;
+    for (int g = 0; g < groups; ++g) {
+      const int rows = s_starts[g + 1] - s_starts[g];
+      if (rows <= 0) continue;
+      const int cuts = (rows + 255) / 256;
+      const int per = ((rows + cuts - 1) / cuts + 31) / 32 * 32;
+      for (int r = 0; r < rows && n < GROUPED_PAIR_SLOTS; r += per, ++n) {
+        s_group[n] = g;
+        s_row0[n] = s_starts[g] + r;
+        s_rows[n] = min(per, rows - r);
+      }
+    }
+    s_slots = n;
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_barrier();  // the peer's barriers exist before anything arrives on them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int tiles_w = rows_w / (2 * BM);
+  const int total_units = s_slots * tiles_w;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      const uint32_t full_leader = cluster_address(&full[0], 0);
+      int it = 0;
+      bool ok = true;
+      for (int u = cluster; u < total_units && ok; u += clusters, it += nkb) {
+        const int slot = u / tiles_w, tw = u - slot * tiles_w;
+        const int half = (s_rows[slot] + 31) / 32 * 16;  // tokens of a CTA
+        const int row0 = s_row0[slot] + (int)rank * half;
+        const CUtensorMap* map_t = half > 64 ? &maps.rows128 : half > 32 ? &maps.rows64 : &maps.rows32;
+        const int box = half > 64 ? 128 : half > 32 ? 64 : 32;
+        const int w_row = s_group[slot] * rows_w +
+                          (GLU ? tw * BM + (int)rank * (BM / 2) : tw * 2 * BM + (int)rank * BM);
+        for (int kb = 0; kb < nkb; ++kb) {
+          const int use = it + kb;
+          const int s = use % S::STAGES;
+          const uint32_t phase = (uint32_t)(use / S::STAGES) & 1u;
+          if (!mbar_wait(&empty[s], phase ^ 1u, abort_flag, 1, kb)) { ok = false; break; }
+          uint8_t* w_dst = tiles + s * S::STAGE_BYTES;
+          uint8_t* t_dst = w_dst + S::A_BYTES;
+          if (leader) mbar_expect_tx(&full[s], 2 * (S::A_BYTES + box * BK * 2));
+          const uint32_t bar = full_leader + (uint32_t)(s * 8);
+          tma_load_2d_pair(w_dst, &map_w, bar, kb * BK, w_row);
+          if constexpr (GLU)
+            tma_load_2d_pair(w_dst + S::A_BYTES / 2, &map_w, bar, kb * BK, w_row + rows_w / 2);
+          tma_load_2d_pair(t_dst, map_t, bar, kb * BK, row0);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------- MMA issuer (leader only)
+    if (lane == 0 && leader) {
+      int it = 0, j = 0;
+      bool ok = true;
+      for (int u = cluster; u < total_units && ok; u += clusters, ++j, it += nkb) {
+        const uint32_t idesc = make_idesc(2 * BM, (s_rows[u / tiles_w] + 31) / 32 * 32);
+        const int buf = j & 1;
+        ok = mbar_wait_cluster(&acc_empty[buf], (uint32_t)((j >> 1) & 1) ^ 1u, abort_flag, 4, j);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * 256);
+        for (int kb = 0; kb < nkb; ++kb) {
+          const int use = it + kb;
+          const int s = use % S::STAGES;
+          const uint32_t phase = (uint32_t)(use / S::STAGES) & 1u;
+          ok = mbar_wait_cluster(&full[s], phase, abort_flag, 2, kb);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t w_addr = smem_u32(tiles + s * S::STAGE_BYTES);
+          const uint32_t t_addr = w_addr + S::A_BYTES;
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_pair(d_tmem, make_desc(w_addr + k * UMMA_K * 2),
+                      make_desc(t_addr + k * UMMA_K * 2), idesc, (kb | k) != 0 ? 1u : 0u);
+          tc_commit_pair(&empty[s]);
+        }
+        if (!ok) break;
+        tc_commit_pair(&acc_full[buf]);
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------- epilogue
+    const int quarter = warp & 3;
+    float* out_f = (float*)out;
+    __nv_bfloat16* out_h = (__nv_bfloat16*)out;
+    const uint32_t acc_empty_leader = cluster_address(&acc_empty[0], 0);
+    int j = 0;
+    for (int u = cluster; u < total_units; u += clusters, ++j) {
+      const int slot = u / tiles_w, tw = u - slot * tiles_w;
+      const int rows = s_rows[slot];
+      const long long row0 = s_row0[slot];
+      const int buf = j & 1;
+      if (!epilogue_all(mbar_wait(&acc_full[buf], (uint32_t)((j >> 1) & 1), abort_flag, 3, j))) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256);
+#pragma unroll 1
+      for (int c = 0; c < rows; c += 32) {
+        uint32_t r[32];
+        tmem_ld32(taddr + (uint32_t)c, r);
+        tmem_ld_wait();
+        if constexpr (GLU) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {  // 16 tokens at a time, [token][64 gates, 64 ups]
+            float* there = exchange + h * 16 * BM;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) there[e * BM + quarter * 32 + lane] = __uint_as_float(r[16 * h + e]);
+            // the half before this one has been read by all when they meet here
+            asm volatile("barrier.cta.sync.aligned 1, 128;" ::: "memory");
+            const int t = quarter * 4 + (lane >> 3), col = c + 16 * h + t;
+            __nv_bfloat16* dst = out_h + (row0 + col) * ldo + (long long)tw * BM + (int)rank * (BM / 2);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const int f = k * 32 + 4 * (lane & 7);
+              const float4 g4 = *reinterpret_cast<const float4*>(there + t * BM + f);
+              const float4 u4 = *reinterpret_cast<const float4*>(there + t * BM + BM / 2 + f);
+              const float g[4] = {g4.x, g4.y, g4.z, g4.w}, v[4] = {u4.x, u4.y, u4.z, u4.w};
+              float y[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const float gate = fminf(g[q], glu.limit);
+                const float up = fminf(fmaxf(v[q], -glu.limit), glu.limit);
+                y[q] = fb_quotient(gate, 1.0f + __expf(-glu.alpha * gate)) * (up + glu.shift);
+              }
+              const __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]);
+              const __nv_bfloat162 hi = __floats2bfloat162_rn(y[2], y[3]);
+              uint2 pk;
+              pk.x = *reinterpret_cast<const uint32_t*>(&lo);
+              pk.y = *reinterpret_cast<const uint32_t*>(&hi);
+              if (col < rows) *reinterpret_cast<uint2*>(dst + f) = pk;
+            }
+          }
+        } else {
+          const long long f = (long long)tw * 2 * BM + (int)rank * BM + quarter * 32 + lane;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            if (c + e < rows) {
+              const float v = __uint_as_float(r[e]);
+              if (out_f32) out_f[(row0 + c + e) * ldo + f] = v;
+              else out_h[(row0 + c + e) * ldo + f] = __float2bfloat16(v);
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(acc_empty_leader + (uint32_t)(buf * 8));
+    }
+  }
+  // ------------------------------------------------------------------ teardown
+  tc_fence_before();
+  __syncthreads();
+  cluster_barrier();  // nothing of the peer's may still be on its way to this CTA
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u)
+                 : "memory");
+  }
+}
+
+template <bool GLU>
+int launch_grouped_pair(const CUtensorMap& mw, const TokenMaps& maps, const int* starts, int groups,
+                        int rows_w, int K, void* out, long long ldo, int out_f32,
+                        const GroupedGlu& glu, long long most_units, cudaStream_t stream) {
+  static int clusters_of_device[64] = {};  // CTA pairs that run at once, per device
+  int device = 0;
+  cudaGetDevice(&device);
+  if (device < 0 || device >= 64) device = 63;
+  int& clusters_max = clusters_of_device[device];
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = SmemGroupedPair::BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  if (clusters_max == 0) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_grouped_pair_kernel<GLU>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SmemGroupedPair::BYTES);
+    if (e != cudaSuccess)
+      return fb_fail(2, "gemm_tc_grouped: shared memory opt-in: %s", cudaGetErrorString(e));
+    cfg.gridDim = dim3(sm_count() / 2 * 2);
+    cfg.numAttrs = 1;
+    int n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, gemm_tc_grouped_pair_kernel<GLU>, &cfg);
+    if (e != cudaSuccess || n <= 0)
+      return fb_fail(2, "gemm_tc_grouped: no CTA pair of this kernel fits the device (%s)",
+                     cudaGetErrorString(e));
+    clusters_max = n;
+  }
+  cfg.gridDim = dim3(2 * (unsigned)(most_units < clusters_max ? most_units : clusters_max));
+  cfg.numAttrs = g_fb_pdl ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, gemm_tc_grouped_pair_kernel<GLU>, mw, maps, starts, groups, rows_w, K, out,
+                     ldo, out_f32, glu);
+  return fb_check_launch("gemm_tc_grouped_pair");
+}
+
 }  // namespace
+
+// Whether the form above takes these sizes: whole tiles of 256 weight rows, a table of all tiles.
+bool fb_grouped_pair_takes(int rows_a, int rows_b, int groups) {
+  return rows_b % (2 * BM) == 0 && groups <= 256 && rows_a / 256 + groups <= GROUPED_PAIR_SLOTS;
+}
+
+// The grouped product in pairs; arguments as checked by fb_gemm_tc_grouped.
+int fb_gemm_tc_grouped_pair(const void* a, long long lda, int rows_a, const void* b, long long ldb,
+                            int rows_b, int K, const int* starts, int groups, void* out,
+                            long long ldo, int out_f32, int glu, float limit, float alpha,
+                            float shift, cudaStream_t stream) {
+  bind_status_mirror(stream);
+  CUtensorMap mw;
+  TokenMaps maps;
+  int rc = make_map(&mw, b, (long long)groups * rows_b, K, ldb, glu ? BM / 2 : BM);
+  if (!rc) rc = make_map(&maps.rows128, a, rows_a, K, lda, 128);
+  if (!rc) rc = make_map(&maps.rows64, a, rows_a, K, lda, 64);
+  if (!rc) rc = make_map(&maps.rows32, a, rows_a, K, lda, 32);
+  if (rc) return rc;
+  const long long most = (long long)(rows_a / 256 + groups) * (rows_b / (2 * BM));
+  const GroupedGlu rule{limit, alpha, shift};
+  return glu ? launch_grouped_pair<true>(mw, maps, starts, groups, rows_b, K, out, ldo, out_f32, rule,
+                                         most, stream)
+             : launch_grouped_pair<false>(mw, maps, starts, groups, rows_b, K, out, ldo, out_f32,
+                                          rule, most, stream);
+}
 
 // a, b as in fb_gemm_tc; `p` filled by it. A in blocks of 256 rows, each CTA of a
 // pair loads half of a B tile (bn / 2 rows).

@@ -3246,14 +3246,16 @@ def moe_grouped_tc_fits(x: torch.Tensor, *sizes: int) -> bool:
 
 def gemm_tc_grouped(rows: torch.Tensor, w: torch.Tensor, order: "ExpertOrder",
                     out_dtype: torch.dtype = torch.float32, glu: Optional[tuple] = None,
-                    persistent: Optional[bool] = None) -> torch.Tensor:
+                    persistent: Optional[int] = None) -> torch.Tensor:
     """out[i] = rows[i] @ w[expert of row i]^T for rows sorted by expert (`order.starts`):
     rows [pairs, K] bfloat16, w [E, N, K] bfloat16 -> [pairs, N], in one launch on the
     tensor cores (csrc/gemm_tcgen05.cu, `gemm_tc_grouped_kernel`). Nothing of the launch
     depends on the experts' counts, so a captured step may hold it. `glu` = (limit, alpha,
     shift): an expert's rows are N / 2 gate rows and then as many up rows, and the result is
     bfloat16 [pairs, N / 2] = min(g, limit) sigmoid(alpha min(g, limit)) (clamp(u, +-limit) +
-    shift), made in the product's epilogue."""
+    shift), made in the product's epilogue. `persistent`: the form (0: a CTA a tile; 1: a CTA
+    an SM; 2: pairs of SMs with the weights as rows, csrc/gemm_tcgen05_pair.cu); each passes
+    on to the one before where it does not apply."""
     pairs, K = rows.shape
     E, N, Kw = w.shape
     if Kw != K or E != order.experts or pairs != order.pairs or not w.is_contiguous():
@@ -3268,12 +3270,19 @@ def gemm_tc_grouped(rows: torch.Tensor, w: torch.Tensor, order: "ExpertOrder",
     if pairs == 0:
         return out
     limit, alpha, shift = glu if glu is not None else (0.0, 0.0, 0.0)
+    form = persistent
+    if form is None:
+        # pairs of SMs from 128 rows an expert on average. Gated + plain product of 16 experts of
+        # 2,048 over 3,072, even counts, against one CTA an SM: 16 rows each 154 us for 143, 125
+        # 163 for 163, 250 190 for 191, 500 261 for 311; 64 experts of 1,024, 125 rows 210 for 222.
+        # A router's counts are less even, which these tiles mind less: the whole feed-forward of
+        # 2,000 tokens of 3,072 (250 rows an expert on average) 258 us for 280.
+        form = 0 if not MOE_GROUPED_TC_PERSISTENT else 2 if pairs >= 128 * E else 1
     _call("fb_gemm_tc_grouped", _dev(rows, "rows", contiguous=False), _rows(rows, "rows"), pairs,
           _dev(w, "w"), K, N, K, order.starts.data_ptr(), E, pairs // 128 + E, _dev(out, "out"),
           width, 1 if out_dtype == torch.float32 else 0, 0 if glu is None else 1, float(limit),
           float(alpha), float(shift),
-          1 if (MOE_GROUPED_TC_PERSISTENT if persistent is None else persistent) else 0, _stream(),
-          tag=("m{} k{} n{}", pairs, K, N))
+          int(form), _stream(), tag=("m{} k{} n{}", pairs, K, N))
     return out
 
 
