@@ -323,7 +323,7 @@ __device__ __forceinline__ void sort_pairs(const int* chosen, int n_pairs, int E
 #pragma unroll
       for (int k = 0; k < AHEAD; ++k) {
         const int i = base + 32 * k + lane;
-        e[k] = i < last ? __ldcg(chosen + i) : -2;
+        e[k] = i < last ? __ldcg(chosen + i) : -1;
       }
 #pragma unroll
       for (int k = 0; k < AHEAD; ++k) {
@@ -381,7 +381,7 @@ __device__ __forceinline__ void sort_pairs(const int* chosen, int n_pairs, int E
     if (has && rank == 0) held[warp][e] += __popc(same);
     if (has) pair_at[where] = i;
     // pairs without an expert among the first E (identity experts) are put nowhere
-    if (e != -2) place[i] = where;
+    if (i < last) place[i] = where;
   });
 }
 

@@ -32,6 +32,18 @@ def test_sort_of_the_pairs(ops, pairs, E, experts):
     assert order.place.flatten().cpu().tolist() == place.tolist()
 
 
+def test_choices_that_name_no_expert_have_no_place(ops):
+    """Any number outside the experts, on either side of the table."""
+    chosen = torch.tensor([[-2, 0], [-1, 3], [4, -2], [2, -2 ** 31], [3, 2 ** 31 - 1]],
+                          dtype=torch.int32).to(DEV)
+    order = ops.ExpertOrder(chosen, 4, sort=False)
+    order.place.fill_(7)  # a place that would be read as a row
+    ops._call("fb_moe_sort", chosen.data_ptr(), 10, 4, order.counts.data_ptr(), order.starts.data_ptr(),
+              order.place.data_ptr(), order.pair_at.data_ptr(), ops._stream())
+    assert order.place.cpu().tolist() == [[-1, 0], [-1, 2], [-1, -1], [1, -1], [3, -1]]
+    assert order.pair_at.cpu().tolist()[:4] == [1, 6, 3, 8] and order.counts.cpu().tolist() == [1, 0, 1, 2]
+
+
 @pytest.mark.parametrize("T", [1, 65, 70])
 @pytest.mark.parametrize("W", [64, 1028, 70])
 def test_gather_and_combine(ops, T, W):
