@@ -3152,7 +3152,7 @@ def moe_router_fits(x, router: torch.Tensor) -> bool:
     also applies a norm's pending scale, and that block are two launches, too)."""
     return (isinstance(x, torch.Tensor) and x.shape[0] > MOE_ROUTE_SORT_ROWS
             and x.dtype == router.dtype == torch.bfloat16 and router.shape[0] <= 64
-            and x.shape[1] % 64 == 0 and x.stride(1) == router.stride(1) == 1
+            and x.shape[1] == router.shape[1] and x.shape[1] % 64 == 0 and x.stride(1) == router.stride(1) == 1
             and x.stride(0) % 8 == 0 and router.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0 and router.data_ptr() % 16 == 0)
 
@@ -3166,6 +3166,9 @@ def moe_router_sorted(x: torch.Tensor, router: torch.Tensor, bias: Optional[torc
     """The router's product in 32 bits, the choice (`moe_route`) and the sort of the chosen pairs."""
     T, K = x.shape
     E = router.shape[0]
+    if router.shape != (E, K) or tuple(chosen.shape) != (T, top) or tuple(weights.shape) != (T, top):
+        raise KernelError(f"moe_router: x {tuple(x.shape)}, router {tuple(router.shape)}, choices "
+                          f"{tuple(chosen.shape)} and weights {tuple(weights.shape)}")
     if correction is not None and tuple(correction.shape) != (E,):
         raise KernelError(f"moe_router: a correction of {tuple(correction.shape)} for {E} experts")
     z = torch.empty((T, E), dtype=torch.float32, device=x.device)
