@@ -2556,12 +2556,16 @@ def attention_maps_paged(ctx, q, out, page_table, k_cache, v_cache, H: int, G: i
 def _tc_rows_blocks(ctx, q, out, k, k_shared, v, k1: int, k2: int, vdim: int, softcap: float) -> int:
     """128-row query blocks of a step that the tcgen05 kernel over rows takes, else 0: some
     sequence brings 64 tokens or more, keys of 64 or 128 elements and up to 64 shared ones, no
-    soft cap, and 16-byte rows throughout."""
+    soft cap, heads side by side in rows of 16-byte pieces throughout (a head or a row that all
+    read, an expanded view, is no box of a tensor map)."""
     if not PREFILL_TC or softcap or k_shared is None or k1 not in (64, 128) or not 0 < k2 <= 64 \
             or k2 % 8 or vdim % 8 or vdim > 128:
         return 0
     for t in (q, out, k, k_shared, v):
         if t.data_ptr() % 16 or any(n % 8 for n in t.stride()[:-1]):
+            return 0
+        heads = (t.shape[1] - 1) * t.stride(1) if t.dim() == 3 else 0
+        if t.stride(0) < heads + t.shape[-1] or (t.dim() == 3 and t.stride(1) < t.shape[2]):
             return 0
     if ctx.cu_tokens_host is None:  # a replayed step: bounds that its bucket gives
         return (ctx.query_blocks_bound + 1) // 2 + ctx.n_seqs if ctx.long_queries else 0

@@ -1,5 +1,7 @@
 """Which kernel a call goes to: rules that read shapes, strides and counts alone, so that tensors on
 the CPU show them."""
+import types
+
 import pytest
 import torch
 
@@ -20,3 +22,28 @@ def test_router_kernel_takes_rows_of_the_routers_width_only():
     with pytest.raises(ops.KernelError, match="choices"):
         ops.moe_router_sorted(x, router, None, 2, torch.zeros(99, 2, dtype=torch.int32),
                               torch.zeros(99, 2), 8)
+
+
+def rows_of(T, H=3, k1=64, k2=32, e=64):
+    bf = dict(dtype=torch.bfloat16)
+    return [torch.zeros(T, H * (k1 + k2), **bf), torch.zeros(T, H * e, **bf), torch.zeros(T, H, k1, **bf),
+            torch.zeros(T, k2, **bf), torch.zeros(T, H, e, **bf)]
+
+
+def rows_step(lens):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    return types.SimpleNamespace(n_seqs=len(lens), cu_tokens_host=cu)
+
+
+def test_rows_attention_on_tensor_maps_takes_heads_side_by_side_only():
+    T, ctx = 96, rows_step([96])
+    q, out, k, shared, v = rows_of(T)
+    assert ops._tc_rows_blocks(ctx, q, out, k, shared, v, 64, 32, 64, 0.0) == 1
+    for other in (dict(k=k[:, :1].expand(T, 3, 64)), dict(v=v[:, :1].expand(T, 3, 64)),
+                  dict(shared=shared[:1].expand(T, 32)), dict(k=k[:1].expand(T, 3, 64)),
+                  dict(v=torch.zeros(3, T, 64, dtype=torch.bfloat16).transpose(0, 1)),
+                  dict(k=torch.zeros(T, 96, dtype=torch.bfloat16).as_strided((T, 3, 64), (96, 16, 1)))):
+        args = dict(dict(k=k, shared=shared, v=v), **other)
+        assert ops._tc_rows_blocks(ctx, q, out, args["k"], args["shared"], args["v"], 64, 32, 64, 0.0) == 0

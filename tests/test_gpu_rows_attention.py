@@ -73,3 +73,38 @@ def test_another_sequences_numbers_do_not_matter(ops):
         ops.attention_maps_rows(ctx, q, out, kv[:, :, :64], low, kv[:, :, 64:], H, 96, 64, 0.1)
         results.append(out[cu[1]:cu[2]].clone())
     assert bool(torch.isfinite(results[0]).all()) and torch.equal(*results)
+
+
+def plain(q, k, shared, v, H, scale):
+    n = q.shape[0]
+    keys = torch.cat([k, shared[:, None].expand(n, H, shared.shape[1])], -1).double()
+    w = torch.einsum("ihd,jhd->hij", q.double().view(n, H, -1), keys) * scale
+    w = w.masked_fill(torch.triu(torch.ones(n, n, dtype=torch.bool, device=DEV), 1), -torch.inf)
+    return torch.einsum("hij,jhe->ihe", torch.softmax(w, -1), v.double()).reshape(n, -1)
+
+
+@pytest.mark.parametrize("form", ["one head's keys for all", "one head's values for all", "one row of keys",
+                                  "overlapping heads", "heads outside"])
+def test_views_of_any_strides(ops, form):
+    """Views whose heads or rows are no boxes side by side, too, as the kernel without tensor maps
+    reads them."""
+    H, T, e = 3, 96, 64
+    ctx, _ = step_of([T])
+    gen = torch.Generator().manual_seed(7)
+    rnd = lambda *s: torch.randn(*s, generator=gen).to(torch.bfloat16).to(DEV)  # noqa: E731
+    q, k, v, shared = rnd(T, H * 96), rnd(T, H, 64), rnd(T, H, e), rnd(T, 32)
+    if form == "one head's keys for all":
+        k = k[:, :1].expand(T, H, 64)
+    elif form == "one head's values for all":
+        v = v[:, :1].expand(T, H, e)
+    elif form == "one row of keys":
+        k, shared = k[:1].expand(T, H, 64), shared[:1].expand(T, 32)
+    elif form == "overlapping heads":
+        k = rnd(T, 96).as_strided((T, H, 64), (96, 16, 1))
+    else:  # a head's rows together
+        k, v = rnd(H, T, 64).transpose(0, 1), rnd(H, T, e).transpose(0, 1)
+    out = torch.full((T, H * e), 9.0, dtype=torch.bfloat16, device=DEV)
+    ops.attention_maps_rows(ctx, q, out, k, shared, v, H, 96, e, 0.1)
+    want = plain(q, k, shared, v, H, 0.1)
+    # weights and outputs rounded to bfloat16 (2^-9 each) of values of up to about four
+    assert float((out.double() - want).abs().max()) < 4 * 2.0 ** -7
