@@ -260,8 +260,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
       fb_pdl_wait();  // the queries and this step's keys and values come from earlier kernels
       mbar_expect_tx(q_full, Smem::Q_BYTES);
 #pragma unroll
-      for (int sb = 0; sb < KS; ++sb)
-        tma_load_2d(sQ + sb * Q_SUB, &map_q, q_full, head * p.D + sb * 64, tok0 + row0);
+      for (int sb = 0; sb < KS; ++sb) {
+        // (ROWS: a head of its own in the map, so that what lies behind a head's last element is
+        // zero and not the next head's: the keys' zeros there would not hide a number that is none)
+        if constexpr (ROWS) tma_load_3d(sQ + sb * Q_SUB, &map_q, q_full, sb * 64, head, tok0 + row0);
+        else tma_load_2d(sQ + sb * Q_SUB, &map_q, q_full, head * p.D + sb * 64, tok0 + row0);
+      }
       for (int j = 0; j < n_pages; ++j) {
         const int s = j % RING;
         const uint32_t parity = (uint32_t)((j / RING) & 1) ^ 1u;
@@ -719,7 +723,9 @@ FB_API int fb_attention_prefill_rows(const void* q, long long q_stride, int T, v
     const int box[2] = {64, rows};
     return make_map(map, at, 2, dims, strides, box);
   };
-  int rc = rows_map(&mq, q, (long long)A * (K1 + K2), q_stride, BQ);
+  const long long qdims[3] = {K1 + K2, A, T}, qstrides[2] = {K1 + K2, q_stride};
+  const int qbox[3] = {64, 1, BQ};
+  int rc = make_map(&mq, q, 3, qdims, qstrides, qbox);
   if (!rc) rc = rows_map(&mk, k, (long long)(A - 1) * k_head + K1, k_row, FB_PAGE);
   if (!rc) rc = rows_map(&ms, k_shared, K2, ks_row, FB_PAGE);
   if (!rc) rc = rows_map(&mv, v, (long long)(A - 1) * v_head + DV, v_row, FB_PAGE);

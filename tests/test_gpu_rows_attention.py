@@ -75,6 +75,25 @@ def test_another_sequences_numbers_do_not_matter(ops):
     assert bool(torch.isfinite(results[0]).all()) and torch.equal(*results)
 
 
+@pytest.mark.parametrize("k1,k2,e", [(64, 32, 64), (64, 8, 72), (128, 16, 64)])
+def test_another_heads_numbers_do_not_matter(ops, k1, k2, e):
+    """Queries, keys and values of one head that are no numbers leave the other heads as they are."""
+    H, T = 3, 200
+    ctx, _ = step_of([T])
+    gen = torch.Generator().manual_seed(11)
+    rnd = lambda *s: torch.randn(*s, generator=gen).to(torch.bfloat16).to(DEV)  # noqa: E731
+    q, kv, low = rnd(T, H, k1 + k2), rnd(T, H, k1 + e), rnd(T, k2)
+    results = []
+    for spoil in (False, True):
+        if spoil:
+            q[:, 1], kv[:, 1] = float("nan"), float("inf")
+        out = torch.empty(T, H, e, dtype=torch.bfloat16, device=DEV)
+        ops.attention_maps_rows(ctx, q.view(T, -1), out.view(T, -1), kv[:, :, :k1], low, kv[:, :, k1:], H,
+                                k1 + k2, e, 0.1)
+        results.append(out[:, [0, 2]].clone())
+    assert bool(torch.isfinite(results[0]).all()) and torch.equal(*results)
+
+
 def plain(q, k, shared, v, H, scale):
     n = q.shape[0]
     keys = torch.cat([k, shared[:, None].expand(n, H, shared.shape[1])], -1).double()
