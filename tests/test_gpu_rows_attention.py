@@ -127,3 +127,21 @@ def test_views_of_any_strides(ops, form):
     want = plain(q, k, shared, v, H, 0.1)
     # weights and outputs rounded to bfloat16 (2^-9 each) of values of up to about four
     assert float((out.double() - want).abs().max()) < 4 * 2.0 ** -7
+
+
+@pytest.mark.parametrize("k1,k2,e", [(64, 32, 64), (128, 64, 128)])
+def test_as_close_to_float64_as_the_kernel_without_tensor_maps(ops, k1, k2, e, monkeypatch):
+    """Both round weights and outputs to bfloat16; a weight of one, a row's largest, is exact in both."""
+    H, T = 8, 900
+    ctx, _ = step_of([T])
+    gen = torch.Generator().manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=gen).to(torch.bfloat16).to(DEV)  # noqa: E731
+    q, k, v, shared = rnd(T, H * (k1 + k2)), rnd(T, H, k1), rnd(T, H, e), rnd(T, k2)
+    scale = (k1 + k2) ** -0.5
+    want, off = plain(q, k, shared, v, H, scale), []
+    for tensor_maps in (True, False):
+        monkeypatch.setattr(ops, "PREFILL_TC", tensor_maps)
+        out = torch.empty(T, H * e, dtype=torch.bfloat16, device=DEV)
+        ops.attention_maps_rows(ctx, q, out, k, shared, v, H, k1 + k2, e, scale)
+        off.append(float((out.double() - want).norm() / want.norm()))
+    assert off[0] <= off[1], off
