@@ -36,15 +36,16 @@ __device__ __forceinline__ float exp_below(float a, float b) {
 
 // ------------------------------------------------------------------- few tokens a sequence
 // Eight lanes share a key (a lane holds D / 8 elements of every query head and of its sums, in
-// runs of 4), a warp takes four keys side by side and U of each lane group's keys at a time;
+// runs of 4), W warps share a pair, each takes four keys side by side and U of each lane group's
+// keys at a time (two where four would not fit the registers);
 // lane groups, warps and CTAs keep a maximum and a sum of their own and are merged in a fixed
 // order at the end.
-constexpr int SPLIT_WARPS = 4, SPLIT_GROUPS = SPLIT_WARPS * 4, U = 4;
-
-template <int D, int GH, int S>
-__global__ void __launch_bounds__(SPLIT_WARPS * 32)
+template <int D, int GH, int S, int W>
+__global__ void __launch_bounds__(W * 32)
 split_kernel(FbAttentionF32 p, int head_chunks) {
-  constexpr int V4 = D / 32;
+  constexpr int V4 = D / 32, SPLIT_WARPS = W, SPLIT_GROUPS = W * 4;
+  constexpr bool FEW = W < 4;  // mostly few keys
+  constexpr int U = FEW && D >= 128 ? 2 : 4;
   __shared__ float stat_m[SPLIT_GROUPS][GH], stat_l[SPLIT_GROUPS][GH];
   __shared__ __align__(16) float sums[SPLIT_GROUPS][GH][D];
   __shared__ float cta_m[GH], cta_l[GH];
@@ -90,6 +91,11 @@ split_kernel(FbAttentionF32 p, int head_chunks) {
     float4 kk[U][V4], vv[U][V4];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
+      if (FEW && u > 0 && j0 + u * SPLIT_GROUPS >= end) {  // no group has a key there
+#pragma unroll
+        for (int i = 0; i < V4; ++i) kk[u][i] = vv[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        continue;
+      }
       const int j = min(j0 + u * SPLIT_GROUPS + group, end - 1);  // beyond the end: masked below
       const long long row = row_of(pages, j, p.ring_pages, p.page_stride, D);
 #pragma unroll
@@ -162,14 +168,18 @@ split_kernel(FbAttentionF32 p, int head_chunks) {
       *reinterpret_cast<float4*>(&sums[group][h][part * 4 + 32 * i]) = acc[h][i];
   }
   __syncthreads();
-  // the block's groups into group 0's place (each element by one thread)
+  // the block's groups into group 0's place (each element by one thread); groups that saw no key
+  // hold nothing
+  const int seen = FEW ? max(1, min(SPLIT_GROUPS, end - begin)) : SPLIT_GROUPS;
   for (int i = threadIdx.x; i < GH * D; i += SPLIT_WARPS * 32) {
     const int h = i / D, d = i % D;
     float top = -INFINITY, sum = 0.f, total = 0.f;
 #pragma unroll
-    for (int g = 0; g < SPLIT_GROUPS; ++g) top = fmaxf(top, stat_m[g][h]);
+    for (int g = 0; g < SPLIT_GROUPS; ++g)
+      if (g < seen) top = fmaxf(top, stat_m[g][h]);
 #pragma unroll
     for (int g = 0; g < SPLIT_GROUPS; ++g) {
+      if (g >= seen) break;
       const float f = exp_below(stat_m[g][h], top);
       sum = fmaf(f, sums[g][h][d], sum);
       total = fmaf(f, stat_l[g][h], total);
@@ -262,6 +272,7 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
     qt[d + 2][r] = v.z;
     qt[d + 3][r] = v.w;
   }
+  const int warp_row = warp * 16;  // a warp's 16 rows
   for (int first = 0, run = 0; first < rows; ++run) {
     const int seq = seq_of[first];
     int last = first;  // the run's last row
@@ -291,6 +302,8 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
       inner_to = min(inner_to, pos_of[r]);
       inner_from = max(inner_from, lo);
     }
+    // a warp without a row of the run only helps to load
+    const bool mine_here = warp_row <= last && warp_row + 15 >= begin_row;
     const int* pages = p.page_table + (size_t)seq * p.max_pages;
     const float* kbase = p.k + (long long)kvh * p.head_stride;
     const float* vbase = p.v + (long long)kvh * p.head_stride;
@@ -328,6 +341,8 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
                  : make_float4(0.f, 0.f, 0.f, 0.f);
       }
       __syncthreads();
+      if (!mine_here) continue;
+      const int keys = min(BKEY, to - j0 + 1);  // (the rest of the tile counts as nothing)
       float s[4][4 * NK];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -338,13 +353,15 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
         float x[4], y[4 * NK];
         *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(&qt[d][ty * 4]);
 #pragma unroll
-        for (int q = 0; q < NK; ++q)
+        for (int q = 0; q < NK; ++q) {
+          if (q > 0 && q * 32 >= keys) break;
           *reinterpret_cast<float4*>(y + 4 * q) =
               *reinterpret_cast<const float4*>(&kt[d][q * 32 + tx * 4]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+          for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int c = 0; c < 4 * NK; ++c) s[i][c] = fmaf(x[i], y[c], s[i][c]);
+            for (int c = 4 * q; c < 4 * q + 4; ++c) s[i][c] = fmaf(x[i], y[c], s[i][c]);
+        }
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -385,7 +402,7 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
       // no number (a later token's): tiles on the edge of what the run sees leave such values out.
       auto add_values = [&](auto edge) {
 #pragma unroll 4
-        for (int key = 0; key < BKEY; ++key) {
+        for (int key = 0; key < (decltype(edge)::value ? keys : BKEY); ++key) {
           float x[4];
           *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(&pt[key][ty * 4]);
 #pragma unroll
@@ -425,15 +442,14 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
   }
 }
 
-template <int D, int GH, int S>
+template <int D, int GH, int S, int W = 4>
 int launch_split(const FbAttentionF32& p, cudaStream_t stream) {
   const int chunks = (p.A / p.Kh + GH - 1) / GH;
   const dim3 grid(p.T, p.Kh * chunks, S);
   if (S == 1)
-    fb_launch(split_kernel<D, GH, S>, grid, dim3(SPLIT_WARPS * 32), 0, stream, p, chunks);
+    fb_launch(split_kernel<D, GH, S, W>, grid, dim3(W * 32), 0, stream, p, chunks);
   else
-    fb_launch_cluster(split_kernel<D, GH, S>, grid, dim3(SPLIT_WARPS * 32), 0, stream, S, p,
-                      chunks);
+    fb_launch_cluster(split_kernel<D, GH, S, W>, grid, dim3(W * 32), 0, stream, S, p, chunks);
   return fb_check_launch("attention_f32_split");
 }
 
@@ -454,9 +470,21 @@ int launch_d(const FbAttentionF32& p, cudaStream_t stream) {
   if (tokens <= 16 * seqs) {
     const int G = p.A / p.Kh;
     const long long pairs = (long long)tokens * p.Kh * (G == 1 ? 1 : (G + 3) / 4);
-    // ranges until two blocks an SM are there, each of two pages and more
+    // ranges until two blocks an SM are there, each of two pages and more; several tokens a
+    // sequence with no more than eight pages mostly have few keys each (no more than 16 tokens may
+    // also be single ones, padded)
+    const bool several = tokens > 16 && tokens > seqs;
     int S = 1;
-    while (S < 8 && pairs * S < 2 * 148 && S * 2 * 2 <= width) S *= 2;
+    while (S < 8 && pairs * S < 2 * 148 && S * 2 * 2 <= width && !(several && width <= 8)) S *= 2;
+    // With few keys, 16 lane groups of four warps have more to merge than to add, and the pairs
+    // fill the SMs without them. 100 x 8 tokens, 32 heads over 8 of 64: 25 us with one warp a pair,
+    // 60 with four (attention_simt.cu 35); 4 x 8 tokens: 6.1 with two, 11.3 with four in two ranges
+    // (8.2). Single tokens keep four warps: 128 of them over 600 keys 94 us, 117 with two.
+    if (several && S == 1) {
+      if (pairs >= 1024)
+        return G == 1 ? launch_split<D, 1, 1, 1>(p, stream) : launch_split<D, 4, 1, 1>(p, stream);
+      return G == 1 ? launch_split<D, 1, 1, 2>(p, stream) : launch_split<D, 4, 1, 2>(p, stream);
+    }
     if (G == 1)
       return S == 8   ? launch_split<D, 1, 8>(p, stream)
              : S == 4 ? launch_split<D, 1, 4>(p, stream)

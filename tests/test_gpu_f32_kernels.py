@@ -121,6 +121,22 @@ def test_attention_of_prompts(ops, D, runs):
     check_attention(ops, paged_case(runs, 2, 2, D), 2, 2, D)
 
 
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("Kh,G", [(1, 1), (2, 3), (8, 4), (3, 6)])
+@pytest.mark.parametrize("runs", [
+    [(0, 0, 8), (1, 0, 3), (2, 61, 9), (3, 250, 2)],                     # one or two warps a pair
+    [(i, 3 * i, 1 + i % 16) for i in range(18)] + [(-1, 0, 5)],
+    [(i, 0, 17) for i in range(5)] + [(5, 30, 20)],                      # runs between warps' rows
+])
+def test_attention_of_short_prompts(ops, D, Kh, G, runs):
+    check_attention(ops, paged_case(runs, Kh, G, D), Kh, G, D)
+
+
+def test_attention_of_short_prompts_with_a_window(ops):
+    runs = [(i, 7 * i, 6) for i in range(12)]
+    check_attention(ops, paged_case(runs, 2, 4, 64, ring=3), 2, 4, 64, 5, 3)
+
+
 @pytest.mark.parametrize("runs", [[(0, 0, 1), (1, 250, 1)], [(0, 180, 70)]])
 @pytest.mark.parametrize("window", [1, 20, 90])
 def test_attention_with_a_window_on_a_ring(ops, runs, window):
