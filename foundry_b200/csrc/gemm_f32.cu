@@ -45,13 +45,16 @@ __device__ __forceinline__ float4 ld_stream(const float* p) {
 // weight rows). WK warps share the K of the same rows, the others own other rows; a result is
 // the sum over lanes by halving exchanges, then over the WK warps in order, whatever M is.
 constexpr int ROWS_WARPS = 8, ROWS_R = 4;
+// K that is staged at a time (one warp a row group: no more than there is, see launch_rows_by_shape)
+template <int WK>
+constexpr int ROWS_CHUNK = WK == 1 ? 128 : 512;
 
 template <int MR, int WK>
 __global__ void __launch_bounds__(ROWS_WARPS * 32, 2)
 rows_kernel(const float* x /* written by the kernel before: no read-only promise */,
             const float* __restrict__ w, float* out, int M, int N, int K, long long ldx,
             long long ldw, long long ldo) {
-  constexpr int WR = ROWS_WARPS / WK, KB = 128 * WK, CH = KB > 512 ? KB : 512, IT = CH / KB;
+  constexpr int WR = ROWS_WARPS / WK, KB = 128 * WK, CH = ROWS_CHUNK<WK>, IT = CH / KB;
   constexpr int V = MR * ROWS_R;
   extern __shared__ __align__(16) float smem[];  // [2][MR][CH]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -337,7 +340,7 @@ tile_kernel(const float* x /* written by the kernel before: no read-only promise
 
 template <int MR, int WK>
 int launch_rows(const FbGemmF32& p, cudaStream_t stream) {
-  constexpr int KB = 128 * WK, CH = KB > 512 ? KB : 512, WR = ROWS_WARPS / WK;
+  constexpr int CH = ROWS_CHUNK<WK>, WR = ROWS_WARPS / WK;
   constexpr int bytes = 2 * MR * CH * 4;
   static_assert(bytes >= ROWS_WARPS * MR * ROWS_R * 4, "room for the sums");
   static bool seen[64] = {};
@@ -353,8 +356,14 @@ int launch_rows(const FbGemmF32& p, cudaStream_t stream) {
 
 template <int MR>
 int launch_rows_by_shape(const FbGemmF32& p, cudaStream_t stream) {
-  // WK from N alone, so that a result's order of summation does not depend on M
-  if (p.N <= 8192) return launch_rows<MR, 4>(p, stream);
+  // WK from N and K alone, so that a result's order of summation does not depend on M. Up to 128 of
+  // K is one warp's: the others of four had nothing to do, and blocks of 8 rows of w each staged a
+  // whole chunk (32 rows, 64 -> 2048: 2.6 us for 7.2; 16 rows, 64 -> 16384: 6.1 for 14.0; the general
+  // kernel 5.3 and 7.6).
+  if (p.K <= 128) return launch_rows<MR, 1>(p, stream);
+  if constexpr (MR <= 8) {  // (16 rows a pass go with N > 8192)
+    if (p.N <= 8192) return launch_rows<MR, 4>(p, stream);
+  }
   return launch_rows<MR, 2>(p, stream);
 }
 
@@ -391,7 +400,10 @@ bool fb_gemm_f32_fits(const FbGemmF32& p) {
 }
 
 int fb_gemm_f32_launch(const FbGemmF32& p, cudaStream_t stream) {
-  if (p.count == 1 && p.M <= FB_GEMM_F32_ROWS) {
+  // (17 to 32 rows of many short columns are a tile's: 32 rows, 64 -> 16384 7.0 us against 10.1, 96
+  // 9.4 against 10.2, 128 11.9 against 10.4, 256 20.7 against 27.0)
+  const bool thin = p.M > 16 && p.N > 8192 && (p.K <= 96 || (p.K > 128 && p.K <= 256));
+  if (p.count == 1 && p.M <= FB_GEMM_F32_ROWS && !thin) {
     if (p.M == 1) return launch_rows_by_shape<1>(p, stream);
     if (p.M == 2) return launch_rows_by_shape<2>(p, stream);
     if (p.M <= 4) return launch_rows_by_shape<4>(p, stream);

@@ -29,7 +29,7 @@ def check_product(x, w, out):
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 129])
 @pytest.mark.parametrize("N,K", [(1, 4), (7, 132), (65, 516), (130, 1028), (8196, 260), (8190, 128),
-                                 (3, 4096)])
+                                 (3, 4096), (8193, 64), (8200, 200), (34, 124)])
 def test_product_of_16_byte_rows(ops, M, N, K):
     x, w = rnd(M, K), rnd(N, K, seed=1)
     wide = torch.full((M + 1, N + 5), 7.0, device=DEV)
