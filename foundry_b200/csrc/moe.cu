@@ -429,16 +429,19 @@ __global__ void moe_gather_kernel(const T* x, const int* pair_at, const int* sta
   for (int i = threadIdx.x; i < W; i += blockDim.x) out[(size_t)at * W + i] = x[(size_t)t * W + i];
 }
 
-// The same for rows of whole 16-byte pieces.
-__global__ void __launch_bounds__(256)
+// The same for rows of whole 16-byte pieces: a row's threads ask for four pieces together.
+constexpr int GATHER_THREADS = 64, GATHER_ROWS = 4;
+__global__ void __launch_bounds__(GATHER_THREADS * GATHER_ROWS)
 moe_gather_rows_kernel(const uint4* x, const int* pair_at, const int* starts, int E, int top,
                        uint4* __restrict__ out, int pieces) {
   fb_pdl_launch();
   fb_pdl_wait();
-  const int at = blockIdx.x;
+  const int at = blockIdx.x * GATHER_ROWS + threadIdx.y;
   if (at >= __ldcg(starts + E)) return;
   const uint4* row = x + (size_t)(__ldcg(pair_at + at) / top) * pieces;
-  for (int i = threadIdx.x; i < pieces; i += blockDim.x) out[(size_t)at * pieces + i] = __ldcg(row + i);
+  uint4* to = out + (size_t)at * pieces;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < pieces; i += GATHER_THREADS) to[i] = __ldcg(row + i);
 }
 
 __device__ __forceinline__ float glu_act(float g, float u, float limit, float alpha, float shift) {
@@ -907,8 +910,9 @@ FB_API int fb_moe_gather(const void* x, int dtype, const int* pair_at, const int
   if ((dtype == FB_BF16 || dtype == FB_F32) && bytes % 16 == 0 && ((uintptr_t)x % 16) == 0 &&
       ((uintptr_t)out % 16) == 0) {
     const int pieces = (int)(bytes / 16);
-    fb_launch(moe_gather_rows_kernel, dim3(n_pairs), dim3(pieces < 256 ? (pieces + 31) / 32 * 32 : 256),
-              0, stream, (const uint4*)x, pair_at, starts, E, top, (uint4*)out, pieces);
+    fb_launch(moe_gather_rows_kernel, dim3((n_pairs + GATHER_ROWS - 1) / GATHER_ROWS),
+              dim3(GATHER_THREADS, GATHER_ROWS), 0, stream, (const uint4*)x, pair_at, starts, E, top,
+              (uint4*)out, pieces);
     return fb_check_launch("moe_gather");
   }
   FB_DISPATCH_DTYPE(dtype, T_, (fb_launch(moe_gather_kernel<T_>, dim3(n_pairs), dim3(256), 0,

@@ -45,7 +45,7 @@ def test_choices_that_name_no_expert_have_no_place(ops):
 
 
 @pytest.mark.parametrize("T", [1, 65, 70])
-@pytest.mark.parametrize("W", [64, 1028, 70])
+@pytest.mark.parametrize("W", [64, 1028, 70, 4120])
 def test_gather_and_combine(ops, T, W):
     gen = torch.Generator().manual_seed(T + W)
     chosen = torch.randint(0, 6, (T, 3), generator=gen, dtype=torch.int32).to(DEV)
