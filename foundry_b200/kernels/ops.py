@@ -2555,7 +2555,7 @@ def attention_maps_paged(ctx, q, out, page_table, k_cache, v_cache, H: int, G: i
 
 def _tc_rows_blocks(ctx, q, out, k, k_shared, v, k1: int, k2: int, vdim: int, softcap: float) -> int:
     """128-row query blocks of a step that the tcgen05 kernel over rows takes, else 0: some
-    sequence brings 64 tokens or more, keys of 64 or 128 elements and up to 64 shared ones, no
+    sequence brings 64 tokens or more and all of them enough on average, keys of 64 or 128 elements and up to 64 shared ones, no
     soft cap, heads side by side in rows of 16-byte pieces throughout (a head or a row that all
     read, an expanded view, is no box of a tensor map)."""
     if not PREFILL_TC or softcap or k_shared is None or k1 not in (64, 128) or not 0 < k2 <= 64 \
@@ -2567,6 +2567,14 @@ def _tc_rows_blocks(ctx, q, out, k, k_shared, v, k1: int, k2: int, vdim: int, so
         heads = (t.shape[1] - 1) * t.stride(1) if t.dim() == 3 else 0
         if t.stride(0) < heads + t.shape[-1] or (t.dim() == 3 and t.stride(1) < t.shape[2]):
             return 0
+    # Its blocks are 128 rows, so sequences of up to 64 leave half of them empty (graph replays, 32
+    # heads of 64 + 32 and 64: one of 64 beside 31 of 8 tokens 24.6 us against 17.2, 64 of 64 50
+    # against 38, 16 of 64 11.7 each, 8 of 70 8.5 against 13.5). With keys of 128 it holds its own
+    # down to 16 a sequence (24 heads of 128 + 64 and 128: 16 a sequence 18.4 us against 18.3, 12
+    # 36 against 35, 36 46 against 70).
+    tokens, seqs = _padded_tokens(q.shape[0]), _padded(ctx.n_seqs, 1)
+    if tokens < (64 if k1 == 64 else 16) * seqs or (k1 == 64 and seqs > 16 and tokens == 64 * seqs):
+        return 0
     if ctx.cu_tokens_host is None:  # a replayed step: bounds that its bucket gives
         return (ctx.query_blocks_bound + 1) // 2 + ctx.n_seqs if ctx.long_queries else 0
     lens = [b - a for a, b in zip(ctx.cu_tokens_host, ctx.cu_tokens_host[1:])]
@@ -2883,13 +2891,18 @@ def _padded(n: int, least: int) -> int:
     return least
 
 
+def _padded_tokens(n: int) -> int:
+    """Tokens as a replayed step pads them: rules that go by them choose alike for both forms."""
+    return _padded(n, 16) if n <= 128 else (n + 127) // 128 * 128
+
+
 def chunk_scan_unit(ctx, mode: int, T: int, H: int, dim: int, vdim: int, rows, state: StateRows,
                     field: str) -> int:
     """Floats of workspace a chunk takes, or 0 where `chunk_scan.cu` does not fit: another
     recurrence, single tokens, few of them, other sizes, `rows` that no 16-byte piece can address."""
     if mode != SCAN_DELTA or ctx.is_decode or SCAN_CHUNK_TOKENS <= 0:
         return 0
-    tokens = _padded(T, 16) if T <= 128 else (T + 127) // 128 * 128
+    tokens = _padded_tokens(T)
     if tokens < CHUNK_SCAN_LEAST * _padded(ctx.n_seqs, 1):
         return 0
     if any(t.data_ptr() % 16 or t.stride(0) % 4 for t in rows) or state.stride % 4 or \

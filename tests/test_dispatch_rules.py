@@ -47,3 +47,21 @@ def test_rows_attention_on_tensor_maps_takes_heads_side_by_side_only():
                   dict(k=torch.zeros(T, 96, dtype=torch.bfloat16).as_strided((T, 3, 64), (96, 16, 1)))):
         args = dict(dict(k=k, shared=shared, v=v), **other)
         assert ops._tc_rows_blocks(ctx, q, out, args["k"], args["shared"], args["v"], 64, 32, 64, 0.0) == 0
+
+
+@pytest.mark.parametrize("lens,k64,k128", [
+    ([64], 1, 1), ([63], 0, 0), ([129, 1, 63], 4, 4), ([70] * 8, 8, 8), ([64] * 16, 16, 16),
+    ([64] * 64, 0, 64), ([64] + [8] * 31, 0, 0), ([64] + [16] * 15, 0, 16), ([200] + [5] * 7, 0, 9),
+    ([1000] + [5] * 15, 23, 23)])
+def test_rows_attention_on_tensor_maps_by_tokens_a_sequence(lens, k64, k128):
+    """The same for a plain step and for the padded one that replays it."""
+    from foundry_b200.engine.decode import bucket_of
+    from foundry_b200.engine.prompt import token_bucket
+    T = sum(lens)
+    for k1, want in ((64, k64), (128, k128)):
+        args = (k1, 32, 64, 0.0)
+        assert ops._tc_rows_blocks(rows_step(lens), *rows_of(T, k1=k1), *args) == want
+        t, n = token_bucket(T), bucket_of(len(lens))
+        replay = types.SimpleNamespace(n_seqs=n, cu_tokens_host=None, query_blocks_bound=(t + 63) // 64 + n,
+                                       long_queries=max(lens) >= 64)
+        assert (ops._tc_rows_blocks(replay, *rows_of(t, k1=k1), *args) > 0) == (want > 0)
