@@ -2962,8 +2962,10 @@ def state_scan(ctx, mode: int, q, k, v, g, state: StateRows, field: str, out: to
     if out.shape != (T, H * vdim) or out.dtype != torch.float32 or not out.is_contiguous():
         raise KernelError("state_scan: out must be contiguous float32 [T, heads * vdim]")
     f32 = torch.float32
-    unit = chunk_scan_unit(ctx, mode, T, H, dim, vdim, (q, k, out) if decay_per_head else
-                           (q, k, out, g), state, field)
+    unit = 0
+    if beta is not None and out_scale == 1.0:  # (else `fb_state_scan` refuses the delta rule)
+        unit = chunk_scan_unit(ctx, mode, T, H, dim, vdim, (q, k, out) if decay_per_head else
+                               (q, k, out, g), state, field)
     if unit:
         total = T // CHUNK_SCAN_TOKENS + ctx.n_seqs
         room = min(total, max(1, CHUNK_SCAN_ROOM // unit))

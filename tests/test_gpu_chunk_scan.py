@@ -100,3 +100,17 @@ def test_a_later_token_that_is_no_number_does_not_reach_earlier_ones(ops):
     out, want, _, _ = run(ops, [128], 2, 2, 64, 64, True, DECAYS["slow"], nan_at=70)
     assert bool(torch.isfinite(out[:70]).all()) and bool(torch.isnan(out[70:]).all())
     near(out[:70], want[:70])
+
+
+def test_what_the_delta_rule_does_not_take_is_refused(ops):
+    """A constant on the outputs, or no step sizes: the same for chunks as token by token."""
+    H, d, T = 2, 64, 128
+    x, g = torch.randn(T, H * d, device=DEV), torch.rand(T, H * d, device=DEV)
+    beta, out = torch.randn(T, H, device=DEV), torch.empty(T, H * d, device=DEV)
+    state = ops.StateRows(torch.zeros(1, H * d * d, device=DEV), [("S", H * d * d)])
+    ctx = types.SimpleNamespace(is_decode=False, n_seqs=1, max_q_len=T,
+                                slots=torch.zeros(1, dtype=torch.int32, device=DEV),
+                                cu_tokens=torch.tensor([0, T], dtype=torch.int32, device=DEV))
+    for more in (dict(beta=beta, out_scale=2.0), dict(beta=None)):
+        with pytest.raises(ops.KernelError, match="state_scan"):
+            ops.state_scan(ctx, ops.SCAN_DELTA, x, x, x, g, state, "S", out, H, 1, d, d, **more)
