@@ -2879,9 +2879,14 @@ def scan_chunks(ctx, mode: int, H: int, dim: int, vdim: int):
 # The delta rule over prompts whose heads have 64 or 128 key channels goes 32 tokens at a time as
 # small matrix products (csrc/chunk_scan.cu) where sequences bring about this many tokens and more
 # (one of 128 tokens, 32 heads of 64 x 64: 26 us against 47 token by token; eight of 60: 72 and 68).
+# With small heads the walk token by token fills the SMs once there are more than about 128 heads
+# over all sequences, and chunks only add work then: 16 sequences of 200 tokens, 32 heads of 64 x 64
+# 348 us in chunks against 301, of 64 x 32 264 against 180, of 64 x 16 225 against 99; with 64 x 128,
+# 128 x 64 and larger ones chunks stay ahead (1,072 us against 707 for 24 heads of 128 x 128).
 # Tokens and sequences count as a replayed step pads them, so that both forms of a step take the
 # same path. The workspace holds at most so many floats (256 MB); longer steps are worked in parts.
 CHUNK_SCAN_LEAST = 96
+CHUNK_SCAN_HEADS, CHUNK_SCAN_ANY = 128, 64 * 128  # heads of all sequences; sizes from which any number
 CHUNK_SCAN_TOKENS, CHUNK_SCAN_ROOM = 32, 1 << 26
 
 
@@ -2902,8 +2907,10 @@ def chunk_scan_unit(ctx, mode: int, T: int, H: int, dim: int, vdim: int, rows, s
     recurrence, single tokens, few of them, other sizes, `rows` that no 16-byte piece can address."""
     if mode != SCAN_DELTA or ctx.is_decode or SCAN_CHUNK_TOKENS <= 0:
         return 0
-    tokens = _padded_tokens(T)
-    if tokens < CHUNK_SCAN_LEAST * _padded(ctx.n_seqs, 1):
+    tokens, seqs = _padded_tokens(T), _padded(ctx.n_seqs, 1)
+    if tokens < CHUNK_SCAN_LEAST * seqs:
+        return 0
+    if seqs * H > CHUNK_SCAN_HEADS and dim * vdim < CHUNK_SCAN_ANY:
         return 0
     if any(t.data_ptr() % 16 or t.stride(0) % 4 for t in rows) or state.stride % 4 or \
             (state.rows.data_ptr() + 4 * state.offset[field]) % 16:

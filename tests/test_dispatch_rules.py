@@ -65,3 +65,19 @@ def test_rows_attention_on_tensor_maps_by_tokens_a_sequence(lens, k64, k128):
         replay = types.SimpleNamespace(n_seqs=n, cu_tokens_host=None, query_blocks_bound=(t + 63) // 64 + n,
                                        long_queries=max(lens) >= 64)
         assert (ops._tc_rows_blocks(replay, *rows_of(t, k1=k1), *args) > 0) == (want > 0)
+
+
+@pytest.mark.parametrize("H,dim,vdim,lens,chunks", [
+    (32, 64, 64, [128], True), (32, 64, 64, [95], True), (32, 64, 64, [64], False), (32, 64, 64, [200] * 4, True),
+    (32, 64, 64, [200] * 5, False), (4, 64, 64, [200] * 32, True), (4, 64, 64, [200] * 33, False),
+    (32, 64, 128, [200] * 16, True), (24, 128, 128, [100] * 16, True), (24, 128, 48, [100] * 16, False)])
+def test_delta_rule_in_chunks_by_tokens_and_heads(H, dim, vdim, lens, chunks, monkeypatch):
+    """The same for a plain step and for the padded one that replays it."""
+    from foundry_b200.engine.decode import bucket_of
+    from foundry_b200.engine.prompt import token_bucket
+    monkeypatch.setattr(ops, "_fn", lambda name: lambda h, d, e: 1)
+    for T, n in ((sum(lens), len(lens)), (token_bucket(sum(lens)), bucket_of(len(lens)))):
+        state = ops.StateRows(torch.zeros(1, 4), [("S", 4)])
+        ctx = types.SimpleNamespace(is_decode=False, n_seqs=n)
+        rows = [torch.zeros(1, 4)]
+        assert bool(ops.chunk_scan_unit(ctx, ops.SCAN_DELTA, T, H, dim, vdim, rows, state, "S")) == chunks
