@@ -2884,7 +2884,9 @@ def scan_chunks(ctx, mode: int, H: int, dim: int, vdim: int):
 # 348 us in chunks against 301, of 64 x 32 264 against 180, of 64 x 16 225 against 99; with 64 x 128,
 # 128 x 64 and larger ones chunks stay ahead (1,072 us against 707 for 24 heads of 128 x 128).
 # Tokens and sequences count as a replayed step pads them, so that both forms of a step take the
-# same path. The workspace holds at most so many floats (256 MB); longer steps are worked in parts.
+# same path. The workspace holds at most so many floats (256 MB; 1,500 tokens of 24 heads of 128 x 128
+# 355 us, with 128 MB 375, with 64 MB 405), fewer where memory is short; longer steps are worked in
+# parts.
 CHUNK_SCAN_LEAST = 96
 CHUNK_SCAN_HEADS, CHUNK_SCAN_ANY = 128, 64 * 128  # heads of all sequences; sizes from which any number
 CHUNK_SCAN_TOKENS, CHUNK_SCAN_ROOM = 32, 1 << 26
@@ -2899,6 +2901,19 @@ def _padded(n: int, least: int) -> int:
 def _padded_tokens(n: int) -> int:
     """Tokens as a replayed step pads them: rules that go by them choose alike for both forms."""
     return _padded(n, 16) if n <= 128 else (n + 127) // 128 * 128
+
+
+def _chunk_workspace(unit: int, total: int, device):
+    """(floats, chunks they hold) for a step of `total` chunks of `unit` floats: as many chunks as
+    memory has room for (the results do not depend on it), or None where there is none for one."""
+    room = min(total, max(1, CHUNK_SCAN_ROOM // unit))
+    while True:
+        try:
+            return torch.empty(room * unit, dtype=torch.float32, device=device), room
+        except torch.cuda.OutOfMemoryError:
+            if room == 1:
+                return None
+            room = (room + 1) // 2
 
 
 def chunk_scan_unit(ctx, mode: int, T: int, H: int, dim: int, vdim: int, rows, state: StateRows,
@@ -2973,10 +2988,10 @@ def state_scan(ctx, mode: int, q, k, v, g, state: StateRows, field: str, out: to
     if beta is not None and out_scale == 1.0:  # (else `fb_state_scan` refuses the delta rule)
         unit = chunk_scan_unit(ctx, mode, T, H, dim, vdim, (q, k, out) if decay_per_head else
                                (q, k, out, g), state, field)
-    if unit:
-        total = T // CHUNK_SCAN_TOKENS + ctx.n_seqs
-        room = min(total, max(1, CHUNK_SCAN_ROOM // unit))
-        ws = torch.empty(room * unit, dtype=f32, device=out.device)
+    total = T // CHUNK_SCAN_TOKENS + ctx.n_seqs
+    space = _chunk_workspace(unit, total, out.device) if unit else None
+    if space is not None:
+        ws, room = space
         _call("fb_chunk_scan", _dev(q, "q", f32, contiguous=False), _rows(q, "q"),
               _dev(k, "k", f32, contiguous=False), _rows(k, "k"),
               _dev(v, "v", f32, contiguous=False), _rows(v, "v"),

@@ -81,3 +81,20 @@ def test_delta_rule_in_chunks_by_tokens_and_heads(H, dim, vdim, lens, chunks, mo
         ctx = types.SimpleNamespace(is_decode=False, n_seqs=n)
         rows = [torch.zeros(1, 4)]
         assert bool(ops.chunk_scan_unit(ctx, ops.SCAN_DELTA, T, H, dim, vdim, rows, state, "S")) == chunks
+
+
+@pytest.mark.parametrize("free,room", [(10 ** 9, 5), (45, 3), (25, 2), (15, 1), (5, None)])
+def test_workspace_of_the_chunks_fits_the_memory_there_is(free, room, monkeypatch):
+    """Fewer chunks at a time where memory is short; token by token where there is none for one."""
+    asked = []
+
+    def empty(count, **kw):
+        asked.append(count)
+        if count > free:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return [0.0] * count
+
+    monkeypatch.setattr(ops.torch, "empty", empty)
+    got = ops._chunk_workspace(10, 5, "cuda")
+    assert got is None if room is None else (len(got[0]), got[1]) == (10 * room, room)
+    assert asked == sorted(asked, reverse=True)

@@ -95,6 +95,20 @@ def test_steps_in_parts(ops, room, monkeypatch):
     near(out, want)
     near(rows, states)
 
+def test_parts_do_not_change_the_numbers(ops, monkeypatch):
+    whole, _, moved, _ = run(ops, [200, 96, 130], 2, 1, 64, 32, True, DECAYS["any"])
+    monkeypatch.setattr(ops, "CHUNK_SCAN_ROOM", 3 * ops._fn("fb_chunk_scan_unit")(2, 64, 32))
+    out, _, rows, _ = run(ops, [200, 96, 130], 2, 1, 64, 32, True, DECAYS["any"])
+    assert torch.equal(out, whole) and torch.equal(rows, moved)
+
+
+def test_no_memory_for_the_chunks(ops, monkeypatch):
+    """Token by token, then."""
+    monkeypatch.setattr(ops, "_chunk_workspace", lambda *a: None)
+    out, want, rows, states = run(ops, [200, 96], 2, 1, 64, 32, True, DECAYS["any"])
+    near(out, want)
+    near(rows, states)
+
 
 def test_a_later_token_that_is_no_number_does_not_reach_earlier_ones(ops):
     out, want, _, _ = run(ops, [128], 2, 2, 64, 64, True, DECAYS["slow"], nan_at=70)
