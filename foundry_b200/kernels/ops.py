@@ -2944,8 +2944,9 @@ def low_rank(x: torch.Tensor, weight: torch.Tensor, act: str = "identity",
     n = weight.shape[0]
     if rank % 8 or rank > 512 or weight.data_ptr() % 16 or not weight.is_contiguous():
         return None
-    if weight.shape[1] != rank or (bias is not None and bias.numel() != n):
-        raise KernelError(f"low_rank: {tuple(x.shape)} x {tuple(weight.shape)}")
+    if weight.shape[1] != rank or (bias is not None and bias.numel() != n) or \
+            (A is not None and (bias is None or per_head <= 0 or A.numel() * per_head < n)):
+        raise KernelError(f"low_rank: {tuple(x.shape)} x {tuple(weight.shape)} and its decays")
     out = torch.empty((T, n), dtype=torch.float32, device=x.device)
     _call("fb_low_rank", _dev(x, "x", torch.float32, contiguous=False), _rows(x, "x"),
           {"identity": 0, "tanh": 1}[act], _dev(weight, "weight"), code_of(weight.dtype), rank,

@@ -98,3 +98,11 @@ def test_workspace_of_the_chunks_fits_the_memory_there_is(free, room, monkeypatc
     got = ops._chunk_workspace(10, 5, "cuda")
     assert got is None if room is None else (len(got[0]), got[1]) == (10 * room, room)
     assert asked == sorted(asked, reverse=True)
+
+
+@pytest.mark.parametrize("more", [dict(A=torch.zeros(3), per_head=4), dict(A=torch.zeros(16), per_head=0),
+                                  dict(bias=torch.zeros(15)), dict(A=torch.zeros(16), bias=None)])
+def test_decays_that_do_not_cover_the_channels_are_refused(more):
+    args = dict(dict(bias=torch.zeros(16)), **more)
+    with pytest.raises(ops.KernelError, match="low_rank"):
+        ops.low_rank(torch.zeros(5, 8), torch.zeros(16, 8), **args)

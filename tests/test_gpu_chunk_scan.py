@@ -95,6 +95,7 @@ def test_steps_in_parts(ops, room, monkeypatch):
     near(out, want)
     near(rows, states)
 
+
 def test_parts_do_not_change_the_numbers(ops, monkeypatch):
     whole, _, moved, _ = run(ops, [200, 96, 130], 2, 1, 64, 32, True, DECAYS["any"])
     monkeypatch.setattr(ops, "CHUNK_SCAN_ROOM", 3 * ops._fn("fb_chunk_scan_unit")(2, 64, 32))
