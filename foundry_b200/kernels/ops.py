@@ -2933,6 +2933,20 @@ def chunk_scan_unit(ctx, mode: int, T: int, H: int, dim: int, vdim: int, rows, s
     return _fn("fb_chunk_scan_unit")(H, dim, vdim)
 
 
+def low_rank_pays(T: int, dtype: torch.dtype, *ranks: int) -> bool:
+    """Whether `low_rank` beats cast, product and decay as launches of their own. The product takes
+    the tensor cores from ranks of 64 on, and the one kernel, an FMA a token, rank and channel, lost
+    at every size there (rank 64 -> 2,048 channels in graph replays, with a decay: 8 tokens 6.3 us
+    against 4.5, 300 12.7 against 11.1; without one 5.2 against 2.9, 1,500 tokens 23 against 12;
+    rank 512 -> 4,096: 8 tokens 55 against 11, 1,500 346 against 66). Below, in bfloat16 it is ahead
+    throughout (rank 32: 4.3 against 5.7, 1,500 tokens 17 against 32), in float32 up to rank 40 and
+    128 tokens, up to rank 24 at any number (rank 32, 1,500 tokens without a decay 17 against 13).
+    Tokens count as a replayed step pads them."""
+    if dtype == torch.bfloat16:
+        return max(ranks) < 64
+    return max(ranks) <= 24 or (max(ranks) <= 40 and _padded_tokens(T) <= 128)
+
+
 def low_rank(x: torch.Tensor, weight: torch.Tensor, act: str = "identity",
              bias: Optional[torch.Tensor] = None, A: Optional[torch.Tensor] = None,
              per_head: int = 1) -> Optional[torch.Tensor]:

@@ -122,8 +122,10 @@ class GatedDeltaChannel(Part):
                                   n_scaled=G, extra=d ** -0.5, unit_eps=self.unit_eps):
             ops.state_tail_update(ctx, p, state, "tail", self.taps - 1, C)
         at = C + H + self.decay_rank
-        decay = ops.low_rank(p[:, C + H:at], self.a2, bias=self.dt_bias, A=self.A_log, per_head=d)
-        gate = ops.low_rank(p[:, at:at + self.gate_rank], self.g2)
+        decay = gate = None
+        if ops.low_rank_pays(T, x.dtype, self.decay_rank, self.gate_rank):
+            decay = ops.low_rank(p[:, C + H:at], self.a2, bias=self.dt_bias, A=self.A_log, per_head=d)
+            gate = ops.low_rank(p[:, at:at + self.gate_rank], self.g2)
         if decay is None or gate is None:
             low = torch.empty((T, self.decay_rank + self.gate_rank), dtype=x.dtype, device=x.device)
             ops.unary_cast(p[:, C + H:], low)
@@ -330,7 +332,9 @@ class WkvTimeMix(Part):
             ops.state_tail_update(ctx, x, state, "prev", 1, W)
         r, k, v, g, raw = products_f32([(mixes[i], w) for i, w in enumerate(
             (self.r, self.k, self.v, self.g, self.w1))])
-        decay = ops.low_rank(raw, self.w2, "tanh", bias=self.w0)
+        decay = None
+        if ops.low_rank_pays(T, x.dtype, self.decay_rank):
+            decay = ops.low_rank(raw, self.w2, "tanh", bias=self.w0)
         if decay is None:
             low = torch.empty((T, self.decay_rank), dtype=x.dtype, device=x.device)
             ops.unary_cast(raw, low, "tanh")

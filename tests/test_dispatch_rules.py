@@ -106,3 +106,14 @@ def test_decays_that_do_not_cover_the_channels_are_refused(more):
     args = dict(dict(bias=torch.zeros(16)), **more)
     with pytest.raises(ops.KernelError, match="low_rank"):
         ops.low_rank(torch.zeros(5, 8), torch.zeros(16, 8), **args)
+
+
+def test_low_rank_kernel_by_rank_tokens_and_type():
+    """The same for a plain step and for the padded one that replays it."""
+    from foundry_b200.engine.prompt import token_bucket
+    for dtype, ranks, most in ((torch.bfloat16, (32, 48), 5000), (torch.bfloat16, (64,), 0),
+                               (torch.bfloat16, (8, 512), 0), (torch.float32, (24, 8), 5000),
+                               (torch.float32, (40,), 128), (torch.float32, (48,), 0)):
+        for T in (1, 8, 100, 128, 129, 5000):
+            assert ops.low_rank_pays(T, dtype, *ranks) == (T <= most)
+            assert ops.low_rank_pays(token_bucket(T), dtype, *ranks) == (T <= most)
