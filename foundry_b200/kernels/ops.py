@@ -3303,6 +3303,21 @@ def moe_grouped_tc_fits(x: torch.Tensor, *sizes: int) -> bool:
             and all(n % 32 == 0 for n in sizes))
 
 
+def grouped_form(pairs: int, experts: int, K: int, gated: bool) -> int:
+    """The form of `gemm_tc_grouped`: Pairs of SMs, gated from 128 rows an expert on average: 16
+    experts of 2,048 over 3,072, 125 rows each 163 us for 163 (gated and plain product, even
+    counts), 250 190 for 191, 500 261 for 311; 64 experts of 1,024, 125 rows 210 for 222. A
+    router's counts are less even, which these tiles mind less: the whole feed-forward of 2,000
+    tokens of 3,072 (250 rows an expert on average) 258 us for 280. The plain product has fewer
+    units, and more so of long K, where a few full experts leave most pairs idle in the last
+    round: with one expert of half the rows, 200 an expert, 65 us for 63 at 2,048 -> 3,072, 96
+    for 69 at 8,192 -> 2,048 (500 random rows 142 for 128; 700 and 1,000 155 for 178, 211 for
+    245); 160 an expert, 64 experts, 1,024 -> 2,048 100 for 82, 200 105 for 98, 250 evenly 97
+    for 109."""
+    least = 128 if gated else 200 if K <= 4096 else 600
+    return 0 if not MOE_GROUPED_TC_PERSISTENT else 2 if pairs >= least * experts else 1
+
+
 def gemm_tc_grouped(rows: torch.Tensor, w: torch.Tensor, order: "ExpertOrder",
                     out_dtype: torch.dtype = torch.float32, glu: Optional[tuple] = None,
                     persistent: Optional[int] = None) -> torch.Tensor:
@@ -3331,12 +3346,7 @@ def gemm_tc_grouped(rows: torch.Tensor, w: torch.Tensor, order: "ExpertOrder",
     limit, alpha, shift = glu if glu is not None else (0.0, 0.0, 0.0)
     form = persistent
     if form is None:
-        # pairs of SMs from 128 rows an expert on average. Gated + plain product of 16 experts of
-        # 2,048 over 3,072, even counts, against one CTA an SM: 16 rows each 154 us for 143, 125
-        # 163 for 163, 250 190 for 191, 500 261 for 311; 64 experts of 1,024, 125 rows 210 for 222.
-        # A router's counts are less even, which these tiles mind less: the whole feed-forward of
-        # 2,000 tokens of 3,072 (250 rows an expert on average) 258 us for 280.
-        form = 0 if not MOE_GROUPED_TC_PERSISTENT else 2 if pairs >= 128 * E else 1
+        form = grouped_form(pairs, E, K, glu is not None)
     _call("fb_gemm_tc_grouped", _dev(rows, "rows", contiguous=False), _rows(rows, "rows"), pairs,
           _dev(w, "w"), K, N, K, order.starts.data_ptr(), E, pairs // 128 + E, _dev(out, "out"),
           width, 1 if out_dtype == torch.float32 else 0, 0 if glu is None else 1, float(limit),

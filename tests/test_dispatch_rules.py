@@ -117,3 +117,10 @@ def test_low_rank_kernel_by_rank_tokens_and_type():
         for T in (1, 8, 100, 128, 129, 5000):
             assert ops.low_rank_pays(T, dtype, *ranks) == (T <= most)
             assert ops.low_rank_pays(token_bucket(T), dtype, *ranks) == (T <= most)
+
+
+@pytest.mark.parametrize("rows,K,gated,form", [
+    (127, 3072, True, 1), (128, 3072, True, 2), (128, 14336, True, 2), (199, 2048, False, 1),
+    (200, 2048, False, 2), (500, 8192, False, 1), (600, 8192, False, 2)])
+def test_form_of_the_experts_products_by_rows_an_expert(rows, K, gated, form):
+    assert ops.grouped_form(16 * rows, 16, K, gated) == form
