@@ -179,12 +179,13 @@ __device__ __forceinline__ __nv_bfloat16 fb_from_float<__nv_bfloat16>(float v) {
   return __float2bfloat16_rn(v);
 }
 
-// n / d for d >= 1, without the branch that the division operator takes for scaled operands: the
-// hardware's reciprocal, one Newton step, and the quotient corrected by its own remainder
-// (Markstein's method), within an ulp; what no correction fits (infinities, NaN) keeps the plain
-// product. The branch kept the epilogues of the gated products from overlapping one element's
-// latency with the next one's: 2,048 rows of 2,048 -> 2 x 8,192 102.2 -> 100.4 us (300 rows: 52 ->
-// 44), 16 experts of 250 rows of 3,072 -> 2 x 2,048 142 -> 115 us (1,000 rows each: 462 -> 375).
+// n / d for d >= 1 without a branch: the hardware's reciprocal, one Newton step, and the quotient
+// corrected by its own remainder (Markstein's method), which leaves the rounding of the exact
+// quotient but for 2^-19 of its last place; a zero keeps n's sign, and what no correction fits
+// (infinities, NaN) keeps the plain product. Without a branch the epilogues of the gated products
+// overlap one element's latency with the next one's: 2,048 rows of 2,048 -> 2 x 8,192 102.2 ->
+// 100.4 us (300 rows: 52 -> 44), 16 experts of 250 rows of 3,072 -> 2 x 2,048 142 -> 115 us (1,000
+// rows each: 462 -> 375).
 __device__ __forceinline__ float fb_quotient(float n, float d) {
   float r;
   asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
@@ -192,7 +193,7 @@ __device__ __forceinline__ float fb_quotient(float n, float d) {
   r = fmaf(r, fmaf(-d, r, 1.0f), r);
   float q = n * r;
   q = fmaf(r, fmaf(-d, q, n), q);
-  return q == q ? q : plain;
+  return fabsf(q) > 0.0f ? q : plain;
 }
 
 // The activation of a gated feed-forward on its gate: 0 SiLU, g / (1 + exp(-g));

@@ -498,6 +498,27 @@ FB_API int fb_add_into(float* a, const float* b, long long n, cudaStream_t strea
   return fb_check_launch("add_into");
 }
 
+// ------------------------------------------------------------------- quotients
+// out = n / d for d >= 1 as the gated products' epilogues divide (fb_quotient), by itself.
+namespace {
+__global__ void quotient_kernel(const float* n, const float* d, float* __restrict__ out, long long count) {
+  fb_pdl_wait();
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count;
+       i += (long long)gridDim.x * blockDim.x)
+    out[i] = fb_quotient(__ldcg(n + i), __ldcg(d + i));
+}
+}  // namespace
+
+FB_API int fb_quotients(const float* n, const float* d, float* out, long long count,
+                        cudaStream_t stream) {
+  FB_REQUIRE(count >= 0, "quotients: bad size %lld", count);
+  if (count == 0) return 0;
+  const long long want = (count + 255) / 256;
+  const int blocks = (int)(want < 148 * 8 ? want : 148 * 8);
+  fb_launch(quotient_kernel, dim3(blocks), dim3(256), 0, stream, n, d, out, count);
+  return fb_check_launch("quotients");
+}
+
 // ------------------------------------------------------------- cap on values
 // x <- cap * tanh(x / cap), in place, 32-bit (a soft cap on the logits).
 namespace {

@@ -204,6 +204,7 @@ _SIGNATURES = {
                           c_ll, c_float, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "fb_unary_cast": [c_void_p, c_ll, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "fb_add_into": [c_void_p, c_void_p, c_ll, c_void_p],
+    "fb_quotients": [c_void_p, c_void_p, c_void_p, c_ll, c_void_p],
     "fb_sigmoid_gate": [c_void_p, c_int, c_ll, c_void_p, c_ll, c_int, c_int, c_void_p],
     "fb_moe_router": [c_void_p, c_ll, c_void_p, c_ll, c_int, c_void_p, c_void_p, c_int, c_int,
                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float,
@@ -1352,6 +1353,16 @@ def add_into(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     _call("fb_add_into", _dev(a, "a", torch.float32), _dev(b, "b", torch.float32), a.numel(),
           _stream())
     return a
+
+
+def quotients(n: torch.Tensor, d: torch.Tensor) -> torch.Tensor:
+    """n / d for d >= 1 as the gated products' epilogues divide, float32 of one shape."""
+    if n.shape != d.shape:
+        raise KernelError(f"quotients: {tuple(n.shape)} / {tuple(d.shape)}")
+    out = torch.empty_like(n)
+    _call("fb_quotients", _dev(n, "n", torch.float32), _dev(d, "d", torch.float32), out.data_ptr(),
+          n.numel(), _stream())
+    return out
 
 
 def _tc_usable(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
