@@ -28,9 +28,9 @@ def plain(q, k, v, g, beta, S):
     return torch.stack(out), S
 
 
-def run(ops, lens, H, G, d, e, channels, decay, seed=0, nan_at=None):
+def run(ops, lens, H, G, d, e, channels, decay, seed=0, nan_at=None, padding=0):
     gen = torch.Generator().manual_seed(seed)
-    T, n = sum(lens), len(lens)
+    T, n = sum(lens) + padding, len(lens)
     wide = torch.randn(T, 2 * G * d + H * e, generator=gen).to(DEV)  # q | k | v of one product
     for a in (0, G * d):
         part = wide[:, a:a + G * d].view(T, G, d)
@@ -59,11 +59,14 @@ def run(ops, lens, H, G, d, e, channels, decay, seed=0, nan_at=None):
     values = wide[:, 2 * G * d:].double().view(T, H, e)
     want, states = [], before[:, 4:].double().view(n + 3, H, d, e).clone()
     for s, a, b in zip(slots.tolist(), cu, cu[1:]):
+        if a == b:
+            continue
         part, states[s] = plain(heads[0][a:b], heads[1][a:b], values[a:b],
                                 g[a:b].double().view(b - a, H, -1), beta[a:b].double(), states[s])
         want.append(part)
     assert torch.equal(rows[:, :4], before[:, :4])
-    return out.double().view(T, H, e), torch.cat(want), rows[:, 4:].double().view_as(states), states
+    assert bool((out[cu[-1]:] == 9.0).all())  # padding rows stay as they were
+    return out[:cu[-1]].double().view(-1, H, e), torch.cat(want), rows[:, 4:].double().view_as(states), states
 
 
 def near(a, b):
@@ -129,3 +132,23 @@ def test_what_the_delta_rule_does_not_take_is_refused(ops):
     for more in (dict(beta=beta, out_scale=2.0), dict(beta=None)):
         with pytest.raises(ops.KernelError, match="state_scan"):
             ops.state_scan(ctx, ops.SCAN_DELTA, x, x, x, g, state, "S", out, H, 1, d, d, **more)
+
+
+def test_many_sequences_in_parts(ops, monkeypatch):
+    """More than a warp's lanes of sequences: the search for a chunk's sequence and the count of the
+    chunks in front of one go on for a second round."""
+    gen = torch.Generator().manual_seed(4)
+    lens = torch.randint(100, 220, (40,), generator=gen).tolist()
+    monkeypatch.setattr(ops, "CHUNK_SCAN_ROOM", 37 * ops._fn("fb_chunk_scan_unit")(2, 64, 16))
+    out, want, rows, states = run(ops, lens, 2, 1, 64, 16, True, DECAYS["any"])
+    near(out, want)
+    near(rows, states)
+
+
+@pytest.mark.parametrize("lens,padding", [([300, 0, 161, 0], 51), ([0, 0, 400], 1), ([129] + [0] * 3, 255),
+                                          ([0] * 33 + [6200] + [0] * 5, 120)])
+def test_empty_sequences_and_padding_tokens(ops, lens, padding):
+    """A replayed step's form: sequences without tokens, and tokens behind the last sequence."""
+    out, want, rows, states = run(ops, lens, 2, 1, 64, 32, False, DECAYS["slow"], padding=padding)
+    near(out, want)
+    near(rows, states)

@@ -38,6 +38,21 @@ def test_product_of_16_byte_rows(ops, M, N, K):
     assert bool((wide[:, N:] == 7.0).all()) and bool((wide[M] == 7.0).all())  # nothing beyond
 
 
+@pytest.mark.parametrize("M", [1, 8, 16, 32, 33, 64, 129])
+@pytest.mark.parametrize("K", [1028, 4096, 4100])
+def test_no_term_of_a_long_sum_is_lost(ops, M, K):
+    """Products of independent signs: a sum of i of them is about sqrt(i) of their root mean square,
+    |x||w| / K, and each addition rounds it by up to 2^-24, errors of independent signs again: 0.41 *
+    2^-24 * |x||w| in the root mean square where they are added one by one. Seven times that is far
+    below one product."""
+    x, w = rnd(M, K), rnd(70, K, seed=1)
+    out = torch.empty(M, 70, device=DEV)
+    ops.gemm_simt(x, w, out)
+    want = x.double() @ w.double().T
+    norms = x.double().norm(dim=1)[:, None] * w.double().norm(dim=1)
+    assert float(((out.double() - want).abs() / norms).max()) < 3 * 2.0 ** -24
+
+
 @pytest.mark.parametrize("M,N,K", [(3000, 4700, 64), (700, 70, 20)])
 def test_product_of_large_tiles_and_views(ops, M, N, K):
     x, w = rnd(M, K + 8)[:, 4:K + 4], rnd(N, K + 12, seed=2)[:, 8:K + 8]  # strides, 16-byte bases
