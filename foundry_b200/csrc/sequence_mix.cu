@@ -869,8 +869,7 @@ void launch_linear_chunks(const ScanArgs& a, bool wkv, int n_seqs, cudaStream_t 
     if (a.g_scalar) fb_launch_serial(linear_chunk_kernel<1, RG, true>, grid, block, 0, stream, a);
     else fb_launch_serial(linear_chunk_kernel<1, RG, false>, grid, block, 0, stream, a);
   } else if (wkv) {
-    if (a.g_scalar) fb_launch(linear_chunk_kernel<2, RG, true, true>, grid, block, 0, stream, a);
-    else fb_launch(linear_chunk_kernel<2, RG, false, true>, grid, block, 0, stream, a);
+    fb_launch(linear_chunk_kernel<2, RG, false, true>, grid, block, 0, stream, a);
   } else {
     if (a.g_scalar) fb_launch(linear_chunk_kernel<2, RG, true>, grid, block, 0, stream, a);
     else fb_launch(linear_chunk_kernel<2, RG, false>, grid, block, 0, stream, a);
@@ -1356,8 +1355,9 @@ FB_API int fb_state_scan(int mode, const float* q, long long q_ld, const float* 
   ScanArgs a{q, q_ld, k, k_ld, v, v_ld, g, g_ld, beta, beta_ld, bonus, state, state_stride,
              s_offset, out, cu_tokens, slots, H, rep, dim, vdim, g_scalar ? 1 : 0, out_scale,
              n_chunks, chunk, ws, wg};
-  // (mode 1 reads no step sizes)
-  if (mode != 0 && n_chunks > 1 && linear_chunks_fit(a) && (mode == 2 || beta == nullptr)) {
+  // (mode 1 reads no step sizes; one decay a head, which no mixer gives it, is the scan's)
+  if (mode != 0 && n_chunks > 1 && linear_chunks_fit(a) &&
+      (mode == 2 || (beta == nullptr && !g_scalar))) {
     launch_linear_pass<1>(a, mode == 1, n_seqs, stream);
     fb_launch(scan_chunk_starts_kernel<4>, dim3(n_seqs, H, (dim * vdim / 4 + 127) / 128), dim3(128), 0,
               stream, a);

@@ -152,3 +152,34 @@ def test_empty_sequences_and_padding_tokens(ops, lens, padding):
     out, want, rows, states = run(ops, lens, 2, 1, 64, 32, False, DECAYS["slow"], padding=padding)
     near(out, want)
     near(rows, states)
+
+
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("H,d,e", [(2, 64, 64), (3, 128, 40), (4, 16, 24), (1, 256, 20)])
+def test_wkv_over_prompts(ops, H, d, e, per_head):
+    """The recurrence with a bonus, its tokens in chunks where the decay is a channel's, token by
+    token where it is a head's: o = q . (S + bonus k v), S <- g S + k v."""
+    gen = torch.Generator().manual_seed(d + e)
+    lens = [300, 7, 129]
+    T, n = sum(lens), len(lens)
+    q, k, v = (torch.randn(T, H * x, generator=gen).to(DEV) for x in (d, d, e))
+    g = torch.exp(-torch.exp(torch.randn(T, H if per_head else H * d, generator=gen) - 3)).to(DEV)
+    bonus = torch.randn(H, d, generator=gen).to(DEV)
+    rows = (0.3 * torch.randn(n, H * d * e, generator=gen)).to(DEV)
+    states = rows.double().view(n, H, d, e).clone()
+    cu = [0, 300, 307, 436]
+    ctx = types.SimpleNamespace(is_decode=False, n_seqs=n, max_q_len=300,
+                                slots=torch.arange(n, dtype=torch.int32, device=DEV),
+                                cu_tokens=torch.tensor(cu, dtype=torch.int32, device=DEV))
+    out = torch.empty(T, H * e, device=DEV)
+    ops.state_scan(ctx, ops.SCAN_WKV, q, k, v, g, ops.StateRows(rows, [("S", H * d * e)]), "S", out, H, 1, d,
+                   e, bonus=bonus, decay_per_head=per_head)
+    want = []
+    for s, a, b in zip(range(n), cu, cu[1:]):
+        for t in range(a, b):
+            kv = k[t].double().view(H, d, 1) * v[t].double().view(H, 1, e)
+            want.append(torch.einsum("hd,hde->he", q[t].double().view(H, d),
+                                     states[s] + bonus.double()[:, :, None] * kv).flatten())
+            states[s] = states[s] * g[t].double().view(H, -1, 1) + kv
+    near(out.double(), torch.stack(want))
+    near(rows.double().view_as(states), states)
