@@ -475,7 +475,7 @@ int launch_d(const FbAttentionF32& p, cudaStream_t stream) {
     // also be single ones, padded)
     const bool several = tokens > 16 && tokens > seqs;
     int S = 1;
-    while (S < 8 && pairs * S < 2 * 148 && S * 2 * 2 <= width && !(several && width <= 8)) S *= 2;
+    while (S < 8 && pairs * S < 2 * sm_count() && S * 2 * 2 <= width && !(several && width <= 8)) S *= 2;
     // With few keys, 16 lane groups of four warps have more to merge than to add, and the pairs
     // fill the SMs without them. 100 x 8 tokens, 32 heads over 8 of 64: 25 us with one warp a pair,
     // 60 with four (attention_simt.cu 35); 4 x 8 tokens: 6.1 with two, 11.3 with four in two ranges

@@ -36,6 +36,18 @@ inline bool fb_first_use_on_device(bool (&seen)[64]) {
   return true;
 }
 
+// SMs of the device (of one kind where there are several).
+inline int sm_count() {
+  static int count = 0;
+  if (count == 0) {
+    int device = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
+    if (count <= 0) count = 148;
+  }
+  return count;
+}
+
 #define FB_REQUIRE(cond, ...)                      \
   do {                                             \
     if (!(cond)) return fb_fail(1, __VA_ARGS__);   \

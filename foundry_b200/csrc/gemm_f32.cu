@@ -420,7 +420,7 @@ int fb_gemm_f32_launch(const FbGemmF32& p, cudaStream_t stream) {
   // and 827; 128 rows, 2048 -> 64: 14 against 230 and 125). Rows count in whole 128s: a step that
   // is padded to a bucket sums as the plain one does.
   const long long big = (long long)((p.M + 127) / 128) * ((p.N + 127) / 128) * p.count;
-  if (big >= 3 * 2 * 148) return launch_tile<128, 128, 8, 1, 2>(p, stream);
+  if (big >= 3 * 2 * sm_count()) return launch_tile<128, 128, 8, 1, 2>(p, stream);
   if (p.K >= 1024) return launch_tile<64, 64, 4, 8, 4>(p, stream);
   if (p.K >= 512) return launch_tile<64, 64, 4, 4, 4>(p, stream);
   if (p.K >= 256) return launch_tile<64, 64, 4, 2, 4>(p, stream);

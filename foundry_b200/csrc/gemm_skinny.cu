@@ -522,17 +522,6 @@ gemm_skinny_kernel(const __nv_bfloat16* x, long long ldx,
   }
 }
 
-int sm_count() {
-  static int count = 0;
-  if (count == 0) {
-    int device = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
-    if (count <= 0) count = 148;
-  }
-  return count;
-}
-
 int launch_skinny(const void* x, long long ldx, const void* w, long long ldw, void* out,
                   long long ldo, int out_f32, int T, int N, int K, int epilogue, const void* next,
                   long long next_bytes, int ksplit, long long plane_stride, int warps,

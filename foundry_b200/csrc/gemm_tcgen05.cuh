@@ -445,15 +445,4 @@ int make_map(CUtensorMap* map, const void* ptr, long long rows, long long cols, 
   return 0;
 }
 
-int sm_count() {
-  static int count = 0;
-  if (count == 0) {
-    int device = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
-    if (count <= 0) count = 148;
-  }
-  return count;
-}
-
 }  // namespace
