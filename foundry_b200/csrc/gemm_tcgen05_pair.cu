@@ -55,6 +55,18 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Tensor memory of both CTAs of a pair: one warp of each calls them, whole; all tcgen05
+// instructions of a kernel have one cta_group.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
+               "r"(columns)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t base, uint32_t columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns)
+               : "memory");
+}
 // A tile load whose completion is counted on a barrier of the CTA pair (its
 // address in the cluster window), not necessarily this CTA's own.
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map,
@@ -174,16 +186,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
-                 "r"((uint32_t)TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  __syncthreads();
+  cluster_barrier();  // the peer is there, and its barriers exist before anything arrives on them
+  if (warp == 1) tmem_alloc_pair(tmem_slot, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
-  cluster_barrier();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -389,9 +396,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   cluster_barrier();  // nothing of the peer's may still be on its way to this CTA
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"((uint32_t)TMEM_COLS)
-                 : "memory");
+    tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
 }
 
@@ -557,13 +562,9 @@ gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
-                 "r"(512u)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  __syncthreads();
+  cluster_barrier();  // the peer is there, and its barriers exist before anything arrives on them
+  if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
   fb_pdl_wait();  // `starts` is the work of an earlier kernel
   for (int g = threadIdx.x; g <= groups; g += blockDim.x) s_starts[g] = __ldcg(starts + g);
   __syncthreads();
@@ -584,7 +585,6 @@ gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w,
   }
   tc_fence_before();
   __syncthreads();
-  cluster_barrier();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const int tiles_w = rows_w / (2 * BM);
@@ -725,8 +725,7 @@ gemm_tc_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w,
   cluster_barrier();  // nothing of the peer's may still be on its way to this CTA
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u)
-                 : "memory");
+    tmem_dealloc_pair(tmem_base, 512);
   }
 }
 
