@@ -15,13 +15,15 @@
 // 16 columns of a head's state a block, with the two products that the next chunk waits for, and
 // leaves u and every chunk's S0; `output_kernel` makes all outputs from them side by side. The
 // token-by-token scan has 32 dependent steps of two dot products each where a walk has one chunk:
-// 0.35 us a step whatever its size (latency: two warps a scheduler in one chain).
+// 0.35 us a step with heads of 64 x 64, 0.59 with 128 x 128 (latency: a few warps a scheduler in
+// one chain). A step's heads that fill the SMs that way need no chunks (`ops.chunk_scan_unit`).
 // All of it is 32-bit arithmetic on the FMA pipe, reordered.
 //
 // Measured: 2,048 tokens, 32 heads of 64 x 64: 199 us (89, 82 and 35), token by token 709. 1,500
 // tokens, 24 heads of 128 x 128: 355 us (93, 210 and 57) against 892. Outputs made in the walk
-// itself, from the same registers: 217 and 378 us. Error against 64 bits: 1.1e-7, token by token
-// 1.2e-7.
+// itself, from the same registers: 217 and 378 us. Error against 64 bits with a decay a channel:
+// outputs 1.29e-7 and 1.37e-7, token by token 1.39e-7 and 1.40e-7; states 1.09e-7 and 1.00e-7 for
+// 1.02e-7 and 0.99e-7 (a chunk's own sum, added to the decayed state last, left that as it was).
 #include "common.cuh"
 
 namespace {
