@@ -113,6 +113,18 @@ def test_low_rank(ops, T, rank, n, dtype):
     assert ops.low_rank(x[:, :rank - 1], w[:, :rank - 1].contiguous()) is None
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,rank,n", [(300, 512, 130), (700, 48, 200), (1025, 8, 64)])
+def test_low_rank_at_its_limits(ops, T, rank, n, dtype):
+    gen = torch.Generator().manual_seed(rank)
+    x = torch.randn(T, rank, generator=gen).to(DEV)
+    w = (torch.randn(n, rank, generator=gen) / rank ** 0.5).to(dtype).to(DEV)
+    want = x.to(dtype).double() @ w.double().T
+    # 2^-24 * 0.41 * |x||w| in the root mean square for terms added one by one (|w| near one)
+    assert float(((ops.low_rank(x, w).double() - want).abs() / x.double().norm(dim=1)[:, None]).max()) \
+        < 3 * 2.0 ** -24 * float(w.double().norm(dim=1).max())
+
+
 @pytest.mark.parametrize("T", [1, 8, 9, 16])
 def test_several_products_in_one_launch(ops, T):
     gen = torch.Generator().manual_seed(T)
