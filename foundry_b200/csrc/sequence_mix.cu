@@ -1068,7 +1068,9 @@ __global__ void low_rank_decay_kernel(const float* low, long long ld, const T* _
 // exp(-exp(A[head]) softplus(z + bias[c])), 2 a decay exp(-exp(z + bias[c])). Three launches as
 // cast, product, decay. A block takes up to TOKENS rows, staged in shared memory; a thread a
 // channel, whose weights it reads once for all of them. Bound by issue (an FMA a token and rank,
-// a 16-byte shared-memory read for four of them) from some hundred tokens on, by its launch below.
+// a 16-byte shared-memory read for four of them) from some hundred tokens on, by its launch and the
+// chain of its weights' loads below: for ranks under those that the tensor cores take (32 -> 2,048,
+// 8 tokens 4.3 us against 5.7 in three launches; 64: 6.3 against 4.5, see ops.low_rank_pays).
 constexpr int LOW_RANK = 8;  // weights a thread holds at a time
 template <typename T, int TOKENS, int ACT, int LAST>
 __global__ void __launch_bounds__(128)
