@@ -1,5 +1,5 @@
-// out[M,N] = x[M,K] * w[N,K]^T in 32 bits on the CUDA cores (IEEE FFMA; no tensor cores, no TF32)
-// for operands that 16-byte loads can address:
+// out[M,N] = x[M,K] * w[N,K]^T in 32 bits on the CUDA cores (IEEE FFMA), for operands that 16-byte
+// loads can address; large products of more than 32 rows are gemm_f32_tcgen05.cu's.
 //
 // few rows (single-token steps): the weights stream once, and that stream is the bound.
 //   `rows_kernel`: 8 rows of 2048 -> 16384 in 31 us (134 MB, 4.3 TB/s), one row in 22 us
@@ -413,12 +413,21 @@ int fb_gemm_f32_launch(const FbGemmF32& p, cudaStream_t stream) {
     if (p.M <= 8 || p.N <= 8192) return launch_rows_by_shape<8>(p, stream);
     return launch_rows_by_shape<16>(p, stream);
   }
+  // The tensor cores (gemm_f32_tcgen05.cu) from 33 rows on, where there is enough to do: their kernel
+  // starts 4 us later (tensor memory, a pair of SMs, the first split). 64 rows of 2048 -> 128 20.5 us
+  // against 24.6 with tiles, -> 2048 22.6 against 32.8; 1000 rows of 256 -> 2048 20.5 against 45; but
+  // 512 rows of 512 -> 512 22.5 against 18.4, 1000 rows of 64 -> 1024 16.4 against 12.3, 300 rows of
+  // 2048 -> 64 both 24.6. Rows count in whole 128s: a step that is padded to a bucket sums as the
+  // plain one does.
+  const long long rows = (p.M + 127) / 128 * 128;
+  if (p.count == 1 && p.ldx >= p.K && p.ldw >= p.K && p.N >= 128 &&
+      (p.K >= 1024 || rows * p.N * p.K >= 1LL << 28))
+    return fb_gemm_f32_tc_launch(p, stream);
   // 128 x 128 tiles move the least through shared memory (46 TFLOP/s at 2048 x 2048 -> 16384
   // against 37 with 64 x 64 and 24 before) and need three full rounds of two blocks an SM to hide
   // their last one; below that 64 x 64 tiles with K shared eightfold (777 rows, 2048 -> 3072:
   // 305 us against 412 with 128 x 128 and 491 before; 300 rows, 8192 -> 2048: 357 against 1068
-  // and 827; 128 rows, 2048 -> 64: 14 against 230 and 125). Rows count in whole 128s: a step that
-  // is padded to a bucket sums as the plain one does.
+  // and 827; 128 rows, 2048 -> 64: 14 against 230 and 125). Rows count in whole 128s here, too.
   const long long big = (long long)((p.M + 127) / 128) * ((p.N + 127) / 128) * p.count;
   if (big >= 3 * 2 * sm_count()) return launch_tile<128, 128, 8, 1, 2>(p, stream);
   if (p.K >= 1024) return launch_tile<64, 64, 4, 8, 4>(p, stream);

@@ -17,4 +17,5 @@ struct FbGemmF32 {
 constexpr int FB_GEMM_F32_ROWS = 32;
 
 bool fb_gemm_f32_fits(const FbGemmF32& p);
+int fb_gemm_f32_tc_launch(const FbGemmF32& p, cudaStream_t stream);  // gemm_f32_tcgen05.cu
 int fb_gemm_f32_launch(const FbGemmF32& p, cudaStream_t stream);

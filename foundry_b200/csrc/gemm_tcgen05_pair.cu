@@ -2,6 +2,7 @@
 // and the entry point `fb_gemm_tc` are in gemm_tcgen05.cu.
 #define FB_STATUS_KERNEL 2
 #include "gemm_tcgen05.cuh"
+#include "tcgen05_pair.cuh"
 
 namespace {
 
@@ -39,84 +40,6 @@ struct SmemPair {
   static constexpr int STAGES = BUDGET / STAGE_BYTES > 12 ? 12 : BUDGET / STAGE_BYTES;
   static constexpr int BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256;
 };
-
-__device__ __forceinline__ uint32_t cluster_cta_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// The address, in the cluster's shared-memory window, of `local` in CTA `rank`.
-__device__ __forceinline__ uint32_t cluster_address(const void* local, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(local)), "r"(rank));
-  return out;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Tensor memory of both CTAs of a pair: one warp of each calls them, whole; all tcgen05
-// instructions of a kernel have one cta_group.
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t columns) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
-               "r"(columns)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t base, uint32_t columns) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns)
-               : "memory");
-}
-// A tile load whose completion is counted on a barrier of the CTA pair (its
-// address in the cluster window), not necessarily this CTA's own.
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map,
-                                                 uint32_t bar_cluster, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(bar_cluster), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Arrives, when the MMAs issued so far are complete, on the barrier at this
-// shared-memory offset in both CTAs of the pair.
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
-      "[%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3)
-      : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster)
-               : "memory");
-}
-// mbar_wait for a barrier that the peer CTA arrives on: acquire at cluster scope.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity,
-                                                  volatile int* abort_flag, int where, int kb) {
-  for (uint32_t spin = 0; spin < SPIN_LIMIT; ++spin) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((spin & 1023u) == 1023u && *abort_flag) return false;
-  }
-  *abort_flag = 1;
-  record_failure(where, (int)blockIdx.x, kb);
-  return false;
-}
 
 constexpr int MAX_TAIL_SHARES = 4;
 

@@ -101,6 +101,7 @@ _SIGNATURES = {
                      c_void_p, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_ll, c_int, c_int,
                      c_int, c_int, c_int, c_float, c_float, c_float, c_void_p, c_void_p],
     "fb_gemm_rows_status": [c_void_p],
+    "fb_gemm_f32_status": [c_void_p],
     "fb_row_scales": [c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p],
     "fb_select_tokens": [c_void_p, c_ll, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                          c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
@@ -1281,12 +1282,12 @@ if _os.environ.get("FOUNDRY_B200_PDL", "1") == "0":
 
 
 _STATUS_READERS = ("fb_gemm_tc_status", "fb_gemm_tc_pair_status", "fb_attention_tc_status",
-                   "fb_gemm_rows_status")
+                   "fb_gemm_rows_status", "fb_gemm_f32_status")
 # kernel codes of the host-visible failure record (FB_STATUS_KERNEL in csrc)
 _STATUS_KERNELS = {1: "tcgen05 product", 2: "paired tcgen05 product", 3: "tcgen05 prompt attention",
-                   4: "tcgen05 product for few token rows"}
+                   4: "tcgen05 product for few token rows", 5: "32-bit tcgen05 product"}
 _STATUS_ROLES = {1: "tile loads", 2: "matrix instructions", 3: "epilogue",
-                 20: "shared-memory alignment"}
+                 4: "accumulators", 5: "tiles to split", 6: "room for pieces", 20: "shared-memory alignment"}
 _MIRROR = []
 
 

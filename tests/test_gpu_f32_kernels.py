@@ -61,6 +61,66 @@ def test_product_of_large_tiles_and_views(ops, M, N, K):
     check_product(x, w, out)
 
 
+@pytest.mark.parametrize("M", [33, 64, 65, 128, 209, 417])
+@pytest.mark.parametrize("N,K", [(128, 1024), (257, 1028), (300, 4100), (2100, 1056), (8200, 1060)])
+def test_product_of_pieces(ops, M, N, K):
+    """Edges of the tensor cores' tiles (256 weight rows, 16 to 208 tokens, 32 of K), with and without
+    several pairs of SMs on a tile's K, as a view into a wider matrix."""
+    x, w = rnd(M, K + 8)[:, 4:K + 4], rnd(N, K, seed=1)
+    wide = torch.full((M + 1, N + 5), 7.0, device=DEV)
+    ops.gemm_simt(x, w, wide[:M, :N])
+    check_product(x, w, wide[:M, :N])
+    assert bool((wide[:, N:] == 7.0).all()) and bool((wide[M] == 7.0).all())  # nothing beyond
+    assert ops.gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("N", [300, 9000])
+def test_product_of_pieces_rounds_no_more_than_a_chain(ops, N):
+    """A chain of K additions is off by about 0.41 * 2^-24 * |x||w| in the root mean square (see
+    test_no_term_of_a_long_sum_is_lost); 32 of K at a time, a sum is off by less than half of that."""
+    x, w = rnd(100, 4096), rnd(N, 4096, seed=1)
+    out = torch.empty(100, N, device=DEV)
+    ops.gemm_simt(x, w, out)
+    norms = x.double().norm(dim=1)[:, None] * w.double().norm(dim=1)
+    off = (out.double() - x.double() @ w.double().T) / norms
+    assert float(off.square().mean().sqrt()) < 0.2 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("N", [300, 9000])
+def test_product_of_pieces_of_what_pieces_cannot_carry(ops, N):
+    """Infinities, NaN, overflow and operands near the smallest normal number come out as a chain of
+    32-bit FMAs gives them."""
+    x, w = rnd(64, 1024), rnd(N, 1024, seed=1)
+    x[3, 5], x[7, 9], w[100, 77] = float("inf"), float("nan"), float("-inf")
+    w[5] = 2.0 ** torch.randint(-3, 3, (1024,)).float()  # one piece each: the others are zero
+    x[9], w[11] = 3e38, 1.0
+    x[20] *= 1e-36
+    w[21] *= 1e-35
+    out = torch.empty(64, N, device=DEV)
+    ops.gemm_simt(x, w, out)
+    plain = torch.empty(64, N, device=DEV)
+    for r in range(0, 64, 32):  # up to 32 rows: FMAs
+        ops.gemm_simt(x[r:r + 32], w, plain[r:r + 32])
+    assert float(out[9, 11]) == float("inf")
+    out[9], plain[9] = 0, 0  # elsewhere in the row the order decides what overflows first
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf())
+    assert torch.equal(out.isposinf(), plain.isposinf())
+    whole = plain.isfinite()
+    size = (x.double().abs() @ w.double().abs().T)[whole]
+    # (1024 + 2) * 2^-24 of the magnitudes for either sum, and what rounding below 2^-126 takes
+    gap = (out.double() - plain.double()).abs()[whole] - 2 * 1026 * 2.0 ** -24 * size
+    assert float(gap.max()) <= 2.0 ** -126
+
+
+@pytest.mark.parametrize("M,N,K", [(900, 500, 64), (700, 300, 1028)])
+def test_many_batched_products(ops, M, N, K):
+    x, w = rnd(M, 32, K), rnd(32, N, K, seed=4)
+    out = torch.empty(M, 32, N, device=DEV)
+    ops.gemm_simt_batched(x, w, out)
+    for b in (0, 13, 31):
+        check_product(x[:, b], w[b], out[:, b])
+
+
 @pytest.mark.parametrize("M,off", [(3, 1), (40, 2), (5, 0)])
 def test_views_without_16_byte_rows_take_the_general_kernel(ops, M, off):
     K = 130 if off == 0 else 128  # a K of no whole pieces, or a base that is not aligned
