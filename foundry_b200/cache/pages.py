@@ -155,6 +155,16 @@ class SlotTable:
             group.grow(slot, length)
         self.length[slot] = length
 
+    def grow_in_place(self, slots, lengths) -> bool:
+        """One more token for each of the slots, which hold `lengths` tokens, if every one has room for
+        it on the pages it holds: else nothing changes, and `grow` decides. Between two pages, that is
+        (a held slot has the pages of its length in every group)."""
+        if any(n % PAGE == 0 for n in lengths) or not all(self.slots.is_held(s) for s in slots):
+            return False
+        for slot, n in zip(slots, lengths):
+            self.length[slot] = n + 1
+        return True
+
     def forget_from(self, slot: int, length: int) -> None:
         """The slot's tokens from `length` on are given up: a step that was run
         on a guess and is not wanted leaves the sequence as it was before it.

@@ -206,8 +206,13 @@ class SequenceCache:
     # --------------------------------------------------------------- slots
     def open_sequence(self) -> int:
         slot = self.table.open()
-        for rows in self.state.values():
-            rows[slot].zero_()
+        rows = [rows[slot] for rows in self.state.values()]
+        if rows and rows[0].is_cuda:
+            from ..kernels import ops  # (the cache itself needs no kernels, nor a GPU)
+            ops.zero_rows(rows)
+        else:
+            for row in rows:
+                row.zero_()
         return slot
 
     def close_sequence(self, slot: int) -> None:

@@ -1,6 +1,7 @@
 // The error channel of the kernel library.
 #include "common.cuh"
 
+#include <cstring>
 #include <mutex>
 
 static thread_local char g_error[1024] = "";
@@ -47,6 +48,41 @@ int* fb_status_mirror_host() {
 // The record's host address for the caller to read (and to zero after a
 // failure has been reported); null if it could not be made.
 FB_API int* fb_status_mirror() { return fb_status_mirror_host(); }
+
+// ---------------------------------------------------------------- host side of a step
+// One call each for what a step's host side does between two launches; through torch a step's
+// upload took four calls and about 25 us, its wait 10 (a stream object, its device looked up).
+
+FB_API int fb_event_create(void** event) {
+  const cudaError_t e = cudaEventCreateWithFlags((cudaEvent_t*)event, cudaEventDisableTiming);
+  return e == cudaSuccess ? 0 : fb_fail(2, "event_create: %s", cudaGetErrorString(e));
+}
+
+FB_API int fb_event_synchronize(void* event) {
+  return cudaEventSynchronize((cudaEvent_t)event) == cudaSuccess ? 0 : 2;
+}
+
+FB_API int fb_event_destroy(void* event) {
+  return cudaEventDestroy((cudaEvent_t)event) == cudaSuccess ? 0 : 2;
+}
+
+// Sends `bytes` from ordinary host memory through a pinned buffer, once the copy that last read the
+// buffer (`event` is recorded behind it) has run.
+FB_API int fb_upload(void* dst, void* pinned, const void* src, long long bytes, void* event,
+                     cudaStream_t stream) {
+  cudaError_t e = cudaEventSynchronize((cudaEvent_t)event);
+  if (e == cudaSuccess) {
+    memcpy(pinned, src, (size_t)bytes);
+    e = cudaMemcpyAsync(dst, pinned, (size_t)bytes, cudaMemcpyHostToDevice, stream);
+  }
+  if (e == cudaSuccess) e = cudaEventRecord((cudaEvent_t)event, stream);
+  return e == cudaSuccess ? 0 : fb_fail(2, "upload: %s", cudaGetErrorString(e));
+}
+
+FB_API int fb_wait_for_stream(cudaStream_t stream) {
+  const cudaError_t e = cudaStreamSynchronize(stream);
+  return e == cudaSuccess ? 0 : fb_fail(2, "wait_for_stream: %s", cudaGetErrorString(e));
+}
 
 int g_fb_pdl = 1;
 

@@ -539,3 +539,44 @@ FB_API int fb_softcap(float* x, long long n, float cap, cudaStream_t stream) {
   fb_launch(softcap_kernel, dim3(blocks), dim3(256), 0, stream, x, n, cap);
   return fb_check_launch("softcap");
 }
+
+// --------------------------------------------------------------- rows to zero
+// Up to 32 rows of memory become zero: a new sequence's state rows in one launch (a launch a tensor
+// was 5 us of host time each; 10 tensors, 8 sequences: 64 launches).
+namespace {
+constexpr int ZERO_ROWS = 32;
+struct ZeroRows {
+  unsigned char* row[ZERO_ROWS];
+  long long bytes[ZERO_ROWS];
+};
+__global__ void zero_rows_kernel(const __grid_constant__ ZeroRows rows) {
+  fb_pdl_wait();
+  unsigned char* row = rows.row[blockIdx.y];
+  const long long bytes = rows.bytes[blockIdx.y];
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  long long done = 0;
+  if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+    done = bytes / 16 * 16;
+    for (long long i = first; i < bytes / 16; i += step)
+      reinterpret_cast<uint4*>(row)[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  for (long long i = done + first; i < bytes; i += step) row[i] = 0;
+}
+}  // namespace
+
+FB_API int fb_zero_rows(void* const* row, const long long* bytes, int count, cudaStream_t stream) {
+  FB_REQUIRE(count >= 0 && count <= ZERO_ROWS, "zero_rows: %d rows, at most %d", count, ZERO_ROWS);
+  ZeroRows rows = {};
+  long long most = 0;
+  for (int i = 0; i < count; ++i) {
+    FB_REQUIRE(bytes[i] >= 0, "zero_rows: bad size %lld", bytes[i]);
+    rows.row[i] = (unsigned char*)row[i];
+    rows.bytes[i] = bytes[i];
+    if (bytes[i] > most) most = bytes[i];
+  }
+  if (most == 0) return 0;
+  const long long want = (most + 256 * 16 - 1) / (256 * 16);
+  fb_launch(zero_rows_kernel, dim3((unsigned)(want < 64 ? want : 64), (unsigned)count), dim3(256), 0,
+            stream, rows);
+  return fb_check_launch("zero_rows");
+}

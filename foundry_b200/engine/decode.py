@@ -80,6 +80,7 @@ class DecodeRunner:
             self.ctx._tables[id(group)] = part[7 + i].view(b, width)
         self.h_tables = [self.h[7 + i].reshape(b, width) for i in range(len(groups))]
         self.row_sig: List[Optional[Tuple[int, int, int]]] = [None] * b
+        self.filled_for: Optional[List[int]] = None  # the slots that the rows stand for
         self.h[3][:] = np.arange(b)  # every row's logits are wanted
         self.h[5][:] = np.arange(b + 1)
         # sampling inputs: temperature per row; random stream and step count per row
@@ -119,7 +120,7 @@ class DecodeRunner:
             self.kernel_histogram = {k: n - counted.get(k, 0) for k, n in after.items()
                                      if n != counted.get(k, 0)}
             plain_logits = self.logits
-            torch.cuda.current_stream().synchronize()
+            ops.wait_for_stream()
             graph = torch.cuda.CUDAGraph()
             # "relaxed": torch's pinned-memory allocator may query an event of an
             # earlier host copy while the capture is open; that call touches
@@ -165,16 +166,17 @@ class DecodeSession:
     def _prepare(self) -> DecodeRunner:
         """Reserve one more token per sequence and refresh the host buffers."""
         engine, cache = self.engine, self.engine.cache
-        n = len(self.slots)
-        lengths = [cache.length(s) for s in self.slots]
+        slots, table = self.slots, self.engine.cache.table
+        n = len(slots)
+        lengths = [table.length[s] for s in slots]
         limit = engine.spec.max_positions
-        for s, length in zip(self.slots, lengths):
-            if length + 1 > limit:
-                raise ValueError(f"slot {s} would pass the model's {limit} positions")
-        cache.reserve({s: length + 1 for s, length in zip(self.slots, lengths)})
-        need = 1
-        for g in cache.groups:
-            need = max(need, max(len(g.pages.pages(s)) for s in self.slots))
+        if max(lengths) + 1 > limit:
+            s = next(s for s, length in zip(slots, lengths) if length + 1 > limit)
+            raise ValueError(f"slot {s} would pass the model's {limit} positions")
+        if not table.grow_in_place(slots, lengths):
+            cache.reserve({s: length + 1 for s, length in zip(slots, lengths)})
+        held = [[g.pages.pages(s) for g in cache.groups] for s in slots]
+        need = max([1] + [len(pages) for groups in held for pages in groups])
         bucket = bucket_of(n)
         unequal = lengths_are_unequal(lengths)
         runner = self.runner
@@ -189,26 +191,24 @@ class DecodeSession:
                 # tokens that stay on the device (`step`) move on with the session
                 runner.ctx.token_ids.copy_(previous.next_tokens)
         h = runner.h
+        if runner.filled_for != slots:  # what the same rows leave as it is, and the padding
+            h[1][n:] = 0
+            h[2][:n] = np.arange(n)
+            h[2][n:] = -1
+            h[4][:n] = slots
+            h[4][n:] = cache.scratch_slot
+            h[6][n:] = 0
+            runner.row_sig[n:] = [None] * (bucket - n)
+            runner.filled_for = list(slots)
         h[1][:n] = lengths
-        h[1][n:] = 0
-        h[2][:n] = np.arange(n)
-        h[2][n:] = -1
-        h[4][:n] = self.slots
-        h[4][n:] = cache.scratch_slot
-        h[6][:n] = lengths
-        h[6][:n] += 1
-        h[6][n:] = 0
-        epoch = cache.table.epoch
-        for i, s in enumerate(self.slots):
-            count = sum(len(g.pages.pages(s)) for g in cache.groups)
-            sig = (s, epoch[s], count)
+        h[6][:n] = h[1][:n] + 1
+        epoch = table.epoch
+        for i, s in enumerate(slots):
+            sig = (s, epoch[s], sum([len(pages) for pages in held[i]]))
             if runner.row_sig[i] != sig:
                 runner.row_sig[i] = sig
-                for table, group in zip(runner.h_tables, cache.groups):
-                    pages = group.pages.pages(s)
-                    table[i, :len(pages)] = pages
-        for i in range(n, bucket):
-            runner.row_sig[i] = None
+                for rows, pages in zip(runner.h_tables, held[i]):
+                    rows[i, :len(pages)] = pages
         if not runner.capturable:  # plain launches: the parts may read the step on the host
             pad = bucket - n
             runner.ctx.slots_host = self.slots + [cache.scratch_slot] * pad
@@ -285,6 +285,31 @@ class DecodeSession:
                 self.engine.cache.forget_from(slot, length)
         self.counts = list(ahead["counts"])
 
+    def _started(self, tokens: List[int], counts: Optional[Sequence[int]] = None) -> DecodeRunner:
+        """The runner of the step for these tokens, which is on its way: from before, on
+        a guess that was right, or from now."""
+        ahead = self._ahead
+        if ahead is not None and (ahead["tokens"] != tokens or
+                                  (counts is not None and list(counts) != ahead["counts"])):
+            self.cancel_ahead()
+            ahead = None
+        self._ahead = None
+        if ahead is not None:
+            return self.runner
+        if counts is not None:
+            self.counts = list(counts)
+        return self._launch(tokens)
+
+    def step_logits(self, tokens: Sequence[int]) -> torch.Tensor:
+        """One step fed from the host; returns its float32 logits [rows, vocab], the
+        caller's own. Their copy is queued behind the step, and one wait covers both (the
+        tokens fetched, waited for, then the logits waited for and copied: 40 us more a step)."""
+        runner = self._started([int(t) for t in tokens])
+        logits = runner.logits[:len(self.slots)].clone()
+        ops.wait_for_stream()
+        ops.raise_on_device_failure()
+        return logits
+
     def step_host(self, tokens: Sequence[int], more: bool = False,
                   counts: Optional[Sequence[int]] = None) -> List[int]:
         """One step fed from the host; returns the chosen tokens on the host.
@@ -292,19 +317,7 @@ class DecodeSession:
         (sampling only). `more`: the caller expects to come back with the same
         rows and the tokens returned here, so the step after this one is
         started before this one's tokens are handed out."""
-        tokens = [int(t) for t in tokens]
-        ahead = self._ahead
-        if ahead is not None and (ahead["tokens"] != tokens or
-                                  (counts is not None and list(counts) != ahead["counts"])):
-            self.cancel_ahead()
-            ahead = None
-        self._ahead = None
-        if ahead is None:
-            if counts is not None:
-                self.counts = list(counts)
-            runner = self._launch(tokens)
-        else:
-            runner = self.runner  # the step for these tokens is already on its way
+        runner = self._started([int(t) for t in tokens], counts)
         n = len(self.slots)
         runner.tokens_host[:n].copy_(runner.next_tokens[:n], non_blocking=True)
         self._read.record()
@@ -329,6 +342,6 @@ class DecodeSession:
         if self._ahead is not None:
             raise RuntimeError("a step was started ahead: its logits have replaced the last "
                                "step's (use step_host(..., more=False) where logits are read)")
-        torch.cuda.current_stream().synchronize()
+        ops.wait_for_stream()
         ops.raise_on_device_failure()
         return self.runner.logits[:len(self.slots)]

@@ -148,7 +148,8 @@ class Engine:
         """Run the given tokens from the cache; float32 logits [wanted, vocab]
         in the order of `steps` and of each `want`."""
         if self._is_decode(steps):
-            return self._decode(steps, SamplingParams(), None, None)[1].logits().clone()
+            return self._session_of(steps, SamplingParams(), None, None).step_logits(
+                [int(s.tokens[0]) for s in steps])
         self._settle()
         limit = self.cache.step_token_limit()
         if limit is not None and any(len(s.tokens) > limit for s in steps):
@@ -165,7 +166,7 @@ class Engine:
         if logits.shape[0]:
             # logits leave the engine: wait for them, and let none out after a
             # kernel gave up on a bounded wait
-            torch.cuda.current_stream().synchronize()
+            ops.wait_for_stream()
             ops.raise_on_device_failure()
         return logits
 
@@ -207,7 +208,8 @@ class Engine:
         (a generation loop whose rows all go on unless a stop token ends one);
         single-token steps then start the next step before they return."""
         if self._is_decode(steps):
-            return self._decode(steps, params, keys, counts, more)[0]
+            session = self._session_of(steps, params, keys, counts)
+            return session.step_host([int(s.tokens[0]) for s in steps], more, counts)
         logits = self.step(steps)
         tokens = self.sampler.select(logits, params, keys, counts)
         return tokens.tolist()
@@ -216,9 +218,9 @@ class Engine:
     def _is_decode(steps: Sequence[SequenceStep]) -> bool:
         return len(steps) > 0 and all(len(s.tokens) == 1 and list(s.want) == [0] for s in steps)
 
-    def _decode(self, steps, params, keys, counts, more: bool = False):
-        """One token per sequence, through a `DecodeSession` (fixed buffers,
-        replayed graph); returns (host tokens, the session)."""
+    def _session_of(self, steps, params, keys, counts) -> "DecodeSession":
+        """The `DecodeSession` (fixed buffers, replayed graph) for one more token of
+        each sequence: the last one, if it is these sequences'."""
         slots = [s.slot for s in steps]
         if len(set(slots)) != len(slots):
             raise ValueError("a slot appears twice in one step")
@@ -234,8 +236,7 @@ class Engine:
                 or session.keys != keys:
             self._settle()
             session = self._session = DecodeSession(self, slots, params, keys, counts)
-        tokens = session.step_host([int(s.tokens[0]) for s in steps], more, counts)
-        return tokens, session
+        return session
 
     # -------------------------------------------------------------- decode
     def decode_session(self, slots: Sequence[int], sampling: SamplingParams = SamplingParams(),

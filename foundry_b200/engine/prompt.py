@@ -122,7 +122,7 @@ class PromptRunner:
             self.kernel_histogram = {k: n - counted.get(k, 0) for k, n in after.items()
                                      if n != counted.get(k, 0)}
             plain_logits = self.logits
-            torch.cuda.current_stream().synchronize()
+            ops.wait_for_stream()
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph, pool=self.engine.graph_pool(),
                                   capture_error_mode="relaxed"):

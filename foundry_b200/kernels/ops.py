@@ -9,7 +9,8 @@ from __future__ import annotations
 
 import ctypes
 import threading
-from typing import Optional
+import weakref
+from typing import Optional, Sequence
 
 import os as _os
 
@@ -101,6 +102,12 @@ _SIGNATURES = {
                      c_void_p, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_ll, c_int, c_int,
                      c_int, c_int, c_int, c_float, c_float, c_float, c_void_p, c_void_p],
     "fb_gemm_rows_status": [c_void_p],
+    "fb_event_create": [c_void_p],
+    "fb_event_synchronize": [c_void_p],
+    "fb_event_destroy": [c_void_p],
+    "fb_upload": [c_void_p, c_void_p, c_void_p, c_ll, c_void_p, c_void_p],
+    "fb_wait_for_stream": [c_void_p],
+    "fb_zero_rows": [c_void_p, c_void_p, c_int, c_void_p],
     "fb_gemm_f32_status": [c_void_p],
     "fb_row_scales": [c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p],
     "fb_select_tokens": [c_void_p, c_ll, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -342,14 +349,64 @@ def _call(name: str, *args, tag=None) -> None:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream() -> int:
     """The current CUDA stream's handle. This is called once per launch: the raw
     getter costs a fraction of a microsecond, `torch.cuda.current_stream()` ten."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_current_device())
     return torch.cuda.current_stream().cuda_stream
+
+
+def _host_call(name: str, *args) -> None:
+    """A call of the library that launches no kernel."""
+    if _fn(name)(*args) != 0:
+        message = library.load().fb_last_error().decode(errors="replace")
+        raise KernelError(f"{name}: {message}")
+
+
+def wait_for_stream() -> None:
+    """Wait for all work of the current stream."""
+    _host_call("fb_wait_for_stream", _stream())
+
+
+class UploadBuffer:
+    """A pinned buffer for uploads of up to `size` bytes: each goes through it once the copy that
+    last read it has run (csrc/common.cu)."""
+
+    def __init__(self, size: int):
+        self.size = size
+        self._pinned = torch.empty(max(1, size), dtype=torch.uint8).pin_memory()
+        self._address = self._pinned.data_ptr()
+        event = ctypes.c_void_p()
+        _host_call("fb_event_create", ctypes.addressof(event))
+        self._event = event.value
+        # (the copy that is under way holds on to the pinned memory: torch's allocator does not know it)
+        weakref.finalize(self, _end_upload_buffer, self._event, self._pinned)
+
+    def send(self, dst: int, src: int, size: int) -> None:
+        """Queue a copy of `size` bytes from the host address `src` to the device address `dst` on
+        the current stream."""
+        if size > self.size:
+            raise KernelError(f"an upload of {size} bytes through a buffer of {self.size}")
+        _host_call("fb_upload", dst, self._address, src, size, self._event, _stream())
+
+
+def _end_upload_buffer(event: int, pinned: torch.Tensor) -> None:
+    _fn("fb_event_synchronize")(event)
+    _fn("fb_event_destroy")(event)
+    del pinned
+
+
+def zero_rows(rows: Sequence[torch.Tensor]) -> None:
+    """Contiguous tensors become zero, up to 32 in a launch."""
+    for a in range(0, len(rows), 32):
+        part = rows[a:a + 32]
+        where = (c_void_p * len(part))(*[_dev(t, "row") for t in part])
+        size = (c_ll * len(part))(*[t.numel() * t.element_size() for t in part])
+        _call("fb_zero_rows", ctypes.addressof(where), ctypes.addressof(size), len(part), _stream())
 
 
 def code_of(dtype: torch.dtype) -> int:
@@ -731,7 +788,7 @@ _SM_OF_DEVICE = {}
 def sm_count() -> int:
     """SMs of the current device (asked once per device): the plans below size
     their grids to cover the SMs once."""
-    device = torch.cuda.current_device()
+    device = _current_device()
     count = _SM_OF_DEVICE.get(device)
     if count is None:
         count = _SM_OF_DEVICE[device] = torch.cuda.get_device_properties(device).multi_processor_count

@@ -166,3 +166,28 @@ def test_a_step_can_be_taken_back():
     with pytest.raises(CacheMisuse):
         table.forget_from(slot, 0)
     table.check()
+
+
+@pytest.mark.parametrize("window", [None, 100])
+@pytest.mark.parametrize("lengths", [[1, 63], [64, 5], [65, 200, 127], [128, 128]])
+def test_a_token_more_on_the_pages_held_is_what_growing_gives(lengths, window):
+    """Between two pages a token needs no page; at a page's edge, or for a slot that is not held, the
+    short way declines and changes nothing."""
+    def table():
+        t = SlotTable(4, [GroupPages(12), GroupPages(12, window)])
+        for n in lengths:
+            t.grow(t.open(), n)
+        return t
+    short, long = table(), table()
+    slots = list(range(3, 3 - len(lengths), -1)) if short.slots.is_held(3) else list(range(len(lengths)))
+    took = short.grow_in_place(slots, [short.length[s] for s in slots])
+    assert took == all(short.groups[0].pages_needed(n) == short.groups[0].pages_needed(n + 1) for n in lengths)
+    if took:
+        for s in slots:
+            long.grow(s, long.length[s] + 1)
+    assert short.length == long.length
+    for a, b in zip(short.groups, long.groups):
+        assert [a.pages(s) for s in slots] == [b.pages(s) for s in slots]
+    short.close(slots[0])
+    before = list(short.length)
+    assert not short.grow_in_place(slots, [short.length[s] for s in slots]) and short.length == before

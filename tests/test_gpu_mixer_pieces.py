@@ -138,3 +138,13 @@ def test_several_products_in_one_launch(ops, T):
             size = x.double().abs() @ w.double().abs().T
             assert bool(((out.double() - want).abs() <= x.shape[1] * 2.0 ** -23 * size).all())
     assert not ops.skinny_many_fits(pairs + pairs[:1])
+
+
+def test_zero_rows(ops):
+    """Rows of several tensors, types and alignments, more than fit one launch; nothing beside them."""
+    held = [torch.ones(3, n, dtype=d, device=DEV) for n, d in
+            [(1, torch.float32), (7, torch.bfloat16), (4096, torch.float32), (100001, torch.bfloat16)] * 9]
+    ops.zero_rows([t[1] for t in held])
+    for t in held:
+        assert bool((t[1] == 0).all()) and bool((t[0] == 1).all()) and bool((t[2] == 1).all())
+
