@@ -148,3 +148,45 @@ def test_zero_rows(ops):
     for t in held:
         assert bool((t[1] == 0).all()) and bool((t[0] == 1).all()) and bool((t[2] == 1).all())
 
+
+@pytest.mark.parametrize("W", [4, 100, 1024, 1028, 2048, 3072, 4100, 8192, 8196])
+@pytest.mark.parametrize("has_y,norm_y,has_out", [(1, 1, 1), (1, 0, 1), (0, 0, 1), (1, 1, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_layer_norms_around_a_sum(ops, W, has_y, norm_y, has_out, dtype):
+    """Rows at the edges of what a block's threads hold, against float64: sums of W terms in 32 bits
+    (W * 2^-24 of them at worst, sqrt(W) of order), 16 roundings besides, and bfloat16's half place."""
+    T = 3
+    rnd = lambda *s, seed: torch.randn(*s, generator=torch.Generator().manual_seed(seed)).to(DEV)  # noqa: E731
+    resid, y = rnd(T, W, seed=1) + 0.5, (rnd(T, W, seed=2) * 3 - 1).to(dtype)
+    w1, b1, w2, b2 = (rnd(W, seed=s) for s in (3, 4, 5, 6))
+    norm = lambda x, w, b: (x - x.mean(-1, keepdim=True)) / torch.sqrt(  # noqa: E731
+        x.var(-1, unbiased=False, keepdim=True) + 1e-5) * w.double() + b.double()
+    want = resid.double()
+    if has_y:
+        want = want + (norm(y.double(), w1, b1) if norm_y else 0.7 * y.double())
+    pending = types.SimpleNamespace(values=y, weight=w1 if norm_y else None, bias=b1 if norm_y else None,
+                                    eps=1e-5, scale=1.0 if norm_y else 0.7) if has_y else None
+    out = torch.empty(T, W, dtype=dtype, device=DEV) if has_out else None
+    ops.ln_add_ln(resid, pending, w2 if has_out else None, b2 if has_out else None, 1e-5, out)
+    room = (16 + 2 * W ** 0.5) * 2.0 ** -24
+    assert float((resid.double() - want).abs().max()) <= room * float(want.abs().max() + 4)
+    if has_out:
+        end = norm(want, w2, b2)
+        slack = 0 if dtype == torch.float32 else 2.0 ** -8
+        assert bool(((out.double() - end).abs() <= room * 16 + slack * end.abs() + 16 * room * end.abs()).all())
+
+
+@pytest.mark.parametrize("W", [2, 250, 2048])
+def test_embedding_with_sines_and_cosines(ops, W):
+    """Both of a pair from one thread; positions far out keep their 32 bits."""
+    table, ids = torch.randn(7, W, generator=torch.Generator().manual_seed(1)).to(DEV), [0, 6, 3, 9, -1]
+    positions = [0, 1, 77, 131071, 5]
+    freq = torch.pow(10000.0, -2.0 * torch.arange(W // 2, dtype=torch.float64) / W).to(DEV)
+    out, copy = (torch.empty(5, W, device=DEV) for _ in range(2))
+    as_int = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    ops.embed_sinusoid(table, as_int(ids), as_int(positions), freq, 1.5, out, copy)
+    angle = torch.tensor(positions, dtype=torch.float64, device=DEV)[:, None] * freq
+    pe = torch.stack([angle.sin(), angle.cos()], -1).flatten(1).float()
+    rows = torch.stack([table[i] * 1.5 if 0 <= i < 7 else torch.zeros(W, device=DEV) for i in ids])
+    # the sine's own rounding and the sum's: half a place each of numbers up to 1 and 8
+    assert float((out - (rows + pe)).abs().max()) <= 2.0 ** -24 + 2.0 ** -21 and torch.equal(out, copy)
