@@ -202,6 +202,11 @@ _SIGNATURES = {
                       c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p],
     "fb_chunk_scan_unit": [c_int, c_int, c_int],
     "fb_linear_step_fits": [c_int, c_int, c_int],
+    "fb_state_step_fits": [c_int, c_int],
+    "fb_state_step": [c_int, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_ll, c_void_p,
+                      c_void_p, c_int, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_int, c_void_p,
+                      c_int, c_void_p, c_ll, c_ll, c_void_p, c_ll, c_int, c_void_p, c_void_p, c_int,
+                      c_int, c_int, c_int, c_int, c_float, c_void_p],
     "fb_linear_step": [c_void_p, c_ll, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
                        c_void_p, c_int, c_void_p, c_ll, c_ll, c_void_p, c_ll, c_int, c_void_p,
                        c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float,
@@ -3133,6 +3138,46 @@ def linear_step(ctx, p: torch.Tensor, at, a2: torch.Tensor, a2_bias: torch.Tenso
           code_of(out.dtype), _dev(ctx.cu_tokens, "cu_tokens", torch.int32),
           _dev(ctx.slots, "slots", torch.int32), ctx.n_seqs, H, dim, vdim, rank, float(q_scale),
           float(eps), float(out_scale), _stream())
+    return out
+
+
+def state_step_fits(ctx, mode: int, state: StateRows, field: str, dim: int, vdim: int) -> bool:
+    """Whether `state_step` takes this step (single tokens, heads and states of whole 16-byte pieces)."""
+    return (LINEAR_STEP and ctx.is_decode and mode in (SCAN_DELTA, SCAN_WKV) and state.stride % 4 == 0
+            and (state.rows.data_ptr() + 4 * state.offset[field]) % 16 == 0
+            and bool(_fn("fb_state_step_fits")(dim, vdim)))
+
+
+def state_step(ctx, mode: int, q, k, v, g, decay, state: StateRows, field: str, norm: torch.Tensor,
+               gate: torch.Tensor, act: str, eps: float, out: torch.Tensor, H: int, rep: int, dim: int,
+               vdim: int, beta=None, bonus=None, decay_per_head: bool = False) -> torch.Tensor:
+    """One token a sequence of the delta rule or the wkv between its products (csrc/state_step.cu):
+    `decay_gate`, `state_scan` and `head_norm_gate` in one launch; arguments as theirs. `decay`: None
+    (g holds decays), or (A or None, bias) with the projection in g. `norm`: [vdim], or [H * vdim]."""
+    f32 = torch.float32
+    form, A, bias = 0, None, None
+    if decay is not None:
+        A, bias = decay
+        form = 2 if A is None else 1
+    n, decays = ctx.n_seqs, H if decay_per_head else H * dim
+    if norm.numel() not in (vdim, H * vdim) or out.shape[0] < n or out.shape[1] < H * vdim \
+            or g.shape[1] < decays or gate.shape[1] < H * vdim \
+            or (A is not None and A.numel() != H) or (bias is not None and bias.numel() != decays) \
+            or (bonus is not None and bonus.numel() != H * dim):
+        raise KernelError(f"state_step: a parameter's size is not that of {H} heads of {dim} x {vdim}")
+
+    def rows(t, name):
+        return (0, 0) if t is None else (_dev(t, name, f32, contiguous=False), _rows(t, name))
+
+    def flat(t, name):
+        return 0 if t is None else _dev(t, name, f32)
+    _call("fb_state_step", 1 if mode == SCAN_DELTA else 0, *rows(q, "q"), *rows(k, "k"), *rows(v, "v"),
+          *rows(g, "g"), flat(A, "A"), flat(bias, "bias"), form, 1 if decay_per_head else 0,
+          *rows(beta, "beta"), flat(bonus, "bonus"), *rows(gate, "gate"), {"sigmoid": 0, "silu": 1}[act],
+          flat(norm, "norm"), 0 if norm.numel() == vdim else vdim, state.rows.data_ptr(), state.stride,
+          state.offset[field], _dev(out, "out", contiguous=False), _rows(out, "out"),
+          code_of(out.dtype), _dev(ctx.cu_tokens, "cu_tokens", torch.int32),
+          _dev(ctx.slots, "slots", torch.int32), n, H, rep, dim, vdim, float(eps), _stream())
     return out
 
 

@@ -122,7 +122,7 @@ class GatedDeltaChannel(Part):
                                   n_scaled=G, extra=d ** -0.5, unit_eps=self.unit_eps):
             ops.state_tail_update(ctx, p, state, "tail", self.taps - 1, C)
         at = C + H + self.decay_rank
-        decay = gate = None
+        decay, gate, raw = None, None, False
         if ops.low_rank_pays(T, x.dtype, self.decay_rank, self.gate_rank):
             decay = ops.low_rank(p[:, C + H:at], self.a2, bias=self.dt_bias, A=self.A_log, per_head=d)
             gate = ops.low_rank(p[:, at:at + self.gate_rank], self.g2)
@@ -131,6 +131,14 @@ class GatedDeltaChannel(Part):
             ops.unary_cast(p[:, C + H:], low)
             decay = product_f32(low[:, :self.decay_rank], self.a2)
             gate = product_f32(low[:, self.decay_rank:], self.g2)
+            raw = True
+        if ops.state_step_fits(ctx, ops.SCAN_DELTA, state, "S", d, v):
+            y = torch.empty((T, H * v), dtype=x.dtype, device=x.device)
+            ops.state_step(ctx, ops.SCAN_DELTA, qkv, qkv[:, G * d:], qkv[:, 2 * G * d:], decay,
+                           (self.A_log, self.dt_bias) if raw else None, state, "S", self.norm, gate,
+                           "sigmoid", self.eps, y, H, H // G, d, v, beta=p[:, C:])
+            return product_f32(y, self.o)
+        if raw:
             ops.decay_gate(decay, d, self.dt_bias, self.A_log)
         o = torch.empty((T, H * v), **f32)
         ops.state_scan(ctx, ops.SCAN_DELTA, qkv, qkv[:, G * d:], qkv[:, 2 * G * d:], decay, state,
@@ -198,6 +206,12 @@ class GatedDelta(Part):
                                   n_scaled=G, extra=d ** -0.5, unit_eps=self.unit_eps):
             ops.state_tail_update(ctx, p, state, "tail", self.taps - 1, C)
         at = C + H * v
+        if ops.state_step_fits(ctx, ops.SCAN_DELTA, state, "S", d, v):
+            y = torch.empty((T, H * v), dtype=x.dtype, device=x.device)
+            ops.state_step(ctx, ops.SCAN_DELTA, qkv, qkv[:, G * d:], qkv[:, 2 * G * d:], p[:, at + H:],
+                           (self.A_log, self.dt_bias), state, "S", self.norm, p[:, C:], self.gate,
+                           self.eps, y, H, H // G, d, v, beta=p[:, at:], decay_per_head=True)
+            return product_to_residual(ctx, y, self.o)
         decay = torch.empty((T, H), **f32)
         ops.decay_gate(p[:, at + H:at + 2 * H], 1, self.dt_bias, self.A_log, out=decay)
         o = torch.empty((T, H * v), **f32)
@@ -332,13 +346,20 @@ class WkvTimeMix(Part):
             ops.state_tail_update(ctx, x, state, "prev", 1, W)
         r, k, v, g, raw = products_f32([(mixes[i], w) for i, w in enumerate(
             (self.r, self.k, self.v, self.g, self.w1))])
-        decay = None
+        decay, projected = None, False
         if ops.low_rank_pays(T, x.dtype, self.decay_rank):
             decay = ops.low_rank(raw, self.w2, "tanh", bias=self.w0)
         if decay is None:
             low = torch.empty((T, self.decay_rank), dtype=x.dtype, device=x.device)
             ops.unary_cast(raw, low, "tanh")
             decay = product_f32(low, self.w2)
+            projected = True
+        if ops.state_step_fits(ctx, ops.SCAN_WKV, state, "S", d, d):
+            y = torch.empty((T, H * d), dtype=x.dtype, device=x.device)
+            ops.state_step(ctx, ops.SCAN_WKV, r, k, v, decay, (None, self.w0) if projected else None,
+                           state, "S", self.norm, g, "silu", self.eps, y, H, 1, d, d, bonus=self.u)
+            return product_f32(y, self.o)
+        if projected:
             ops.decay_gate(decay, d, self.w0, None)
         o = torch.empty((T, H * d), dtype=torch.float32, device=x.device)
         ops.state_scan(ctx, ops.SCAN_WKV, r, k, v, decay, state, "S", o, H, 1, d, d, bonus=self.u)

@@ -149,6 +149,81 @@ def test_zero_rows(ops):
         assert bool((t[1] == 0).all()) and bool((t[0] == 1).all()) and bool((t[2] == 1).all())
 
 
+def sigmoid64(x):
+    return torch.sigmoid(x.double())
+
+
+@pytest.mark.parametrize("mode,H,rep,dim,vdim,per_head", [
+    ("delta", 4, 2, 64, 64, False), ("delta", 3, 1, 128, 128, False), ("delta", 2, 1, 30, 8, True),
+    ("delta", 2, 2, 100, 32, True), ("delta", 2, 1, 61, 256, False), ("wkv", 4, 1, 64, 64, False),
+    ("wkv", 2, 1, 128, 128, False), ("wkv", 3, 1, 16, 16, False)])
+@pytest.mark.parametrize("form", [0, 1, 2])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_state_step(ops, mode, H, rep, dim, vdim, per_head, form, dtype):
+    """A token's decays, step, norm and gate in one kernel against float64. Every 32-bit sum here has up
+    to `dim` terms, each off by at most dim * 2^-24 of the magnitudes; the norm makes them of order one
+    and adds a few roundings: 64 + dim of them bound the state and the output (bfloat16: its own half
+    place, 2^-9, on top)."""
+    n, slots_n, n_decay = 3, 5, H if per_head else H * dim
+    rnd = lambda *s, seed: torch.randn(*s, generator=torch.Generator().manual_seed(seed)).to(DEV)  # noqa: E731
+    slots = [4, 0, 2]
+    q, k = rnd(n, H // rep * dim + 3, seed=1), rnd(n, H // rep * dim, seed=2) * dim ** -0.5
+    v, gate = rnd(n, H * vdim, seed=3), rnd(n, H * vdim + 5, seed=4)
+    raw, beta = rnd(n, n_decay, seed=5), rnd(n, H, seed=6)
+    A, bias = rnd(H, seed=7) * 0.3, rnd(n_decay, seed=8)
+    bonus, wide_norm = rnd(H, dim, seed=9), mode == "wkv"
+    norm = 1 + 0.1 * rnd(H * vdim if wide_norm else vdim, seed=10)
+    g = torch.sigmoid(raw) if form == 0 else raw
+    rows = rnd(slots_n, 4 + H * dim * vdim, seed=11)
+    before = rows.clone()
+    state = ops.StateRows(rows, [("front", 4), ("S", H * dim * vdim)])
+    as_int = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    ctx = types.SimpleNamespace(is_decode=True, n_seqs=n, cu_tokens=as_int([0, 1, 2, 3]), slots=as_int(slots))
+    which = ops.SCAN_DELTA if mode == "delta" else ops.SCAN_WKV
+    assert ops.state_step_fits(ctx, which, state, "S", dim, vdim)
+    out = torch.empty(n, H * vdim, dtype=dtype, device=DEV)
+    act = "sigmoid" if mode == "delta" else "silu"
+    ops.state_step(ctx, which, q, k, v, g, None if form == 0 else (A if form == 1 else None, bias), state,
+                   "S", norm, gate, act, 1e-5, out, H, rep, dim, vdim, beta=beta, bonus=bonus,
+                   decay_per_head=per_head)
+    d64 = g.double()
+    if form == 1:
+        each = A.double() if per_head else A.double().repeat_interleave(dim)
+        d64 = torch.exp(-torch.exp(each) * torch.nn.functional.softplus(d64 + bias.double()))
+    if form == 2:
+        d64 = torch.exp(-torch.exp(d64 + bias.double()))
+    room = (64 + dim) * 2.0 ** -24
+    for i in range(n):
+        S0 = before[slots[i], 4:].double().view(H, dim, vdim)
+        for h in range(H):
+            S, a = S0[h], (h // rep) * dim
+            qq, kk = q[i, a:a + dim].double(), k[i, a:a + dim].double()
+            vv = v[i, h * vdim:(h + 1) * vdim].double()
+            gg = d64[i, h] if per_head else d64[i, h * dim:(h + 1) * dim, None]
+            if mode == "delta":
+                new = gg * S
+                new = new + kk[:, None] * (sigmoid64(beta[i, h]) * (vv - kk @ new))
+                o, size = qq @ new, qq.abs() @ new.abs()
+            else:
+                kv = kk[:, None] * vv
+                o = qq @ (S + bonus[h].double()[:, None] * kv)
+                size = qq.abs() @ (S.abs() + (bonus[h].double()[:, None] * kv).abs())
+                new = gg * S + kv
+            got = rows[slots[i], 4 + h * dim * vdim:4 + (h + 1) * dim * vdim].double().view(dim, vdim)
+            assert float((got - new).abs().max()) <= room * float(S.abs().max() + vv.abs().max()) * 4
+            scale = 1 / torch.sqrt((o * o).mean() + 1e-5)
+            z = gate[i, h * vdim:(h + 1) * vdim].double()
+            z = torch.sigmoid(z) if act == "sigmoid" else z * torch.sigmoid(z)
+            w = (norm[h * vdim:(h + 1) * vdim] if wide_norm else norm).double() * z
+            want = o * scale * w
+            bound = room * (size * scale * w.abs() + want.abs() * (1 + size.max() * scale))
+            if dtype == torch.bfloat16:
+                bound = bound + want.abs() * 2.0 ** -8
+            assert bool(((out[i, h * vdim:(h + 1) * vdim].double() - want).abs() <= bound + 1e-7).all())
+    untouched = [s for s in range(slots_n) if s not in slots]
+    assert torch.equal(rows[untouched], before[untouched]) and torch.equal(rows[:, :4], before[:, :4])
+
+
 @pytest.mark.parametrize("W", [4, 100, 1024, 1028, 2048, 3072, 4100, 8192, 8196])
 @pytest.mark.parametrize("has_y,norm_y,has_out", [(1, 1, 1), (1, 0, 1), (0, 0, 1), (1, 1, 0)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
