@@ -20,9 +20,8 @@
 // instruction's first operand, the tokens' to shared memory: with both in shared memory, its
 // bandwidth was the bound (raw tiles in and out, pieces in, and out again for six products; 777 rows
 // -> 16384 473 us). Roles of a CTA's 20 warps: TMA producer, MMA issuer (leader only), two idle, 8
-// that split raw 32-bit stages, 8 that add accumulators up in registers and store. Barriers of the
-// pair order shared and tensor memory of the CTA that arrives only (the default scope): arrivals at
-// cluster scope took about 1,000 cycles each. Every wait is bounded, as elsewhere.
+// that split raw 32-bit stages, 8 that add accumulators up in registers and store. Every wait is
+// bounded, as elsewhere.
 //
 // What a piece cannot carry is summed again by the thread that would store it, one product after the
 // other: results that are not finite (an infinity's pieces are not numbers, and what overflows has to
@@ -86,12 +85,6 @@ __device__ __forceinline__ uint32_t last_piece(float a, float b) {
   uint32_t h;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
   return h;
-}
-
-// An arrival on a barrier of either CTA that orders this CTA's own shared and tensor memory only,
-// which is what the MMAs of a pair read and write.
-__device__ __forceinline__ void mbar_arrive_pair(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }
 
 __device__ __forceinline__ bool elect_one() {

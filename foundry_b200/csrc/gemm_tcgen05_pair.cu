@@ -177,7 +177,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       for (int u = cluster; u < total_units && ok; u += clusters, ++j) {
         const PairUnit w = pair_unit(p, u, tiles_a, nkb);
         const int buf = j & 1;
-        ok = mbar_wait_cluster(&acc_empty[buf], (uint32_t)((j >> 1) & 1) ^ 1u, abort_flag, 4, j);
+        ok = mbar_wait(&acc_empty[buf], (uint32_t)((j >> 1) & 1) ^ 1u, abort_flag, 4, j);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
@@ -185,7 +185,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           const int use = it + (kb - w.kb0);
           const int s = use % STAGES;
           const uint32_t phase = (uint32_t)(use / STAGES) & 1u;
-          ok = mbar_wait_cluster(&full[s], phase, abort_flag, 2, kb);
+          ok = mbar_wait(&full[s], phase, abort_flag, 2, kb);
           if (!ok) break;
           tc_fence_after();
           const uint32_t a_addr = smem_u32(tiles + s * SmemPair<BN>::STAGE_BYTES);
@@ -262,7 +262,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       // this warp has read its lanes of the accumulator: tell the leader's MMA warp
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(acc_empty_leader + (uint32_t)(buf * 8));
+      if (lane == 0) mbar_arrive_pair(acc_empty_leader + (uint32_t)(buf * 8));
       if (mine != nullptr) {
         // publish this warp's 32 rows of the share; the warp that completes the set
         // (the same rows of every share) sums them and stores the result
