@@ -8,8 +8,9 @@
 //   another. 4 tokens over 600 keys, 32 heads over 8 of 64: 11 us against 511.
 // `tile_kernel`, many tokens a sequence (prompts): 64 neighbouring tokens of one sequence and one
 //   query head a block, keys in tiles through shared memory, register tiles for both products.
-//   Bound by the FMA pipe and the shared-memory reads beside it. 777 tokens, 32 heads over 8 of
-//   64: 199 us against 1405.
+//   Bound by latency with three warps a scheduler (the issue slots are 38 % busy; registers and
+//   shared memory hold no more). 777 tokens, 32 heads over 8 of 64: 169 us, 204 before a tile's
+//   product lost a branch a channel and two blocks shared the keys, 1405 in attention_simt.cu.
 //
 // Queries, keys and values are read with coherent (L2) loads: the kernel that wrote this step's
 // rows may have overlapped this kernel's start.
@@ -232,7 +233,9 @@ split_kernel(FbAttentionF32 p, int head_chunks) {
 // time (`runs`: z of the grid shares a block's runs among neighbours, so that many short
 // sequences side by side are not walked one after another). A thread owns 4 rows; the 8 threads
 // of a row lie in one warp, so the weights between the two products pass through shared memory
-// that only the warp reads.
+// that only the warp reads. A causal prompt's blocks have one tile of keys to many: the S blocks of a
+// cluster (neighbours in z) take every S-th tile of the same rows and merge what they hold, in rank
+// order, each a share of the rows.
 constexpr int BQ = 64, TILE_THREADS = 128;
 
 template <int D, int BKEY>
@@ -241,7 +244,31 @@ struct AttnTile {
   static constexpr int BYTES = (D * PQ + D * PK + BKEY * PV + BKEY * PP) * 4;
 };
 
-template <int D, int BKEY>
+__device__ __forceinline__ void meet_cluster() {
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned shared_of(const float* mine, int rank) {
+  unsigned there;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(there)
+               : "r"((unsigned)__cvta_generic_to_shared(mine)), "r"(rank));
+  return there;
+}
+__device__ __forceinline__ float ld_peer(unsigned there) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(there) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_peer4(unsigned there) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(there)
+               : "memory");
+  return v;
+}
+
+template <int D, int BKEY, int S>
 __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(FbAttentionF32 p) {
   using G = AttnTile<D, BKEY>;
   constexpr int NK = BKEY / 32, NV = D / 32;
@@ -257,12 +284,19 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
   const int tx = lane % 8, ty = warp * 4 + lane / 8;
   const int t0 = (gridDim.x - 1 - blockIdx.x) * BQ;  // later tokens see more keys: first
   const int a = blockIdx.y, kvh = a / (p.A / p.Kh);
-  const int rows = min(BQ, p.T - t0);
+  const int rows = min(BQ, p.T - t0), rank = S > 1 ? blockIdx.z % S : 0;
+  // (a cluster's own results, over the tiles of keys and values: rows of D, maxima, sums)
+  float* held = smem + D * G::PQ;
+  float* held_m = held + BQ * D;
+  float* held_l = held_m + BQ;
+  static_assert(BQ * D + 2 * BQ <= D * G::PK + BKEY * G::PV, "room for a cluster's results");
   if (tid < BQ) {
     seq_of[tid] = tid < rows ? p.seq_of_token[t0 + tid] : -1;
     pos_of[tid] = tid < rows ? p.positions[t0 + tid] : 0;
   }
   __syncthreads();
+  const int breaks = __syncthreads_count(tid > 0 && tid < rows && seq_of[tid] != seq_of[tid - 1]);
+  if ((int)blockIdx.z / S > breaks) return;  // no run for this block, nor for its cluster
   for (int i = tid; i < BQ * (D / 4); i += TILE_THREADS) {
     const int r = i % BQ, d = (i / BQ) * 4;
     const float4 v = seq_of[r] >= 0 ? ldcg4(p.q + (size_t)(t0 + r) * p.q_stride + (size_t)a * D + d)
@@ -279,7 +313,8 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
     while (last + 1 < rows && seq_of[last + 1] == seq) ++last;
     const int begin_row = first;
     first = last + 1;
-    if (run % gridDim.z != blockIdx.z) continue;
+    if (run % (gridDim.z / S) != blockIdx.z / S) continue;
+    if (seq < 0 && rank > 0) continue;
     if (seq < 0) {  // padding tokens: defined output, no cache access
       for (int i = tid; i < (last - begin_row + 1) * D; i += TILE_THREADS)
         p.out[(size_t)(t0 + begin_row + i / D) * p.out_stride + (size_t)a * D + i % D] = 0.f;
@@ -316,7 +351,7 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
 #pragma unroll
       for (int q = 0; q < NV; ++q) acc[i][q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int j0 = from / BKEY * BKEY; j0 <= to; j0 += BKEY) {
+    for (int j0 = (from / BKEY + rank) * BKEY; j0 <= to; j0 += S * BKEY) {
       __syncthreads();  // the tile before is no longer read (and the queries are in)
 #pragma unroll 4
       for (int i = tid; i < BKEY * (D / 4); i += TILE_THREADS) {
@@ -348,13 +383,13 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int c = 0; c < 4 * NK; ++c) s[i][c] = 0.f;
+      // (a short tile's second half is multiplied, too: it is zeros)
 #pragma unroll 8
       for (int d = 0; d < D; ++d) {
         float x[4], y[4 * NK];
         *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(&qt[d][ty * 4]);
 #pragma unroll
         for (int q = 0; q < NK; ++q) {
-          if (q > 0 && q * 32 >= keys) break;
           *reinterpret_cast<float4*>(y + 4 * q) =
               *reinterpret_cast<const float4*>(&kt[d][q * 32 + tx * 4]);
 #pragma unroll
@@ -425,6 +460,59 @@ __global__ void __launch_bounds__(TILE_THREADS, D >= 128 ? 2 : 3) tile_kernel(Fb
         add_values(std::true_type{});
       __syncwarp();  // the weights are read before the next tile's replace them
     }
+    if constexpr (S > 1) {
+      __syncthreads();  // the last tile is no longer read
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = ty * 4 + i;
+        if (tx == 0) {
+          held_m[r] = m[i];
+          held_l[r] = l[i];
+        }
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+          *reinterpret_cast<float4*>(held + r * D + q * 32 + tx * 4) = acc[i][q];
+      }
+      meet_cluster();
+      unsigned sums[S], tops[S], totals[S];
+#pragma unroll
+      for (int k = 0; k < S; ++k) {
+        sums[k] = shared_of(held, k);
+        tops[k] = shared_of(held_m, k);
+        totals[k] = shared_of(held_l, k);
+      }
+      for (int e = tid; e < BQ / S * (D / 4); e += TILE_THREADS) {
+        const int r = rank * (BQ / S) + e / (D / 4), d = e % (D / 4) * 4;
+        if (r < begin_row || r > last) continue;
+        float pm[S], pl[S], top = -INFINITY, total = 0.f;
+        float4 ps[S], sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+          pm[k] = ld_peer(tops[k] + r * 4);
+          pl[k] = ld_peer(totals[k] + r * 4);
+          ps[k] = ld_peer4(sums[k] + (r * D + d) * 4);
+        }
+#pragma unroll
+        for (int k = 0; k < S; ++k) top = fmaxf(top, pm[k]);
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+          const float f = exp_below(pm[k], top);
+          total = fmaf(f, pl[k], total);
+          sum.x = fmaf(f, ps[k].x, sum.x);
+          sum.y = fmaf(f, ps[k].y, sum.y);
+          sum.z = fmaf(f, ps[k].z, sum.z);
+          sum.w = fmaf(f, ps[k].w, sum.w);
+        }
+        const float inv = 1.0f / total;
+        float* o = p.out + (size_t)(t0 + r) * p.out_stride + (size_t)a * D + d;
+        o[0] = sum.x * inv;
+        o[1] = sum.y * inv;
+        o[2] = sum.z * inv;
+        o[3] = sum.w * inv;
+      }
+      meet_cluster();  // a peer may still read this block's results
+      continue;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = ty * 4 + i;
@@ -451,6 +539,20 @@ int launch_split(const FbAttentionF32& p, cudaStream_t stream) {
   else
     fb_launch_cluster(split_kernel<D, GH, S, W>, grid, dim3(W * 32), 0, stream, S, p, chunks);
   return fb_check_launch("attention_f32_split");
+}
+
+template <int D, int S>
+int launch_tiles(const FbAttentionF32& p, cudaStream_t stream) {
+  constexpr int BKEY = D >= 128 ? 32 : 64, bytes = AttnTile<D, BKEY>::BYTES;
+  static bool seen[64] = {};
+  if (fb_first_use_on_device(seen) &&
+      cudaFuncSetAttribute(tile_kernel<D, BKEY, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           bytes) != cudaSuccess)
+    return fb_fail(2, "attention: cannot set %d bytes of shared memory", bytes);
+  const dim3 grid((p.T + BQ - 1) / BQ, p.A, (p.n_seqs < 4 ? p.n_seqs : 4) * S);
+  if (S == 1) fb_launch(tile_kernel<D, BKEY, S>, grid, dim3(TILE_THREADS), (size_t)bytes, stream, p);
+  else fb_launch_cluster(tile_kernel<D, BKEY, S>, grid, dim3(TILE_THREADS), (size_t)bytes, stream, S, p);
+  return fb_check_launch("attention_f32_tile");
 }
 
 int power_of_two(int n, int from) {
@@ -495,15 +597,13 @@ int launch_d(const FbAttentionF32& p, cudaStream_t stream) {
            : S == 2 ? launch_split<D, 4, 2>(p, stream)
                     : launch_split<D, 4, 1>(p, stream);
   }
-  constexpr int BKEY = D >= 128 ? 32 : 64, bytes = AttnTile<D, BKEY>::BYTES;
-  static bool seen[64] = {};
-  if (fb_first_use_on_device(seen) &&
-      cudaFuncSetAttribute(tile_kernel<D, BKEY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           bytes) != cudaSuccess)
-    return fb_fail(2, "attention: cannot set %d bytes of shared memory", bytes);
-  const dim3 grid((p.T + BQ - 1) / BQ, p.A, p.n_seqs < 4 ? p.n_seqs : 4);
-  fb_launch(tile_kernel<D, BKEY>, grid, dim3(TILE_THREADS), (size_t)bytes, stream, p);
-  return fb_check_launch("attention_f32_tile");
+  // One sequence: two blocks share a row block's keys (777 tokens, 32 heads over 8 of 64: 169 us for
+  // 191; 400: 54 for 85; 33: 15 for 14), four where the cache holds eight times the step's tokens and
+  // more (64 tokens behind 3,000: 127 for 471, with two 242). The blocks of several sequences fill the
+  // SMs as they are (2 x 400: 99 us, 107 with two, 4 x 200: 57 and 84).
+  if (seqs == 1 && width >= 16 && width * FB_PAGE >= 8 * tokens) return launch_tiles<D, 4>(p, stream);
+  if (seqs == 1 && tokens > BQ) return launch_tiles<D, 2>(p, stream);
+  return launch_tiles<D, 1>(p, stream);
 }
 }  // namespace
 

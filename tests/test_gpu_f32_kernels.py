@@ -191,6 +191,7 @@ def test_attention_of_single_tokens(ops, D, G):
     [(0, 0, 130)],                                                     # blocks' and tiles' edges
     [(0, 37, 64), (1, 0, 65)],                                         # continued; ends in a block
     [(0, 0, 17), (1, 200, 20), (2, 3, 16), (3, 0, 40), (-1, 0, 30)],   # runs in one block, padding
+    [(0, 0, 65), (-1, 0, 63)], [(0, 590, 1), (-1, 0, 20), (0, 591, 50)],  # blocks that share the keys
 ])
 def test_attention_of_prompts(ops, D, runs):
     check_attention(ops, paged_case(runs, 2, 2, D), 2, 2, D)
