@@ -756,11 +756,12 @@ moe_combine_rows_kernel(const float* y, const int* place, const float* weights, 
 }
 
 // The router's product and the choice in one kernel, for rows of whole 64s in 16 bits and up to 64
-// outputs: a block takes 16 tokens, its eight warps share K, token rows and router rows go
+// outputs: a block takes 16 tokens, its warps share K, token rows and router rows go
 // straight from memory into mma.sync fragments (K permuted within 64 so that a thread's fragment is
 // 16-byte pieces, as in gemm_skinny.cu), the warps' sums meet in shared memory in order, and the
-// tokens' logits are routed where they were made. Bound by its loads' latency: 2,000 tokens of
-// 3,072, 16 outputs 21 us; the product alone took 27 on the tcgen05 kernel, whose 16 tiles
+// tokens' logits are routed where they were made. Bound by its loads' latency and by a token's choice,
+// a chain of one warp's: 16 warps a block (eight from 33 outputs on, for their shared memory).
+// 2,000 tokens of 3,072, 16 outputs with the sort behind it 14.2 us, 16.6 with eight; the product alone took 27 on the tcgen05 kernel, whose 16 tiles
 // walk all of K on 16 SMs, and the choice 6.
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                           uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -770,18 +771,21 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-constexpr int ROUTER_WARPS = 8, ROUTER_TOKENS = 16;
+constexpr int ROUTER_TOKENS = 16;
 template <int NT>
-__global__ void __launch_bounds__(ROUTER_WARPS * 32)
+constexpr int ROUTER_WARPS = NT <= 4 ? 16 : 8;
+template <int NT>
+__global__ void __launch_bounds__(ROUTER_WARPS<NT> * 32)
 moe_router_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __restrict__ w,
                   long long ldw, int K, float* z, const float* __restrict__ bias, int E, int top,
                   int* __restrict__ chosen, float* __restrict__ weights, int score, int groups,
                   int keep, const float* __restrict__ correction, int normalise, float sum_floor,
                   float weight_scale, int group_best, int T) {
+  constexpr int WARPS = ROUTER_WARPS<NT>;
   fb_pdl_launch();
-  __shared__ float part[ROUTER_WARPS][ROUTER_TOKENS][8 * NT + 1];
-  __shared__ float s_all[ROUTER_WARPS][8 * NT], s_group[ROUTER_WARPS][8 * NT],
-      s_plain[ROUTER_WARPS][8 * NT];
+  __shared__ float part[WARPS][ROUTER_TOKENS][8 * NT + 1];
+  __shared__ float s_all[WARPS][8 * NT], s_group[WARPS][8 * NT],
+      s_plain[WARPS][8 * NT];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int t0 = blockIdx.x * ROUTER_TOKENS;
   const __nv_bfloat16* rows[2] = {x + (long long)min(t0 + g, T - 1) * ldx + q * 8,
@@ -794,7 +798,7 @@ moe_router_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __
   for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
   fb_pdl_wait();
 #pragma unroll 2
-  for (int c = warp; c < K / 64; c += ROUTER_WARPS) {
+  for (int c = warp; c < K / 64; c += WARPS) {
     uint4 a[2][2], b[NT][2];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
@@ -821,15 +825,15 @@ moe_router_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* __
 #pragma unroll
     for (int i = 0; i < 4; ++i) part[warp][g + (i >> 1) * 8][j * 8 + 2 * q + (i & 1)] = acc[j][i];
   __syncthreads();
-  for (int i = threadIdx.x; i < ROUTER_TOKENS * 8 * NT; i += ROUTER_WARPS * 32) {
+  for (int i = threadIdx.x; i < ROUTER_TOKENS * 8 * NT; i += WARPS * 32) {
     const int t = i / (8 * NT), e = i % (8 * NT);
     float sum = 0.f;
 #pragma unroll
-    for (int k = 0; k < ROUTER_WARPS; ++k) sum += part[k][t][e];
+    for (int k = 0; k < WARPS; ++k) sum += part[k][t][e];
     if (t0 + t < T && e < E) z[(long long)(t0 + t) * E + e] = sum;
   }
   __syncthreads();  // the block's own writes of z are visible to all its threads
-  for (int t = t0 + warp; t < min(T, t0 + ROUTER_TOKENS); t += ROUTER_WARPS)
+  for (int t = t0 + warp; t < min(T, t0 + ROUTER_TOKENS); t += WARPS)
     route_token(z, E, bias, E, top, chosen, weights, score, groups, keep, correction, normalise,
                 sum_floor, weight_scale, group_best, t, lane, s_all[warp], s_group[warp],
                 s_plain[warp]);
@@ -856,16 +860,16 @@ FB_API int fb_moe_router(const void* x, long long ldx, const void* w, long long 
              "moe_router: groups, a correction, shares of the sum and a constant on the weights need "
              "scores of their own");
   if (T == 0) return 0;
-  auto go = [&](auto kernel) {
-    fb_launch(kernel, dim3((T + ROUTER_TOKENS - 1) / ROUTER_TOKENS), dim3(ROUTER_WARPS * 32), 0, stream,
+  auto go = [&](auto kernel, int warps) {
+    fb_launch(kernel, dim3((T + ROUTER_TOKENS - 1) / ROUTER_TOKENS), dim3(warps * 32), 0, stream,
               (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, ldw, K, z, bias, E, top, chosen,
               weights, score, groups, keep, correction, normalise, sum_floor, weight_scale,
               group_best, T);
   };
-  if (E <= 8) go(moe_router_kernel<1>);
-  else if (E <= 16) go(moe_router_kernel<2>);
-  else if (E <= 32) go(moe_router_kernel<4>);
-  else go(moe_router_kernel<8>);
+  if (E <= 8) go(moe_router_kernel<1>, ROUTER_WARPS<1>);
+  else if (E <= 16) go(moe_router_kernel<2>, ROUTER_WARPS<2>);
+  else if (E <= 32) go(moe_router_kernel<4>, ROUTER_WARPS<4>);
+  else go(moe_router_kernel<8>, ROUTER_WARPS<8>);
   return fb_check_launch("moe_router");
 }
 
