@@ -265,3 +265,60 @@ def test_embedding_with_sines_and_cosines(ops, W):
     rows = torch.stack([table[i] * 1.5 if 0 <= i < 7 else torch.zeros(W, device=DEV) for i in ids])
     # the sine's own rounding and the sum's: half a place each of numbers up to 1 and 8
     assert float((out - (rows + pe)).abs().max()) <= 2.0 ** -24 + 2.0 ** -21 and torch.equal(out, copy)
+
+
+@pytest.mark.parametrize("T,n,per_head", [(1, 5, 1), (3, 32, 1), (9, 33, 11), (130, 300, 100), (5, 2048, 64)])
+@pytest.mark.parametrize("with_A", [True, False])
+def test_decays(ops, T, n, per_head, with_A):
+    """Channels and tokens at the edges of a block's, from a wider row and in place, against float64: the
+    exponent is off by a few roundings of its own size (up to 30), and so is the decay, relatively."""
+    rnd = lambda *s, seed: torch.randn(*s, generator=torch.Generator().manual_seed(seed)).to(DEV)  # noqa: E731
+    wide, bias, A = rnd(T, n + 3, seed=1) * 2, rnd(n, seed=2), rnd(-(-n // per_head), seed=3) * 0.5
+    z = wide[:, :n].double() + bias.double()
+    steps = torch.empty(T, n, device=DEV) if with_A else None
+    out = torch.empty(T, n, device=DEV)
+    ops.decay_gate(wide[:, :n], per_head, bias, A if with_A else None, out=out, steps=steps)
+    if with_A:
+        soft = torch.nn.functional.softplus(z)
+        want = torch.exp(-torch.exp(A.double()).repeat_interleave(per_head)[:n] * soft)
+        assert float((steps.double() - soft).abs().max()) <= 16 * 2.0 ** -24 * float(soft.max() + 1)
+    else:
+        want = torch.exp(-torch.exp(z))
+    room = 16 * 2.0 ** -24 * (1 + want.clamp_min(1e-30).log().abs())
+    assert bool(((out.double() - want).abs() <= room * want + 1e-37).all())
+    own = wide[:, :n].contiguous()
+    ops.decay_gate(own, per_head, bias, A if with_A else None)
+    assert torch.equal(own, out)
+
+
+@pytest.mark.parametrize("H,G,dim,vdim", [(32, 8, 64, 64), (24, 8, 128, 128), (3, 1, 20, 12), (32, 16, 128, 128),
+                                          (3, 1, 10, 6), (40, 8, 128, 128)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_query_and_key_norms_into_the_cache(ops, H, G, dim, vdim, dtype):
+    """Rows in registers and, for sizes those do not take, by elements; a padding token writes no cache. A
+    norm's sum of n squares is off by at most n * 2^-24 of itself, its root by half of that; eight
+    roundings besides, and bfloat16's half place."""
+    T, nq, nk, nv = 3, H * dim, G * dim, G * vdim
+    rnd = lambda *s, seed: torch.randn(*s, generator=torch.Generator().manual_seed(seed)).to(DEV)  # noqa: E731
+    qkv = rnd(T, nq + nk + nv + 4, seed=1)
+    wq, wk = rnd(nq, seed=2), rnd(nk, seed=3)
+    k, v = torch.full((4, G, 64, dim), 7.0, device=DEV, dtype=dtype), torch.full((4, G, 64, vdim), 7.0, device=DEV, dtype=dtype)
+    as_int = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    table, seqs, pos = as_int([[2, 0], [3, 1]]), [0, -1, 1], [63, 0, 70]
+    q_out = torch.empty(T, nq, device=DEV, dtype=dtype)
+    ops.qk_norm_cache_write(qkv, q_out, wq, wk, 1e-5, as_int(pos), as_int(seqs), table, k, v, H, G, dim, vdim)
+    norm = lambda x, w: x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w.double()  # noqa: E731
+    x = qkv.double()
+    room = (8 + nq / 2) * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0)
+
+    def close(got, want):
+        assert bool(((got.double() - want).abs() <= room * want.abs() + 1e-30).all())
+    close(q_out, norm(x[:, :nq], wq))
+    keys, values = norm(x[:, nq:nq + nk], wk), x[:, nq + nk:nq + nk + nv]
+    seen = torch.zeros(4, 64, dtype=torch.bool, device=DEV)
+    for t in (0, 2):
+        page, r = int(table[seqs[t], pos[t] // 64]), pos[t] % 64
+        close(k[page, :, r].flatten(), keys[t])
+        close(v[page, :, r].flatten(), values[t])
+        seen[page, r] = True
+    assert bool((k.transpose(1, 2)[~seen] == 7).all()) and bool((v.transpose(1, 2)[~seen] == 7).all())
