@@ -54,6 +54,15 @@
 // are masked, and the softmax warps put zeros over the values before the product reads them.
 // 2,048 tokens, 32 heads of 64 + 32 and 64: 58 us against 182 on mma.sync (attention_maps_mma.cu).
 //
+// The form with two maps a head (MAPS): a query head has two query vectors and a key row two key
+// vectors of 64 side by side, over the same values; each (head, map) is a block row of its own, scores
+// may be capped, and the 32-bit results of both maps are combined by a kernel behind it
+// (`combine_maps_kernel`): o = a1 - lambda a2, normalised. The cap, c tanh(x), is a polynomial of odd
+// powers where a warp's |x| stay below a quarter (the next term is below 1e-8 of it), else an
+// exponential and a division: 2,048 tokens, 16 heads of 2 x 64 and 128 91 us with its combination, 229
+// on mma.sync (attention_maps_mma.cu), which holds both maps' sums in registers; 2.49e-3 off float64
+// either way (2.61e-3 and 78 us with a reference maximum that stays behind).
+//
 // Shared memory (96 KB at head size 128) and tensor memory (256 columns) are
 // sized so that two CTAs share an SM: the second CTA's warps fill the gaps that
 // a row's long dependent chain leaves on the schedulers and the tensor pipe.
@@ -103,6 +112,9 @@ struct FaParams {
   long long gate_stride;
   // The form over rows: elements from one head's key (value) to the next in a row.
   int k_head, v_head;
+  // The form with two maps: A counts (head, map) pairs; [T, A, DV], and the cap (0: none).
+  float* maps_out;
+  float softcap, scale;
 };
 constexpr int TABLE_FRONT = 192;  // a query row may lie 127 in front of a page, a key 63 into it
 constexpr int TABLE_BACK = 96;    // a warp's rows span 32, a page 64 keys
@@ -157,7 +169,7 @@ struct FaSmem {
   static_assert(BYTES <= LIMIT || KS > 2, "two CTAs must fit an SM");
 };
 
-template <int KS, int VS, bool ONE, bool ROWS = false>
+template <int KS, int VS, bool ONE, bool ROWS = false, bool MAPS = false>
 __global__ void __launch_bounds__(THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                        const __grid_constant__ CUtensorMap map_k,
@@ -292,8 +304,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         mbar_expect_tx(&k_full[s], Smem::K_BYTES);
 #pragma unroll
         for (int sb = 0; sb < KS; ++sb)
-          tma_load_3d(sK + s * Smem::K_BYTES + sb * KV_SUB, &map_k, &k_full[s], sb * 64,
-                      ONE ? 0 : kvh * FB_PAGE, ONE ? page * p.Kh + kvh : page);
+          tma_load_3d(sK + s * Smem::K_BYTES + sb * KV_SUB, &map_k, &k_full[s],
+                      MAPS ? (head & 1) * 64 : sb * 64, ONE ? 0 : kvh * FB_PAGE, ONE ? page * p.Kh + kvh : page);
         if (ONE) continue;
         if (!mbar_wait(&v_empty[s], parity, abort_flag, 10, j)) break;
         mbar_expect_tx(&v_full[s], Smem::V_BYTES);
@@ -354,7 +366,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
     const int qpos = pos0 + row;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     float m_ref = -INFINITY, l = 0.f;
-    if (p.sink_logits != nullptr) { m_ref = p.sink_logits[head] * LOG2E; l = 1.f; }
+    if (p.sink_logits != nullptr) { m_ref = p.sink_logits[MAPS ? head >> 1 : head] * LOG2E; l = 1.f; }
     bool ok = true;
     fb_pdl_wait();
     // ONE: a page's key factors go to the warp's own copy, read a page ahead
@@ -433,7 +445,31 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
           }
         }
       }
-      const float to_log2 = ONE ? 1.0f : p.scale_log2;
+      if (MAPS && p.softcap > 0.f) {  // to cap * tanh(score * scale / cap), in powers of two
+        const float in = p.scale / p.softcap, to = p.softcap * LOG2E;
+        float far = 0.f;
+#pragma unroll
+        for (int e = 0; e < FB_PAGE; ++e) {
+          sc[e] *= in;
+          far = fmaxf(far, fabsf(sc[e]));
+        }
+        if (__any_sync(0xffffffffu, !(far <= 0.25f))) {
+#pragma unroll
+          for (int e = 0; e < FB_PAGE; ++e)
+            sc[e] = to * (1.0f - __fdividef(2.0f, fast_exp2(2.0f * LOG2E * sc[e]) + 1.0f));
+        } else {
+#pragma unroll
+          for (int e = 0; e < FB_PAGE; ++e) {
+            const float x2 = sc[e] * sc[e];
+            float t = fmaf(x2, 62.0f / 2835.0f, -17.0f / 315.0f);
+            t = fmaf(x2, t, 2.0f / 15.0f);
+            t = fmaf(x2, t, -1.0f / 3.0f);
+            const float y = sc[e] * to;
+            sc[e] = fmaf(y * x2, t, y);
+          }
+        }
+      }
+      const float to_log2 = ONE || (MAPS && p.softcap > 0.f) ? 1.0f : p.scale_log2;
       const bool diagonal = key0 + FB_PAGE - 1 > pos0 + quarter * 32;  // some key may be masked
       if (diagonal) {
 #pragma unroll
@@ -459,11 +495,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         mx4[3] = fmaxf(mx4[3], sc[e + 3]);
       }
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * to_log2;
-      // (also the first page: m_ref = -inf). ROWS moves the reference with every new maximum, so
+      // (also the first page: m_ref = -inf). ROWS and MAPS move the reference with every new maximum, so
       // that a row's largest probability is one, which bfloat16 holds: as close to float64 as the
       // mma.sync kernel (2,048 tokens, 32 heads of 64 + 32 and 64: 1.99e-3 against 2.01e-3, 58 us
       // against 182; a reference that stays behind 2.07e-3, 52 us).
-      const bool grow = mx > m_ref + (ROWS ? 0.f : RESCALE_STEP);
+      const bool grow = mx > m_ref + (ROWS || MAPS ? 0.f : RESCALE_STEP);
       if (__any_sync(0xffffffffu, grow)) {
         const float corr = grow ? exp2f(m_ref - mx) : 1.0f;  // 0 on the row's first page
         if (j > 0) {
@@ -507,7 +543,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         const float p1 = fast_exp2(sc[2 * c + 1]);
         const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
         packed[c] = *reinterpret_cast<const uint32_t*>(&h);
-        if (ROWS) {
+        if (ROWS || MAPS) {
           // the sum of what the product takes: part of the rounding cancels in the quotient
           const float2 r = __bfloat1622float2(h);
           sum4[c & 1] += r.x;
@@ -567,7 +603,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
             r[e] = __float_as_uint(__fdividef(__uint_as_float(r[e]), 1.0f + __expf(-gate[e])));
           ask_gate(c + 32);
         }
-        if (row < rows_valid) {
+        if (MAPS) {
+          float* to = p.maps_out + ((long long)(tok0 + row0 + row) * p.A + head) * p.DV + c;
+#pragma unroll
+          for (int e = 0; e < 32; e += 4)
+            if (row < rows_valid && c + e < p.DV)
+              *reinterpret_cast<float4*>(to + e) =
+                  make_float4(__uint_as_float(r[e]) * inv, __uint_as_float(r[e + 1]) * inv,
+                              __uint_as_float(r[e + 2]) * inv, __uint_as_float(r[e + 3]) * inv);
+        } else if (row < rows_valid) {
 #pragma unroll
           for (int e = 0; e < 32; e += 8) {
             if (c + e >= p.DV) break;  // (whole pieces: DV is a multiple of 8)
@@ -597,6 +641,35 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
   }
 }
 
+// o = a1 - lambda a2;  out = o / sqrt(mean(o^2) + eps) * scale: a warp a (token, head), a lane pieces of
+// four. Bound by its bytes.
+__global__ void __launch_bounds__(256)
+combine_maps_kernel(const float* maps, __nv_bfloat16* out, long long out_stride, long long count, int H,
+                    int DV, float lambda, float eps, float scale) {
+  fb_pdl_launch();
+  fb_pdl_wait();
+  const long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (i >= count) return;
+  const int d = (threadIdx.x & 31) * 4;
+  const float* a = maps + i * 2 * DV;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (d < DV) {
+    const float4 x = __ldcg(reinterpret_cast<const float4*>(a + d));
+    const float4 y = __ldcg(reinterpret_cast<const float4*>(a + DV + d));
+    o = make_float4(fmaf(-lambda, y.x, x.x), fmaf(-lambda, y.y, x.y), fmaf(-lambda, y.z, x.z),
+                    fmaf(-lambda, y.w, x.w));
+  }
+  const float ss = fb_warp_sum((o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w));
+  const float r = 1.0f / sqrtf(ss / (float)DV + eps) * scale;
+  if (d < DV) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * r, o.y * r), hi = __floats2bfloat162_rn(o.z * r, o.w * r);
+    uint2 raw;
+    raw.x = *reinterpret_cast<const uint32_t*>(&lo);
+    raw.y = *reinterpret_cast<const uint32_t*>(&hi);
+    *reinterpret_cast<uint2*>(out + i / H * out_stride + i % H * DV + d) = raw;
+  }
+}
+
 // ------------------------------------------------------------- host: tensor maps
 // bf16 tensor of rank 2 or 3, innermost dimension contiguous, 128-byte swizzle.
 int make_map(CUtensorMap* map, const void* ptr, int rank, const long long* dims,
@@ -614,7 +687,7 @@ int make_map(CUtensorMap* map, const void* ptr, int rank, const long long* dims,
   return 0;
 }
 
-template <int KS, int VS, bool ONE = false, bool ROWS = false>
+template <int KS, int VS, bool ONE = false, bool ROWS = false, bool MAPS = false>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
            const CUtensorMap& shared, const FaParams& p, int q_blocks, cudaStream_t stream) {
   using Smem = FaSmem<KS, VS, ONE>;
@@ -624,12 +697,12 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
     bytes = Smem::USED + p.table_pitch * 4;
   static bool configured[64] = {};
   if (fb_first_use_on_device(configured)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<KS, VS, ONE, ROWS>,
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<KS, VS, ONE, ROWS, MAPS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          ONE ? Smem::LIMIT : Smem::BYTES);
     if (e != cudaSuccess) return fb_fail(2, "attention_tc: %s", cudaGetErrorString(e));
   }
-  fb_launch(attn_prefill_tc_kernel<KS, VS, ONE, ROWS>, dim3(p.A, q_blocks), dim3(THREADS), bytes,
+  fb_launch(attn_prefill_tc_kernel<KS, VS, ONE, ROWS, MAPS>, dim3(p.A, q_blocks), dim3(THREADS), bytes,
             stream, mq, mk, mv, shared, p);
   return fb_check_launch("attention_prefill_tc");
 }
@@ -734,6 +807,59 @@ FB_API int fb_attention_prefill_rows(const void* q, long long q_stride, int T, v
                                 : launch<2, 2, false, true>(mq, mk, mv, ms, p, q_blocks, stream);
   return DV <= 64 ? launch<3, 1, false, true>(mq, mk, mv, ms, p, q_blocks, stream)
                   : launch<3, 2, false, true>(mq, mk, mv, ms, p, q_blocks, stream);
+}
+
+// The form with two maps a head (see the file's notes): q [T, H * 2 * 64] rows, keys [n_pages, G, 64,
+// 2 * 64], values [n_pages, G, 64, DV], `maps` float32 [T, H, 2, DV] between the two kernels.
+FB_API int fb_attention_prefill_maps(const void* q, long long q_stride, int T, float* maps, void* out,
+                                     long long out_stride, const int* cu_tokens, const int* kv_lens,
+                                     const int* page_table, int max_pages, const void* k_cache,
+                                     const void* v_cache, long long k_page, long long k_head,
+                                     long long v_page, long long v_head, int n_pages, int n_seqs,
+                                     int q_blocks, int H, int G, int DV, float scale, float softcap,
+                                     const float* sink_logits, float lambda, float eps,
+                                     float post_scale, cudaStream_t stream) {
+  constexpr int D = 64;
+  FB_REQUIRE((DV == 64 || DV == 128) && n_seqs > 0 && H > 0 && G > 0 && H % G == 0 && T > 0 && n_pages > 0 &&
+                 softcap >= 0.f && scale > 0.f,
+             "attention_maps_tc: %d heads over %d with values of %d are not built", H, G, DV);
+  FB_REQUIRE(k_head == (long long)FB_PAGE * 2 * D && v_head == (long long)FB_PAGE * DV,
+             "attention_maps_tc: the heads of a page must be contiguous");
+  FB_REQUIRE(q_stride % 8 == 0 && out_stride % 4 == 0 && k_page % 8 == 0 && v_page % 8 == 0 &&
+                 ((uintptr_t)q % 16) == 0 && ((uintptr_t)out % 8) == 0 && ((uintptr_t)maps % 16) == 0 &&
+                 ((uintptr_t)k_cache % 16) == 0 && ((uintptr_t)v_cache % 16) == 0,
+             "attention_maps_tc: pointers and strides must keep 16-byte alignment");
+  if (q_blocks <= 0) return 0;
+  bind_status_mirror(stream);
+  CUtensorMap mq, mk, mv;
+  {
+    const long long dims[2] = {(long long)H * 2 * D, T}, strides[1] = {q_stride};
+    const int box[2] = {64, BQ};
+    int rc = make_map(&mq, q, 2, dims, strides, box);
+    if (rc) return rc;
+  }
+  {
+    const int box[3] = {64, FB_PAGE, 1};
+    const long long kdims[3] = {2 * D, (long long)G * FB_PAGE, n_pages}, kstrides[2] = {2 * D, k_page};
+    int rc = make_map(&mk, k_cache, 3, kdims, kstrides, box);
+    if (rc) return rc;
+    const long long vdims[3] = {DV, (long long)G * FB_PAGE, n_pages}, vstrides[2] = {DV, v_page};
+    rc = make_map(&mv, v_cache, 3, vdims, vstrides, box);
+    if (rc) return rc;
+  }
+  FaParams p{};
+  p.cu_tokens = cu_tokens; p.kv_lens = kv_lens; p.page_table = page_table;
+  p.max_pages = max_pages; p.n_seqs = n_seqs; p.A = 2 * H; p.Kh = G;
+  p.D = D; p.DV = DV; p.maps_out = maps;
+  p.scale_log2 = scale * LOG2E; p.scale = scale; p.softcap = softcap;
+  p.sink_logits = sink_logits;
+  const int rc = DV == 64 ? launch<1, 1, false, false, true>(mq, mk, mv, mk, p, q_blocks, stream)
+                          : launch<1, 2, false, false, true>(mq, mk, mv, mk, p, q_blocks, stream);
+  if (rc) return rc;
+  const long long count = (long long)T * H;
+  fb_launch(combine_maps_kernel, dim3((unsigned)((count + 7) / 8)), dim3(256), 0, stream, maps,
+            (__nv_bfloat16*)out, out_stride, count, H, DV, lambda, eps, post_scale);
+  return fb_check_launch("combine_maps");
 }
 
 // The form with shared rows (see the file's notes): `rows` are one cache entry's

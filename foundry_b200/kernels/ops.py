@@ -162,6 +162,10 @@ _SIGNATURES = {
                             c_void_p, c_void_p],
     "fb_attention_sink_merge": [c_void_p, c_void_p, c_ll, c_int, c_void_p, c_int, c_int, c_int,
                                 c_int, c_void_p, c_void_p],
+    "fb_attention_prefill_maps": [c_void_p, c_ll, c_int, c_void_p, c_void_p, c_ll, c_void_p, c_void_p,
+                                  c_void_p, c_int, c_void_p, c_void_p, c_ll, c_ll, c_ll, c_ll, c_int,
+                                  c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_float,
+                                  c_float, c_float, c_void_p],
     "fb_attention_maps": [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_int,
                           c_void_p, c_void_p, c_void_p, c_ll, c_ll, c_ll, c_ll, c_ll, c_ll, c_ll,
                           c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
@@ -2610,11 +2614,66 @@ def attention_folded(ctx, q: torch.Tensor, out: torch.Tensor, page_table, cache:
     return out
 
 
+MAPS_WORKSPACE = 1 << 27  # floats of both maps' results at most (a step of more keeps mma.sync)
+
+
+def _maps_workspace(floats: int, device) -> Optional[torch.Tensor]:
+    """Memory for both maps' results, or None where there is too little."""
+    if floats > MAPS_WORKSPACE:
+        return None
+    try:
+        return torch.empty(floats, dtype=torch.float32, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
+def _tc_maps_blocks(ctx, q, out, k_cache, v_cache, G: int, dim: int, vdim: int, maps: int,
+                    scale: float) -> int:
+    """128-row query blocks of a step that the tcgen05 kernel with two maps takes, else 0: two maps of
+    64, whole pages of heads side by side, 16-byte pieces; some sequence brings 64 tokens or more and
+    all of them 128 on average, which is a block of it (16 heads of 2 x 64 and 128: 8 of 100 tokens
+    16.2 us against 15.3 on mma.sync, 16 of 64 19.9 against 11.0; 400 19.2 against 35.7)."""
+    if not PREFILL_TC or maps != 2 or dim != 64 or vdim not in (64, 128) or scale <= 0:
+        return 0
+    if k_cache.stride(1) != PAGE * 2 * dim or v_cache.stride(1) != PAGE * vdim:
+        return 0
+    for t in (q, out, k_cache, v_cache):
+        if t.data_ptr() % 16 or any(n % 8 for n in t.stride()[:-1]):
+            return 0
+    if q.stride(0) < q.shape[1] or out.stride(0) < out.shape[1] \
+            or k_cache.stride(0) < G * k_cache.stride(1) or v_cache.stride(0) < G * v_cache.stride(1):
+        return 0
+    tokens, seqs = _padded_tokens(q.shape[0]), _padded(ctx.n_seqs, 1)
+    if tokens < 128 * seqs:
+        return 0
+    if ctx.cu_tokens_host is None:  # a replayed step: bounds that its bucket gives
+        return (ctx.query_blocks_bound + 1) // 2 + ctx.n_seqs if ctx.long_queries else 0
+    lens = [b - a for a, b in zip(ctx.cu_tokens_host, ctx.cu_tokens_host[1:])]
+    return sum((n + 127) // 128 for n in lens) if max(lens) >= 64 else 0
+
+
 def attention_maps_paged(ctx, q, out, page_table, k_cache, v_cache, H: int, G: int, dim: int,
                          vdim: int, maps: int, scale: float, softcap: float, sink_logits,
                          combine) -> torch.Tensor:
-    """The tensor-core prompt kernel over the paged cache (key rows of maps * dim)."""
+    """The tensor-core prompt kernel over the paged cache (key rows of maps * dim); where it fits, the
+    tcgen05 kernel in its form with two maps (csrc/attention_tcgen05.cu)."""
     lam, post_eps, post_scale = combine if combine is not None else (0.0, 0.0, 1.0)
+    blocks128 = _tc_maps_blocks(ctx, q, out, k_cache, v_cache, G, dim, vdim, maps, scale)
+    if blocks128:
+        both = _maps_workspace(q.shape[0] * H * 2 * vdim, q.device)
+        if both is not None:
+            _call("fb_attention_prefill_maps", _dev(q, "q", torch.bfloat16, contiguous=False),
+                  _rows(q, "q"), q.shape[0], both.data_ptr(),
+                  _dev(out, "out", torch.bfloat16, contiguous=False), _rows(out, "out"),
+                  _dev(ctx.cu_tokens, "cu_tokens", torch.int32), _dev(ctx.kv_lens, "kv_lens", torch.int32),
+                  _dev(page_table, "page_table", torch.int32), page_table.shape[1], k_cache.data_ptr(),
+                  v_cache.data_ptr(), k_cache.stride(0), k_cache.stride(1), v_cache.stride(0),
+                  v_cache.stride(1), k_cache.shape[0], ctx.n_seqs, blocks128, H, G, vdim, float(scale),
+                  float(softcap),
+                  0 if sink_logits is None else _dev(sink_logits, "sink_logits", torch.float32),
+                  float(lam), float(post_eps), float(post_scale), _stream())
+            add_launches(1)  # two kernels
+            return out
     _call("fb_attention_maps", _dev(q, "q", torch.bfloat16, contiguous=False), _rows(q, "q"),
           _dev(out, "out", torch.bfloat16, contiguous=False), _rows(out, "out"),
           _dev(ctx.cu_tokens, "cu_tokens", torch.int32), _dev(ctx.kv_lens, "kv_lens", torch.int32),
