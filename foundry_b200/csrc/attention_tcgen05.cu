@@ -63,6 +63,10 @@
 // on mma.sync (attention_maps_mma.cu), which holds both maps' sums in registers; 2.49e-3 off float64
 // either way (2.61e-3 and 78 us with a reference maximum that stays behind).
 //
+// The masked form (MASK): a window that keeps the first tokens, a bias that falls with distance by a
+// slope a head, and a sink whose score is 0. 1,500 tokens, 24 heads over 8 of 128, a window of 1,024 that
+// keeps 4: 32 us, 87 on mma.sync (attention_mma.cu); 1.89e-3 off float64, 1.92e-3 there.
+//
 // Shared memory (96 KB at head size 128) and tensor memory (256 columns) are
 // sized so that two CTAs share an SM: the second CTA's warps fill the gaps that
 // a row's long dependent chain leaves on the schedulers and the tensor pipe.
@@ -115,6 +119,10 @@ struct FaParams {
   // The form with two maps: A counts (head, map) pairs; [T, A, DV], and the cap (0: none).
   float* maps_out;
   float softcap, scale;
+  // The masked form: head h's scores lose 2^(-steep (h + 1) / A) a token of distance (0: nothing);
+  // sink: the sum has one more term exp(0).
+  float steep;
+  int sink;
 };
 constexpr int TABLE_FRONT = 192;  // a query row may lie 127 in front of a page, a key 63 into it
 constexpr int TABLE_BACK = 96;    // a warp's rows span 32, a page 64 keys
@@ -169,13 +177,14 @@ struct FaSmem {
   static_assert(BYTES <= LIMIT || KS > 2, "two CTAs must fit an SM");
 };
 
-template <int KS, int VS, bool ONE, bool ROWS = false, bool MAPS = false>
+template <int KS, int VS, bool ONE, bool ROWS = false, bool MAPS = false, bool MASK = false>
 __global__ void __launch_bounds__(THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                        const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v,
                        const __grid_constant__ CUtensorMap map_shared, const FaParams p) {
   using Smem = FaSmem<KS, VS, ONE>;
+  constexpr bool KEEP = ONE || MASK;  // the window may keep the first tokens
   constexpr int RING = Smem::RING;
   constexpr int Q_SUB = BQ * 128;              // bytes of one query sub-tile
   constexpr int KV_SUB = FB_PAGE * 128;        // bytes of one K or V sub-tile
@@ -261,10 +270,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
   // the pages the block walks: those of the kept first tokens that lie in front of the
   // window's, then from the first row's window on; the j-th of them is page_at(j)
   const int first_page = p.window > 0 ? max(0, pos0 - p.window + 1) / FB_PAGE : 0;
-  const int kept = ONE ? min((p.keep_first + FB_PAGE - 1) / FB_PAGE, first_page) : 0;
+  const int kept = KEEP ? min((p.keep_first + FB_PAGE - 1) / FB_PAGE, first_page) : 0;
   const int n_pages = kept + (pos0 + rows_valid - 1) / FB_PAGE + 1 - first_page;
   const int* pages = p.page_table + (size_t)seq * p.max_pages;
-  auto page_at = [&](int j) { return ONE && j < kept ? j : first_page + j - kept; };
+  auto page_at = [&](int j) { return KEEP && j < kept ? j : first_page + j - kept; };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -367,6 +376,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     float m_ref = -INFINITY, l = 0.f;
     if (p.sink_logits != nullptr) { m_ref = p.sink_logits[MAPS ? head >> 1 : head] * LOG2E; l = 1.f; }
+    else if (MASK && p.sink) { m_ref = 0.f; l = 1.f; }
+    const float slope = MASK && p.steep > 0.f ? exp2f(-p.steep * (float)(head + 1) / (float)p.A) * LOG2E : 0.f;
     bool ok = true;
     fb_pdl_wait();
     // ONE: a page's key factors go to the warp's own copy, read a page ahead
@@ -469,7 +480,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
           }
         }
       }
-      const float to_log2 = ONE || (MAPS && p.softcap > 0.f) ? 1.0f : p.scale_log2;
+      if (MASK) {
+        const float near = (float)(key0 - qpos);  // minus the first key's distance
+#pragma unroll
+        for (int e = 0; e < FB_PAGE; ++e) sc[e] = fmaf(slope, near + (float)e, sc[e] * p.scale_log2);
+      }
+      const float to_log2 = KEEP || (MAPS && p.softcap > 0.f) ? 1.0f : p.scale_log2;
       const bool diagonal = key0 + FB_PAGE - 1 > pos0 + quarter * 32;  // some key may be masked
       if (diagonal) {
 #pragma unroll
@@ -479,10 +495,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
       // some key may lie behind some row's window (rows of the warp reach 31 further)
       if (p.window > 0 && key0 <= pos0 + quarter * 32 + 31 - p.window) {
         const int behind = qpos - p.window - key0;  // keys of the page up to this one are behind it
-        const int held = ONE ? p.keep_first - key0 : 0;  // keys of the page in front of this one stay
+        const int held = KEEP ? p.keep_first - key0 : 0;  // keys of the page in front of this one stay
 #pragma unroll
         for (int e = 0; e < FB_PAGE; ++e)
-          if (e <= behind && (!ONE || e >= held)) sc[e] = -INFINITY;
+          if (e <= behind && (!KEEP || e >= held)) sc[e] = -INFINITY;
       }
       // the row maximum of the raw scores, by four independent chains; the scale is
       // positive, so it can be applied to the maximum afterwards
@@ -495,11 +511,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         mx4[3] = fmaxf(mx4[3], sc[e + 3]);
       }
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * to_log2;
-      // (also the first page: m_ref = -inf). ROWS and MAPS move the reference with every new maximum, so
+      // (also the first page: m_ref = -inf). ROWS, MAPS and MASK move the reference with every new maximum, so
       // that a row's largest probability is one, which bfloat16 holds: as close to float64 as the
       // mma.sync kernel (2,048 tokens, 32 heads of 64 + 32 and 64: 1.99e-3 against 2.01e-3, 58 us
       // against 182; a reference that stays behind 2.07e-3, 52 us).
-      const bool grow = mx > m_ref + (ROWS || MAPS ? 0.f : RESCALE_STEP);
+      const bool grow = mx > m_ref + (ROWS || MAPS || MASK ? 0.f : RESCALE_STEP);
       if (__any_sync(0xffffffffu, grow)) {
         const float corr = grow ? exp2f(m_ref - mx) : 1.0f;  // 0 on the row's first page
         if (j > 0) {
@@ -533,7 +549,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
       for (int c = 0; c < 32; ++c) {
         // 2^(s * scale - m_ref): one multiply-add and one ex2; the result is at most 2^8
         // and is rounded to bfloat16 next, so the approximate ex2 costs no accuracy
-        if (ONE) {
+        if (KEEP) {
           add2(sc[2 * c], sc[2 * c + 1], neg_ref);
         } else {
           sc[2 * c] = fmaf(sc[2 * c], to_log2, neg_ref);
@@ -543,7 +559,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
         const float p1 = fast_exp2(sc[2 * c + 1]);
         const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
         packed[c] = *reinterpret_cast<const uint32_t*>(&h);
-        if (ROWS || MAPS) {
+        if (ROWS || MAPS || MASK) {
           // the sum of what the product takes: part of the rounding cancels in the quotient
           const float2 r = __bfloat1622float2(h);
           sum4[c & 1] += r.x;
@@ -687,7 +703,7 @@ int make_map(CUtensorMap* map, const void* ptr, int rank, const long long* dims,
   return 0;
 }
 
-template <int KS, int VS, bool ONE = false, bool ROWS = false, bool MAPS = false>
+template <int KS, int VS, bool ONE = false, bool ROWS = false, bool MAPS = false, bool MASK = false>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
            const CUtensorMap& shared, const FaParams& p, int q_blocks, cudaStream_t stream) {
   using Smem = FaSmem<KS, VS, ONE>;
@@ -697,12 +713,12 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
     bytes = Smem::USED + p.table_pitch * 4;
   static bool configured[64] = {};
   if (fb_first_use_on_device(configured)) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<KS, VS, ONE, ROWS, MAPS>,
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<KS, VS, ONE, ROWS, MAPS, MASK>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          ONE ? Smem::LIMIT : Smem::BYTES);
     if (e != cudaSuccess) return fb_fail(2, "attention_tc: %s", cudaGetErrorString(e));
   }
-  fb_launch(attn_prefill_tc_kernel<KS, VS, ONE, ROWS, MAPS>, dim3(p.A, q_blocks), dim3(THREADS), bytes,
+  fb_launch(attn_prefill_tc_kernel<KS, VS, ONE, ROWS, MAPS, MASK>, dim3(p.A, q_blocks), dim3(THREADS), bytes,
             stream, mq, mk, mv, shared, p);
   return fb_check_launch("attention_prefill_tc");
 }
@@ -714,13 +730,18 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
 // [n_pages, Kh, 64, D] with strides (k_page, 64*D, D, 1), and with DV and v_page for the
 // values. `q_blocks` bounds the number of 128-row query blocks: the sum over sequences of
 // ceil(q_len / 128). D and DV: multiples of 8 up to 128. `window`: see the file's notes.
-FB_API int fb_attention_prefill_tc(const void* q, long long q_stride, int T, void* out,
-                                   long long out_stride, const int* cu_tokens, const int* kv_lens,
-                                   const int* page_table, int max_pages, const void* k_cache,
-                                   const void* v_cache, long long k_page, long long k_head,
-                                   long long v_page, long long v_head, int n_pages, int n_seqs,
-                                   int q_blocks, int A, int Kh, int D, int DV, int window,
-                                   float scale, const float* sink_logits, cudaStream_t stream) {
+namespace {
+struct MaskRule {
+  bool on;
+  int keep_first, sink;
+  float steep;
+};
+int prefill_tc(const void* q, long long q_stride, int T, void* out, long long out_stride,
+               const int* cu_tokens, const int* kv_lens, const int* page_table, int max_pages,
+               const void* k_cache, const void* v_cache, long long k_page, long long k_head,
+               long long v_page, long long v_head, int n_pages, int n_seqs, int q_blocks, int A, int Kh,
+               int D, int DV, int window, float scale, const float* sink_logits, const MaskRule& mask,
+               cudaStream_t stream) {
   FB_REQUIRE(D > 0 && DV > 0 && D <= 128 && DV <= 128 && D % 8 == 0 && DV % 8 == 0 && window >= 0,
              "attention_tc: head sizes %d and %d are not built (multiples of 8 up to 128)", D, DV);
   FB_REQUIRE(n_seqs > 0 && A > 0 && Kh > 0 && A % Kh == 0 && T > 0 && n_pages > 0,
@@ -756,10 +777,48 @@ FB_API int fb_attention_prefill_tc(const void* q, long long q_stride, int T, voi
   p.D = D; p.DV = DV; p.window = window;
   p.scale_log2 = scale * LOG2E;
   p.sink_logits = sink_logits;
+  if (mask.on) {
+    p.keep_first = window > 0 ? mask.keep_first : 0;
+    p.steep = mask.steep;
+    p.sink = mask.sink;
+    return D <= 64 ? launch<1, 1, false, false, false, true>(mq, mk, mv, mk, p, q_blocks, stream)
+                   : launch<2, 2, false, false, false, true>(mq, mk, mv, mk, p, q_blocks, stream);
+  }
   if (D <= 64) return DV <= 64 ? launch<1, 1>(mq, mk, mv, mk, p, q_blocks, stream)
                                : launch<1, 2>(mq, mk, mv, mk, p, q_blocks, stream);
   return DV <= 64 ? launch<2, 1>(mq, mk, mv, mk, p, q_blocks, stream)
                   : launch<2, 2>(mq, mk, mv, mk, p, q_blocks, stream);
+}
+}  // namespace
+
+FB_API int fb_attention_prefill_tc(const void* q, long long q_stride, int T, void* out,
+                                   long long out_stride, const int* cu_tokens, const int* kv_lens,
+                                   const int* page_table, int max_pages, const void* k_cache,
+                                   const void* v_cache, long long k_page, long long k_head,
+                                   long long v_page, long long v_head, int n_pages, int n_seqs,
+                                   int q_blocks, int A, int Kh, int D, int DV, int window,
+                                   float scale, const float* sink_logits, cudaStream_t stream) {
+  return prefill_tc(q, q_stride, T, out, out_stride, cu_tokens, kv_lens, page_table, max_pages, k_cache,
+                    v_cache, k_page, k_head, v_page, v_head, n_pages, n_seqs, q_blocks, A, Kh, D, DV,
+                    window, scale, sink_logits, MaskRule{false, 0, 0, 0.f}, stream);
+}
+
+// The masked form (see the file's notes): heads of 64 or 128, `sink` without `sink_logits` a term
+// exp(0), with them exp(sink_logits[head]).
+FB_API int fb_attention_prefill_mask_tc(const void* q, long long q_stride, int T, void* out,
+                                        long long out_stride, const int* cu_tokens, const int* kv_lens,
+                                        const int* page_table, int max_pages, const void* k_cache,
+                                        const void* v_cache, long long page_stride,
+                                        long long head_stride, int n_pages, int n_seqs, int q_blocks,
+                                        int A, int Kh, int D, int window, int keep_first, int sink,
+                                        float steep, float scale, const float* sink_logits,
+                                        cudaStream_t stream) {
+  FB_REQUIRE((D == 64 || D == 128) && keep_first >= 0 && steep >= 0.f && scale > 0.f,
+             "attention_mask_tc: heads of %d, %d kept tokens", D, keep_first);
+  return prefill_tc(q, q_stride, T, out, out_stride, cu_tokens, kv_lens, page_table, max_pages, k_cache,
+                    v_cache, page_stride, head_stride, page_stride, head_stride, n_pages, n_seqs,
+                    q_blocks, A, Kh, D, D, window, scale, sink ? sink_logits : nullptr,
+                    MaskRule{true, keep_first, sink, steep}, stream);
 }
 
 // The form over rows (see the file's notes): q [T, A * (K1 + K2)] rows; a head's K1 key elements at

@@ -330,9 +330,13 @@ embed_sinusoid_kernel(const T* __restrict__ table, const int* __restrict__ ids,
   double sine, cosine;
   sincos((double)positions[t] * f, &sine, &cosine);
   const size_t at = (size_t)t * W + 2 * i;
-  const float2 v = make_float2(e0 + (float)sine, e1 + (float)cosine);
-  *reinterpret_cast<float2*>(out + at) = v;
-  if (copy != nullptr) *reinterpret_cast<float2*>(copy + at) = v;
+  const float v0 = e0 + (float)sine, v1 = e1 + (float)cosine;
+  out[at] = v0;
+  out[at + 1] = v1;
+  if (copy != nullptr) {
+    copy[at] = v0;
+    copy[at + 1] = v1;
+  }
 }
 
 // out[t, :W] = resid[t, :] (+ nothing), out[t, W:] = x0[t, :], rounded to the
@@ -418,8 +422,6 @@ FB_API int fb_embed_sinusoid(const void* table, int table_dtype, const int* ids,
   FB_REQUIRE(T >= 0 && W > 0 && W % 2 == 0 && V > 0, "embed_sinusoid: bad sizes T=%d W=%d V=%d", T,
              W, V);
   if (T == 0) return 0;
-  FB_REQUIRE(((uintptr_t)out % 8) == 0 && ((uintptr_t)copy % 8) == 0,
-             "embed_sinusoid: rows are not on 8-byte boundaries");
   FB_DISPATCH_DTYPE(table_dtype, E, (fb_launch(embed_sinusoid_kernel<E>,
       dim3(T, (W / 2 + 127) / 128), dim3(128), 0, stream, (const E*)table, ids, positions, freq, scale, out, copy, W, V)));
   return fb_check_launch("embed_sinusoid");

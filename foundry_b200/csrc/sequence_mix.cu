@@ -369,24 +369,26 @@ decay_gate_kernel(const float* in, long long ld, float* out, int T, int n, int p
                   const float* __restrict__ A, const float* __restrict__ bias, int mode, float* steps) {
   fb_pdl_launch();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t0 = (blockIdx.y * blockDim.y + threadIdx.y) * DECAY_RUN;
   const bool mine = c < n;
   const float shift = mine ? bias[c] : 0.f, rate = mine && mode == 0 ? expf(A[c / per_head]) : 0.f;
   fb_pdl_wait();
   if (!mine) return;
-  float v[DECAY_RUN];
+  for (int t0 = (blockIdx.y * blockDim.y + threadIdx.y) * DECAY_RUN; t0 < T;
+       t0 += gridDim.y * blockDim.y * DECAY_RUN) {
+    float v[DECAY_RUN];
 #pragma unroll
-  for (int i = 0; i < DECAY_RUN; ++i) v[i] = t0 + i < T ? __ldcg(in + (long long)(t0 + i) * ld + c) + shift : 0.f;
+    for (int i = 0; i < DECAY_RUN; ++i) v[i] = t0 + i < T ? __ldcg(in + (long long)(t0 + i) * ld + c) + shift : 0.f;
 #pragma unroll
-  for (int i = 0; i < DECAY_RUN; ++i) {
-    if (t0 + i >= T) break;
-    const long long at = (long long)(t0 + i) * n + c;
-    if (mode == 0) {
-      const float sp = softplusf_(v[i]);
-      out[at] = expf(-rate * sp);
-      if (steps != nullptr) steps[at] = sp;
-    } else {
-      out[at] = expf(-expf(v[i]));
+    for (int i = 0; i < DECAY_RUN; ++i) {
+      if (t0 + i >= T) break;
+      const long long at = (long long)(t0 + i) * n + c;
+      if (mode == 0) {
+        const float sp = softplusf_(v[i]);
+        out[at] = expf(-rate * sp);
+        if (steps != nullptr) steps[at] = sp;
+      } else {
+        out[at] = expf(-expf(v[i]));
+      }
     }
   }
 }
@@ -1345,8 +1347,8 @@ FB_API int fb_decay_gate(const float* x, long long ld, float* out, int T, int n,
   int wide = 32;  // channels of a block; its other threads take other tokens
   while (wide < 256 && wide < n) wide *= 2;
   const int tokens = 256 / wide * DECAY_RUN;
-  const dim3 grid((n + wide - 1) / wide, (T + tokens - 1) / tokens);
-  FB_REQUIRE(grid.y <= 65535, "decay_gate: T=%d exceeds the grid limit", T);
+  const int rows = (T + tokens - 1) / tokens;
+  const dim3 grid((n + wide - 1) / wide, rows < 65535 ? rows : 65535);
   fb_launch(decay_gate_kernel, grid, dim3(wide, 256 / wide), 0, stream, x, ld, out, T, n, per_head, A,
             bias, mode, steps);
   return fb_check_launch("decay_gate");

@@ -162,6 +162,10 @@ _SIGNATURES = {
                             c_void_p, c_void_p],
     "fb_attention_sink_merge": [c_void_p, c_void_p, c_ll, c_int, c_void_p, c_int, c_int, c_int,
                                 c_int, c_void_p, c_void_p],
+    "fb_attention_prefill_mask_tc": [c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_void_p,
+                                     c_int, c_void_p, c_void_p, c_ll, c_ll, c_int, c_int, c_int, c_int,
+                                     c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p,
+                                     c_void_p],
     "fb_attention_prefill_maps": [c_void_p, c_ll, c_int, c_void_p, c_void_p, c_ll, c_void_p, c_void_p,
                                   c_void_p, c_int, c_void_p, c_void_p, c_ll, c_ll, c_ll, c_ll, c_int,
                                   c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_float,
@@ -2288,6 +2292,17 @@ def attention_sink(ctx, q: torch.Tensor, out: torch.Tensor, page_table, k_cache,
             and dim == vdim
             and dim in FAST_HEAD_DIMS and H // G <= 16 and k_cache.stride() == v_cache.stride()
             and _tc_attention_ok(q, out)):
+        blocks128 = _tc_mask_blocks(ctx, q, out, k_cache, v_cache, G, dim, scale, steep)
+        if blocks128:
+            _call("fb_attention_prefill_mask_tc", _dev(q, "q", contiguous=False), _rows(q, "q"), T,
+                  _dev(out, "out", contiguous=False), _rows(out, "out"),
+                  _dev(ctx.cu_tokens, "cu_tokens", torch.int32), _dev(ctx.kv_lens, "kv_lens", torch.int32),
+                  _dev(page_table, "page_table", torch.int32), page_table.shape[1], k_cache.data_ptr(),
+                  v_cache.data_ptr(), k_cache.stride(0), k_cache.stride(1), k_cache.shape[0], ctx.n_seqs,
+                  blocks128, H, G, dim, window, keep_first, 1 if sink or sink_logits is not None else 0,
+                  float(steep), float(scale),
+                  0 if sink_logits is None else _dev(sink_logits, "sink_logits", torch.float32), _stream())
+            return out
         q_blocks = ctx.query_blocks_bound
         if q_blocks is None:
             cu = ctx.cu_tokens_host
@@ -2627,15 +2642,10 @@ def _maps_workspace(floats: int, device) -> Optional[torch.Tensor]:
         return None
 
 
-def _tc_maps_blocks(ctx, q, out, k_cache, v_cache, G: int, dim: int, vdim: int, maps: int,
-                    scale: float) -> int:
-    """128-row query blocks of a step that the tcgen05 kernel with two maps takes, else 0: two maps of
-    64, whole pages of heads side by side, 16-byte pieces; some sequence brings 64 tokens or more and
-    all of them 128 on average, which is a block of it (16 heads of 2 x 64 and 128: 8 of 100 tokens
-    16.2 us against 15.3 on mma.sync, 16 of 64 19.9 against 11.0; 400 19.2 against 35.7)."""
-    if not PREFILL_TC or maps != 2 or dim != 64 or vdim not in (64, 128) or scale <= 0:
-        return 0
-    if k_cache.stride(1) != PAGE * 2 * dim or v_cache.stride(1) != PAGE * vdim:
+def _tc_paged_blocks(ctx, q, out, k_cache, v_cache, G: int, row: int, vdim: int) -> int:
+    """128-row query blocks of a prompt step over whole pages of heads side by side, in 16-byte pieces,
+    in which some sequence brings 64 tokens or more and all of them 128 on average; else 0."""
+    if k_cache.stride(1) != PAGE * row or v_cache.stride(1) != PAGE * vdim:
         return 0
     for t in (q, out, k_cache, v_cache):
         if t.data_ptr() % 16 or any(n % 8 for n in t.stride()[:-1]):
@@ -2650,6 +2660,26 @@ def _tc_maps_blocks(ctx, q, out, k_cache, v_cache, G: int, dim: int, vdim: int, 
         return (ctx.query_blocks_bound + 1) // 2 + ctx.n_seqs if ctx.long_queries else 0
     lens = [b - a for a, b in zip(ctx.cu_tokens_host, ctx.cu_tokens_host[1:])]
     return sum((n + 127) // 128 for n in lens) if max(lens) >= 64 else 0
+
+
+def _tc_maps_blocks(ctx, q, out, k_cache, v_cache, G: int, dim: int, vdim: int, maps: int,
+                    scale: float) -> int:
+    """Query blocks of a step that the tcgen05 kernel with two maps takes, else 0: two maps of 64. A
+    block is 128 rows (16 heads of 2 x 64 and 128: 8 of 100 tokens 16.2 us against 15.3 on mma.sync, 16
+    of 64 19.9 against 11.0; 400 19.2 against 35.7)."""
+    if not PREFILL_TC or maps != 2 or dim != 64 or vdim not in (64, 128) or scale <= 0:
+        return 0
+    return _tc_paged_blocks(ctx, q, out, k_cache, v_cache, G, maps * dim, vdim)
+
+
+def _tc_mask_blocks(ctx, q, out, k_cache, v_cache, G: int, dim: int, scale: float, steep: float) -> int:
+    """Query blocks of a step that the tcgen05 kernel in its masked form takes, else 0: heads of 64 or
+    128, more than 256 tokens (graph replays, 32 heads over 8 of 64, a window of 1,024: 65 tokens 6.1 us
+    against 5.3 on mma.sync, 130 7.2 against 6.9, 4 of 128 6.8 against 7.4, 2,048 47 against 103)."""
+    if not PREFILL_TC or dim not in TC_HEAD_DIMS or scale <= 0 or steep < 0 \
+            or _padded_tokens(q.shape[0]) <= 256:
+        return 0
+    return _tc_paged_blocks(ctx, q, out, k_cache, v_cache, G, dim, dim)
 
 
 def attention_maps_paged(ctx, q, out, page_table, k_cache, v_cache, H: int, G: int, dim: int,

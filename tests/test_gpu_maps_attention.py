@@ -1,4 +1,4 @@
-"""Prompt attention with two maps a head on tcgen05, at the edges of its 128-row blocks and 64-key
+"""Prompt attention with two maps a head, and with masks, on tcgen05, at the edges of its 128-row blocks and 64-key
 pages, against float64 and beside the mma.sync kernel that it takes the place of."""
 import types
 
@@ -102,3 +102,65 @@ def test_what_the_form_does_not_take_stays(ops):
     assert takes(long, q2, k2[:, :1].expand(-1, 2, -1, -1), v2) == 0  # heads that lie over one another
     shifted = torch.empty(100 * 520 + 8, dtype=torch.bfloat16, device=DEV)[4:100 * 520 + 4].view(100, 520)[:, :512]
     assert takes(long, shifted, k2, v2) == 0  # rows that are not on 16-byte boundaries
+    # the masked form: more than 256 tokens, heads of 64 or 128
+    masked = lambda c, q, k, v, dim=128, steep=8.0: ops._tc_mask_blocks(c, q, q, k, v, 2, dim, 0.1, steep)  # noqa: E731
+    few, q3, k3, v3, _ = make([200], [0], 4, 2, 128)
+    many, q4, k4, v4, _ = make([300], [0], 4, 2, 128)
+    assert masked(few, q3, k3, v3) == 0 and masked(many, q4, k4, v4) == 3
+    assert masked(many, q4, k4, v4, dim=96) == 0 and masked(many, q4, k4, v4, steep=-1.0) == 0
+
+
+def exact_masked(q, k, v, table, lens, starts, H, G, D, scale, window, keep, sink, logits, steep):
+    outs, sizes, t0 = [], [], 0
+    for i, (n, s) in enumerate(zip(lens, starts)):
+        j = torch.arange(s + n, device=DEV)
+        kk, vv = (c[table[i][j // PAGE].long(), :, j % PAGE].double().repeat_interleave(H // G, 1) for c in (k, v))
+        qq = q[t0:t0 + n].double().view(n, H, D)
+        t0 += n
+        back = (s + torch.arange(n, device=DEV))[:, None] - j[None]
+        z = torch.einsum("thd,jhd->htj", qq, kk) * scale
+        if steep:
+            slope = 2.0 ** (-steep * torch.arange(1, H + 1, device=DEV).double() / H)
+            z = z - slope[:, None, None] * back
+        seen = back >= 0
+        if window:
+            seen &= (back < window) | (j[None] < keep)
+        z = z.masked_fill(~seen, -float("inf"))
+        if sink:
+            term = torch.zeros(H, device=DEV).double() if logits is None else logits.double()
+            z = torch.cat([z, term[:, None, None].expand(H, n, 1)], -1)
+        w = torch.softmax(z, -1)[..., :s + n]
+        outs.append(torch.einsum("htj,jhe->the", w, vv).flatten(1))
+        sizes.append(torch.einsum("htj,jhe->the", w, vv.abs()).flatten(1))
+    return torch.cat(outs), torch.cat(sizes)
+
+
+@pytest.mark.parametrize("lens,starts", [([390], [0]), ([300, 65, 70], [0, 0, 0]), ([200, 64], [37, 128]),
+                                         ([300, 1, 90], [0, 500, 63])])
+@pytest.mark.parametrize("H,G,D,window,keep,sink,logits,steep", [
+    (4, 2, 64, 0, 0, 0, False, 8.0), (3, 1, 128, 100, 4, 1, False, 8.0), (4, 4, 64, 64, 0, 1, False, 0.0),
+    (2, 2, 128, 129, 70, 1, True, 2.0), (4, 2, 64, 1, 0, 0, False, 0.0)])
+def test_masked(ops, lens, starts, H, G, D, window, keep, sink, logits, steep):
+    ctx, _, _, _, table = make(lens, starts, H, G, 64)
+    g = torch.Generator().manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV).bfloat16()  # noqa: E731
+    T = sum(lens)
+    q, kv = rnd(T, H * D + 8)[:, :H * D], rnd(table.numel(), 2, G, PAGE, D)
+    k, v = kv[:, 0], kv[:, 1]
+    terms = torch.randn(H, generator=g).to(DEV) if logits else None
+    out, old = (torch.full((T, H * D + 8), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    scale = D ** -0.5
+    assert ops._tc_mask_blocks(ctx, q, out, k, v, G, D, scale, steep) > 0
+    args = dict(window=window, keep_first=keep, sink=bool(sink and not logits), steep=steep, sink_logits=terms)
+    ops.attention_sink(ctx, q, out[:, :H * D], table, k, v, H, G, D, D, scale, **args)
+    ops.PREFILL_TC, before = False, ops.PREFILL_TC
+    try:
+        ops.attention_sink(ctx, q, old[:, :H * D], table, k, v, H, G, D, D, scale, **args)
+    finally:
+        ops.PREFILL_TC = before
+    assert bool((out[:, H * D:] == 7).all()) and ops.gemm_tc_status() == 0
+    want, size = exact_masked(q, k, v, table, lens, starts, H, G, D, scale, window, keep, sink, terms, steep)
+    off, was = (x[:, :H * D].double() - want for x in (out, old))
+    # weights and the result rounded to bfloat16: half a place of each, twice for what else is 32-bit
+    assert bool((off.abs() <= 2.0 ** -8 * size + 2.0 ** -8 * want.abs()).all())
+    assert float(off.norm()) <= 1.05 * float(was.norm()) + 1e-9
