@@ -12,16 +12,16 @@
 //
 // `prepare_kernel` makes W, U0, A and the decayed copies of q and k for every chunk of the prompt
 // side by side; they do not depend on the state. `walk_kernel` goes through the chunks in order,
-// 16 columns of a head's state a block, with the two products that the next chunk waits for, and
-// leaves u and every chunk's S0; `output_kernel` makes all outputs from them side by side. The
+// 16 or 24 columns of a head's state a block, with the two products that the next chunk waits for,
+// and leaves u and every chunk's S0; `output_kernel` makes all outputs from them side by side. The
 // token-by-token scan has 32 dependent steps of two dot products each where a walk has one chunk:
 // 0.35 us a step with heads of 64 x 64, 0.59 with 128 x 128 (latency: a few warps a scheduler in
 // one chain). A step's heads that fill the SMs that way need no chunks (`ops.chunk_scan_unit`).
 // All of it is 32-bit arithmetic on the FMA pipe, reordered.
 //
 // Measured: 2,048 tokens, 32 heads of 64 x 64: 199 us (89, 82 and 35), token by token 709. 1,500
-// tokens, 24 heads of 128 x 128: 355 us (93, 210 and 57) against 892. Outputs made in the walk
-// itself, from the same registers: 217 and 378 us. Error against 64 bits with a decay a channel:
+// tokens, 24 heads of 128 x 128: 301 us (91, 155 and 55) against 892. Outputs made in the walk
+// itself, from the same registers (blocks of 16 columns): 217 for 199 and 378 for 355 us. Error against 64 bits with a decay a channel:
 // outputs 1.29e-7 and 1.37e-7, token by token 1.39e-7 and 1.40e-7; states 1.09e-7 and 1.00e-7 for
 // 1.02e-7 and 0.99e-7 (a chunk's own sum, added to the decayed state last, left that as it was).
 #include "common.cuh"
@@ -29,7 +29,6 @@
 namespace {
 
 constexpr int C = 32, SUB = 16;  // tokens a chunk; tokens whose decays are multiplied out pairwise
-constexpr int COLS = 16;         // columns of the state a walking block owns
 constexpr int MAX_VDIM = 128;
 
 struct ChunkArgs {
@@ -273,7 +272,10 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(ChunkArgs a) {
 // columns and half the channels; then the state, a thread one channel by 4 or 8 columns in
 // registers. Two neighbouring terms of a sum share an instruction (fma.rn.f32x2). The next
 // chunk's matrices arrive by asynchronous copies while this one is multiplied.
-constexpr int WALK_THREADS = 256;
+// COLS: columns of the state a block owns, 16 threads each; the last block of a head may have fewer.
+// The walk takes as long as its slowest SM: 24 heads of 128 x 128 are 192 blocks of 16 columns, two of
+// them on 44 SMs, or 144 of 24, one an SM: 1,500 tokens 155 us, 207 with 16. (1,000 tokens, 40 heads
+// of 64 x 64, all three kernels: 151 us, 170 with 16.)
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ void fma2(f32x2& d, f32x2 x, f32x2 y) {
@@ -302,16 +304,17 @@ __device__ __forceinline__ ulonglong2 lds2(const float* p) {
   return *reinterpret_cast<const ulonglong2*>(p);
 }
 
-template <int D>
+template <int D, int COLS>
 struct Walk {
   static constexpr int P = D + 4, PU = COLS + 4;
   static constexpr int W = 0, K = W + C * P, U = K + C * D, G = U + C * PU, BUFFER = G + D;
   static constexpr int S = 2 * BUFFER, US = S + COLS * P, FLOATS = US + C * PU;  // S by columns
 };
 
-template <int D>
-__global__ void __launch_bounds__(WALK_THREADS, 2) walk_kernel(ChunkArgs a) {
-  using B = Walk<D>;
+template <int D, int COLS>
+__global__ void __launch_bounds__(16 * COLS, COLS > 16 ? 1 : 2) walk_kernel(ChunkArgs a) {
+  constexpr int WALK_THREADS = 16 * COLS;
+  using B = Walk<D, COLS>;
   constexpr int P = B::P, PU = B::PU;
   extern __shared__ __align__(16) float smem[];
   float(*S)[P] = reinterpret_cast<float(*)[P]>(smem + B::S);
@@ -346,7 +349,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) walk_kernel(ChunkArgs a) {
     }
     if (tid < C * COLS / 4) {
       const int t = tid / (COLS / 4), c = tid % (COLS / 4) * 4;
-      copy16(dst + B::U + t * PU + c, u + Unit<D>::U + (long long)t * a.vdim + col0 + c);
+      if (col0 + c < a.vdim)
+        copy16(dst + B::U + t * PU + c, u + Unit<D>::U + (long long)t * a.vdim + col0 + c);
     } else if (tid - C * COLS / 4 < D / 4) {
       const int c = (tid - C * COLS / 4) * 4;
       copy16(dst + B::G + c, u + Unit<D>::G + c);
@@ -358,19 +362,21 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) walk_kernel(ChunkArgs a) {
   constexpr int OWN = D * COLS / WALK_THREADS;  // columns of a channel that a thread holds
   const int ch = tid % D, own0 = tid / D * OWN;
   const long long mine = (long long)ch * a.vdim + col0 + own0;  // its place in a head's state
+  const bool inside = col0 + own0 < a.vdim;  // (whole runs of columns: a.vdim is a multiple of 16)
   float* state = a.state + (long long)a.slots[seq] * a.state_stride + a.s_offset +
                  (long long)h * D * a.vdim + mine;
   f32x2 s[OWN / 2];
   fetch(0, ws);
 #pragma unroll
   for (int j = 0; j < OWN; j += 4) {
-    const float4 x = ldcg4(state + j);
+    const float4 x = inside ? ldcg4(state + j) : make_float4(0.f, 0.f, 0.f, 0.f);
     s[j / 2] = pack2(x.x, x.y);
     s[j / 2 + 1] = pack2(x.z, x.w);
     S[own0 + j][ch] = x.x; S[own0 + j + 1][ch] = x.y;
     S[own0 + j + 2][ch] = x.z; S[own0 + j + 3][ch] = x.w;
   }
   auto put_state = [&](float* to_) {
+    if (!inside) return;
 #pragma unroll
     for (int j = 0; j < OWN; j += 4) {
       const float2 x = unpack2(s[j / 2]), y = unpack2(s[j / 2 + 1]);
@@ -380,7 +386,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) walk_kernel(ChunkArgs a) {
   // in the first product: tokens t0 and t0 + 4, columns j0 and j0 + 4, half the channels. (The
   // second half starts 16 channels on, so that the halves' reads lie in other banks.)
   const int lane = tid & 31, warp = tid >> 5, half = lane / 16;
-  const int t0 = warp / 2 * 8 + lane / 4 % 4, j0 = warp % 2 * 8 + lane % 4;
+  constexpr int CW = COLS / 8;  // warps side by side over the columns, four over the tokens
+  const int t0 = warp / CW * 8 + lane / 4 % 4, j0 = warp % CW * 8 + lane % 4;
   for (int c0 = from; c0 < to; ++c0, ws += unit) {
     const int b = (c0 - from) & 1;
     const float* buf = smem + b * B::BUFFER;
@@ -413,8 +420,9 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) walk_kernel(ChunkArgs a) {
     __syncthreads();  // u is whole; the state and W have been read
     {
       const int t = tid / (COLS / 2), col = tid % (COLS / 2) * 2;
-      *reinterpret_cast<float2*>(ws + Unit<D>::U + (long long)t * a.vdim + col0 + col) =
-          *reinterpret_cast<const float2*>(&Us[t][col]);
+      if (col0 + col < a.vdim)
+        *reinterpret_cast<float2*>(ws + Unit<D>::U + (long long)t * a.vdim + col0 + col) =
+            *reinterpret_cast<const float2*>(&Us[t][col]);
     }
     const f32x2 decay = pack2(buf[B::G + ch], buf[B::G + ch]);
 #pragma unroll
@@ -531,7 +539,7 @@ __global__ void __launch_bounds__(OUT_GROUPS * 32, 2) output_kernel(ChunkArgs a)
 
 template <int D>
 int run(ChunkArgs a, int total, cudaStream_t stream) {
-  constexpr int prep = Prep<D>::FLOATS * 4, walk = Walk<D>::FLOATS * 4;
+  constexpr int prep = Prep<D>::FLOATS * 4;
   constexpr int most = (C * (D + 4) + C * (C + 4) + (D + C) * (MAX_VDIM + 4)) * 4;
   const int outs = (C * (D + 4) + C * (C + 4) + (D + C) * (a.vdim + 4)) * 4;
   static bool seen[64] = {};
@@ -540,15 +548,25 @@ int run(ChunkArgs a, int total, cudaStream_t stream) {
            cudaSuccess;
   };
   if (fb_first_use_on_device(seen) &&
-      !(room_for((const void*)prepare_kernel<D>, prep) && room_for((const void*)walk_kernel<D>, walk) &&
+      !(room_for((const void*)prepare_kernel<D>, prep) &&
+        room_for((const void*)walk_kernel<D, 16>, Walk<D, 16>::FLOATS * 4) &&
+        room_for((const void*)walk_kernel<D, 24>, Walk<D, 24>::FLOATS * 4) &&
         room_for((const void*)output_kernel<D>, most)))
     return fb_fail(2, "chunk_scan: cannot set %d bytes of shared memory", most);
   const int room = a.chunks;
+  const long long heads = (long long)a.n_seqs * a.H;
+  // 24 columns only where 16 would put two blocks on some SMs and 24 puts at most one on each: with
+  // more blocks than that, two a SM hide each other's waits (2 sequences of 750: 315 us both ways)
+  const bool wide = heads * (a.vdim / 16) > sm_count() && heads * ((a.vdim + 23) / 24) <= sm_count();
   for (a.first_chunk = 0; a.first_chunk < total; a.first_chunk += room) {
     a.chunks = total - a.first_chunk < room ? total - a.first_chunk : room;
     fb_launch(prepare_kernel<D>, dim3(a.chunks, a.H), dim3(PREP_THREADS), (size_t)prep, stream, a);
-    fb_launch(walk_kernel<D>, dim3(a.n_seqs, a.H, a.vdim / COLS), dim3(WALK_THREADS),
-              (size_t)walk, stream, a);
+    if (wide)
+      fb_launch(walk_kernel<D, 24>, dim3(a.n_seqs, a.H, (a.vdim + 23) / 24), dim3(16 * 24),
+                (size_t)Walk<D, 24>::FLOATS * 4, stream, a);
+    else
+      fb_launch(walk_kernel<D, 16>, dim3(a.n_seqs, a.H, a.vdim / 16), dim3(16 * 16),
+                (size_t)Walk<D, 16>::FLOATS * 4, stream, a);
     fb_launch(output_kernel<D>, dim3(a.chunks, a.H), dim3(OUT_GROUPS * a.vdim / 4), (size_t)outs,
               stream, a);
   }
@@ -559,7 +577,7 @@ int run(ChunkArgs a, int total, cudaStream_t stream) {
 // Floats of workspace that one chunk of 32 tokens takes over all heads (0: sizes that the chunked
 // kernels are not built for).
 FB_API int fb_chunk_scan_unit(int H, int dim, int vdim) {
-  if (vdim <= 0 || vdim % COLS != 0 || vdim > MAX_VDIM || H > 4096) return 0;
+  if (vdim <= 0 || vdim % 16 != 0 || vdim > MAX_VDIM || H > 4096) return 0;
   if (dim == 64) return (int)(H * Unit<64>::size(vdim));
   if (dim == 128) return (int)(H * Unit<128>::size(vdim));
   return 0;

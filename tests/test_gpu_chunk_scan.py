@@ -89,6 +89,18 @@ def test_chunks_equal_token_by_token(ops, H, G, d, e, channels, decay):
         near(rows, states)  # every slot's: the sequences' moved on, the others as they were
 
 
+@pytest.mark.parametrize("H,G,d,e", [(24, 24, 128, 128), (60, 30, 128, 48), (28, 28, 128, 112), (40, 20, 64, 64)])
+def test_blocks_of_24_columns(ops, H, G, d, e):
+    """Heads whose blocks of 16 columns are more than the SMs, those of 24 are not; the last block of a
+    head has 8, 24 or 16 columns."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if not H * (e // 16) > sms >= H * -(-e // 24):
+        pytest.skip("another number of SMs")
+    out, want, rows, states = run(ops, [131], H, G, d, e, True, DECAYS["slow"], seed=e)
+    near(out, want)
+    near(rows, states)
+
+
 @pytest.mark.parametrize("room", [1, 2, 5])
 def test_steps_in_parts(ops, room, monkeypatch):
     """A workspace of so many chunks: parts that begin and end inside sequences."""
