@@ -30,6 +30,12 @@ __device__ __forceinline__ long long row_of(const int* pages, int j, int ring_pa
   if (ring_pages > 0) lp %= ring_pages;
   return (long long)pages[lp] * page_stride + (long long)(j % FB_PAGE) * D;
 }
+// All threads of the cluster's blocks meet. (The aligned form wants whole warps: some lanes may still
+// be in the branch or the loop in front.)
+__device__ __forceinline__ void meet_cluster() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
 // exp(a - b) for a running maximum b that is -inf while nothing has been seen (a NaN stays one)
 __device__ __forceinline__ float exp_below(float a, float b) {
   return a == -INFINITY ? 0.f : expf(a - b);
@@ -196,7 +202,7 @@ split_kernel(FbAttentionF32 p, int head_chunks) {
     }
   }
   if (S == 1) return;
-  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+  meet_cluster();
   auto peer = [](const float* mine, int r) {
     unsigned there;
     float v;
@@ -225,7 +231,7 @@ split_kernel(FbAttentionF32 p, int head_chunks) {
     }
     o[i] = sum / total;
   }
-  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+  meet_cluster();
 }
 
 // ------------------------------------------------------------------ many tokens a sequence
@@ -244,9 +250,6 @@ struct AttnTile {
   static constexpr int BYTES = (D * PQ + D * PK + BKEY * PV + BKEY * PP) * 4;
 };
 
-__device__ __forceinline__ void meet_cluster() {
-  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
-}
 __device__ __forceinline__ unsigned shared_of(const float* mine, int rank) {
   unsigned there;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"

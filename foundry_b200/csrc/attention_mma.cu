@@ -431,6 +431,7 @@ __device__ void merge_if_last(const AttnParams& p, int seq, int kvh, int token, 
 // memory, no counters. Every CTA of the cluster calls this exactly once (also
 // one whose range is empty): the two barriers need all of them.
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();  // the aligned form wants whole warps
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

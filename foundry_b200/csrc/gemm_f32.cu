@@ -175,6 +175,7 @@ rows_kernel(const float* x /* written by the kernel before: no read-only promise
 constexpr int BK = 16;
 
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();  // the aligned form wants whole warps
   asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float4 ld_peer(unsigned addr, unsigned rank) {

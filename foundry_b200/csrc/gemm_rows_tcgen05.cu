@@ -116,6 +116,7 @@ __device__ __forceinline__ void epi_barrier() {  // the four epilogue warps
   asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 __device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();  // the aligned form wants whole warps
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -42,6 +42,7 @@ __device__ __forceinline__ float read_peer(const float* mine, unsigned rank) {
   return v;
 }
 __device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();  // the aligned form wants whole warps
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -18,6 +18,7 @@ __device__ __forceinline__ uint32_t cluster_address(const void* local, uint32_t 
   return out;
 }
 __device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();  // the aligned form wants whole warps
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
