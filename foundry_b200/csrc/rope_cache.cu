@@ -19,6 +19,11 @@
 // windowed group, else unbounded).
 #include "common.cuh"
 
+// A pair turned by an angle. The multiply-adds are written out, so that the kernels below round alike.
+__device__ __forceinline__ float2 turn_pair(float x1, float x2, float c, float s) {
+  return make_float2(fmaf(x1, c, -(x2 * s)), fmaf(x1, s, x2 * c));
+}
+
 // `src` is the fused projection output: T elements, or float32 when it is
 // `planes` partial results of a split-K product (summed here in plane order).
 // Rotated queries go to `q_out` (row stride q_stride), which may be `src`
@@ -94,15 +99,14 @@ __global__ void rope_kv_write_kernel(const TS* src, long long src_stride, int pl
       const int e1 = interleaved ? 2 * i : i, e2 = interleaved ? 2 * i + 1 : i + half;
       float x1, x2;
       load2(h * D + e1, h * D + e2, x1, x2);
-      const float y1 = x1 * c - x2 * s;
-      const float y2 = x2 * c + x1 * s;
+      const float2 y = turn_pair(x1, x2, c, s);
       if (h < A) {
-        qrow[h * D + e1] = fb_from_float<T>(y1);
-        qrow[h * D + e2] = fb_from_float<T>(y2);
+        qrow[h * D + e1] = fb_from_float<T>(y.x);
+        qrow[h * D + e2] = fb_from_float<T>(y.y);
       } else {
         T* dst = k_cache + cache_row + (long long)(h - A) * head_stride;
-        dst[e1] = fb_from_float<T>(y1);
-        dst[e2] = fb_from_float<T>(y2);
+        dst[e1] = fb_from_float<T>(y.x);
+        dst[e2] = fb_from_float<T>(y.y);
       }
     } else if (idx < n_rot + n_val) {
       const int j = idx - n_rot;
@@ -134,7 +138,7 @@ __global__ void rope_kv_write_kernel(const TS* src, long long src_stride, int pl
 // The same for float32 sources (planes of a split product among them) with interleaved pairs, a
 // rotary part as wide as the head and rows of whole 16-byte pieces: a thread takes two neighbouring
 // pairs, asks for all their planes before it knows its position, and makes its own two angles, so
-// that no barrier stands between. Bound by the chain of its loads: 128 tokens of 32 + 2 x 8 heads of
+// that no barrier stands between; the same bits. Bound by the chain of its loads: 128 tokens of 32 + 2 x 8 heads of
 // 64, six planes 3.5 us, 5.7 above; 384, two planes 3.8 for 9.6; 777, one plane, 32 bits 6.3 for 15.3.
 template <typename T>
 __device__ __forceinline__ void put_four(T* p, float4 v);
@@ -187,7 +191,8 @@ rope_kv_write_four_kernel(const float* src, long long src_stride, int planes, lo
     float s0, c0, s1, c1;
     sincosf((float)pos * freq.x, &s0, &c0);
     sincosf((float)pos * freq.y, &s1, &c1);
-    x = make_float4(x.x * c0 - x.y * s0, x.y * c0 + x.x * s0, x.z * c1 - x.w * s1, x.w * c1 + x.z * s1);
+    const float2 lo = turn_pair(x.x, x.y, c0, s0), hi = turn_pair(x.z, x.w, c1, s1);
+    x = make_float4(lo.x, lo.y, hi.x, hi.y);
   }
   if (h < A) {
     put_four<T>(q_out + (size_t)t * q_stride + at, x);

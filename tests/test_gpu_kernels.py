@@ -510,6 +510,34 @@ def test_rope_kv_write(ops, dtype, A, Kh, D, rot, source, pairing):
     assert float(k_cache.float().abs().sum(dim=(1, 3)).cpu()[mask].max()) == 0.0
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("planes", [1, 2, 4, 5, 9])
+@pytest.mark.parametrize("A,Kh,D", [(32, 8, 64), (5, 2, 4), (3, 1, 20), (8, 2, 128)])
+@pytest.mark.parametrize("write_cache,ring", [(True, 0), (True, 2), (False, 0)])
+def test_rope_kv_write_of_two_pairs_a_thread(ops, dtype, planes, A, Kh, D, write_cache, ring):
+    """Whole rows of float32 planes, interleaved, have a kernel of their own, with the bits of the general
+    one, which takes the same call where the frequencies do not lie on 8 bytes."""
+    positions, seqs = [0, 1, 63, 64, 5000, 7, 130], [0, 0, 1, 1, 2, -1, 0]
+    as_int = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    parts = torch.stack([rnd(len(seqs), (A + 2 * Kh) * D, seed=s) for s in range(planes)])
+    table = torch.randperm(3 * 80, generator=torch.Generator().manual_seed(1)).view(3, 80).to(torch.int32).to(DEV)
+    held = torch.empty(D // 2 + 2, device=DEV)
+    got = []
+    for shift in (0, 1):
+        inv_freq = held[shift:shift + D // 2]
+        inv_freq.copy_(torch.from_numpy((10000.0 ** (-np.arange(0, D, 2, dtype=np.float32) / D)).astype(np.float32)))
+        k_cache, v_cache = (torch.full((240, Kh, 64, D), 7.0, dtype=dtype, device=DEV) for _ in range(2))
+        q_out = torch.full((len(seqs), A * D), 7.0, dtype=dtype, device=DEV)
+        ops.rope_kv_write(ops.Planes(parts.clone()), as_int(positions), as_int(seqs), table, inv_freq, D, k_cache,
+                          v_cache, A, Kh, D, ring_pages=ring, write_cache=write_cache, q_out=q_out, dtype=dtype,
+                          pairing="interleaved")
+        got.append((q_out, k_cache, v_cache))
+    for two, general in zip(*got):
+        assert torch.equal(two, general)
+    assert bool((got[0][0][5] == 7).all()) and bool((got[0][0][:5] != 7).any())  # a padding token
+    assert write_cache == bool((got[0][1] != 7).any()) == bool((got[0][2] != 7).any())
+
+
 @pytest.mark.parametrize("A,Kh,D,rot", [(4, 2, 16, 16), (6, 3, 32, 32), (3, 1, 48, 32), (8, 2, 128, 128),
                                         (2, 2, 64, 0), (5, 1, 80, 48)])
 @pytest.mark.parametrize("T", [6, 13])
