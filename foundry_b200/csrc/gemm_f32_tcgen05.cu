@@ -23,8 +23,8 @@
 // that split raw 32-bit stages, 8 that add accumulators up in registers and store. Every wait is
 // bounded, as elsewhere.
 //
-// What a piece cannot carry is summed again by the thread that would store it, one product after the
-// other: results that are not finite (an infinity's pieces are not numbers, and what overflows has to
+// What a piece cannot carry is summed again behind all tiles, as chains of FMAs (`repair`): results that
+// are not finite (an infinity's pieces are not numbers, and what overflows has to
 // do so where 32 bits do), and those below 2^-100, whose operands may have pieces below the smallest
 // normal number, which the tensor cores take as zero.
 #define FB_STATUS_KERNEL 5
@@ -38,6 +38,7 @@ constexpr int W_ROWS = 128;       // weight rows of a CTA
 constexpr int PIECES = 3;
 constexpr int MAX_STAGES = 8, MAX_PIECE_STAGES = 4;
 constexpr int MAX_SHARES = 4;     // pairs of a cluster (8 CTAs, the portable size)
+constexpr int ROUNDS = 32;
 constexpr int SPLIT_WARPS = 8, SUM_WARPS = 8;
 constexpr int THREADS = 32 * (4 + SPLIT_WARPS + SUM_WARPS);
 // Tensor memory: two accumulators of tn columns, then the weights' pieces, 16 columns each.
@@ -143,6 +144,10 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr) {
   return v;
 }
 
+__device__ __forceinline__ void or_cluster(uint32_t addr, uint32_t bits) {
+  asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(addr), "r"(bits) : "memory");
+}
+
 // A warp's wait for two barriers, asked after together (one after the other cost twice the latency).
 __device__ __forceinline__ bool wait_both(uint64_t* bar_a, uint32_t parity_a, int where_a, uint64_t* bar_b,
                                           uint32_t parity_b, int where_b, volatile int* abort_flag,
@@ -179,12 +184,77 @@ __device__ __forceinline__ bool stands(float v) {
   return size <= 3.402823466e38f && (size >= 7.888609052e-31f || size == 0.f);
 }
 
-// A result as a chain of FMAs.
-__device__ __forceinline__ float plain_sum(const Params& p, int t, int f) {
-  const float *x = p.x + (long long)t * p.ldx, *w = p.w + (long long)f * p.ldw;
-  float v = 0.f;
-  for (int k = 0; k < p.K; ++k) v = fmaf(__ldcg(x + k), w[k], v);
-  return v;
+// The summing warps' threads meet; whether one of them said yes.
+__device__ __forceinline__ bool any_of_sums(bool mine) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"((uint32_t)mine), "n"(32 * SUM_WARPS)
+      : "memory");
+  return any != 0;
+}
+
+// A run of 16 tokens (from t0) by this CTA's weight rows (from f0) once more, results that do not stand
+// as chains of FMAs over K: 256 threads, a weight row and 8 tokens each, REPAIR_K of K at a time through
+// `stage`. A token that holds a NaN has its results already, all NaN. (Behind all tiles, where nobody
+// waits for these warps.)
+constexpr int REPAIR_K = 256, REPAIR_PITCH = REPAIR_K + 4;
+static_assert((W_ROWS + 16) * REPAIR_PITCH * 4 <= SMEM_TILES, "room for a stage of the repair");
+__device__ __forceinline__ void repair(const Params& p, float* stage, uint32_t* nan_tokens, int f0, int t0) {
+  const int tid = (int)threadIdx.x - 32 * (4 + SPLIT_WARPS), lane = tid & 31;
+  const int row = tid % W_ROWS, half = tid / W_ROWS, f = f0 + row;
+  uint32_t wanted = 0;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int t = t0 + half * 8 + e;
+    if (t < p.M && f < p.N && !stands(__ldcg(p.out + (long long)t * p.ldo + f))) wanted |= 1u << e;
+  }
+  if (tid == 0) *nan_tokens = 0;
+  if (!any_of_sums(wanted != 0)) return;
+  for (int i = tid / 32; i < 16 && t0 + i < p.M; i += SUM_WARPS) {
+    const float* x = p.x + (long long)(t0 + i) * p.ldx;
+    bool none = true;
+    for (int k = lane * 4; k < p.K; k += 128) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(x + k));
+      none = none && v.x == v.x && v.y == v.y && v.z == v.z && v.w == v.w;
+    }
+    if (!none) atomicOr(nan_tokens, 1u << i);
+  }
+  any_of_sums(false);
+  wanted &= ~(*nan_tokens >> (8 * half));
+  if (!any_of_sums(wanted != 0)) return;
+  float* xs = stage + W_ROWS * REPAIR_PITCH;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int k0 = 0; k0 < p.K; k0 += REPAIR_K) {
+    const int k = k0 + tid % 64 * 4;
+    any_of_sums(false);  // the numbers before have been read
+#pragma unroll 4
+    for (int r = tid / 64; r < W_ROWS + 16; r += 4) {  // weight rows, then tokens
+      const int at = r < W_ROWS ? f0 + r : t0 + r - W_ROWS;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (at < (r < W_ROWS ? p.N : p.M) && k < p.K)
+        v = __ldcg(reinterpret_cast<const float4*>(
+            r < W_ROWS ? p.w + (long long)at * p.ldw + k : p.x + (long long)at * p.ldx + k));
+      *reinterpret_cast<float4*>(stage + r * REPAIR_PITCH + tid % 64 * 4) = v;
+    }
+    any_of_sums(false);
+    const int some = min(REPAIR_K, p.K - k0);
+    for (int q = 0; q < some; q += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(stage + row * REPAIR_PITCH + q);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float4 x = *reinterpret_cast<const float4*>(xs + (half * 8 + e) * REPAIR_PITCH + q);
+        acc[e] = fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, acc[e]))));
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (wanted >> e & 1u) p.out[(long long)(t0 + half * 8 + e) * p.ldo + f] = acc[e];
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -200,6 +270,9 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
   __shared__ __align__(8) uint64_t piece_empty[MAX_PIECE_STAGES];
   __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];  // acc_empty: used in the leader
   __shared__ uint32_t tmem_slot;
+  // runs of 16 tokens of this CTA's tiles, round by round (rounds ROUNDS apart share a word), in which
+  // some result does not stand
+  __shared__ uint32_t fallen[ROUNDS], nan_tokens;
   __shared__ int s_abort;
   volatile int* abort_flag = &s_abort;
 
@@ -225,6 +298,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 2 * SUM_WARPS);
     }
+    for (int r = 0; r < ROUNDS; ++r) fallen[r] = 0;
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -375,10 +449,10 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
     const uint32_t acc_empty_leader = cluster_address(&acc_empty[0], lead_cta);
     const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16);
     fb_pdl_wait();
-    int b = 0;
+    int b = 0, round = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int u = cluster; u < p.units && ok; u += clusters) {
+    for (int u = cluster; u < p.units && ok; u += clusters, ++round) {
       float acc[RUNS][16];  // this thread's weight row, every other run of 16 tokens
 #pragma unroll
       for (int g = 0; g < RUNS; ++g)
@@ -418,11 +492,12 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
           for (int e = 0; e < 16; ++e) mine[(c + e) * W_ROWS] = acc[g][e];
         }
       } else if (f < p.N) {
-        bool whole = true;
+        uint32_t fell = 0;
 #pragma unroll
         for (int g = 0; g < RUNS; ++g) {
           const int c = (2 * g + which) * 16;
           if (c >= p.tn) break;
+          bool whole = true;
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const int t = t0 + c + e;
@@ -431,13 +506,9 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
               whole = whole && stands(acc[g][e]);
             }
           }
+          if (!whole) fell |= 1u << (2 * g + which);
         }
-        if (!whole) {
-          for (int t = t0; t < min(t0 + p.tn, p.M); ++t) {
-            float* o = p.out + (long long)t * p.ldo + f;
-            if ((((t - t0) >> 4) & 1) == which && !stands(*o)) *o = plain_sum(p, t, f);
-          }
-        }
+        if (fell != 0) atomicOr(&fallen[round % ROUNDS], fell);
       }
     }
   }
@@ -451,6 +522,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
 #pragma unroll
       for (int i = 0; i < MAX_SHARES; ++i)
         from[i] = cluster_address(tiles, (uint32_t)min(i, p.shares - 1) * 2 + rank);
+      uint32_t fell = 0;
       // every pair stores its tokens of the tile: the sums of all shares, in their order
 #pragma unroll 4
       for (int t = (int)share * 2 + which; t < tokens; t += ctas) {
@@ -460,19 +532,32 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
         for (int i = 1; i < MAX_SHARES; ++i)
           if (i < p.shares) v += ld_cluster(from[i] + at);
         if (f < p.N) {
-          if (!stands(v)) v = plain_sum(p, t0 + t, f);
           p.out[(long long)(t0 + t) * p.ldo + f] = v;
+          if (!stands(v)) fell |= 1u << (t >> 4);
         }
       }
+      if (fell != 0)  // every pair repairs some runs of the tile, whoever stored them
+        for (int i = 0; i < p.shares; ++i)
+          or_cluster(cluster_address(&fallen[0], (uint32_t)i * 2 + rank), fell);
     }
   }
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
-  cluster_barrier();  // nothing of the peer's may still be on its way to this CTA
+  cluster_barrier();  // nothing of the peers' may still be on its way to this CTA; results are stored
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, TMEM_COLS);
+  }
+  if (warp >= 4 + SPLIT_WARPS && !*abort_flag) {
+    int round = 0;
+    for (int u = cluster; u < p.units; u += clusters, ++round) {
+      const uint32_t fell = fallen[round % ROUNDS];
+      for (int run = (int)share; fell >> run != 0; run += p.shares)
+        if (fell >> run & 1u)
+          repair(p, reinterpret_cast<float*>(tiles), &nan_tokens,
+                 (u / p.tiles_t) * 2 * W_ROWS + (int)rank * W_ROWS, (u % p.tiles_t) * p.tn + run * 16);
+    }
   }
 }
 

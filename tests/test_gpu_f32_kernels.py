@@ -112,6 +112,21 @@ def test_product_of_pieces_of_what_pieces_cannot_carry(ops, N):
     assert float(gap.max()) <= 2.0 ** -126
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("M,N,K", [(100, 300, 4096), (777, 300, 1024), (777, 9000, 1028), (1500, 20000, 512)])
+def test_product_of_pieces_of_tokens_that_are_no_numbers(ops, M, N, K, value):
+    """Every result of every tile falls (with and without several pairs on a tile's K, several tiles a
+    pair): they are summed again behind the tiles, and no wait of the others runs out meanwhile."""
+    x, w = torch.full((M, K), value, device=DEV), rnd(N, K, seed=1).abs() + 0.1
+    w[7, 3] = 0.0
+    out = torch.zeros(M, N, device=DEV)
+    ops.gemm_simt(x, w, out)
+    want = torch.full((M, N), value, device=DEV)
+    want[:, 7] = float("nan")
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isposinf(), want.isposinf())
+    assert ops.gemm_tc_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(900, 500, 64), (700, 300, 1028)])
 def test_many_batched_products(ops, M, N, K):
     x, w = rnd(M, 32, K), rnd(32, N, K, seed=4)
