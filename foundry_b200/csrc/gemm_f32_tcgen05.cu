@@ -1,15 +1,17 @@
 // out[M,N] = x[M,K] * w[N,K]^T in 32 bits on the tensor cores, for many rows.
 //
 // A 32-bit number is the sum of three bfloat16 numbers, exactly (its 24 bits are three times 8; each
-// piece is what rounding leaves of the one before). A product of two such sums is nine products of
-// pieces; the six that are not below 2^-24 of the result go through tcgen05.mma (bf16 x bf16, whose
-// products are exact in 32 bits), the other three are dropped. Tensor memory truncates where it
+// piece is what rounding leaves of the one before; Henry, Tang and Heinecke, "Leveraging the bfloat16
+// artificial intelligence datatype for higher-precision computations", 2019). A product of two such sums
+// is nine products of pieces; six go through tcgen05.mma (bf16 x bf16, whose products are exact in 32
+// bits), the other three, below 2^-24 of |x w| each, are dropped. Tensor memory truncates where it
 // accumulates, so a sum stays there for 32 of K only, its small products first, and the partial sums
 // are added in registers, rounded to nearest. Relative error against 64 bits (2-norm, normal
 // operands): K = 2048 1.6e-7 (1.0e-7 where four pairs share K), K = 8192 2.9e-7 (1.6e-7); FFMA tiles
 // (gemm_f32.cu) 8.1e-7 or 2.9e-7, and 5.8e-7. Sums over 64 of K: 3.3e-7, hence 32.
 //
-// Bound by the tensor pipe: six bf16 products for one. 777 rows of 2048 -> 16384 256 us (204 TFLOP/s
+// Bound by the tensor pipe, six bf16 products for one, and close behind it by the issue slots of the
+// warps that split and add (two more instructions an operand: 777 rows of 2048 -> 16384 280 us). 777 rows of 2048 -> 16384 256 us (204 TFLOP/s
 // of the product, 1.22 PFLOP/s of bf16) where FFMA tiles took 1524, -> 3072 59 for 311, 8192 -> 2048
 // 156 for 789; 64 rows of 2048 -> 2048 23 for 33; 2048 rows -> 16384 621 for 3010 (74 TFLOP/s is all
 // that FFMA could give). The weights are split tile by tile, not once to memory, which would move 16
@@ -23,10 +25,14 @@
 // that split raw 32-bit stages, 8 that add accumulators up in registers and store. Every wait is
 // bounded, as elsewhere.
 //
-// What a piece cannot carry is summed again behind all tiles, as chains of FMAs (`repair`): results that
-// are not finite (an infinity's pieces are not numbers, and what overflows has to
-// do so where 32 bits do), and those below 2^-100, whose operands may have pieces below the smallest
-// normal number, which the tensor cores take as zero.
+// What pieces cannot carry is summed again behind all tiles, as chains of FMAs (`repair`): results that are
+// not finite (an infinity's pieces are not numbers, and what overflows has to do so where 32 bits do),
+// and those of operands so small that their pieces, or products of them, fall below the smallest normal
+// number, which the tensor cores take as zero: x of 1e-36 times w of 1e10 would be off by 1e-3. The
+// splitting warps keep the largest first piece (half an instruction an operand; 777 rows of 2048 ->
+// 16384 252 -> 257 us); unless it is huge, a finite result of 2^-64 or more stands, and the rows of the
+// others are looked at, which settles most (`falls`). Zeros cost that look: a token in seven of zeros,
+// 777 rows of 8192 -> 16384 990 -> 1,600 us; all of x NaN 1,900, all of it infinite 30,000.
 #define FB_STATUS_KERNEL 5
 #include "gemm_f32.h"
 #include "tcgen05_pair.cuh"
@@ -144,6 +150,9 @@ __device__ __forceinline__ float ld_cluster(uint32_t addr) {
   return v;
 }
 
+__device__ __forceinline__ void max_cluster(uint32_t addr, uint32_t v) {
+  asm volatile("red.relaxed.cluster.shared::cluster.max.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void or_cluster(uint32_t addr, uint32_t bits) {
   asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(addr), "r"(bits) : "memory");
 }
@@ -178,15 +187,85 @@ __device__ __forceinline__ void fewer_registers() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// Whether a sum of pieces stands (see above).
+// The roles end in branches of their own (a role's registers are its own there): all threads of the
+// cluster meet, with shares twice.
+__device__ __forceinline__ void shares_meet() { cluster_barrier(); }
+__device__ __forceinline__ void roles_meet() {
+  tc_fence_before();
+  __syncwarp();
+  asm volatile("barrier.cta.sync 0;" ::: "memory");
+  cluster_barrier();  // nothing of the peers' may still be on its way to this CTA; results are stored
+}
+__device__ __forceinline__ void all_meet(const Params& p) {
+  if (p.shares > 1) shares_meet();
+  roles_meet();
+}
+
+// Whether a sum of pieces needs no look at its operands: finite, and of 2^-64 or more (see above).
 __device__ __forceinline__ bool stands(float v) {
+  return (__float_as_uint(v) & 0x7fffffffu) - 0x1f800000u < 0x7f800000u - 0x1f800000u;
+}
+
+// The larger magnitudes of two pairs of first pieces (of a number and a NaN the number's).
+__device__ __forceinline__ uint32_t larger_pieces(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t largest_of_warp(uint32_t pieces) {  // as the bits of a float
+  const uint32_t a = (pieces & 0x7fffu) << 16, b = pieces & 0x7fff0000u;
+  return __reduce_max_sync(0xffffffffu, max(a, b));
+}
+
+// What a row of operands is: the largest magnitude (not a NaN's), the smallest that is not zero (as twice
+// its bits less one, so that a zero is the largest), whether it holds a NaN.
+struct RowFacts {
+  float most;
+  uint32_t least;
+  int nan;
+};
+constexpr float LEAST_WHOLE = 1.0f / (1 << 30) / (1 << 30) / (1 << 30) / (1 << 12);  // 2^-102
+
+// Whether a result is to be summed again. Pieces and products of pieces below 2^-126 may have been taken as
+// zero: nothing beyond 2^-24 of an operand of 2^-102 or more, nothing beyond 2^-25 of a product of 2^-98
+// or more; else K terms lose up to 2^-126 of the largest other operand each way, and six products of
+// 2^-126. The result stands where it is 2^24 times that. (A row with a NaN has its results.)
+__device__ __forceinline__ bool falls(float v, const RowFacts& w, const RowFacts& x, int K) {
+  if (w.nan || x.nan) return false;
   const float size = fabsf(v);
-  return size <= 3.402823466e38f && (size >= 7.888609052e-31f || size == 0.f);
+  if (!(size <= 3.402823466e38f)) return true;
+  if (w.least == 0xffffffffu || x.least == 0xffffffffu) return false;  // a row of zeros
+  const float least_w = __uint_as_float((w.least >> 1) + 1u), least_x = __uint_as_float((x.least >> 1) + 1u);
+  if (least_w >= LEAST_WHOLE && least_x >= LEAST_WHOLE && least_w * least_x >= 16.f * LEAST_WHOLE) return false;
+  return !(size >= (float)K * LEAST_WHOLE * (w.most + x.most + 8.f));
+}
+// Whether one operand's row alone settles a result: all are NaN, or it is the zero that a row of zeros makes.
+__device__ __forceinline__ bool settles(const RowFacts& of, float v) {
+  return of.nan || (of.least == 0xffffffffu && v == 0.f);
+}
+// One warp looks at a row.
+__device__ __forceinline__ void look_at_row(RowFacts* to, const float* row, int K, int lane) {
+  float most = 0.f;
+  uint32_t least = 0xffffffffu;
+  bool nan = false;
+#pragma unroll 2
+  for (int k = lane * 4; k < K; k += 128) {
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(row + k));
+    most = fmaxf(most, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    least = min(least, min(min(2u * __float_as_uint(v.x) - 1u, 2u * __float_as_uint(v.y) - 1u),
+                           min(2u * __float_as_uint(v.z) - 1u, 2u * __float_as_uint(v.w) - 1u)));
+    nan = nan || !(v.x == v.x && v.y == v.y && v.z == v.z && v.w == v.w);
+  }
+  most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most)));
+  least = __reduce_min_sync(0xffffffffu, least);
+  nan = __any_sync(0xffffffffu, nan);
+  if (lane == 0) *to = RowFacts{most, least, nan};
 }
 
 // The summing warps' threads meet; whether one of them said yes.
 __device__ __forceinline__ bool any_of_sums(bool mine) {
   uint32_t any;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
@@ -198,51 +277,93 @@ __device__ __forceinline__ bool any_of_sums(bool mine) {
   return any != 0;
 }
 
-// A run of 16 tokens (from t0) by this CTA's weight rows (from f0) once more, results that do not stand
-// as chains of FMAs over K: 256 threads, a weight row and 8 tokens each, REPAIR_K of K at a time through
-// `stage`. A token that holds a NaN has its results already, all NaN. (Behind all tiles, where nobody
-// waits for these warps.)
-constexpr int REPAIR_K = 256, REPAIR_PITCH = REPAIR_K + 4;
-static_assert((W_ROWS + 16) * REPAIR_PITCH * 4 <= SMEM_TILES, "room for a stage of the repair");
-__device__ __forceinline__ void repair(const Params& p, float* stage, uint32_t* nan_tokens, int f0, int t0) {
-  const int tid = (int)threadIdx.x - 32 * (4 + SPLIT_WARPS), lane = tid & 31;
+// A run of 16 tokens (from t0) by this CTA's weight rows (from f0) once more, results that fall as chains of
+// FMAs over K: 256 threads, a weight row and 8 tokens each, REPAIR_K of K at a time through shared memory.
+// All of it is behind all tiles, where nobody waits for these warps. Which results fall: of those that do
+// not stand by themselves (or of all) the rows are looked at, first the operand's of which fewer are
+// asked about (weight rows once a tile), then, for what is left, the other's.
+constexpr int REPAIR_K = 256, REPAIR_PITCH = REPAIR_K + 4, REPAIR_ROWS = W_ROWS + 16;
+static_assert(REPAIR_ROWS % 48 == 0, "whole rounds of loads");
+struct RepairRoom {
+  float stage[REPAIR_ROWS * REPAIR_PITCH];  // weight rows, then tokens
+  RowFacts facts[REPAIR_ROWS];
+  uint32_t asked[W_ROWS / 32 + 1], known[W_ROWS / 32];  // weight rows (tokens last); weight rows looked at
+};
+static_assert(sizeof(RepairRoom) <= SMEM_TILES, "room for the repair");
+__device__ __forceinline__ void repair(const Params& p, RepairRoom& room, bool all, int f0, int t0) {
+  constexpr int WORDS = W_ROWS / 32;
+  const int tid = (int)threadIdx.x - 32 * (4 + SPLIT_WARPS);
   const int row = tid % W_ROWS, half = tid / W_ROWS, f = f0 + row;
+  RowFacts* facts = room.facts;
+  auto result = [&](int e) { return __ldcg(p.out + (long long)(t0 + half * 8 + e) * p.ldo + f); };
   uint32_t wanted = 0;
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int t = t0 + half * 8 + e;
-    if (t < p.M && f < p.N && !stands(__ldcg(p.out + (long long)t * p.ldo + f))) wanted |= 1u << e;
-  }
-  if (tid == 0) *nan_tokens = 0;
-  if (!any_of_sums(wanted != 0)) return;
-  for (int i = tid / 32; i < 16 && t0 + i < p.M; i += SUM_WARPS) {
-    const float* x = p.x + (long long)(t0 + i) * p.ldx;
-    bool none = true;
-    for (int k = lane * 4; k < p.K; k += 128) {
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(x + k));
-      none = none && v.x == v.x && v.y == v.y && v.z == v.z && v.w == v.w;
+  for (int e = 0; e < 8; ++e)
+    if (t0 + half * 8 + e < p.M && f < p.N && (all || !stands(result(e)))) wanted |= 1u << e;
+  auto ask = [&]() {
+    if (tid <= WORDS) room.asked[tid] = 0;
+    if (!any_of_sums(wanted != 0)) return false;
+    if (wanted != 0) {
+      atomicOr(&room.asked[row / 32], 1u << (row % 32));
+      atomicOr(&room.asked[WORDS], wanted << (8 * half));
     }
-    if (!none) atomicOr(nan_tokens, 1u << i);
-  }
-  any_of_sums(false);
-  wanted &= ~(*nan_tokens >> (8 * half));
+    any_of_sums(false);
+    return true;
+  };
+  auto look = [&](bool tokens) {
+    if (tokens) {
+      for (int i = tid / 32; i < 16; i += SUM_WARPS)
+        if (room.asked[WORDS] >> i & 1u)
+          look_at_row(facts + W_ROWS + i, p.x + (long long)(t0 + i) * p.ldx, p.K, tid & 31);
+    } else {
+      for (int r = tid / 32; r < W_ROWS; r += SUM_WARPS)
+        if ((room.asked[r / 32] & ~room.known[r / 32]) >> (r % 32) & 1u) {
+          look_at_row(facts + r, p.w + (long long)(f0 + r) * p.ldw, p.K, tid & 31);
+          if ((tid & 31) == 0) atomicOr(&room.known[r / 32], 1u << (r % 32));
+        }
+    }
+    any_of_sums(false);
+  };
+  if (!ask()) return;
+  int rows = 0;
+#pragma unroll
+  for (int i = 0; i < WORDS; ++i) rows += __popc(room.asked[i] & ~room.known[i]);
+  const bool tokens_first = any_of_sums(__popc(room.asked[WORDS]) <= rows);
+  look(tokens_first);
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if ((wanted >> e & 1u) && settles(facts[tokens_first ? W_ROWS + half * 8 + e : row], result(e)))
+      wanted &= ~(1u << e);
+  if (!ask()) return;
+  look(!tokens_first);
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if ((wanted >> e & 1u) && !falls(result(e), facts[row], facts[W_ROWS + half * 8 + e], p.K))
+      wanted &= ~(1u << e);
   if (!any_of_sums(wanted != 0)) return;
+  float* stage = room.stage;
   float* xs = stage + W_ROWS * REPAIR_PITCH;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int k0 = 0; k0 < p.K; k0 += REPAIR_K) {
     const int k = k0 + tid % 64 * 4;
     any_of_sums(false);  // the numbers before have been read
-#pragma unroll 4
-    for (int r = tid / 64; r < W_ROWS + 16; r += 4) {  // weight rows, then tokens
-      const int at = r < W_ROWS ? f0 + r : t0 + r - W_ROWS;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (at < (r < W_ROWS ? p.N : p.M) && k < p.K)
-        v = __ldcg(reinterpret_cast<const float4*>(
-            r < W_ROWS ? p.w + (long long)at * p.ldw + k : p.x + (long long)at * p.ldx + k));
-      *reinterpret_cast<float4*>(stage + r * REPAIR_PITCH + tid % 64 * 4) = v;
+    for (int r0 = tid / 64; r0 < REPAIR_ROWS; r0 += 48) {  // weight rows, then tokens; 12 loads at once
+      float4 v[12];
+#pragma unroll
+      for (int i = 0; i < 12; ++i) {
+        const int r = r0 + 4 * i, at = r < W_ROWS ? f0 + r : t0 + r - W_ROWS;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (at < (r < W_ROWS ? p.N : p.M) && k < p.K)
+          v[i] = __ldcg(reinterpret_cast<const float4*>(
+              r < W_ROWS ? p.w + (long long)at * p.ldw + k : p.x + (long long)at * p.ldx + k));
+      }
+#pragma unroll
+      for (int i = 0; i < 12; ++i)
+        *reinterpret_cast<float4*>(stage + (r0 + 4 * i) * REPAIR_PITCH + tid % 64 * 4) = v[i];
     }
     any_of_sums(false);
     const int some = min(REPAIR_K, p.K - k0);
+#pragma unroll 4
     for (int q = 0; q < some; q += 4) {
       const float4 w = *reinterpret_cast<const float4*>(stage + row * REPAIR_PITCH + q);
 #pragma unroll
@@ -272,7 +393,8 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
   __shared__ uint32_t tmem_slot;
   // runs of 16 tokens of this CTA's tiles, round by round (rounds ROUNDS apart share a word), in which
   // some result does not stand
-  __shared__ uint32_t fallen[ROUNDS], nan_tokens;
+  __shared__ uint32_t fallen[ROUNDS];
+  __shared__ uint32_t largest[2];  // first piece of a weight, of a token that the cluster multiplied
   __shared__ int s_abort;
   volatile int* abort_flag = &s_abort;
 
@@ -299,6 +421,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
       mbar_init(&acc_empty[b], 2 * SUM_WARPS);
     }
     for (int r = 0; r < ROUNDS; ++r) fallen[r] = 0;
+    largest[0] = largest[1] = 0u;
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -379,6 +502,11 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
         if ((sum ^= 1) == 0) sum_phase ^= 1u;
       }
     }
+    all_meet(p);
+    if (warp == 1) {
+      tc_fence_after();
+      tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    }
   } else if (warp < 4 + SPLIT_WARPS) {
     // ---------------------------------------------------------------- splitting
     fewer_registers<REGS_SPLIT>();
@@ -389,6 +517,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
     const uint32_t w_lanes = tmem_w + ((uint32_t)((warp & 3) * 32) << 16);
     int s = which, b = which;
     uint32_t raw_phase = 0, phase = 0;
+    uint32_t most_w = 0, most_x = 0;
     for (int it = which; it < total; it += 2) {
       if (!wait_both(&raw_full[s], raw_phase, 5, &piece_empty[b], phase ^ 1u, 6, abort_flag, it)) break;
       tc_fence_after();
@@ -409,6 +538,10 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
           for (int e = 0; e < 8; ++e)
             to[e] = piece + 1 < PIECES ? take_piece(v[2 * e], v[2 * e + 1])
                                        : last_piece(v[2 * e], v[2 * e + 1]);
+          if (piece == 0) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) most_w = larger_pieces(most_w, to[e]);
+          }
           tmem_st8(w_lanes + (uint32_t)((b * PIECES + piece) * W_PIECE_COLS + h * 8), to);
         }
       }
@@ -428,6 +561,10 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
           for (int e = 0; e < 4; ++e)
             to[e] = piece + 1 < PIECES ? take_piece(v[2 * e], v[2 * e + 1])
                                        : last_piece(v[2 * e], v[2 * e + 1]);
+          if (piece == 0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) most_x = larger_pieces(most_x, to[e]);
+          }
           st_shared(dst, make_uint4(to[0], to[1], to[2], to[3]));
         }
       }
@@ -442,6 +579,13 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
       if ((s += 2) >= p.stages) { s -= p.stages; raw_phase ^= 1u; }
       if ((b += 2) >= p.piece_stages) { b -= p.piece_stages; phase ^= 1u; }
     }
+    const uint32_t of_w = largest_of_warp(most_w), of_x = largest_of_warp(most_x);
+    if (lane < 2 * p.shares) {  // a lane tells a CTA of the cluster
+      const uint32_t at = cluster_address(&largest[0], (uint32_t)lane);
+      max_cluster(at, of_w);
+      max_cluster(at + 4, of_x);
+    }
+    all_meet(p);
   } else {
     // --------------------------------------------------------------------- sums
     more_registers<REGS_SUM>();
@@ -511,11 +655,8 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
         if (fell != 0) atomicOr(&fallen[round % ROUNDS], fell);
       }
     }
-  }
-  if (p.shares > 1) {
-    cluster_barrier();  // every share's sums are in place (all threads come here)
-    if (warp >= 4 + SPLIT_WARPS) {
-      const int quarter = warp & 3, which = (warp - 4 - SPLIT_WARPS) >> 2;
+    if (p.shares > 1) {
+      shares_meet();  // every share's sums are in place
       const int f = (cluster / p.tiles_t) * 2 * W_ROWS + (int)rank * W_ROWS + quarter * 32 + lane;
       const int t0 = (cluster % p.tiles_t) * p.tn, tokens = min(p.tn, p.M - t0);
       uint32_t from[MAX_SHARES];
@@ -540,23 +681,25 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
         for (int i = 0; i < p.shares; ++i)
           or_cluster(cluster_address(&fallen[0], (uint32_t)i * 2 + rank), fell);
     }
-  }
-  // ------------------------------------------------------------------ teardown
-  tc_fence_before();
-  __syncthreads();
-  cluster_barrier();  // nothing of the peers' may still be on its way to this CTA; results are stored
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc_pair(tmem_base, TMEM_COLS);
-  }
-  if (warp >= 4 + SPLIT_WARPS && !*abort_flag) {
-    int round = 0;
-    for (int u = cluster; u < p.units; u += clusters, ++round) {
-      const uint32_t fell = fallen[round % ROUNDS];
-      for (int run = (int)share; fell >> run != 0; run += p.shares)
-        if (fell >> run & 1u)
-          repair(p, reinterpret_cast<float*>(tiles), &nan_tokens,
-                 (u / p.tiles_t) * 2 * W_ROWS + (int)rank * W_ROWS, (u % p.tiles_t) * p.tn + run * 16);
+    roles_meet();
+    if (!*abort_flag) {
+      // A result of 2^-64 and more stands by itself while K terms of 2^-102 of the largest operands stay
+      // below that (a first piece is off by 2^-8 at most); else every result is looked at.
+      const float most = __uint_as_float(largest[0]) + __uint_as_float(largest[1]);
+      const bool all = !((float)p.K * (1.01f * most + 8.f) < 274877906944.f);  // 2^38
+      RepairRoom& room = *reinterpret_cast<RepairRoom*>(tiles);
+      round = 0;
+      for (int u = cluster; u < p.units; u += clusters, ++round) {
+        const uint32_t fell = all ? (1u << (p.tn / 16)) - 1u : fallen[round % ROUNDS];
+        if (fell == 0) continue;
+        any_of_sums(false);  // the tile before is done
+        if (threadIdx.x < 32 * (4 + SPLIT_WARPS) + W_ROWS / 32)
+          room.known[threadIdx.x - 32 * (4 + SPLIT_WARPS)] = 0;
+        for (int run = (int)share; fell >> run != 0; run += p.shares)
+          if (fell >> run & 1u)
+            repair(p, room, all, (u / p.tiles_t) * 2 * W_ROWS + (int)rank * W_ROWS,
+                   (u % p.tiles_t) * p.tn + run * 16);
+      }
     }
   }
 }

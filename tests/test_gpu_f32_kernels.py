@@ -112,6 +112,24 @@ def test_product_of_pieces_of_what_pieces_cannot_carry(ops, N):
     assert float(gap.max()) <= 2.0 ** -126
 
 
+@pytest.mark.parametrize("N", [300, 9000])
+@pytest.mark.parametrize("of_x,of_w", [(1e-34, 1e8), (1e-36, 1e10), (1e-38, 1e12), (3e-40, 1e15),
+                                       (1e-39, 1e30), (1e10, 1e-36), (1e-20, 1e-18)])
+def test_product_of_pieces_of_small_times_large(ops, N, of_x, of_w):
+    """Operands whose pieces are below the smallest normal number, times operands that make results of
+    any size of them: all tokens, one of them, one number of a token."""
+    for rows, cols in ((slice(None), slice(None)), (slice(5, 6), slice(None)), (slice(40, 41), slice(9, 10))):
+        x, w = rnd(64, 1024), rnd(N, 1024, seed=1) * of_w
+        x[rows, cols] *= of_x
+        x[50] = 0.0
+        out = torch.empty(64, N, device=DEV)
+        ops.gemm_simt(x, w, out)
+        size = x.double().abs() @ w.double().abs().T
+        # products of 2^-24 of their magnitude each; below the smallest normal number, 2^-149 each
+        gap = (out.double() - x.double() @ w.double().T).abs() - 1026 * (2.0 ** -24 * size + 2.0 ** -149)
+        assert float(gap.max()) <= 0, float(gap.max())
+
+
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 @pytest.mark.parametrize("M,N,K", [(100, 300, 4096), (777, 300, 1024), (777, 9000, 1028), (1500, 20000, 512)])
 def test_product_of_pieces_of_tokens_that_are_no_numbers(ops, M, N, K, value):
