@@ -660,12 +660,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
 // o = a1 - lambda a2;  out = o / sqrt(mean(o^2) + eps) * scale: a warp a (token, head), a lane pieces of
 // four. Bound by its bytes.
 __global__ void __launch_bounds__(256)
-combine_maps_kernel(const float* maps, __nv_bfloat16* out, long long out_stride, long long count, int H,
-                    int DV, float lambda, float eps, float scale) {
+combine_maps_kernel(const float* maps, __nv_bfloat16* out, long long out_stride, const int* cu_tokens,
+                    int n_seqs, int H, int DV, float lambda, float eps, float scale) {
   fb_pdl_launch();
   fb_pdl_wait();
   const long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (i >= count) return;
+  if (i >= (long long)cu_tokens[n_seqs] * H) return;  // (no block has made a padding token's rows)
   const int d = (threadIdx.x & 31) * 4;
   const float* a = maps + i * 2 * DV;
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -917,7 +917,7 @@ FB_API int fb_attention_prefill_maps(const void* q, long long q_stride, int T, f
   if (rc) return rc;
   const long long count = (long long)T * H;
   fb_launch(combine_maps_kernel, dim3((unsigned)((count + 7) / 8)), dim3(256), 0, stream, maps,
-            (__nv_bfloat16*)out, out_stride, count, H, DV, lambda, eps, post_scale);
+            (__nv_bfloat16*)out, out_stride, cu_tokens, n_seqs, H, DV, lambda, eps, post_scale);
   return fb_check_launch("combine_maps");
 }
 

@@ -2632,14 +2632,19 @@ def attention_folded(ctx, q: torch.Tensor, out: torch.Tensor, page_table, cache:
 MAPS_WORKSPACE = 1 << 27  # floats of both maps' results at most (a step of more keeps mma.sync)
 
 
-def _maps_workspace(floats: int, device) -> Optional[torch.Tensor]:
-    """Memory for both maps' results, or None where there is too little."""
-    if floats > MAPS_WORKSPACE:
-        return None
-    try:
-        return torch.empty(floats, dtype=torch.float32, device=device)
-    except torch.cuda.OutOfMemoryError:
-        return None
+def _maps_workspace(rows: int, H: int, G: int, device):
+    """Memory for both maps' results (`rows` floats a head) and how many heads it is for: all of them,
+    fewer where memory is short, whole groups or parts of one. Heads do not know of one another: the
+    numbers are the same."""
+    each = H // G
+    sizes = [n * each for n in range(G, 0, -1) if G % n == 0]
+    sizes += [n for n in range(each - 1, 0, -1) if each % n == 0]
+    for heads in sizes:
+        try:
+            return torch.empty(rows * heads, dtype=torch.float32, device=device), heads
+        except torch.cuda.OutOfMemoryError:
+            if heads == 1:
+                raise
 
 
 def _tc_paged_blocks(ctx, q, out, k_cache, v_cache, G: int, row: int, vdim: int) -> int:
@@ -2689,21 +2694,23 @@ def attention_maps_paged(ctx, q, out, page_table, k_cache, v_cache, H: int, G: i
     tcgen05 kernel in its form with two maps (csrc/attention_tcgen05.cu)."""
     lam, post_eps, post_scale = combine if combine is not None else (0.0, 0.0, 1.0)
     blocks128 = _tc_maps_blocks(ctx, q, out, k_cache, v_cache, G, dim, vdim, maps, scale)
-    if blocks128:
-        both = _maps_workspace(q.shape[0] * H * 2 * vdim, q.device)
-        if both is not None:
-            _call("fb_attention_prefill_maps", _dev(q, "q", torch.bfloat16, contiguous=False),
-                  _rows(q, "q"), q.shape[0], both.data_ptr(),
-                  _dev(out, "out", torch.bfloat16, contiguous=False), _rows(out, "out"),
+    if blocks128 and q.shape[0] * H * 2 * vdim <= MAPS_WORKSPACE:
+        both, heads = _maps_workspace(q.shape[0] * 2 * vdim, H, G, q.device)
+        at_q, at_out = (_dev(t, "rows", torch.bfloat16, contiguous=False) for t in (q, out))
+        at_sink = 0 if sink_logits is None else _dev(sink_logits, "sink_logits", torch.float32)
+        for a in range(0, H, heads):  # (2 bytes an element, 4 a sink's)
+            g = a * G // H
+            _call("fb_attention_prefill_maps", at_q + 2 * a * 2 * dim, _rows(q, "q"), q.shape[0],
+                  both.data_ptr(), at_out + 2 * a * vdim, _rows(out, "out"),
                   _dev(ctx.cu_tokens, "cu_tokens", torch.int32), _dev(ctx.kv_lens, "kv_lens", torch.int32),
-                  _dev(page_table, "page_table", torch.int32), page_table.shape[1], k_cache.data_ptr(),
-                  v_cache.data_ptr(), k_cache.stride(0), k_cache.stride(1), v_cache.stride(0),
-                  v_cache.stride(1), k_cache.shape[0], ctx.n_seqs, blocks128, H, G, vdim, float(scale),
-                  float(softcap),
-                  0 if sink_logits is None else _dev(sink_logits, "sink_logits", torch.float32),
-                  float(lam), float(post_eps), float(post_scale), _stream())
+                  _dev(page_table, "page_table", torch.int32), page_table.shape[1],
+                  k_cache.data_ptr() + 2 * g * k_cache.stride(1),
+                  v_cache.data_ptr() + 2 * g * v_cache.stride(1), k_cache.stride(0), k_cache.stride(1),
+                  v_cache.stride(0), v_cache.stride(1), k_cache.shape[0], ctx.n_seqs, blocks128, heads,
+                  max(1, heads * G // H), vdim, float(scale), float(softcap),
+                  at_sink + 4 * a if at_sink else 0, float(lam), float(post_eps), float(post_scale), _stream())
             add_launches(1)  # two kernels
-            return out
+        return out
     _call("fb_attention_maps", _dev(q, "q", torch.bfloat16, contiguous=False), _rows(q, "q"),
           _dev(out, "out", torch.bfloat16, contiguous=False), _rows(out, "out"),
           _dev(ctx.cu_tokens, "cu_tokens", torch.int32), _dev(ctx.kv_lens, "kv_lens", torch.int32),

@@ -89,6 +89,35 @@ def test_two_maps(ops, lens, starts, H, G, vdim, cap, size, sinks):
     assert float(off.norm()) <= 1.05 * float(before.norm())  # the same roundings, in another order
 
 
+@pytest.mark.parametrize("H,G,heads", [(8, 2, 4), (8, 2, 2), (8, 2, 1), (6, 6, 3), (3, 1, 1)])
+def test_two_maps_with_little_memory(ops, monkeypatch, H, G, heads):
+    """Where memory for all heads is missing, they are worked in parts, with the same bits; rows of padding
+    tokens, which no block makes, are not written from what the memory held."""
+    lens, vdim = [200, 65], 128
+    ctx, q, k, v, table = make(lens, [37, 0], H, G, vdim)
+    T = sum(lens)
+    q = torch.cat([q, torch.zeros_like(q[:20])])[:, :H * 128]
+    sink = torch.randn(H, generator=torch.Generator().manual_seed(9)).to(DEV)
+    args = (table, k, v, H, G, 64, vdim, 2, 0.125, 50.0, sink, (0.3, 1e-5, 0.2))
+    whole, parts = (torch.full((T + 20, H * vdim), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    assert ops._tc_maps_blocks(ctx, q, whole, k, v, G, 64, vdim, 2, 0.125) > 0
+    ops.attention_maps_paged(ctx, q, whole, *args)
+    empty, most = torch.empty, (T + 20) * heads * 2 * vdim
+    asked = []
+
+    def little(*size, **how):
+        if how.get("dtype") == torch.float32:
+            asked.append(size[0])
+            if size[0] > most:
+                raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*size, **how)
+    monkeypatch.setattr(ops.torch, "empty", little)
+    ops.attention_maps_paged(ctx, q, parts, *args)
+    monkeypatch.undo()
+    assert asked[-1] == most and len(asked) > 1 and torch.equal(parts, whole)
+    assert bool((whole[T:] == 7).all())
+
+
 def test_what_the_form_does_not_take_stays(ops):
     ctx, q, k, v, table = make([100, 20, 1], [0, 0, 0], 4, 2, 128)
     out = torch.empty(121, 512, dtype=torch.bfloat16, device=DEV)
