@@ -421,14 +421,17 @@ int fb_gemm_f32_launch(const FbGemmF32& p, cudaStream_t stream) {
   // 2048 -> 64 both 24.6. Rows count in whole 128s: a step that is padded to a bucket sums as the
   // plain one does.
   const long long rows = (p.M + 127) / 128 * 128;
-  if (p.count == 1 && p.ldx >= p.K && p.ldw >= p.K && p.N >= 128 &&
-      (p.K >= 1024 || rows * p.N * p.K >= 1LL << 28))
-    return fb_gemm_f32_tc_launch(p, stream);
-  // 128 x 128 tiles move the least through shared memory (46 TFLOP/s at 2048 x 2048 -> 16384
-  // against 37 with 64 x 64 and 24 before) and need three full rounds of two blocks an SM to hide
-  // their last one; below that 64 x 64 tiles with K shared eightfold (777 rows, 2048 -> 3072:
-  // 305 us against 412 with 128 x 128 and 491 before; 300 rows, 8192 -> 2048: 357 against 1068
-  // and 827; 128 rows, 2048 -> 64: 14 against 230 and 125). Rows count in whole 128s here, too.
+  if (p.count == 1 && p.M > FB_GEMM_F32_ROWS && p.N >= 128 &&
+      (p.K >= 1024 || rows * p.N * p.K >= 1LL << 28)) {
+    const int code = fb_gemm_f32_tc_launch(p, stream);
+    if (code != FB_GEMM_F32_NOT_HERE) return code;
+  }
+  // What is left: batched products, fewer than 128 results a row, little to do. 128 x 128 tiles move
+  // the least through shared memory and need three full rounds of two blocks an SM to hide their last
+  // one; below that 64 x 64 tiles, K shared eightfold from 1,024 on. (The lines were drawn where large
+  // single products were these tiles', too: 2048 rows, 2048 -> 16384 46 TFLOP/s, 37 with 64 x 64; 777
+  // rows, 2048 -> 3072 305 us with 64 x 64, 412 with 128 x 128; 128 rows, 2048 -> 64: 14 and 230.)
+  // Rows count in whole 128s here, too.
   const long long big = (long long)((p.M + 127) / 128) * ((p.N + 127) / 128) * p.count;
   if (big >= 3 * 2 * sm_count()) return launch_tile<128, 128, 8, 1, 2>(p, stream);
   if (p.K >= 1024) return launch_tile<64, 64, 4, 8, 4>(p, stream);

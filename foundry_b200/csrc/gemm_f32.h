@@ -17,5 +17,8 @@ struct FbGemmF32 {
 constexpr int FB_GEMM_F32_ROWS = 32;
 
 bool fb_gemm_f32_fits(const FbGemmF32& p);
-int fb_gemm_f32_tc_launch(const FbGemmF32& p, cudaStream_t stream);  // gemm_f32_tcgen05.cu
+// gemm_f32_tcgen05.cu; FB_GEMM_F32_NOT_HERE: the kernel does not fit this build's registers or this
+// device, and nothing was launched.
+constexpr int FB_GEMM_F32_NOT_HERE = -1;
+int fb_gemm_f32_tc_launch(const FbGemmF32& p, cudaStream_t stream);
 int fb_gemm_f32_launch(const FbGemmF32& p, cudaStream_t stream);

@@ -50,7 +50,7 @@ constexpr int THREADS = 32 * (4 + SPLIT_WARPS + SUM_WARPS);
 // Tensor memory: two accumulators of tn columns, then the weights' pieces, 16 columns each.
 constexpr int W_PIECE_COLS = KB / 2, TMEM_COLS = 512, MAX_TN = 208, RUNS = (MAX_TN / 16 + 1) / 2;
 // registers a thread of the five warpgroups: loads and MMAs, 2 x splitting, 2 x sums (112 sums a
-// thread); their total stays below what the block is launched with (checked by the launcher)
+// thread); their total stays below what the block is launched with (the launcher looks, and leaves it)
 constexpr int REGS_LOAD = 48, REGS_SPLIT = 56, REGS_SUM = 160;
 constexpr int REGS_ALL = REGS_LOAD + 2 * REGS_SPLIT + 2 * REGS_SUM;
 constexpr int SMEM_BYTES = 227 * 1024, SMEM_TILES = SMEM_BYTES - 1024 /*align*/ - 512;
@@ -754,9 +754,8 @@ int fb_gemm_f32_tc_launch(const FbGemmF32& p, cudaStream_t stream) {
   if (clusters_max == 0) {
     cudaFuncAttributes have;
     cudaError_t e = cudaFuncGetAttributes(&have, gemm_f32_pair_kernel);
-    if (e != cudaSuccess || have.numRegs * (THREADS / 128) < REGS_ALL)
-      return fb_fail(2, "gemm_f32: %d registers a thread do not cover the roles' shares (%s)",
-                     have.numRegs, cudaGetErrorString(e));
+    if (e != cudaSuccess) return fb_fail(2, "gemm_f32: attributes: %s", cudaGetErrorString(e));
+    if (have.numRegs * (THREADS / 128) < REGS_ALL) return FB_GEMM_F32_NOT_HERE;  // the roles would wait
     e = cudaFuncSetAttribute(gemm_f32_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)cfg.dynamicSmemBytes);
     if (e != cudaSuccess)
@@ -765,9 +764,8 @@ int fb_gemm_f32_tc_launch(const FbGemmF32& p, cudaStream_t stream) {
     cfg.numAttrs = 1;
     int n = 0;
     e = cudaOccupancyMaxActiveClusters(&n, gemm_f32_pair_kernel, &cfg);
-    if (e != cudaSuccess || n <= 0)
-      return fb_fail(2, "gemm_f32: no cluster of this kernel fits the device (%s)",
-                     cudaGetErrorString(e));
+    if (e != cudaSuccess) return fb_fail(2, "gemm_f32: occupancy: %s", cudaGetErrorString(e));
+    if (n <= 0) return FB_GEMM_F32_NOT_HERE;
     clusters_max = n;
   }
   // Tokens of a tile: the count that costs the fewest rounds times a stage's time, which is 6 * tn

@@ -1,12 +1,11 @@
-// out[M,N] = x[M,K] * w[N,K]^T on the CUDA cores, accumulating in IEEE 32-bit
-// (FFMA; no tensor cores, no TF32). This is the matrix product of the 32-bit
-// path of the whole model, and the plain check of the tensor-core products.
+// out[M,N] = x[M,K] * w[N,K]^T in 32 bits (no TF32): the matrix product of the 32-bit path of the
+// whole model, and, in this file's kernel (FFMA alone), the plain check of the tensor-core products.
 //
 // A projection is `x * W^T` with W stored [out, in] row-major and no bias
 // (src/nn/linear.rs:19-36); accumulation is 32-bit in the reference too
 // (src/metal/kernels/matmul.metal:42-64). Every output element of this kernel sums
 // its K products in order, whatever M is. Operands in 32 bits that 16-byte loads can
-// address take the kernels of gemm_f32.cu instead (see there for how they sum).
+// address take the kernels of gemm_f32.cu and gemm_f32_tcgen05.cu instead (see there for how they sum).
 #include "common.cuh"
 #include "gemm_f32.h"
 

@@ -74,6 +74,19 @@ def test_product_of_pieces(ops, M, N, K):
     assert ops.gemm_tc_status() == 0
 
 
+@pytest.mark.parametrize("M", [17, 32])
+@pytest.mark.parametrize("N,K", [(10504, 200), (21900, 96), (10504, 256)])
+def test_up_to_32_rows_are_multiplied_and_added(ops, M, N, K):
+    """However many columns: the bits are those of the first 8,200 columns alone, which are too few for the
+    tensor cores."""
+    x, w = rnd(M, K), rnd(N, K, seed=1)
+    out, few = torch.empty(M, N, device=DEV), torch.empty(M, 8200, device=DEV)
+    ops.gemm_simt(x, w, out)
+    ops.gemm_simt(x, w[:8200], few)
+    check_product(x, w, out)
+    assert torch.equal(out[:, :8200], few)
+
+
 @pytest.mark.parametrize("N", [300, 9000])
 def test_product_of_pieces_rounds_no_more_than_a_chain(ops, N):
     """A chain of K additions is off by about 0.41 * 2^-24 * |x||w| in the root mean square (see
