@@ -75,7 +75,7 @@ def test_product_of_pieces(ops, M, N, K):
 
 
 @pytest.mark.parametrize("M", [17, 32])
-@pytest.mark.parametrize("N,K", [(10504, 200), (21900, 96), (10504, 256)])
+@pytest.mark.parametrize("N,K", [(10504, 200), (21900, 96), (11000, 204)])
 def test_up_to_32_rows_are_multiplied_and_added(ops, M, N, K):
     """However many columns: the bits are those of the first 8,200 columns alone, which are too few for the
     tensor cores."""
