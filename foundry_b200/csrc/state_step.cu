@@ -12,8 +12,10 @@
 // in sequence_mix.cu) took 13 us for 8 sequences of 32 heads of 64 x 64 (8 MB); eight tokens through
 // four such layers 4,565 -> 4,356 us. A block a
 // (sequence, head); a thread owns four neighbouring columns of every R-th key row, and asks for them
-// before it waits for the kernel in front (the state was written a whole step ago). Sums over the
-// key rows meet in shared memory, in row order. All arithmetic is 32-bit.
+// before it waits for the kernel in front. That is right because what wrote it (the last step's scan or
+// step, or the zeros of a new sequence) let nobody start before its writes, and a kernel behind it that
+// let its successor start had waited for it: every kernel that writes states either never calls
+// fb_pdl_launch or calls it behind its writes. The same goes for the slots. Sums over the key rows meet in shared memory, in row order. All arithmetic is 32-bit.
 #include "common.cuh"
 
 namespace {
@@ -178,7 +180,7 @@ FB_API int fb_state_step(int delta, const float* q, long long q_ld, const float*
                          long long s_offset, void* out, long long out_ld, int out_dtype,
                          const int* cu_tokens, const int* slots, int n_seqs, int H, int rep, int dim,
                          int vdim, float eps, cudaStream_t stream) {
-  FB_REQUIRE(n_seqs >= 0 && H > 0 && H <= 65535 && rep > 0 && eps > 0.f, "state_step: bad sizes");
+  FB_REQUIRE(n_seqs >= 0 && H > 0 && H <= 65535 && rep > 0, "state_step: bad sizes");
   FB_REQUIRE(fb_state_step_fits(dim, vdim), "state_step: heads of %d x %d do not fit", dim, vdim);
   FB_REQUIRE(((uintptr_t)state % 16) == 0 && state_stride % 4 == 0 && s_offset % 4 == 0,
              "state_step: the state is not on 16-byte boundaries");

@@ -224,6 +224,24 @@ def test_state_step(ops, mode, H, rep, dim, vdim, per_head, form, dtype):
     assert torch.equal(rows[untouched], before[untouched]) and torch.equal(rows[:, :4], before[:, :4])
 
 
+def test_state_step_with_no_epsilon(ops):
+    """What the kernels that it takes the place of took: a norm without a constant in its root."""
+    n, H, dim, vdim = 2, 3, 64, 64
+    rnd = lambda *s, seed: torch.randn(*s, generator=torch.Generator().manual_seed(seed)).to(DEV)  # noqa: E731
+    as_int = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    ctx = types.SimpleNamespace(is_decode=True, n_seqs=n, cu_tokens=as_int([0, 1, 2]), slots=as_int([1, 0]))
+    q, k, v, gate, g = (rnd(n, H * dim, seed=s) for s in range(5))
+    args = (q, k, v, torch.sigmoid(g), None)
+    outs = []
+    for eps in (0.0, 1e-12):
+        state = ops.StateRows(rnd(2, H * dim * vdim, seed=9), [("S", H * dim * vdim)])
+        out = torch.empty(n, H * vdim, device=DEV)
+        ops.state_step(ctx, ops.SCAN_WKV, *args, state, "S", torch.ones(vdim, device=DEV), gate, "silu", eps, out,
+                       H, 1, dim, vdim, bonus=rnd(H, dim, seed=7))
+        outs.append(out)
+    assert torch.allclose(*outs, rtol=1e-6) and bool(outs[0].isfinite().all())
+
+
 @pytest.mark.parametrize("W", [4, 100, 1024, 1028, 2048, 3072, 4100, 8192, 8196])
 @pytest.mark.parametrize("has_y,norm_y,has_out", [(1, 1, 1), (1, 0, 1), (0, 0, 1), (1, 1, 0)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
