@@ -761,8 +761,9 @@ moe_combine_rows_kernel(const float* y, const int* place, const float* weights, 
 // 16-byte pieces, as in gemm_skinny.cu), the warps' sums meet in shared memory in order, and the
 // tokens' logits are routed where they were made. Bound by its loads' latency and by a token's choice,
 // a chain of one warp's: 16 warps a block (eight from 33 outputs on, for their shared memory).
-// 2,000 tokens of 3,072, 16 outputs with the sort behind it 14.2 us, 16.6 with eight; the product alone took 27 on the tcgen05 kernel, whose 16 tiles
-// walk all of K on 16 SMs, and the choice 6.
+// Tokens of 3,072, 16 outputs: 2,000 10.9 us, 14.4 with eight warps, 500 7.7 and 10.7 (an experts' call of
+// 254 us: inside its runs' spread); the product alone took 27 on the tcgen05 kernel, whose 16 tiles walk
+// all of K on 16 SMs, and the choice 6.
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                           uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile(

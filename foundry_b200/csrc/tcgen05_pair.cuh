@@ -87,9 +87,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // An arrival on a barrier of either CTA of the pair that orders the shared and tensor memory of the CTA
 // that arrives, which is all that the MMAs and the epilogues of a pair read and write (the default
 // scope, as mbar_wait's): at cluster scope an arrival took about 1,000 cycles, and a wait for a barrier
-// that was complete already some hundred. 2,048 rows of 3,072 -> 16,384 142.5 -> 141.8 us, 8,192 of
-// 2,048 -> 2,048 51.2 -> 50.6, 25,900 tokens of four layers at 1B sizes 16.25 -> 16.03 ms; the grouped
-// product keeps cluster scope: 128 rows an expert 83.2 -> 84.5 us with the default one.
+// that was complete already some hundred. Products alone, in turn: 2,048 rows of 3,072 -> 16,384 140.5 ->
+// 139.3 us, 8,192 of 2,048 -> 2,048 65.3 -> 64.3 (a whole prompt step: inside its runs' spread); the
+// grouped product keeps cluster scope: 128 rows an expert 83.2 -> 84.5 us with the default one.
 __device__ __forceinline__ void mbar_arrive_pair(uint32_t bar_cluster) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }

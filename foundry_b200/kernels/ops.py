@@ -2636,15 +2636,15 @@ def _maps_workspace(rows: int, H: int, G: int, device):
     """Memory for both maps' results (`rows` floats a head) and how many heads it is for: all of them,
     fewer where memory is short, whole groups or parts of one. Heads do not know of one another: the
     numbers are the same."""
-    each = H // G
-    sizes = [n * each for n in range(G, 0, -1) if G % n == 0]
-    sizes += [n for n in range(each - 1, 0, -1) if each % n == 0]
-    for heads in sizes:
+    heads = H
+    while True:
         try:
             return torch.empty(rows * heads, dtype=torch.float32, device=device), heads
         except torch.cuda.OutOfMemoryError:
             if heads == 1:
                 raise
+        each = H // G
+        heads = next(n for n in range(heads - 1, 0, -1) if each % n == 0 or (n % each == 0 and H % n == 0))
 
 
 def _tc_paged_blocks(ctx, q, out, k_cache, v_cache, G: int, row: int, vdim: int) -> int:
@@ -2696,7 +2696,8 @@ def attention_maps_paged(ctx, q, out, page_table, k_cache, v_cache, H: int, G: i
     blocks128 = _tc_maps_blocks(ctx, q, out, k_cache, v_cache, G, dim, vdim, maps, scale)
     if blocks128 and q.shape[0] * H * 2 * vdim <= MAPS_WORKSPACE:
         both, heads = _maps_workspace(q.shape[0] * 2 * vdim, H, G, q.device)
-        at_q, at_out = (_dev(t, "rows", torch.bfloat16, contiguous=False) for t in (q, out))
+        at_q = _dev(q, "q", torch.bfloat16, contiguous=False)
+        at_out = _dev(out, "out", torch.bfloat16, contiguous=False)
         at_sink = 0 if sink_logits is None else _dev(sink_logits, "sink_logits", torch.float32)
         for a in range(0, H, heads):  # (2 bytes an element, 4 a sink's)
             g = a * G // H
