@@ -13,9 +13,9 @@
 // Bound by the tensor pipe, six bf16 products for one, and close behind it by the issue slots of the
 // warps that split and add (two more instructions an operand: 777 rows of 2048 -> 16384 280 us). 777
 // rows of 2048 -> 16384 257 us (203 TFLOP/s of the product, 1.22 PFLOP/s of bf16) where FFMA tiles took
-// 1524, -> 3072 59 for 311, 8192 -> 2048 156 for 789; 64 rows of 2048 -> 2048 23 for 33; 2048 rows -> 16384 700 for 3010 (74 TFLOP/s is all
-// that FFMA could give). The weights are split tile by tile, not once to memory, which would move 16
-// bytes an element where this moves 4.
+// 1524, -> 3072 59 for 311, 8192 -> 2048 156 for 789; 64 rows of 2048 -> 2048 23 for 33; 2048 rows ->
+// 16384 700 for 3010 (74 TFLOP/s is all that FFMA could give). The weights are split tile by tile, not
+// once to memory, which would move 16 bytes an element where this moves 4.
 //
 // Two SMs share a tile of 256 weight rows (the instruction's rows) and up to 208 tokens (its N): each
 // loads 128 weight rows and half of the tokens. The weights' pieces go to tensor memory, as the
