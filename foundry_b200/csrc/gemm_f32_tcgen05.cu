@@ -243,23 +243,41 @@ __device__ __forceinline__ bool falls(float v, const RowFacts& w, const RowFacts
 __device__ __forceinline__ bool settles(const RowFacts& of, float v) {
   return of.nan || (of.least == 0xffffffffu && v == 0.f);
 }
-// One warp looks at a row.
-__device__ __forceinline__ void look_at_row(RowFacts* to, const float* row, int K, int lane) {
-  float most = 0.f;
-  uint32_t least = 0xffffffffu;
-  bool nan = false;
-#pragma unroll 2
-  for (int k = lane * 4; k < K; k += 128) {
-    const float4 v = __ldcg(reinterpret_cast<const float4*>(row + k));
-    most = fmaxf(most, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-    least = min(least, min(min(2u * __float_as_uint(v.x) - 1u, 2u * __float_as_uint(v.y) - 1u),
-                           min(2u * __float_as_uint(v.z) - 1u, 2u * __float_as_uint(v.w) - 1u)));
-    nan = nan || !(v.x == v.x && v.y == v.y && v.z == v.z && v.w == v.w);
+// One warp looks at two rows side by side (a null row is left), up to 16 loads under way.
+__device__ __forceinline__ void look_at_rows(RowFacts* to_a, const float* a, RowFacts* to_b, const float* b,
+                                             int K, int lane) {
+  float most[2] = {0.f, 0.f};
+  uint32_t least[2] = {0xffffffffu, 0xffffffffu};
+  bool nan[2] = {false, false};
+  if (a == nullptr && b == nullptr) return;
+  for (int k0 = lane * 4; k0 < K; k0 += 8 * 128) {
+    float4 v[2][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = k0 + 128 * i;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      v[0][i] = a != nullptr && k < K ? __ldcg(reinterpret_cast<const float4*>(a + k)) : zero;
+      v[1][i] = b != nullptr && k < K ? __ldcg(reinterpret_cast<const float4*>(b + k)) : zero;
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float x[4] = {v[r][i].x, v[r][i].y, v[r][i].z, v[r][i].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          most[r] = fmaxf(most[r], fabsf(x[e]));
+          least[r] = min(least[r], 2u * __float_as_uint(x[e]) - 1u);
+          nan[r] = nan[r] || !(x[e] == x[e]);
+        }
+      }
   }
-  most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most)));
-  least = __reduce_min_sync(0xffffffffu, least);
-  nan = __any_sync(0xffffffffu, nan);
-  if (lane == 0) *to = RowFacts{most, least, nan};
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const RowFacts facts = {__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most[r]))),
+                            __reduce_min_sync(0xffffffffu, least[r]), __any_sync(0xffffffffu, nan[r])};
+    if (lane == 0 && (r == 0 ? a : b) != nullptr) *(r == 0 ? to_a : to_b) = facts;
+  }
 }
 
 // The summing warps' threads meet; whether one of them said yes.
@@ -310,17 +328,25 @@ __device__ __forceinline__ void repair(const Params& p, RepairRoom& room, bool a
     any_of_sums(false);
     return true;
   };
-  auto look = [&](bool tokens) {
-    if (tokens) {
-      for (int i = tid / 32; i < 16; i += SUM_WARPS)
-        if (room.asked[WORDS] >> i & 1u)
-          look_at_row(facts + W_ROWS + i, p.x + (long long)(t0 + i) * p.ldx, p.K, tid & 31);
-    } else {
-      for (int r = tid / 32; r < W_ROWS; r += SUM_WARPS)
-        if ((room.asked[r / 32] & ~room.known[r / 32]) >> (r % 32) & 1u) {
-          look_at_row(facts + r, p.w + (long long)(f0 + r) * p.ldw, p.K, tid & 31);
-          if ((tid & 31) == 0) atomicOr(&room.known[r / 32], 1u << (r % 32));
-        }
+  auto look = [&](bool tokens) {  // a warp takes rows SUM_WARPS apart, two at once
+    const uint32_t* known = tokens ? nullptr : room.known;
+    const float* base = tokens ? p.x + (long long)t0 * p.ldx : p.w + (long long)f0 * p.ldw;
+    const long long pitch = tokens ? p.ldx : p.ldw;
+    const int first = tokens ? W_ROWS : 0, end = tokens ? W_ROWS + 16 : W_ROWS;
+    for (int r = first + tid / 32; r < end; r += 2 * SUM_WARPS) {
+      auto place = [&](int r) -> const float* {
+        const bool asked = room.asked[r / 32] >> (r % 32) & 1u;
+        return asked && (tokens || !(known[r / 32] >> (r % 32) & 1u)) ? base + (long long)(r - first) * pitch
+                                                                      : nullptr;
+      };
+      const int s = r + SUM_WARPS;
+      const float *a = place(r), *b = place(s);
+      look_at_rows(facts + r, a, facts + s, b, p.K, tid & 31);
+      __syncwarp();
+      if (!tokens && (tid & 31) == 0) {
+        if (a != nullptr) atomicOr(&room.known[r / 32], 1u << (r % 32));
+        if (b != nullptr) atomicOr(&room.known[s / 32], 1u << (s % 32));
+      }
     }
     any_of_sums(false);
   };
