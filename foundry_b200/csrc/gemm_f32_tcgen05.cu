@@ -32,7 +32,7 @@
 // splitting warps keep the largest first piece (half an instruction an operand; 777 rows of 2048 ->
 // 16384 252 -> 257 us); unless it is huge, a finite result of 2^-64 or more stands, and the rows of the
 // others are looked at, which settles most (`falls`). Zeros cost that look: a token in seven of zeros,
-// 777 rows of 8192 -> 16384 990 -> 1,600 us; all of x NaN 1,900, all of it infinite 30,000.
+// 777 rows of 8192 -> 16384 990 -> 1,320 us; all of x NaN 1,500, all of it infinite 26,000.
 #define FB_STATUS_KERNEL 5
 #include "gemm_f32.h"
 #include "tcgen05_pair.cuh"
@@ -44,7 +44,9 @@ constexpr int W_ROWS = 128;       // weight rows of a CTA
 constexpr int PIECES = 3;
 constexpr int MAX_STAGES = 8, MAX_PIECE_STAGES = 4;
 constexpr int MAX_SHARES = 4;     // pairs of a cluster (8 CTAs, the portable size)
-constexpr int ROUNDS = 32;
+// Rounds of tiles that are kept apart in what a CTA notes of them (the others share, round % ROUNDS), and
+// words for a bit a token of a tile.
+constexpr int ROUNDS = 32, TOKEN_WORDS = 7;
 constexpr int SPLIT_WARPS = 8, SUM_WARPS = 8;
 constexpr int THREADS = 32 * (4 + SPLIT_WARPS + SUM_WARPS);
 // Tensor memory: two accumulators of tn columns, then the weights' pieces, 16 columns each.
@@ -53,7 +55,7 @@ constexpr int W_PIECE_COLS = KB / 2, TMEM_COLS = 512, MAX_TN = 208, RUNS = (MAX_
 // thread); their total stays below what the block is launched with (the launcher looks, and leaves it)
 constexpr int REGS_LOAD = 48, REGS_SPLIT = 56, REGS_SUM = 160;
 constexpr int REGS_ALL = REGS_LOAD + 2 * REGS_SPLIT + 2 * REGS_SUM;
-constexpr int SMEM_BYTES = 227 * 1024, SMEM_TILES = SMEM_BYTES - 1024 /*align*/ - 512;
+constexpr int SMEM_DYNAMIC = 227 * 1024 - 1536 /*barriers and notes*/, SMEM_TILES = SMEM_DYNAMIC - 1024 /*align*/;
 
 struct Params {
   const float* x;
@@ -216,6 +218,20 @@ __device__ __forceinline__ uint32_t largest_of_warp(uint32_t pieces) {  // as th
   const uint32_t a = (pieces & 0x7fffu) << 16, b = pieces & 0x7fff0000u;
   return __reduce_max_sync(0xffffffffu, max(a, b));
 }
+// Whether a row is zeros alone, by one warp.
+__device__ __forceinline__ bool is_zero_row(const float* row, int K, int lane) {
+  for (int k0 = lane * 4; __any_sync(0xffffffffu, k0 < K); k0 += 16 * 128) {
+    uint32_t bits = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (k0 + 128 * i < K) {
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(row + k0 + 128 * i));
+        bits |= (__float_as_uint(v.x) | __float_as_uint(v.y)) | (__float_as_uint(v.z) | __float_as_uint(v.w));
+      }
+    if (__any_sync(0xffffffffu, bits << 1 != 0)) return false;  // (a zero has a sign)
+  }
+  return true;
+}
 
 // What a row of operands is: the largest magnitude (not a NaN's), the smallest that is not zero (as twice
 // its bits less one, so that a zero is the largest), whether it holds a NaN.
@@ -298,8 +314,9 @@ __device__ __forceinline__ bool any_of_sums(bool mine) {
 // A run of 16 tokens (from t0) by this CTA's weight rows (from f0) once more, results that fall as chains of
 // FMAs over K: 256 threads, a weight row and 8 tokens each, REPAIR_K of K at a time through shared memory.
 // All of it is behind all tiles, where nobody waits for these warps. Which results fall: of those that do
-// not stand by themselves (or of all) the rows are looked at, first the operand's of which fewer are
-// asked about (weight rows once a tile), then, for what is left, the other's.
+// not stand by themselves (or of all; not the zeros of tokens that are not `busy`, which are zeros) the
+// rows are looked at, first the operand's of which fewer are asked about (weight rows once a tile), then,
+// for what is left, the other's.
 constexpr int REPAIR_K = 256, REPAIR_PITCH = REPAIR_K + 4, REPAIR_ROWS = W_ROWS + 16;
 static_assert(REPAIR_ROWS % 48 == 0, "whole rounds of loads");
 struct RepairRoom {
@@ -308,7 +325,15 @@ struct RepairRoom {
   uint32_t asked[W_ROWS / 32 + 1], known[W_ROWS / 32];  // weight rows (tokens last); weight rows looked at
 };
 static_assert(sizeof(RepairRoom) <= SMEM_TILES, "room for the repair");
-__device__ __forceinline__ void repair(const Params& p, RepairRoom& room, bool all, int f0, int t0) {
+// Whether the result of weight row f and a tile's token t is to be looked at: no zero of a token of zeros.
+__device__ __forceinline__ bool falls_maybe(const Params& p, const uint32_t* busy, bool all, int f, int tile0, int t) {
+  if (tile0 + t >= p.M || f >= p.N) return false;
+  const float v = __ldcg(p.out + (long long)(tile0 + t) * p.ldo + f);
+  return v == 0.f ? busy[t >> 5] >> (t & 31) & 1u : all || !stands(v);
+}
+__device__ __forceinline__ void repair(const Params& p, RepairRoom& room, const uint32_t* busy, bool all, int f0,
+                                       int tile0, int run0) {
+  const int t0 = tile0 + run0;
   constexpr int WORDS = W_ROWS / 32;
   const int tid = (int)threadIdx.x - 32 * (4 + SPLIT_WARPS);
   const int row = tid % W_ROWS, half = tid / W_ROWS, f = f0 + row;
@@ -317,7 +342,7 @@ __device__ __forceinline__ void repair(const Params& p, RepairRoom& room, bool a
   uint32_t wanted = 0;
 #pragma unroll
   for (int e = 0; e < 8; ++e)
-    if (t0 + half * 8 + e < p.M && f < p.N && (all || !stands(result(e)))) wanted |= 1u << e;
+    if (falls_maybe(p, busy, all, f, tile0, run0 + half * 8 + e)) wanted |= 1u << e;
   auto ask = [&]() {
     if (tid <= WORDS) room.asked[tid] = 0;
     if (!any_of_sums(wanted != 0)) return false;
@@ -417,9 +442,9 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
   __shared__ __align__(8) uint64_t piece_empty[MAX_PIECE_STAGES];
   __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];  // acc_empty: used in the leader
   __shared__ uint32_t tmem_slot;
-  // runs of 16 tokens of this CTA's tiles, round by round (rounds ROUNDS apart share a word), in which
-  // some result does not stand
-  __shared__ uint32_t fallen[ROUNDS];
+  // of this CTA's tiles, round by round: runs of 16 tokens in which a result does not stand; of a tile: its
+  // tokens that are not zeros alone, the runs in which a result of theirs does not stand
+  __shared__ uint32_t fallen[ROUNDS], busy[TOKEN_WORDS], odd;
   __shared__ uint32_t largest[2];  // first piece of a weight, of a token that the cluster multiplied
   __shared__ int s_abort;
   volatile int* abort_flag = &s_abort;
@@ -433,6 +458,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
   const int stages_k = (p.K + KB - 1) / KB, kb0 = stages_k * (int)share / p.shares;
   const int nkb = stages_k * ((int)share + 1) / p.shares - kb0;  // this pair's part of K
 
+  if (threadIdx.x < ROUNDS) fallen[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(&raw_full[s], 1);
@@ -446,7 +472,6 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 2 * SUM_WARPS);
     }
-    for (int r = 0; r < ROUNDS; ++r) fallen[r] = 0;
     largest[0] = largest[1] = 0u;
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -718,13 +743,34 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap map_w,
       for (int u = cluster; u < p.units; u += clusters, ++round) {
         const uint32_t fell = all ? (1u << (p.tn / 16)) - 1u : fallen[round % ROUNDS];
         if (fell == 0) continue;
+        const int f0 = (u / p.tiles_t) * 2 * W_ROWS + (int)rank * W_ROWS, t0 = (u % p.tiles_t) * p.tn;
+        const int me = warp - 4 - SPLIT_WARPS, tid = me * 32 + lane;
+        // Mostly zeros of tokens of zeros (padding, in a step), which one look at those settles. (Where a
+        // weight is infinite, such a token's results are NaN, by pieces as by FMAs.)
         any_of_sums(false);  // the tile before is done
-        if (threadIdx.x < 32 * (4 + SPLIT_WARPS) + W_ROWS / 32)
-          room.known[threadIdx.x - 32 * (4 + SPLIT_WARPS)] = 0;
+        if (tid < TOKEN_WORDS) busy[tid] = 0;
+        if (tid < W_ROWS / 32) room.known[tid] = 0;
+        if (tid == 0) odd = 0;
+        any_of_sums(false);
+#pragma unroll 1
+        for (int t = me; t < p.tn && t0 + t < p.M; t += SUM_WARPS)
+          if ((fell >> (t >> 4) & 1u) && (t >> 4) % p.shares == (int)share &&
+              !is_zero_row(p.x + (long long)(t0 + t) * p.ldx, p.K, lane) && lane == 0)
+            atomicOr(&busy[t >> 5], 1u << (t & 31));
+        any_of_sums(false);
+#pragma unroll 1
         for (int run = (int)share; fell >> run != 0; run += p.shares)
-          if (fell >> run & 1u)
-            repair(p, room, all, (u / p.tiles_t) * 2 * W_ROWS + (int)rank * W_ROWS,
-                   (u % p.tiles_t) * p.tn + run * 16);
+          if ((fell >> run & 1u) && (busy[run >> 1] >> (16 * (run & 1)) & 0xffffu) != 0) {
+            bool mine = false;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              mine = mine || falls_maybe(p, busy, all, f0 + tid % W_ROWS, t0, run * 16 + tid / W_ROWS * 8 + e);
+            if (mine) atomicOr(&odd, 1u << run);
+          }
+        any_of_sums(false);
+        const uint32_t left = odd;
+        for (int run = (int)share; left >> run != 0; run += p.shares)
+          if (left >> run & 1u) repair(p, room, busy, all, f0, t0, run * 16);
       }
     }
   }
@@ -753,7 +799,7 @@ int fb_gemm_f32_tc_launch(const FbGemmF32& p, cudaStream_t stream) {
   bind_status_mirror(stream);
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = SMEM_BYTES - 512;
+  cfg.dynamicSmemBytes = SMEM_DYNAMIC;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -814,7 +860,7 @@ int fb_gemm_f32_tc_launch(const FbGemmF32& p, cudaStream_t stream) {
   q.units = tiles_w * q.tiles_t;
   q.piece_stages = (TMEM_COLS - 2 * tn) / (PIECES * W_PIECE_COLS);
   if (q.piece_stages > MAX_PIECE_STAGES) q.piece_stages = MAX_PIECE_STAGES;
-  q.stages = (SMEM_TILES - 512 - q.piece_stages * piece_bytes(tn)) / raw_bytes(tn);
+  q.stages = (SMEM_TILES - q.piece_stages * piece_bytes(tn)) / raw_bytes(tn);
   if (q.stages > MAX_STAGES) q.stages = MAX_STAGES;
   CUtensorMap mw, mx;
   int rc = make_map_f32(&mw, p.w, p.N, p.K, p.ldw, W_ROWS);

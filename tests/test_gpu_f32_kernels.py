@@ -127,7 +127,7 @@ def test_product_of_pieces_of_what_pieces_cannot_carry(ops, N):
 
 @pytest.mark.parametrize("N", [300, 9000])
 @pytest.mark.parametrize("of_x,of_w", [(1e-34, 1e8), (1e-36, 1e10), (1e-38, 1e12), (3e-40, 1e15),
-                                       (1e-39, 1e30), (1e10, 1e-36), (1e-20, 1e-18)])
+                                       (1e-39, 1e30), (1e-43, 1e30), (1e10, 1e-36), (1e-20, 1e-18)])
 def test_product_of_pieces_of_small_times_large(ops, N, of_x, of_w):
     """Operands whose pieces are below the smallest normal number, times operands that make results of
     any size of them: all tokens, one of them, one number of a token."""
